@@ -9,9 +9,12 @@
 //              and the TMA writes of the next stages need the same array (measured: main loop at half the instruction
 //              rate).  At 128 x 256 an MMA reads 12 KB per ~136 clk.
 //   pipeline   20 warps.  Warp group 0: warp 0 = TMA producer (operand tiles by tensor map, scale atoms by 1-D bulk copy),
-//              warp 1 = MMA issuer (4 MMAs per stage), warp 2 = scale-factor copier (tcgen05.cp atoms smem -> TMEM; the
-//              copies take tensor-pipe time but overlap the MMAs when another warp issues them), warp 3 idle.  Warp groups
-//              1..4 = 16 epilogue warps.  Registers are re-balanced between the roles (setmaxnreg, per epilogue kind): the three single-thread
+//              warp 1 = MMA issuer (per stage: the scale atoms smem -> TMEM by tcgen05.cp, then 4 MMAs; one thread issues
+//              both, in order, and the hardware overlaps them), warps 2 and 3 idle.  Both issuing warps run warp-uniform
+//              loops with one elected lane per instruction (kf_sm100.cuh): with one-lane loops and the copies issued by a
+//              warp of their own a stage of NVFP4 took 1090 clk on an otherwise idle SM, now 610 (its MMAs: 544); M = 1605,
+//              K = 4096, N = 1024: 14.8 -> 10.6 us, M = 22 470: fc2 75 -> 67 us, plain 69 -> 67 us.  Warp groups
+//              1..4 = 16 epilogue warps.  Registers are re-balanced between the roles (setmaxnreg, per epilogue kind): the issuing
 //              roles give theirs up and every epilogue thread holds its 64 accumulator values plus loads in flight
 //              without spilling.
 //              One 256-column accumulator in TMEM: each epilogue warp takes (32-row TMEM quarter, 64 columns) into
@@ -65,20 +68,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   float* slabs = slices + (g.vec_floats > EPI_WARPS * SLICE_FLOATS ? g.vec_floats : EPI_WARPS * SLICE_FLOATS);   // ROPE only
   uint64_t* bars = reinterpret_cast<uint64_t*>(slabs + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS : 0));
   uint64_t *full = bars, *empty = bars + MAX_STAGES, *tfull = bars + 2 * MAX_STAGES, *tempty = tfull + 1;
-  uint64_t *sf_full = tempty + 1, *sf_empty = sf_full + SF_BUFS;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sf_empty + SF_BUFS);
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   pdl_launch_dependents();                               // the next kernel of the stream may take the SMs this grid leaves
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
-    }
-    for (int b = 0; b < SF_BUFS; ++b) {
-      mbar_init(&sf_full[b], 1);
-      mbar_init(&sf_empty[b], 1);
     }
     mbar_init(tfull, 1);
     mbar_init(tempty, EPI_WARPS);
@@ -110,17 +108,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       // nothing is issued; fall through to the teardown
     } else if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
-        uint32_t s = 0, ph = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-          const int m_blk = tile / g.n_tiles, n_blk = tile - m_blk * g.n_tiles;
-          const int w_halves = (n_blk * BN + 128 < g.N) ? 2 : 1;              // the last column tile may hold only 128 columns
-          int row_end;
-          const int a_row0 = tile_row0(g, m_blk, row_end), w_row0 = tile_wrow0(g, m_blk, n_blk);
-          const uint32_t tx = TILE_BYTES + (SCALED ? (1 + w_halves) * ATOMS * 512 : 0);
-          for (int kt = 0; kt < g.k_tiles; ++kt) {
-            if (!mbar_wait(&empty[s], ph ^ 1, ctx, 1)) { ok = false; break; }
+      uint32_t s = 0, ph = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+        const int m_blk = tile / g.n_tiles, n_blk = tile - m_blk * g.n_tiles;
+        const int w_halves = (n_blk * BN + 128 < g.N) ? 2 : 1;                // the last column tile may hold only 128 columns
+        int row_end;
+        const int a_row0 = tile_row0(g, m_blk, row_end), w_row0 = tile_wrow0(g, m_blk, n_blk);
+        const uint32_t tx = TILE_BYTES + (SCALED ? (1 + w_halves) * ATOMS * 512 : 0);
+        for (int kt = 0; kt < g.k_tiles; ++kt) {
+          if (!mbar_wait_warp(&empty[s], ph ^ 1, ctx, 1)) { ok = false; break; }
+          if (elect_one()) {
             mbar_expect_tx(&full[s], tx);
             uint8_t* ta = tiles + (size_t)s * TILE_BYTES;
             tma_load_2d(ta, &tmA, kt * BKB, a_row0, &full[s]);
@@ -131,35 +129,46 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               for (int h = 0; h < w_halves; ++h)
                 bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(2 * n_blk + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
             }
-            if (++s == STAGES) { s = 0; ph ^= 1; }
           }
+          __syncwarp();
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
-      __syncwarp();
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issuer
-      if (lane == 0) {
-        constexpr uint32_t IDESC = KIND == KIND_BF16 ? idesc_f16(1, BN)
-                                   : KIND == KIND_MX8 ? idesc_bs(0, 1, BN)
-                                   : KIND == KIND_NV4 ? idesc_bs(1, 0, BN)
-                                                      : idesc_bs(1, 1, BN);
-        uint32_t s = 0, ph = 0, lt = 0, sb = 0, sph = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++lt) {
-          if (!mbar_wait(tempty, (lt & 1) ^ 1, ctx, 2)) break;                  // the epilogue has taken the previous tile out of TMEM
+      // Per stage: the scale-factor atoms into one of the SF_BUFS tensor-memory buffers (tcgen05.cp), then four MMAs of 32
+      // K-bytes.  One thread issues both, so the hardware runs them in order (an MMA sees the copies in front of it, a copy
+      // does not overtake the MMAs that read the buffer's previous contents) and overlaps them: twelve copies and four
+      // MMAs take the time of the MMAs alone.
+      constexpr uint32_t IDESC = KIND == KIND_BF16 ? idesc_f16(1, BN)
+                                 : KIND == KIND_MX8 ? idesc_bs(0, 1, BN)
+                                 : KIND == KIND_NV4 ? idesc_bs(1, 0, BN)
+                                                    : idesc_bs(1, 1, BN);
+      uint32_t s = 0, ph = 0, lt = 0, sb = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++lt) {
+        const int n_blk = tile % g.n_tiles;
+        const bool two = n_blk * BN + 128 < g.N;
+        if (!mbar_wait_warp(tempty, (lt & 1) ^ 1, ctx, 2)) break;               // the epilogue has taken the previous tile out of TMEM
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base;
+        for (int kt = 0; kt < g.k_tiles; ++kt) {
+          if (!mbar_wait_warp(&full[s], ph, ctx, 3)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t d_tmem = tmem_base;
-          for (int kt = 0; kt < g.k_tiles; ++kt) {
-            if (!mbar_wait(&full[s], ph, ctx, 3)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t a_addr = smem_u32(tiles + (size_t)s * TILE_BYTES);
-            const uint64_t adesc = smem_desc_sw128(a_addr), bdesc = smem_desc_sw128(a_addr + A_BYTES);
-            // scale factors of this stage: A at +0 (4 columns per atom), W at +16 (8 columns per atom pair: the atom of
-            // columns 0..127 of the tile, then the atom of columns 128..255)
-            const uint32_t sf_t = tmem_base + TMEM_SF_COL + sb * SF_BUF_COLS;
-            if (SCALED) {                          // copied into TMEM by the scale-copy warp, which runs ahead of the MMAs
-              if (!mbar_wait(&sf_full[sb], sph, ctx, 5)) { ok = false; break; }
-              tc_fence_after();
+          const uint32_t a_addr = smem_u32(tiles + (size_t)s * TILE_BYTES);
+          const uint64_t adesc = smem_desc_sw128(a_addr), bdesc = smem_desc_sw128(a_addr + A_BYTES);
+          // scale factors of this stage: A at +0 (4 columns per atom), W at +16 (8 columns per atom pair: the atom of
+          // columns 0..127 of the tile, then the atom of columns 128..255)
+          const uint32_t sf_t = tmem_base + TMEM_SF_COL + sb * SF_BUF_COLS;
+          const uint32_t sa = smem_u32(sfs + (size_t)s * SF_STAGE_BYTES);
+          if (elect_one()) {
+            if (SCALED) {
+#pragma unroll
+              for (int a = 0; a < ATOMS; ++a) {
+                tc_cp_sf(sf_t + 4 * a, smem_desc_sf(sa + a * 512));
+                tc_cp_sf(sf_t + 16 + 8 * a, smem_desc_sf(sa + (ATOMS + a) * 512));
+                if (two) tc_cp_sf(sf_t + 16 + 8 * a + 4, smem_desc_sf(sa + (2 * ATOMS + a) * 512));
+              }
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {                                       // 32 K-bytes per MMA
@@ -176,47 +185,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               }
             }
             tc_commit(&empty[s]);
-            if (SCALED) {
-              tc_commit(&sf_empty[sb]);
-              if (++sb == SF_BUFS) { sb = 0; sph ^= 1; }
-            }
-            if (++s == STAGES) { s = 0; ph ^= 1; }
+            if (kt == g.k_tiles - 1) tc_commit(tfull);
           }
-          if (ok) tc_commit(tfull);
+          __syncwarp();
+          if (SCALED && ++sb == SF_BUFS) sb = 0;
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
-      __syncwarp();
-    } else if (warp == 2) {
-      // ------------------------------------------------------------------ scale-factor copier
-      // tcgen05.cp of one 512-byte atom costs about as much tensor-pipe time as a 128 x 128 MMA, but it overlaps with
-      // the MMAs when it is issued from another warp; issued from the MMA thread the two serialise.  This warp therefore
-      // moves the atoms of stage s (shared memory -> one of SF_BUFS TMEM buffers) as soon as the TMA has landed them and
-      // hands the buffer to the MMA warp through an mbarrier.
-      if (SCALED && lane == 0) {
-        uint32_t s = 0, ph = 0, sb = 0, sph = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-          const int n_blk = tile % g.n_tiles;
-          const int w_halves = (n_blk * BN + 128 < g.N) ? 2 : 1;
-          for (int kt = 0; kt < g.k_tiles; ++kt) {
-            if (!mbar_wait(&sf_empty[sb], sph ^ 1, ctx, 6)) { ok = false; break; }
-            if (!mbar_wait(&full[s], ph, ctx, 7)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t sf_t = tmem_base + TMEM_SF_COL + sb * SF_BUF_COLS;
-            const uint32_t sa = smem_u32(sfs + (size_t)s * SF_STAGE_BYTES);
-#pragma unroll
-            for (int a = 0; a < ATOMS; ++a) {
-              tc_cp_sf(sf_t + 4 * a, smem_desc_sf(sa + a * 512));
-              tc_cp_sf(sf_t + 16 + 8 * a, smem_desc_sf(sa + (ATOMS + a) * 512));
-              if (w_halves == 2) tc_cp_sf(sf_t + 16 + 8 * a + 4, smem_desc_sf(sa + (2 * ATOMS + a) * 512));
-            }
-            tc_commit(&sf_full[sb]);
-            if (++sb == SF_BUFS) { sb = 0; sph ^= 1; }
-            if (++s == STAGES) { s = 0; ph ^= 1; }
-          }
-        }
-      }
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------------ epilogue: 16 warps, warp = (TMEM lane quarter, 64-column group)

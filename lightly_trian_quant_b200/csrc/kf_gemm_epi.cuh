@@ -19,7 +19,7 @@ constexpr int BM = 128, BN = 256, BKB = 128;          // tile rows, tile columns
 constexpr int A_BYTES = BM * BKB, TILE_BYTES = (BM + BN) * BKB;   // 16 KB of A, then 32 KB of W per stage
 constexpr int SF_STAGE_BYTES = 6144;                   // up to 4 atoms for A, then up to 4 + 4 for the two 128-row halves of W
 constexpr int EPI_WARPS = 16;
-constexpr int EPI_WARP0 = 4;                           // warps 0..3: TMA producer, MMA issuer, scale-factor copier, spare
+constexpr int EPI_WARP0 = 4;                           // warps 0..3: TMA producer, MMA issuer, two spares
 constexpr int GEMM_THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
 constexpr int SF_BUFS = 4;                             // scale-factor buffers in TMEM, 48 columns each (A at +0, W at +16)
 constexpr int SF_BUF_COLS = 48;
