@@ -10,10 +10,10 @@
 //            ring, 4-D tensor maps so rows past N read zero); warp 5 issues the PV products (O += P V: 4 MMAs of K=16
 //            with P as the A operand from tensor memory and V as the MN-major B operand), warp 6 the S products
 //            (S = Q K^T: 4 MMAs of K=16 from shared memory); warp 7 idles (it completes the second warp group, whose
-//            registers setmaxnreg hands to the softmax warps: 200 against 56).  One thread issuing both products was
-//            busy for about 1450 of the 1670 clk of a step (each MMA costs it ~55 clk, each commit ~80, each barrier
-//            round trip 60-80 even when the phase completed long ago); with two issuers each waits for its operands
-//            first and for the hand-over last.
+//            registers setmaxnreg hands to the softmax warps: 200 against 56).  The issuing warps run
+//            warp-uniform loops with one elected lane per instruction (kf_sm100.cuh); as one-lane loops they spent ~55 clk
+//            per MMA and ~80 per commit (bf16 B 14, N 1605, quantise-out: 236 -> 214 us; f16 B 8, N 4101: 806 -> 691 us).
+//            Each waits for its operands first and for the hand-over last.
 //   pipeline S and P are double buffered in TMEM: S(j+2) is issued when PV(j) has completed (so a softmax that sees
 //            S(j+2) knows that P buffer j & 1 has been read), also across the end of an item (the next item's Q and
 //            first K tiles are loaded by then).  O accumulates in TMEM over all key tiles.  The exponentials of a tile
@@ -106,7 +106,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   pdl_launch_dependents();                               // the next kernel of the stream may take the SMs this grid leaves
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // Persistent: this CTA works through the (image, head, query tile) items blockIdx.x, blockIdx.x + gridDim.x, ...  All
   // barriers keep running across items: K / V ring stages, S / P buffers and the O barrier are indexed by the CTA's global
   // key-tile count G, the two Q buffers by the item count, so the loads and the first S products of the next item are
@@ -169,81 +169,84 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // nothing was issued; fall through to the teardown
   } else if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmQ);
       prefetch_tmap(&tmK);
       prefetch_tmap(&tmV);
-      uint32_t G = 0;
-      bool ok = true;
-      for (int it = 0; it < n_my && ok; ++it) {
-        const Item I = item_of(it);
-        const int qb = it & 1;
-        if (!mbar_wait(&q_empty[qb], ((it >> 1) & 1) ^ 1, ctx, 10)) break;          // the S products of item it - 2 are done with this buffer
+    }
+    uint32_t G = 0;
+    bool ok = true;
+    for (int it = 0; it < n_my && ok; ++it) {
+      const Item I = item_of(it);
+      const int qb = it & 1;
+      if (!mbar_wait_warp(&q_empty[qb], ((it >> 1) & 1) ^ 1, ctx, 10)) break;       // the S products of item it - 2 are done with this buffer
+      if (elect_one()) {
         mbar_expect_tx(&q_full[qb], AT_QTILE);
         tma_load_4d(smem + AT_OFF_Q + qb * AT_QTILE, &tmQ, 0, I.h, I.qt * AT_BM, I.b, &q_full[qb]);
-        for (int j = 0; j < n_kt; ++j, ++G) {
-          const int st = G % AT_KV;
-          if (!mbar_wait(&kv_empty[st], ((G / AT_KV) & 1) ^ 1, ctx, 11)) { ok = false; break; }
+      }
+      for (int j = 0; j < n_kt; ++j, ++G) {
+        const int st = G % AT_KV;
+        if (!mbar_wait_warp(&kv_empty[st], ((G / AT_KV) & 1) ^ 1, ctx, 11)) { ok = false; break; }
+        if (elect_one()) {
           mbar_expect_tx(&k_full[st], AT_KTILE);
           tma_load_4d(smem + AT_OFF_K + st * AT_KTILE, &tmK, 0, I.h, j * AT_BN, I.b, &k_full[st]);
           mbar_expect_tx(&v_full[st], AT_KTILE);
           tma_load_4d(smem + AT_OFF_V + st * AT_KTILE, &tmV, 0, I.h, j * AT_BN, I.b, &v_full[st]);
         }
+        __syncwarp();
       }
     }
-    __syncwarp();
   } else if (warp == 5) {
     // ------------------------------------------------------------------ issuer of the PV products
-    if (lane == 0) {
-      const uint32_t idesc_o = idesc_f16(F16 ? 0u : 1u, AT_D) | (1u << 16);   // B (= V) is MN-major
-      const uint32_t t_o = tmem_base + AT_COL_O;
-      const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;                // key-tile steps of this CTA over all its items
-      uint32_t j = 0;
-      for (uint32_t G = 0; G < total; ++G) {
-        const uint32_t st = G % AT_KV;
-        if (!mbar_wait(&v_full[st], (G / AT_KV) & 1, ctx, 15)) break;      // V lands long before P: its barrier round trip is off the chain P -> PV -> S
-        if (!mbar_wait(&p_full[G & 1], (G >> 1) & 1, ctx, 14)) break;
-        tc_fence_after();
-        const uint32_t t_p = tmem_base + AT_COL_P + (G & 1) * (AT_BN / 2);
-        const uint64_t vdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_V + st * AT_KTILE));
+    const uint32_t idesc_o = idesc_f16(F16 ? 0u : 1u, AT_D) | (1u << 16);     // B (= V) is MN-major
+    const uint32_t t_o = tmem_base + AT_COL_O;
+    const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;                  // key-tile steps of this CTA over all its items
+    uint32_t j = 0;
+    for (uint32_t G = 0; G < total; ++G) {
+      const uint32_t st = G % AT_KV;
+      if (!mbar_wait_warp(&v_full[st], (G / AT_KV) & 1, ctx, 15)) break;   // V lands long before P: its barrier round trip is off the chain P -> PV -> S
+      if (!mbar_wait_warp(&p_full[G & 1], (G >> 1) & 1, ctx, 14)) break;
+      tc_fence_after();
+      const uint32_t t_p = tmem_base + AT_COL_P + (G & 1) * (AT_BN / 2);
+      const uint64_t vdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_V + st * AT_KTILE));
+      if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)       // A: 16 keys = 8 TMEM columns of P; B: 16 key rows of V = two 8-row groups of 1024 bytes
+        for (int kk = 0; kk < 4; ++kk)         // A: 16 keys = 8 TMEM columns of P; B: 16 key rows of V = two 8-row groups of 1024 bytes
           mma_f16_ta(t_o, t_p + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (j | (uint32_t)kk) != 0);
         tc_commit(&o_full[G & 1]);
-        tc_commit(&kv_empty[st]);            // K of this stage was read by S(G), which completed before the softmax of step G began
-        if (++j == (uint32_t)n_kt) j = 0;
+        tc_commit(&kv_empty[st]);              // K of this stage was read by S(G), which completed before the softmax of step G began
       }
+      __syncwarp();
+      if (++j == (uint32_t)n_kt) j = 0;
     }
-    __syncwarp();
   } else if (warp == 6) {
     // ------------------------------------------------------------------ issuer of the S products
-    // A second issuing thread: one thread issuing both products of a step (eight MMAs, three or four commits, three
-    // barrier round trips) was busy for about 1450 of the 1670 clk of a step.  S(G + 2) goes into the S buffer that the
-    // softmax of step G has read, once PV(G) has completed: then a softmax that sees S(G + 2) also knows that P buffer
-    // G & 1 has been read and may be overwritten, as it did when one thread issued S(G + 2) behind PV(G).
-    if (lane == 0) {
-      const uint32_t idesc_s = idesc_f16(F16 ? 0u : 1u, AT_BN);
-      const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;
-      uint32_t it = 0, j = 0;
-      for (uint32_t G = 0; G < total; ++G) {                               // issues S(G)
-        if (j == 0 && !mbar_wait(&q_full[it & 1], (it >> 1) & 1, ctx, 12)) break;   // the operands first: they land long before PV(G - 2) completes
-        if (!mbar_wait(&k_full[G % AT_KV], (G / AT_KV) & 1, ctx, 13)) break;
-        if (G >= 2 && !mbar_wait(&o_full[G & 1], ((G - 2) >> 1) & 1, ctx, 20)) break;   // PV(G - 2); the barrier's next completion, PV(G), needs this S(G)
-        tc_fence_after();
-        const uint64_t qdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_Q + (it & 1) * AT_QTILE));
-        const uint64_t kdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_K + (G % AT_KV) * AT_KTILE));
-        const uint32_t t_s = tmem_base + AT_COL_S + (G & 1) * AT_BN;
+    // A second issuing warp.  S(G + 2) goes into the S buffer that the softmax of step G has read, once PV(G) has completed:
+    // then a softmax that sees S(G + 2) also knows that P buffer G & 1 has been read and may be overwritten.
+    const uint32_t idesc_s = idesc_f16(F16 ? 0u : 1u, AT_BN);
+    const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;
+    uint32_t it = 0, j = 0;
+    for (uint32_t G = 0; G < total; ++G) {                                 // issues S(G)
+      if (j == 0 && !mbar_wait_warp(&q_full[it & 1], (it >> 1) & 1, ctx, 12)) break;   // the operands first: they land long before PV(G - 2) completes
+      if (!mbar_wait_warp(&k_full[G % AT_KV], (G / AT_KV) & 1, ctx, 13)) break;
+      if (G >= 2 && !mbar_wait_warp(&o_full[G & 1], ((G - 2) >> 1) & 1, ctx, 20)) break;   // PV(G - 2); the barrier's next completion, PV(G), needs this S(G)
+      tc_fence_after();
+      const uint64_t qdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_Q + (it & 1) * AT_QTILE));
+      const uint64_t kdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_K + (G % AT_KV) * AT_KTILE));
+      const uint32_t t_s = tmem_base + AT_COL_S + (G & 1) * AT_BN;
+      const bool last = j + 1 == (uint32_t)n_kt;
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) mma_f16(t_s, qdesc + 2 * kk, kdesc + 2 * kk, idesc_s, kk != 0);
         tc_commit(&s_full[G & 1]);
-        if (++j == (uint32_t)n_kt) {
-          tc_commit(&q_empty[it & 1]);                                     // the item's last S product: its Q buffer is free once it completes
-          j = 0;
-          ++it;
-        }
+        if (last) tc_commit(&q_empty[it & 1]);                             // the item's last S product: its Q buffer is free once it completes
+      }
+      __syncwarp();
+      if (++j == (uint32_t)n_kt) {
+        j = 0;
+        ++it;
       }
     }
-    __syncwarp();
   }   // warp 7 is idle: it completes the second warp group, whose registers go to the softmax warps
   } else {
     setmaxnreg_inc<AT_REGS_SOFTMAX>();
