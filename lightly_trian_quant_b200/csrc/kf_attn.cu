@@ -6,21 +6,28 @@
 //   CTA      persistent, two per SM; an item is 128 query rows of one (batch, head), key tiles of 64; a CTA takes the
 //            items blockIdx.x, blockIdx.x + gridDim.x, ... and keeps every barrier phase running across them
 //   roles    warps 0..3: softmax, one query row per thread (tcgen05.ld of the S row, running max / sum in fp32,
-//            P -> 16 bit -> tensor memory by tcgen05.st); warp 4: TMA producer (Q in two buffers, K / V in a 4-deep
-//            ring, 4-D tensor maps so rows past N read zero); warp 5 issues the PV products (O += P V: 4 MMAs of K=16
-//            with P as the A operand from tensor memory and V as the MN-major B operand), warp 6 the S products
-//            (S = Q K^T: 4 MMAs of K=16 from shared memory); warp 7 idles (it completes the second warp group, whose
-//            registers setmaxnreg hands to the softmax warps: 200 against 56).  The issuing warps run
-//            warp-uniform loops with one elected lane per instruction (kf_sm100.cuh); as one-lane loops they spent ~55 clk
-//            per MMA and ~80 per commit (bf16 B 14, N 1605, quantise-out: 236 -> 214 us; f16 B 8, N 4101: 806 -> 691 us).
-//            Each waits for its operands first and for the hand-over last.
-//   pipeline S and P are double buffered in TMEM: S(j+2) is issued when PV(j) has completed (so a softmax that sees
-//            S(j+2) knows that P buffer j & 1 has been read), also across the end of an item (the next item's Q and
-//            first K tiles are loaded by then).  O accumulates in TMEM over all key tiles.  The exponentials of a tile
+//            P -> 16 bit -> tensor memory by tcgen05.st); warp 4: TMA producer (Q in two buffers, K and V in 4-deep
+//            rings, 4-D tensor maps so rows past N read zero); warp 5 issues the products (S = Q K^T: 4 MMAs of K=16
+//            from shared memory; O += P V: 4 MMAs of K=16 with P as the A operand from tensor memory and V as the
+//            MN-major B operand); warps 6 and 7 idle (they complete the second warp group, whose registers setmaxnreg
+//            hands to the softmax warps: 200 against 56).
+//   pipeline three S buffers in tensor memory, P(j) written over the first half of S(j); O accumulates over all key
+//            tiles.  One thread issues PV(j) and then S(j+3) into the same buffer: the tensor core runs them in order,
+//            so nothing waits for PV(j) to complete, and S runs two steps ahead of the softmax, also across the end of an
+//            item (the next item's Q and first K tiles are loaded by then).  The softmax warps request the next S row as
+//            soon as the registers of the present one are free and ask for its barrier half a step before they look at
+//            the answer: what bounds the kernel is their instruction stream (two of them per scheduler take 983 clk per
+//            64-key step of both in a loop of nothing else, ~1150 here: the exponentials' unit is busy for 768 of them).
+//            The exponentials of a tile
 //            use the running maximum as it is; the tile's own row sum tells whether that was safe (below 2^15 no
 //            element exceeded 2^15), so no maximum is tracked in the common case; only a row whose sum came out larger
 //            finds its maximum, recomputes its P and has its O rescaled (TMEM load, multiply, store), which happens on
 //            the first tiles and then almost never; the O barriers are waited only then and at the end of an item.
+//            Measured (B 14, H 16, NVFP4 out, N 1605 / 1805; B 8, N 4101, f16, MXFP4 out; B 1, N 1605): 200 / 246 / 664 /
+//            25.8 us, against 214 / 264 / 691 / 28.3 us with an issuing warp for each product and S(j+2) behind the
+//            completion of PV(j).  Level with that, and not kept: four CTAs per SM with one S buffer each (202 / 245 /
+//            680 / 34 us), two softmax warps per row with an O each (209 / 258 / 673 / 28 us); the end of a step spread
+//            over the exponentials of the next one broke those into pieces too small to overlap (241 / 296 / 793 / 35 us).
 //   numerics softmax scale 1/8 folded into exp2 (fp32; three of every four element pairs by the special-function unit,
 //            the fourth by a cubic on the FMA pipe: the unit is shared by the softmax warps of both CTAs and is the
 //            busiest pipe of the step; more than a quarter costs more issue slots than it frees); the exponent
@@ -37,7 +44,7 @@
 namespace kf {
 
 constexpr int AT_BM = 128, AT_BN = 64, AT_D = 64;
-constexpr int AT_THREADS = 256;                        // warps 0..3 softmax, 4 TMA, 5 PV issuer, 6 S issuer, 7 idle
+constexpr int AT_THREADS = 256;                        // warps 0..3 softmax, 4 TMA, 5 MMA issuer, 6 and 7 idle
 constexpr int AT_REGS_SOFTMAX = 200, AT_REGS_LEAN = 56; // 128 * 200 + 128 * 56 <= 256 * 128, the allocation at launch
 constexpr int AT_KV = 4;                               // K / V ring depth
 constexpr int AT_QTILE = AT_BM * AT_D * 2;             // 16 KB
@@ -45,8 +52,9 @@ constexpr int AT_KTILE = AT_BN * AT_D * 2;             // 8 KB
 constexpr int AT_OFF_Q = 0, AT_OFF_K = 2 * AT_QTILE, AT_OFF_V = AT_OFF_K + AT_KV * AT_KTILE, AT_OFF_BAR = AT_OFF_V + AT_KV * AT_KTILE;
 constexpr size_t AT_SMEM = (size_t)AT_OFF_BAR + 256;
 constexpr float AT_SUM_LIMIT = 32768.f;                  // a tile's row sum above this sends the row to the exact-maximum path (the largest finite f16 is 65504)
-constexpr int AT_POLY_K = 3;                             // which of every four element pairs takes the polynomial exponential
-constexpr int AT_TMEM_COLS = 256, AT_COL_S = 0, AT_COL_O = 128, AT_COL_P = 192;   // S buffers at columns 0 and 64, P (16-bit pairs) at 192 and 224
+constexpr int AT_POLY_K = 3;                             // element pairs AT_POLY_K .. 3 of every four take the polynomial exponential
+constexpr int AT_SBUF = 3;                               // S buffers in tensor memory
+constexpr int AT_TMEM_COLS = 256, AT_COL_S = 0, AT_COL_O = AT_SBUF * 64;   // P (16-bit pairs, 32 columns) replaces the first half of its S buffer
 
 struct AttnArgs {
   void* O;
@@ -100,15 +108,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const __grid_constant__ AttnArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + AT_OFF_BAR);
-  uint64_t *q_full = bars, *q_empty = bars + 2, *k_full = bars + 4, *v_full = k_full + AT_KV, *kv_empty = v_full + AT_KV, *s_full = kv_empty + AT_KV,
-           *p_full = s_full + 2, *o_full = p_full + 2;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 2);
+  uint64_t *q_full = bars, *q_empty = bars + 2, *k_full = bars + 4, *k_empty = k_full + AT_KV, *v_full = k_empty + AT_KV, *v_empty = v_full + AT_KV,
+           *s_full = v_empty + AT_KV, *p_full = s_full + AT_SBUF, *o_full = p_full + AT_SBUF;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + AT_SBUF);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   pdl_launch_dependents();                               // the next kernel of the stream may take the SMs this grid leaves
   const int warp = warp_index(), lane = threadIdx.x & 31;
   // Persistent: this CTA works through the (image, head, query tile) items blockIdx.x, blockIdx.x + gridDim.x, ...  All
-  // barriers keep running across items: K / V ring stages, S / P buffers and the O barrier are indexed by the CTA's global
+  // barriers keep running across items: K / V ring stages, S / P buffers and the O barriers are indexed by the CTA's global
   // key-tile count G, the two Q buffers by the item count, so the loads and the first S products of the next item are
   // under way while the current one finishes and writes its output.
   const int q_tiles = (a.N + AT_BM - 1) / AT_BM;
@@ -135,15 +143,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     for (int i = 0; i < AT_KV; ++i) {
       mbar_init(&k_full[i], 1);
+      mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
+      mbar_init(&v_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < AT_SBUF; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 128);
+      mbar_init(&o_full[i], 1);                           // PV(G) completes o_full[G % 3]: a waiter is never more than one phase behind
     }
-    mbar_init(&o_full[0], 1);                             // PV(G) completes o_full[G & 1]: a waiter is never more than one phase behind
-    mbar_init(&o_full[1], 1);
     *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;   // the swizzled tiles need a 1024-byte aligned base
     fence_mbar_init();
   }
@@ -186,10 +194,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       for (int j = 0; j < n_kt; ++j, ++G) {
         const int st = G % AT_KV;
-        if (!mbar_wait_warp(&kv_empty[st], ((G / AT_KV) & 1) ^ 1, ctx, 11)) { ok = false; break; }
+        const uint32_t ph = ((G / AT_KV) & 1) ^ 1;
+        if (!mbar_wait_warp(&k_empty[st], ph, ctx, 11)) { ok = false; break; }      // S(G - AT_KV) is complete
         if (elect_one()) {
           mbar_expect_tx(&k_full[st], AT_KTILE);
           tma_load_4d(smem + AT_OFF_K + st * AT_KTILE, &tmK, 0, I.h, j * AT_BN, I.b, &k_full[st]);
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(&v_empty[st], ph, ctx, 15)) { ok = false; break; }      // PV(G - AT_KV) is complete
+        if (elect_one()) {
           mbar_expect_tx(&v_full[st], AT_KTILE);
           tma_load_4d(smem + AT_OFF_V + st * AT_KTILE, &tmV, 0, I.h, j * AT_BN, I.b, &v_full[st]);
         }
@@ -197,57 +210,67 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 5) {
-    // ------------------------------------------------------------------ issuer of the PV products
+    // ------------------------------------------------------------------ MMA issuer
+    // S(0), S(1), S(2), then PV(G) and S(G + 3) for every step.  All come from one thread, so the tensor core runs them in
+    // order: S(G + 3) overwrites the buffer of P(G) behind PV(G) without a wait for its completion.  A softmax that sees
+    // S(G + 3) complete knows that PV(G) is.  S runs two steps ahead of the softmax: issued one step ahead (two buffers) it
+    // came ~700 clk after the hand-over of P, in the middle of the step that wants to prefetch it.
+    const uint32_t idesc_s = idesc_f16(F16 ? 0u : 1u, AT_BN);
     const uint32_t idesc_o = idesc_f16(F16 ? 0u : 1u, AT_D) | (1u << 16);     // B (= V) is MN-major
     const uint32_t t_o = tmem_base + AT_COL_O;
     const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;                  // key-tile steps of this CTA over all its items
-    uint32_t j = 0;
-    for (uint32_t G = 0; G < total; ++G) {
-      const uint32_t st = G % AT_KV;
-      if (!mbar_wait_warp(&v_full[st], (G / AT_KV) & 1, ctx, 15)) break;   // V lands long before P: its barrier round trip is off the chain P -> PV -> S
-      if (!mbar_wait_warp(&p_full[G & 1], (G >> 1) & 1, ctx, 14)) break;
+    const bool leader = elect_one();
+    uint32_t s_it = 0, s_j = 0;                                              // item and key tile of the next S product
+    auto issue_s = [&](uint32_t G, uint32_t buf) {
+      const uint64_t qdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_Q + (s_it & 1) * AT_QTILE));
+      const uint64_t kdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_K + (G % AT_KV) * AT_KTILE));
+      const uint32_t t_s = tmem_base + AT_COL_S + buf * AT_BN;
+      const bool last = s_j + 1 == (uint32_t)n_kt;
+      if (leader) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) mma_f16(t_s, qdesc + 2 * kk, kdesc + 2 * kk, idesc_s, kk != 0);
+        tc_commit(&s_full[buf]);
+        tc_commit(&k_empty[G % AT_KV]);
+        if (last) tc_commit(&q_empty[s_it & 1]);                             // the item's last S product: its Q buffer is free once it completes
+      }
+      __syncwarp();
+      if (++s_j == (uint32_t)n_kt) {
+        s_j = 0;
+        ++s_it;
+      }
+    };
+    bool ok = true;
+    for (uint32_t G = 0; G < AT_SBUF && G < total && ok; ++G) {
+      ok = (s_j != 0 || mbar_wait_warp(&q_full[s_it & 1], (s_it >> 1) & 1, ctx, 12)) && mbar_wait_warp(&k_full[G], 0, ctx, 13);
       tc_fence_after();
-      const uint32_t t_p = tmem_base + AT_COL_P + (G & 1) * (AT_BN / 2);
+      if (ok) issue_s(G, G);
+    }
+    uint32_t j = 0, buf = 0, pph = 0;                                        // buffer of step G and the parity of its P barrier
+    for (uint32_t G = 0; G < total && ok; ++G) {
+      const uint32_t st = G % AT_KV, g3 = G + AT_SBUF;
+      const bool more = g3 < total;
+      if (more && s_j == 0 && !mbar_wait_warp(&q_full[s_it & 1], (s_it >> 1) & 1, ctx, 12)) break;
+      // P(G), V(G) and K(G + 3), asked for together: a barrier costs a round trip of 60 clk also when its phase is complete
+      if (!mbar_wait_warp3(&p_full[buf], pph, &v_full[st], (G / AT_KV) & 1, &k_full[(more ? g3 : G) % AT_KV], ((more ? g3 : G) / AT_KV) & 1, ctx, 14)) break;
+      tc_fence_after();
+      const uint32_t t_p = tmem_base + AT_COL_S + buf * AT_BN;
       const uint64_t vdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_V + st * AT_KTILE));
-      if (elect_one()) {
+      if (leader) {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)         // A: 16 keys = 8 TMEM columns of P; B: 16 key rows of V = two 8-row groups of 1024 bytes
           mma_f16_ta(t_o, t_p + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (j | (uint32_t)kk) != 0);
-        tc_commit(&o_full[G & 1]);
-        tc_commit(&kv_empty[st]);              // K of this stage was read by S(G), which completed before the softmax of step G began
+        tc_commit(&o_full[buf]);
+        tc_commit(&v_empty[st]);
       }
       __syncwarp();
+      if (more) issue_s(g3, buf);
       if (++j == (uint32_t)n_kt) j = 0;
-    }
-  } else if (warp == 6) {
-    // ------------------------------------------------------------------ issuer of the S products
-    // A second issuing warp.  S(G + 2) goes into the S buffer that the softmax of step G has read, once PV(G) has completed:
-    // then a softmax that sees S(G + 2) also knows that P buffer G & 1 has been read and may be overwritten.
-    const uint32_t idesc_s = idesc_f16(F16 ? 0u : 1u, AT_BN);
-    const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;
-    uint32_t it = 0, j = 0;
-    for (uint32_t G = 0; G < total; ++G) {                                 // issues S(G)
-      if (j == 0 && !mbar_wait_warp(&q_full[it & 1], (it >> 1) & 1, ctx, 12)) break;   // the operands first: they land long before PV(G - 2) completes
-      if (!mbar_wait_warp(&k_full[G % AT_KV], (G / AT_KV) & 1, ctx, 13)) break;
-      if (G >= 2 && !mbar_wait_warp(&o_full[G & 1], ((G - 2) >> 1) & 1, ctx, 20)) break;   // PV(G - 2); the barrier's next completion, PV(G), needs this S(G)
-      tc_fence_after();
-      const uint64_t qdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_Q + (it & 1) * AT_QTILE));
-      const uint64_t kdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_K + (G % AT_KV) * AT_KTILE));
-      const uint32_t t_s = tmem_base + AT_COL_S + (G & 1) * AT_BN;
-      const bool last = j + 1 == (uint32_t)n_kt;
-      if (elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) mma_f16(t_s, qdesc + 2 * kk, kdesc + 2 * kk, idesc_s, kk != 0);
-        tc_commit(&s_full[G & 1]);
-        if (last) tc_commit(&q_empty[it & 1]);                             // the item's last S product: its Q buffer is free once it completes
-      }
-      __syncwarp();
-      if (++j == (uint32_t)n_kt) {
-        j = 0;
-        ++it;
+      if (++buf == AT_SBUF) {
+        buf = 0;
+        pph ^= 1;
       }
     }
-  }   // warp 7 is idle: it completes the second warp group, whose registers go to the softmax warps
+  }   // warps 6 and 7 are idle: they complete the second warp group, whose registers go to the softmax warps
   } else {
     setmaxnreg_inc<AT_REGS_SOFTMAX>();
     if (!bad_align) {
@@ -256,112 +279,135 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t t_lane = tmem_base + ((uint32_t)(warp * 32) << 16);
     const float sc = a.scale_log2;
     bool ok = true;
-    uint32_t G = 0;                                              // key-tile steps of this CTA so far, over all its items
+    uint32_t buf = 0, sph = 0;                                   // the next step's S buffer and the parity of its barriers
     // per-tensor scale of an NVFP4 output, its reciprocal and range check: one L2 round trip per CTA, not per item
     const Nv4Scale tsc = nv4_scale(OUT == KF_FMT_NV4 ? __ldg(a.tso) : 1.f);
+    const float2 sc2 = splat2(sc);
+    // P = exp2(s*sc + mneg) of 32 keys as 16-bit pairs; adds the row sum to s0 / s1.  The exponent arguments and the row
+    // sums run as packed pairs: half the issue slots of the scalar form.
+    auto exp_half = [&](const uint32_t (&r)[32], uint32_t* w, float2 mn2, float2& s0, float2& s1) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float2 p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 t = fma2(make_float2(__uint_as_float(r[8 * i + 2 * k]), __uint_as_float(r[8 * i + 2 * k + 1])), sc2, mn2);
+          p[k] = k >= AT_POLY_K ? ex2_poly2(t) : make_float2(ex2(t.x), ex2(t.y));   // one pair in four off the special-function unit
+        }
+        s0 = add2(s0, add2(p[0], p[1]));
+        s1 = add2(s1, add2(p[2], p[3]));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[4 * i + k] = pack16(p[k].x, p[k].y, F16);
+      }
+    };
+    auto row_max = [](const uint32_t (&r)[32], float mx) {
+      float m4[4] = {mx, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < 16; ++i) m4[i & 3] = max3(m4[i & 3], __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+    };
+    auto mask_tail = [&](uint32_t (&r)[32], int key0) {          // columns past N never win the max and give P = 0
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (key0 + i >= a.N) r[i] = 0xff800000u;
+    };
     for (int it = 0; it < n_my && ok; ++it) {
     const Item I = item_of(it);
     const int qt = I.qt, h = I.h, b = I.b;
-    float m_run = -INFINITY, l_run = 0.f;
-    for (int j = 0; j < n_kt; ++j, ++G) {
-      const int sb = G & 1;
-      if (!mbar_wait(&s_full[sb], (G >> 1) & 1, ctx, 17)) { ok = false; break; }
-      tc_fence_after();
-      const int kbase = j * AT_BN;
-      uint32_t r[2][32];
-      tmem_ld32(t_lane + AT_COL_S + sb * AT_BN, r[0]);
-      tmem_ld32(t_lane + AT_COL_S + sb * AT_BN + 32, r[1]);
-      tmem_ld_wait();
-      if (kbase + AT_BN > a.N) {                                // key tail: columns past N never win the max and give P = 0
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (kbase + c * 32 + i >= a.N) r[c][i] = 0xff800000u;
+    float m_run = 0.f, l_run = 0.f;
+    uint32_t ra[32], rb[32];                                     // the S row of this step: keys 0..31 and 32..63 of the tile
+    ok = mbar_wait(&s_full[buf], sph, ctx, 17);
+    if (!ok) break;
+    tc_fence_after();
+    tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
+    tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
+    for (int j = 0; j < n_kt; ++j) {
+      const uint32_t t_s = t_lane + AT_COL_S + buf * AT_BN, cur = buf, cph = sph;
+      if (++buf == AT_SBUF) {
+        buf = 0;
+        sph ^= 1;
       }
-      // the P row of this tile goes to tensor memory (the A operand of the PV product): 64 keys = 32 columns of 16-bit pairs
-      const uint32_t t_p = t_lane + AT_COL_P + sb * (AT_BN / 2);
-      // P = exp2(s*sc + mneg) into tensor memory; returns the row sum.  The exponent arguments and the row sum run as
-      // packed pairs: half the issue slots of the scalar form.
-      auto exp_row = [&](auto is_f16, float mneg) -> float {
-        constexpr int F = decltype(is_f16)::value;
-        const float2 sc2 = splat2(sc), mn2 = splat2(mneg);
-        float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t w[16];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float2 p[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float2 t = fma2(make_float2(__uint_as_float(r[c][8 * i + 2 * k]), __uint_as_float(r[c][8 * i + 2 * k + 1])), sc2, mn2);
-              p[k] = k == AT_POLY_K ? ex2_poly2(t) : make_float2(ex2(t.x), ex2(t.y));   // one pair in four off the special-function unit
-            }
-            s0 = add2(s0, add2(p[0], p[1]));
-            s1 = add2(s1, add2(p[2], p[3]));
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[4 * i + k] = pack16(p[k].x, p[k].y, F);
-          }
-          tmem_st16(t_p + 16 * c, w);
-        }
-        return (s0.x + s0.y) + (s1.x + s1.y);
-      };
-      auto run = [&](float mneg) -> float {
-        return exp_row(std::integral_constant<int, F16>{}, mneg);
-      };
+      const bool prefetch = j + 1 < n_kt;                        // the next step of this item
+      const int kbase = j * AT_BN;
+      // asked for here, looked at half a step later: S(G + 1) was issued more than a step ago and is nearly always there
+      const bool ready = mbar_test_wait(&s_full[buf], sph);
+      tmem_ld_wait();
+      tmem_ld_fence(ra);
+      tmem_ld_fence(rb);
+      if (kbase + AT_BN > a.N) {
+        mask_tail(ra, kbase);
+        mask_tail(rb, kbase + 32);
+      }
+      if (j == 0) m_run = row_max(rb, row_max(ra, -INFINITY));
+      const float2 mn2 = splat2(-m_run * sc);
+      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+      uint32_t w[32];
+      exp_half(ra, w, mn2, s0, s1);
+      // The next step's S row is requested as soon as the registers of this one are free
+      if (prefetch) {
+        if (!ready && !mbar_wait(&s_full[buf], sph, ctx, 17)) { ok = false; break; }
+        __syncwarp();
+        tc_fence_after();
+        tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
+      }
+      exp_half(rb, w + 16, mn2, s0, s1);
+      if (prefetch) tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
       // Lazy maximum without a maximum: the exponentials of tile j > 0 use the running maximum as it is, and the tile's
       // own row sum tells whether that was safe: while it stays below 2^15 no element exceeded 2^15 (bf16 / f16 P, the
       // fp32 sums and O have room for that), so the maximum of the tile is not needed at all.  Only a row whose sum came
       // out larger (or infinite) finds its maximum, raises the running maximum, recomputes its P and has its O rescaled.
       // The first tile has no running maximum yet and finds its own first.
-      float sum = 0.f, alpha = 1.f;
-      bool need = true;
-      if (j > 0) {
-        sum = run(-m_run * sc);
-        need = sum > AT_SUM_LIMIT;
-      }
-      const uint32_t any_need = __ballot_sync(0xffffffffu, need);
-      if (any_need) {                                            // warp-uniform: the tensor-memory stores need the whole warp
+      float sum = (s0.x + s0.y) + (s1.x + s1.y), alpha = 1.f;
+      const bool need = sum > AT_SUM_LIMIT;
+      if (__any_sync(0xffffffffu, need)) {                    // warp-uniform; S is still in tensor memory: P replaces it only below
+        uint32_t r[32];
+        float mx = m_run;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld32(t_s + 32 * c, r);
+          tmem_ld_wait();
+          tmem_ld_fence(r);
+          if (kbase + AT_BN > a.N) mask_tail(r, kbase + 32 * c);
+          mx = row_max(r, mx);
+        }
         if (need) {
-          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-          for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) mx4[i & 3] = max3(mx4[i & 3], __uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1]));
-          const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-          if (mx > m_run) {
-            alpha = ex2((m_run - mx) * sc);                      // 0 on the first tile
-            m_run = mx;
-          }
+          alpha = ex2((m_run - mx) * sc);
+          m_run = mx;
         }
-        sum = run(-m_run * sc);
-      }
-      const uint32_t any = j > 0 ? any_need : 0u;
-      l_run = l_run * alpha + sum;
-      // O is only touched when a row of this warp raised its maximum: PV(G-1) must have landed first.  It completes
-      // o_full[(G-1) & 1], whose next completion, PV(G+1), cannot come before this thread's arrivals of steps G and G+1.
-      // The item's last step always waits, so that the epilogue's wait for the last product is covered as well.
-      if ((any || j == n_kt - 1) && j > 0 && !mbar_wait(&o_full[(G - 1) & 1], ((G - 1) >> 1) & 1, ctx, 18)) { ok = false; break; }
-      if (any) {                                                 // rescale O in TMEM
+        s0 = s1 = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld32(t_s + 32 * c, r);
+          tmem_ld_wait();
+          tmem_ld_fence(r);
+          if (kbase + AT_BN > a.N) mask_tail(r, kbase + 32 * c);
+          if (c == 0) exp_half(r, w, splat2(-m_run * sc), s0, s1);
+          else exp_half(r, w + 16, splat2(-m_run * sc), s0, s1);
+        }
+        sum = (s0.x + s0.y) + (s1.x + s1.y);
+        // rescale O in tensor memory: PV(G - 1) must have landed first (j > 0: the first tile's sum is at most 64).  Its
+        // barrier's previous completion, PV(G - 4), is covered by S(G), which this step has read.
+        const uint32_t pb = cur == 0 ? AT_SBUF - 1 : cur - 1;
+        if (!mbar_wait(&o_full[pb], cur == 0 ? cph ^ 1 : cph, ctx, 18)) { ok = false; break; }
         tc_fence_after();
-        tmem_ld32(t_lane + AT_COL_O, r[0]);
-        tmem_ld32(t_lane + AT_COL_O + 32, r[1]);
-        tmem_ld_wait();
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld32(t_lane + AT_COL_O + 32 * c, r);
+          tmem_ld_wait();
+          tmem_ld_fence(r);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          r[0][i] = __float_as_uint(__uint_as_float(r[0][i]) * alpha);
-          r[1][i] = __float_as_uint(__uint_as_float(r[1][i]) * alpha);
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+          tmem_st32(t_lane + AT_COL_O + 32 * c, r);
         }
-        tmem_st32(t_lane + AT_COL_O, r[0]);
-        tmem_st32(t_lane + AT_COL_O + 32, r[1]);
-        tmem_st_wait();
       }
+      l_run = l_run * alpha + sum;
+      tmem_st32(t_s, w);                                         // the A operand of the PV product: 64 keys = 32 columns of 16-bit pairs
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&p_full[sb]);
+      mbar_arrive(&p_full[cur]);
     }
-    if (ok) ok = mbar_wait(&o_full[(G - 1) & 1], ((G - 1) >> 1) & 1, ctx, 19);     // the item's last PV product
+    // the item's last PV product; its barrier's previous completion, PV(G - 4), is covered by S(G - 1), which has been read
+    if (ok) ok = mbar_wait(&o_full[buf == 0 ? AT_SBUF - 1 : buf - 1], buf == 0 ? sph ^ 1 : sph, ctx, 19);
     const int n = qt * AT_BM + row;
     if (ok) {
       tc_fence_after();

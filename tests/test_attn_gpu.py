@@ -110,3 +110,16 @@ def test_attn_fused_quantise_out(fmt):
     eq, es, _ = qo.quantize(on, fmt, ts)
     assert np.array_equal(out.q.cpu().numpy(), eq)
     assert np.array_equal(out.sf.cpu().numpy(), qo.to_blocked(es).reshape(-1))
+
+
+@pytest.mark.parametrize("B,N,H", [(1, 1, 1), (40, 1, 16), (40, 64, 16), (3, 65, 2), (40, 128, 9), (2, 129, 3), (1, 192, 2), (20, 193, 16), (1, 257, 5)])
+def test_attn_tile_edges_and_items_shorter_than_the_pipeline(B, N, H):
+    """token counts around the 64-key and 128-query tiles, and items of one to three key tiles in a CTA that works through
+    several: S runs ahead of the softmax across item boundaries."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(B + N)
+    qkv = (torch.randn(3, B, N, H, 64, generator=g) * 1.5).to(torch.bfloat16)
+    out = ops.attn_fwd(qkv.cuda())
+    ops.check_device_error()
+    err = go.rel_fro(out.float().cpu().numpy(), ao.attn_ref(qkv.float().numpy()))
+    assert err < 4e-3, err
