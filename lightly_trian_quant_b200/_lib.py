@@ -83,6 +83,18 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def host():
+    """The native operator module over the library (csrc/host/kf_host.cpp)."""
+    lib()                                   # a missing library is reported first
+    try:
+        import torch  # noqa: F401          (its shared libraries are the module's)
+
+        from . import _kf_host
+    except ImportError as e:
+        raise KfError(f"native operator module not built or not loadable ({e}): run `python -m lightly_trian_quant_b200.build` (no fallback path exists)") from e
+    return _kf_host
+
+
 def check(status: int, what: str) -> None:
     if status != 0:
         msg = lib().kf_last_error_string().decode()

@@ -520,18 +520,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // 4-D tensor map over one of q / k / v: dims (64, H, N, B) of 16-bit elements, box (64, 1, rows, 1), 128-byte swizzle;
-// rows past N are out of bounds in their own dimension and read as zero.
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
+// rows past N are out of bounds in their own dimension and read as zero.  Encoding costs about a microsecond of host time and
+// a layer stack asks for the same few maps over and over: kept per thread, direct-mapped by their arguments.
 static int make_tmap_qkv(CUtensorMap* map, const void* base, int B, int N, int H, int box_rows) {
-  void* p = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess || !p) {
+  struct Slot {
+    const void* base;
+    int B, N, H, box_rows;
+    CUtensorMap map;
+  };
+  constexpr int SLOTS = 64;
+  static thread_local Slot cache[SLOTS] = {};
+  const uintptr_t h = (reinterpret_cast<uintptr_t>(base) >> 8) * 0x9E3779B97F4A7C15ull + (uintptr_t)N * 31 + (uintptr_t)B * 7 + (uintptr_t)box_rows;
+  Slot& slot = cache[(h >> 32 ^ h) % SLOTS];
+  if (slot.base == base && slot.B == B && slot.N == N && slot.H == H && slot.box_rows == box_rows) {
+    *map = slot.map;
+    return KF_OK;
+  }
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return KF_ERR_UNSUPPORTED;
   }
-  EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(p);
   cuuint64_t dims[4] = {64, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)B};
   cuuint64_t strides[3] = {128, (cuuint64_t)H * 128, (cuuint64_t)N * H * 128};
   cuuint32_t box[4] = {64, 1, (cuuint32_t)box_rows, 1};
@@ -542,6 +551,7 @@ static int make_tmap_qkv(CUtensorMap* map, const void* base, int B, int N, int H
     set_error("cuTensorMapEncodeTiled (qkv) failed with CUresult %d", (int)r);
     return KF_ERR_BAD_ARGUMENT;
   }
+  slot = Slot{base, B, N, H, box_rows, *map};
   return KF_OK;
 }
 

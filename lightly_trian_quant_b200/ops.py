@@ -9,7 +9,8 @@ Reference counterparts (paths relative to the reference checkout):
 
 Every operator launches on torch's current CUDA stream through the C-ABI, never synchronises and never
 falls back to another implementation: a missing library or a failed launch raises KfError.
-torch is used for device memory and streams only.
+torch is used for device memory and streams only.  The argument checks, the output allocation and the call itself are native
+(csrc/host/kf_host.cpp): in Python they took 12 to 16 us per operator, longer than most kernels of a small model.
 """
 from __future__ import annotations
 
@@ -18,7 +19,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import KF_DT, KF_EPI, KF_FMT, KF_G_GELU, KF_Q_GELU, KF_Q_RECIP_DIV, KF_Q_ROUND_BF16, GemmParams, KfError, check
+from ._lib import KF_DT, KF_FMT, KF_G_GELU, KF_Q_GELU, KF_Q_RECIP_DIV, KF_Q_ROUND_BF16, KfError, check
 
 VEC = {"mx8": 32, "nv4": 16, "mx4": 32}
 
@@ -30,20 +31,37 @@ TIMING = None
 BYTES: dict = {}
 
 
-def _run(name: str, call, nbytes: int = 0) -> None:
+class _NativeHost:
+    """Stands in for the native operator module until the first operator is called, so that this module imports without it."""
+
+    def __getattr__(self, name):
+        global _h
+        _h = _lib.host()
+        return getattr(_h, name)
+
+
+_h = _NativeHost()
+
+
+def _timed(name: str, fn, args: tuple, nbytes: int = 0):
+    """fn(*args) between two CUDA events, under the name of its kernel class (TIMING is a dict)."""
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    r = fn(*args)
+    e1.record()
+    TIMING.setdefault(name, []).append((e0, e1))
+    if nbytes:
+        BYTES[name] = BYTES.get(name, 0) + nbytes
+    return r
+
+
+def _run(name: str, call) -> None:
+    """A launch through the ctypes binding (the operators that are called once per frame)."""
     global LAUNCHES
     LAUNCHES += 1
-    if TIMING is not None:
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        st = call()
-        e1.record()
-        TIMING.setdefault(name, []).append((e0, e1))
-        if nbytes:
-            BYTES[name] = BYTES.get(name, 0) + nbytes
-    else:
-        st = call()
-    check(st, name)
+    check(call() if TIMING is None else _timed(name, call, ()), name)
+
+
 _DT = {torch.float32: KF_DT["f32"], torch.bfloat16: KF_DT["bf16"], torch.float16: KF_DT["f16"]}
 
 
@@ -110,15 +128,12 @@ def quant_rows(x: torch.Tensor, out: ActBuf, *, bias: Optional[torch.Tensor] = N
                round_bf16: bool = False, recip_div: bool = False) -> ActBuf:
     """x [M, K] f32 | bf16 | f16 (last dim contiguous) -> out (codes + blocked scales), format out.fmt.
     gelu=True applies gelu_erf(x + bias) first (the reference's gelu_quant)."""
-    _need_cuda(x, out.q, bias)
-    if x.dim() != 2 or x.stride(1) != 1 or x.shape != (out.M, out.K):
-        raise KfError(f"quant_rows: x must be [M={out.M}, K={out.K}] with a contiguous last dim, got {tuple(x.shape)}")
-    if x.dtype not in _DT:
-        raise KfError(f"quant_rows: unsupported dtype {x.dtype}")
-    _run("quant_rows", lambda: _lib.lib().kf_quant_rows(KF_FMT[out.fmt], _DT[x.dtype], x.data_ptr(), x.stride(0), out.M, out.K, _ptr(out.ts),
-                                                        _ptr(bias), _flags(gelu, round_bf16, recip_div), out.q.data_ptr(), out.sf.data_ptr(), _stream()),
-         x.numel() * x.element_size() + out.q.numel() + out.sf.numel())
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (x, out, bias, _flags(gelu, round_bf16, recip_div))
+    if TIMING is None:
+        return _h.quant_rows(*args)
+    return _timed("quant_rows", _h.quant_rows, args, x.numel() * x.element_size() + out.q.numel() + out.sf.numel())
 
 
 def gelu_quant(y: torch.Tensor, bias: torch.Tensor, out: ActBuf, **kw) -> ActBuf:
@@ -132,15 +147,12 @@ def quantx(x: torch.Tensor, out: ActBuf, **kw) -> ActBuf:
 def ln_quant(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, out: ActBuf, *, round_bf16: bool = False,
              recip_div: bool = False, y_dbg: Optional[torch.Tensor] = None) -> ActBuf:
     """LayerNorm of the fp32 residual stream x [..., d] fused with quantisation into out (ln_mx8 / lnq)."""
-    _need_cuda(x, w, b, out.q)
-    d = x.shape[-1]
-    M = x.numel() // d
-    if x.dtype != torch.float32 or not x.is_contiguous() or (M, d) != (out.M, out.K):
-        raise KfError(f"ln_quant: x must be contiguous fp32 [M={out.M}, d={out.K}], got {tuple(x.shape)} {x.dtype}")
-    _run("ln_quant", lambda: _lib.lib().kf_ln_quant(KF_FMT[out.fmt], x.data_ptr(), w.data_ptr(), b.data_ptr(), float(eps), M, d, _ptr(out.ts),
-                                                    _flags(False, round_bf16, recip_div), out.q.data_ptr(), out.sf.data_ptr(), _ptr(y_dbg), _stream()),
-         x.numel() * 4 + out.q.numel() + out.sf.numel())
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (x, w, b, eps, out, _flags(False, round_bf16, recip_div), y_dbg)
+    if TIMING is None:
+        return _h.ln_quant(*args)
+    return _timed("ln_quant", _h.ln_quant, args, x.numel() * 4 + out.q.numel() + out.sf.numel())
 
 
 def ln_mx8(x, w, b, out: ActBuf, eps: float, **kw) -> ActBuf:
@@ -153,14 +165,10 @@ def lnq(x, w, b, eps: float, out: ActBuf, **kw) -> ActBuf:
 
 def ln_rows(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, dtype=torch.bfloat16) -> torch.Tensor:
     """LayerNorm of fp32 x [..., d] to a bf16 / f16 tensor of the same shape (ln_bf16 / ln16)."""
-    _need_cuda(x, w, b)
-    d = x.shape[-1]
-    M = x.numel() // d
-    if x.dtype != torch.float32 or not x.is_contiguous():
-        raise KfError("ln_rows: x must be contiguous fp32")
-    y = torch.empty(x.shape, dtype=dtype, device=x.device)
-    _run("ln_rows", lambda: _lib.lib().kf_ln_rows(x.data_ptr(), w.data_ptr(), b.data_ptr(), float(eps), M, d, _DT[dtype], y.data_ptr(), _stream()))
-    return y
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (x, w, b, eps, _DT[dtype])
+    return _h.ln_rows(*args) if TIMING is None else _timed("ln_rows", _h.ln_rows, args)
 
 
 ln_bf16 = ln_rows
@@ -209,51 +217,13 @@ class QWeight:
 MXW = QWeight
 
 
-def _gemm(a, W: QWeight, epi: str, *, bias=None, gamma=None, R=None, C=None, sin=None, cos=None, out: Optional[ActBuf] = None,
-          out_dtype=torch.bfloat16, gelu=False, round_bf16=False, recip_div=False, Ntok=0, prefix=0, H=0, tag="block", pre_round=False,
-          fast_nv4=False, y_dbg=None, rope_half=False, row_map=None):
-    p = GemmParams()
-    if isinstance(a, ActBuf):
-        if a.fmt != W.fmt or a.K != W.K:
-            raise KfError(f"gemm: operand mismatch A {a.fmt} K={a.K} vs W {W.fmt} K={W.K}")
-        M = a.M
-        p.A, p.SFA, p.ts_a = a.q.data_ptr(), a.sf.data_ptr(), _ptr(a.ts)
-    else:
-        if W.fmt != "bf16" or a.dtype != torch.bfloat16 or a.dim() != 2 or not a.is_contiguous() or a.shape[1] != W.K:
-            raise KfError("gemm: a plain tensor operand must be contiguous bf16 [M, K] with a bf16 weight")
-        _need_cuda(a)
-        M = a.shape[0]
-        p.A = a.data_ptr()
-    p.fmt, p.epi, p.M, p.N, p.K = KF_FMT[W.fmt], KF_EPI[epi], M, W.N, W.K
-    p.W, p.SFW, p.ts_w = W.q.data_ptr(), _ptr(W.sf), _ptr(W.ts)
-    p.out_dtype = _DT[out_dtype]
-    p.flags = (KF_G_GELU if gelu else 0) | (KF_Q_ROUND_BF16 if round_bf16 else 0) | (KF_Q_RECIP_DIV if recip_div else 0) \
-        | (_lib.KF_G_PRE_ROUND_BF16 if pre_round else 0) | (_lib.KF_Q_FAST_NV4 if fast_nv4 else 0) | (_lib.KF_G_ROPE_HALF if rope_half else 0)
-    p.Ntok, p.prefix, p.H = Ntok, prefix, H
-    _need_cuda(bias, gamma, R, C, sin, cos, y_dbg)
-    p.bias, p.gamma, p.R, p.sin, p.cos, p.C = _ptr(bias), _ptr(gamma), _ptr(R), _ptr(sin), _ptr(cos), _ptr(C)
-    p.y_dbg = _ptr(y_dbg)
-    if row_map is not None:
-        p.out_row_group, p.out_row_stride, p.out_row_offset = row_map
-    if out is not None:
-        p.out_fmt, p.Qo, p.SFo, p.tso = KF_FMT[out.fmt], out.q.data_ptr(), out.sf.data_ptr(), _ptr(out.ts)
-    _run(f"gemm_{tag}_{W.fmt}", lambda: _lib.lib().kf_gemm_bs(p, _stream()))
-
-
-def _f32c(t, n, what):
-    if t is not None and (t.dtype != torch.float32 or not t.is_contiguous() or t.numel() != n):
-        raise KfError(f"gemm: {what} must be contiguous fp32 with {n} elements")
-
-
 def gemm_plain(a, W: QWeight, bias=None, *, gelu: bool = False, out_dtype=torch.bfloat16, out: Optional[torch.Tensor] = None,
                tag: str = "block", pre_round: bool = False) -> torch.Tensor:
     """[M, N] = act(a @ W^T (* ts) + bias) in bf16 / f16 / f32 (mm, gemm_plain, fwd_bias, fwd_gelu, fwd_plain)."""
-    M = a.M if isinstance(a, ActBuf) else a.shape[0]
-    _f32c(bias, W.N, "bias")
-    if out is None:
-        out = torch.empty(M, W.N, dtype=out_dtype, device=W.q.device)
-    _gemm(a, W, "plain", bias=bias, C=out, out_dtype=out.dtype, gelu=gelu, tag=tag, pre_round=pre_round)
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (a, W, bias, out, _DT[out_dtype], (KF_G_GELU if gelu else 0) | (_lib.KF_G_PRE_ROUND_BF16 if pre_round else 0))
+    return _h.gemm_plain(*args) if TIMING is None else _timed(f"gemm_{tag}_{W.fmt}", _h.gemm_plain, args)
 
 
 mm = gemm_plain
@@ -263,55 +233,28 @@ def bmm_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
     """out[b] = a[b] @ w[b]^T for bf16 a [B, Q, K] and w [B, P, K] in one launch (P a multiple of 128): the mask product
     torch.bmm(h, u.transpose(1, 2)) of the head (infer-opt/round11_attn_tier0/impl/head11.py:95).  Bit-identical to B
     gemm_plain calls; one launch fills the SMs where a single image leaves a partial round of tiles."""
-    _need_cuda(a, w)
-    if a.dim() != 3 or w.dim() != 3 or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not a.is_contiguous() or not w.is_contiguous() \
-            or a.shape[0] != w.shape[0] or a.shape[2] != w.shape[2]:
-        raise KfError("bmm_nt: a [B, Q, K] and w [B, P, K] must be contiguous bf16 with equal B and K")
-    B, Q, K = a.shape
-    P = w.shape[1]
-    if out is None:
-        out = torch.empty(B, Q, P, dtype=torch.bfloat16, device=a.device)
-    elif out.shape != (B, Q, P) or out.dtype != torch.bfloat16 or not out.is_contiguous():
-        raise KfError(f"bmm_nt: out must be contiguous bf16 [{B}, {Q}, {P}]")
-    p = GemmParams()
-    p.fmt, p.epi, p.M, p.N, p.K = KF_FMT["bf16"], KF_EPI["plain"], B * Q, P, K
-    p.A, p.W, p.C = a.data_ptr(), w.data_ptr(), out.data_ptr()
-    p.out_dtype = _DT[torch.bfloat16]
-    p.batch, p.a_rows_per_batch, p.w_rows_per_batch = B, Q, P
-    _run(f"gemm_{tag}_bf16", lambda: _lib.lib().kf_gemm_bs(p, _stream()))
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (a, w, out)
+    return _h.bmm_nt(*args) if TIMING is None else _timed(f"gemm_{tag}_bf16", _h.bmm_nt, args)
 
 
 def gemm_res(a, W: QWeight, bias, gamma, res: torch.Tensor, out: Optional[torch.Tensor] = None, row_map=None) -> torch.Tensor:
     """fp32 [M, N] = res + gamma * (a @ W^T (* ts) + bias)   (proj / fc2; gemm_res, fwd_res).
     row_map = (group, stride, offset): row m of the result goes to row (m // group) * stride + offset + m % group of `out`
     (a longer token stream: the rows of each image land behind `offset` rows that are filled separately); not in place."""
-    M = a.M if isinstance(a, ActBuf) else a.shape[0]
-    _f32c(bias, W.N, "bias")
-    _f32c(gamma, W.N, "gamma")
-    _f32c(res, M * W.N, "res")
-    if out is None:
-        if row_map is not None:
-            raise KfError("gemm_res: a row mapping needs the output tensor")
-        out = torch.empty_like(res)
-    if out.dtype != torch.float32 or not out.is_contiguous():
-        raise KfError("gemm_res: out must be contiguous fp32")
-    if row_map is not None:
-        group, stride, offset = row_map
-        if M % group or out.numel() != (M // group) * stride * W.N or offset + group > stride:
-            raise KfError(f"gemm_res: row mapping {row_map} does not fit M={M} rows into {out.numel() // W.N} output rows")
-    _gemm(a, W, "res", bias=bias, gamma=gamma, R=res, C=out, out_dtype=torch.float32, row_map=row_map)
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (a, W, bias, gamma, res, out, row_map)
+    return _h.gemm_res(*args) if TIMING is None else _timed(f"gemm_block_{W.fmt}", _h.gemm_res, args)
 
 
 def broadcast_rows(src: torch.Tensor, dst: torch.Tensor, row_offset: int) -> torch.Tensor:
     """dst[b, row_offset : row_offset + R, :] = src [R, d] for every image b of the fp32 token stream dst [B, Ntok, d]."""
-    _need_cuda(src, dst)
-    if src.dtype != torch.float32 or dst.dtype != torch.float32 or not src.is_contiguous() or not dst.is_contiguous() or dst.dim() != 3 or src.shape[-1] != dst.shape[2]:
-        raise KfError("broadcast_rows: src [R, d] and dst [B, Ntok, d] must be contiguous fp32")
-    R = src.numel() // dst.shape[2]
-    _run("broadcast_rows", lambda: _lib.lib().kf_broadcast_rows(src.data_ptr(), dst.data_ptr(), R, dst.shape[2], dst.shape[0], dst.shape[1] * dst.shape[2], row_offset, _stream()))
-    return dst
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (src, dst, row_offset)
+    return _h.broadcast_rows(*args) if TIMING is None else _timed("broadcast_rows", _h.broadcast_rows, args)
 
 
 def rope_tables_are_half(sin: torch.Tensor, cos: torch.Tensor) -> bool:
@@ -323,16 +266,10 @@ def rope_tables_are_half(sin: torch.Tensor, cos: torch.Tensor) -> bool:
 def qkv_rope(a, W: QWeight, bias, sin, cos, Ntok: int, prefix: int, H: int, out_dtype=torch.bfloat16, half_tables: bool = False) -> torch.Tensor:
     """a [M=B*Ntok, d] -> physical [3, B, Ntok, H, 64] (bias + RoPE in fp32 on q and k of tokens >= prefix).
     half_tables=True promises rope_tables_are_half(sin, cos): the kernel then keeps a tile's table rows in shared memory."""
-    M = a.M if isinstance(a, ActBuf) else a.shape[0]
-    _f32c(bias, W.N, "bias")
-    if sin.dtype != torch.float32 or cos.dtype != torch.float32 or not sin.is_contiguous() or not cos.is_contiguous() \
-            or sin.shape[-1] != 64 or sin.shape[0] < Ntok - prefix or cos.shape != sin.shape:
-        raise KfError("qkv_rope: sin / cos must be contiguous fp32 [>= Ntok - prefix, 64]")
-    if M % Ntok:
-        raise KfError("qkv_rope: M must be a multiple of Ntok")
-    out = torch.empty(3, M // Ntok, Ntok, H, 64, dtype=out_dtype, device=W.q.device)
-    _gemm(a, W, "rope", bias=bias, sin=sin, cos=cos, C=out, out_dtype=out_dtype, Ntok=Ntok, prefix=prefix, H=H, rope_half=half_tables)
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (a, W, bias, sin, cos, Ntok, prefix, H, _DT[out_dtype], _lib.KF_G_ROPE_HALF if half_tables else 0)
+    return _h.qkv_rope(*args) if TIMING is None else _timed(f"gemm_block_{W.fmt}", _h.qkv_rope, args)
 
 
 def gemm_gelu_q(a, W: QWeight, bias, out: ActBuf, *, round_bf16: bool = False, recip_div: bool = False, fast_nv4: bool = False,
@@ -340,27 +277,20 @@ def gemm_gelu_q(a, W: QWeight, bias, out: ActBuf, *, round_bf16: bool = False, r
     """out = quantise(gelu(a @ W^T (* ts) + bias)) in out.fmt: fc1 writes fc2's operand and blocked scales directly.
     The quantisation follows the bit specification (IEEE divisions); fast_nv4=True selects approximate reciprocals for an
     nv4 output.  y_dbg (fp32 [M, N], optional) receives the values that were quantised."""
-    M = a.M if isinstance(a, ActBuf) else a.shape[0]
-    _f32c(bias, W.N, "bias")
-    if (out.M, out.K) != (M, W.N):
-        raise KfError(f"gemm_gelu_q: out must be [{M}, {W.N}], got [{out.M}, {out.K}]")
-    _f32c(y_dbg, M * W.N, "y_dbg")
-    _gemm(a, W, "quant", bias=bias, out=out, round_bf16=round_bf16, recip_div=recip_div, fast_nv4=fast_nv4, y_dbg=y_dbg)
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (a, W, bias, out, _flags(False, round_bf16, recip_div) | (_lib.KF_Q_FAST_NV4 if fast_nv4 else 0), y_dbg)
+    return _h.gemm_gelu_q(*args) if TIMING is None else _timed(f"gemm_block_{W.fmt}", _h.gemm_gelu_q, args)
 
 
 # ------------------------------------------------------------------------------------------------ attention
 def attn_fwd(qkv: torch.Tensor, pre: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """qkv contiguous [3, B, N, H, 64] bf16 | f16 (RoPE applied) -> O [B, N, H*64] of the same dtype.
     Counterpart: attn16_fwd(qkv, kind, pre) (infer-opt/round12_lowp_stack/impl/attn16o.cu:389-404)."""
-    _need_cuda(qkv)
-    if qkv.dim() != 5 or qkv.shape[0] != 3 or qkv.shape[4] != 64 or not qkv.is_contiguous() or qkv.dtype not in (torch.bfloat16, torch.float16):
-        raise KfError("attn_fwd: qkv must be contiguous [3, B, N, H, 64] bf16 or f16")
-    _, B, N, H, _ = qkv.shape
-    if out is None:
-        out = torch.empty(B, N, H * 64, dtype=qkv.dtype, device=qkv.device)
-    _run("attn_fwd", lambda: _lib.lib().kf_attn_fwd(_DT[qkv.dtype], qkv.data_ptr(), out.data_ptr(), B, N, H, float(pre), _stream()))
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (qkv, pre, out)
+    return _h.attn_fwd(*args) if TIMING is None else _timed("attn_fwd", _h.attn_fwd, args)
 
 
 attn16_fwd = attn_fwd
@@ -369,15 +299,10 @@ attn16_fwd = attn_fwd
 def attn_fwd_quant(qkv: torch.Tensor, out: ActBuf, pre: float = 1.0, recip_div: bool = False) -> ActBuf:
     """attention forward whose output is written directly as the quantised [B*N, H*64] operand `out` (codes + blocked
     scales; out.ts is the static nv4 scale): attn16_fwd + quant_rows in one kernel."""
-    _need_cuda(qkv, out.q)
-    if qkv.dim() != 5 or qkv.shape[0] != 3 or qkv.shape[4] != 64 or not qkv.is_contiguous() or qkv.dtype not in (torch.bfloat16, torch.float16):
-        raise KfError("attn_fwd_quant: qkv must be contiguous [3, B, N, H, 64] bf16 or f16")
-    _, B, N, H, _ = qkv.shape
-    if (out.M, out.K) != (B * N, H * 64):
-        raise KfError(f"attn_fwd_quant: out must be [{B * N}, {H * 64}], got [{out.M}, {out.K}]")
-    _run("attn_fwd", lambda: _lib.lib().kf_attn_fwd_quant(_DT[qkv.dtype], qkv.data_ptr(), B, N, H, float(pre), KF_FMT[out.fmt], out.q.data_ptr(),
-                                                          out.sf.data_ptr(), _ptr(out.ts), KF_Q_RECIP_DIV if recip_div else 0, _stream()))
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (qkv, out, pre, KF_Q_RECIP_DIV if recip_div else 0)
+    return _h.attn_fwd_quant(*args) if TIMING is None else _timed("attn_fwd", _h.attn_fwd_quant, args)
 
 
 # ------------------------------------------------------------------------------------------------ patch embed / head / pre / post
@@ -385,16 +310,10 @@ def gemm_tokens(a: torch.Tensor, W: QWeight, bias, out: torch.Tensor, rows_per_i
                 round_bf16: bool = False) -> torch.Tensor:
     """patch-embed GEMM: a bf16 [B*P, K] @ W^T + bias written as fp32 rows row_offset.. of every image of the token
     stream out [B, tokens_per_image, N] (counterpart: PatchEmbedGemm, infer-opt/round11_attn_tier0/impl/patch_embed.py:34-53)."""
-    if out.dtype != torch.float32 or not out.is_contiguous():
-        raise KfError("gemm_tokens: out must be contiguous fp32")
-    p = GemmParams()
-    p.fmt, p.epi, p.M, p.N, p.K = KF_FMT["bf16"], KF_EPI["plain"], a.shape[0], W.N, W.K
-    p.A, p.W, p.bias, p.C = a.data_ptr(), W.q.data_ptr(), _ptr(bias), out.data_ptr()
-    p.out_dtype = KF_DT["f32"]
-    p.flags = _lib.KF_G_ROUND_BF16 if round_bf16 else 0
-    p.out_row_group, p.out_row_stride, p.out_row_offset = rows_per_image, tokens_per_image, row_offset
-    _run("gemm_patch_bf16", lambda: _lib.lib().kf_gemm_bs(p, _stream()))
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (a, W, bias, out, rows_per_image, tokens_per_image, row_offset, _lib.KF_G_ROUND_BF16 if round_bf16 else 0)
+    return _h.gemm_tokens(*args) if TIMING is None else _timed("gemm_patch_bf16", _h.gemm_tokens, args)
 
 
 PATCH_STATIC_MAX_ROWS = 4096
@@ -418,60 +337,35 @@ def patch_embed_static(x: torch.Tensor, W: QWeight, bias, out: torch.Tensor, row
 
 def im2col_patch16(x: torch.Tensor) -> torch.Tensor:
     """x bf16 [B, 3, S, S] -> bf16 [B*(S/16)^2, 768]."""
-    _need_cuda(x)
-    if x.dtype != torch.bfloat16 or x.dim() != 4 or x.shape[1] != 3 or x.shape[2] != x.shape[3] or not x.is_contiguous():
-        raise KfError("im2col_patch16: x must be contiguous bf16 [B, 3, S, S]")
-    B, _, S, _ = x.shape
-    out = torch.empty(B * (S // 16) ** 2, 768, dtype=torch.bfloat16, device=x.device)
-    _run("im2col_patch16", lambda: _lib.lib().kf_im2col_patch16(x.data_ptr(), out.data_ptr(), B, S, _stream()))
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    return _h.im2col_patch16(x) if TIMING is None else _timed("im2col_patch16", _h.im2col_patch16, (x,))
 
 
 def ln_tail(x: torch.Tensor, w, b, eps: float, Q: int, npre: int, wcls: Optional[torch.Tensor] = None, bcls: Optional[torch.Tensor] = None):
     """final LayerNorm + gather: x fp32 [B, Ntok, d] -> (queries bf16 [B*Q, d], patches bf16 [B*(Ntok-Q-npre), d]), and with
     wcls bf16 [ncls1, d] / bcls fp32 [ncls1] the class logits bf16 [B*Q, ncls1] of the query rows as a third result."""
-    _need_cuda(x, w, b, wcls, bcls)
-    B, Ntok, d = x.shape
-    if x.dtype != torch.float32 or not x.is_contiguous():
-        raise KfError("ln_tail: x must be contiguous fp32")
-    qb = torch.empty(B * Q, d, dtype=torch.bfloat16, device=x.device)
-    xb = torch.empty(B * (Ntok - Q - npre), d, dtype=torch.bfloat16, device=x.device)
-    cl, ncls1 = None, 0
-    if wcls is not None:
-        if wcls.dtype != torch.bfloat16 or not wcls.is_contiguous() or wcls.shape[1] != d or bcls is None or bcls.dtype != torch.float32 or bcls.numel() != wcls.shape[0]:
-            raise KfError("ln_tail: wcls must be contiguous bf16 [ncls1, d] and bcls fp32 [ncls1]")
-        ncls1 = wcls.shape[0]
-        cl = torch.empty(B * Q, ncls1, dtype=torch.bfloat16, device=x.device)
-    _run("ln_tail", lambda: _lib.lib().kf_ln_tail(x.data_ptr(), w.data_ptr(), b.data_ptr(), float(eps), B, Ntok, Q, npre, d, qb.data_ptr(), xb.data_ptr(),
-                                                  _ptr(wcls), _ptr(bcls), ncls1, _ptr(cl), _stream()))
-    return (qb, xb) if wcls is None else (qb, xb, cl)
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (x, w, b, eps, Q, npre, wcls, bcls)
+    return _h.ln_tail(*args) if TIMING is None else _timed("ln_tail", _h.ln_tail, args)
 
 
 def dw_ln(g: torch.Tensor, bias, dww, lnw, lnb, B: int, Hs: int, Ws: int, eps: float, pre_act: bool = False) -> torch.Tensor:
     """ScaleBlock tail: g bf16 [B*Hs*Ws, 4C] -> bf16 [B, 2Hs, 2Ws, C] (dw_ln_launch, head11.py:60-67).
     pre_act=True: g already is bf16(gelu(conv + bias)) (fused into the GEMM epilogue), bias may be None."""
-    C = g.shape[1] // 4
-    _need_cuda(g, dww, lnw, lnb)
-    if g.dtype != torch.bfloat16 or not g.is_contiguous() or g.shape[0] != B * Hs * Ws or dww.shape != (9, C) or (bias is None and not pre_act):
-        raise KfError("dw_ln: g must be contiguous bf16 [B*Hs*Ws, 4C] and dww fp32 [9, C]")
-    out = torch.empty(B, 2 * Hs, 2 * Ws, C, dtype=torch.bfloat16, device=g.device)
-    _run("dw_ln", lambda: _lib.lib().kf_dw_ln(g.data_ptr(), _ptr(bias), dww.data_ptr(), lnw.data_ptr(), lnb.data_ptr(), out.data_ptr(), B, Hs, Ws, C,
-                                              float(eps), 1 if pre_act else 0, _stream()))
-    return out
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (g, bias, dww, lnw, lnb, B, Hs, Ws, eps, pre_act)
+    return _h.dw_ln(*args) if TIMING is None else _timed("dw_ln", _h.dw_ln, args)
 
 
 def semantic(mask_logits: torch.Tensor, class_logits: torch.Tensor, want_scores: bool = False):
     """mask_logits bf16 [B, Q, h, w], class_logits bf16 [B, Q, ncls+1] -> (labels uint8 [B, h, w], scores fp32 [B, ncls+1, h, w] | None)."""
-    _need_cuda(mask_logits, class_logits)
-    B, Q, h, w = mask_logits.shape
-    ncls1 = class_logits.shape[-1]
-    if mask_logits.dtype != torch.bfloat16 or class_logits.dtype != torch.bfloat16 or not mask_logits.is_contiguous() or not class_logits.is_contiguous():
-        raise KfError("semantic: logits must be contiguous bf16")
-    labels = torch.empty(B, h, w, dtype=torch.uint8, device=mask_logits.device)
-    scores = torch.empty(B, ncls1, h, w, dtype=torch.float32, device=mask_logits.device) if want_scores else None
-    _run("semantic", lambda: _lib.lib().kf_semantic(mask_logits.data_ptr(), class_logits.data_ptr(), B, Q, ncls1 - 1, h * w, _ptr(scores),
-                                                    labels.data_ptr(), _stream()))
-    return labels, scores
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (mask_logits, class_logits, want_scores)
+    return _h.semantic(*args) if TIMING is None else _timed("semantic", _h.semantic, args)
 
 
 IMAGENET_MEAN = (0.485, 0.456, 0.406)

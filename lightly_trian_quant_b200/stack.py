@@ -24,8 +24,6 @@ infer-opt/round14_fp4_full/impl/fp4util.py:41,68-75; stack14b.py:49-52); that ca
 """
 from __future__ import annotations
 
-import copy
-
 import torch
 
 from . import ops
@@ -78,8 +76,9 @@ def set_ts(ts_dev: torch.Tensor, x: torch.Tensor) -> None:
 
 
 def _with_ts(buf: ops.ActBuf, ts) -> ops.ActBuf:
-    b = copy.copy(buf)
-    b.ts = ts
+    """the same codes and scales under another per-tensor scale."""
+    b = ops.ActBuf.__new__(ops.ActBuf)
+    b.M, b.K, b.fmt, b.q, b.sf, b.ts = buf.M, buf.K, buf.fmt, buf.q, buf.sf, ts
     return b
 
 
@@ -95,6 +94,17 @@ class Layer:
             setattr(self, k, w[k])
         self.ln1_eps, self.ln2_eps = w["ln1_eps"], w["ln2_eps"]
         self.ts_ln1, self.ts_o, self.ts_ln2, self.ts_g = (_site_ts(fmt, dev) for _ in range(4))
+        self._operands = (None, None)
+
+    def operands(self, M: int, device):
+        """The quantised operands of the block's four sites (qkv, proj, fc1, fc2 input) for M rows: the buffers every layer of
+        this shape shares (ops.act_buf) under this layer's scales, put together once per shape."""
+        key = (M, device)
+        if self._operands[0] != key:
+            d, ff = self.qkv.K, self.fc1.N
+            a, o, f = ops.act_buf(M, d, self.fmt, device, 0), ops.act_buf(M, d, self.fmt, device, 1), ops.act_buf(M, ff, self.fmt, device, 0)
+            self._operands = (key, tuple(_with_ts(b, ts) for b, ts in ((a, self.ts_ln1), (o, self.ts_o), (a, self.ts_ln2), (f, self.ts_g))))
+        return self._operands[1]
 
 
 def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, calib: Calib, *, round_bf16: bool, attn_dtype, half_tables: bool = False,
@@ -104,7 +114,6 @@ def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, cali
     returned: how the query tokens join the stream without a copy of it."""
     B, N, d = x.shape
     M = B * N
-    ff = L.fc1.N
     fmt = L.fmt
     nv4, cal = fmt == "nv4", calib.on
     x2 = x.view(M, d)
@@ -119,24 +128,21 @@ def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, cali
     # ---- LN1 + quant -> qkv (bias + RoPE + layout) -> attention
     if cal and nv4:
         set_ts(L.ts_ln1, ops.ln_rows(x, L.ln1_w, L.ln1_b, L.ln1_eps, BF))
-    a = _with_ts(ops.act_buf(M, d, fmt, x.device, 0), L.ts_ln1)
+    a, a2, a3, f = L.operands(M, x.device)
     ops.ln_quant(x, L.ln1_w, L.ln1_b, L.ln1_eps, a, round_bf16=round_bf16)
     qkv = ops.qkv_rope(a, L.qkv, L.bqkv, sin, cos, N, prefix, heads, out_dtype=attn_dtype, half_tables=half_tables)
     # ---- attention with its output quantised in the epilogue -> proj (gamma + residual, in place on the stream)
     if cal and nv4:
         set_ts(L.ts_o, ops.attn_fwd(qkv))
-    a2 = _with_ts(ops.act_buf(M, d, fmt, x.device, 1), L.ts_o)
     ops.attn_fwd_quant(qkv, a2)
     ops.gemm_res(a2, L.proj, L.bproj, L.g1, x2, out=x2)
     # ---- LN2 + quant -> fc1 (GELU + quantise-out) -> fc2 (gamma + residual)
     if cal and nv4:
         set_ts(L.ts_ln2, ops.ln_rows(x, L.ln2_w, L.ln2_b, L.ln2_eps, BF))
-    a = _with_ts(a, L.ts_ln2)
-    ops.ln_quant(x, L.ln2_w, L.ln2_b, L.ln2_eps, a, round_bf16=round_bf16)
+    ops.ln_quant(x, L.ln2_w, L.ln2_b, L.ln2_eps, a3, round_bf16=round_bf16)
     if cal and nv4:
-        set_ts(L.ts_g, ops.gemm_plain(a, L.fc1, L.b1, gelu=True))
-    f = _with_ts(ops.act_buf(M, ff, fmt, x.device, 0), L.ts_g)
-    ops.gemm_gelu_q(a, L.fc1, L.b1, f, round_bf16=round_bf16)
+        set_ts(L.ts_g, ops.gemm_plain(a3, L.fc1, L.b1, gelu=True))
+    ops.gemm_gelu_q(a3, L.fc1, L.b1, f, round_bf16=round_bf16)
     return _fc2(f, L, x, x2, grow_into)
 
 
