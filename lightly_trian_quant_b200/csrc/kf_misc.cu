@@ -513,10 +513,25 @@ extern "C" int kf_dw_ln(const void* g, const float* bias, const float* dww, cons
   int sms = 0;
   int st = device_sm_count(&sms);
   if (st != KF_OK) return st;
-  // items: strips of 8 output pixels in x, cut in y into segments of about 40 rows (each segment re-reads two halo rows:
-  // 5 %); fewer, longer segments when the image count alone fills the CTAs several times over
+  // Items: strips of 8 output pixels in x, cut in y into segments of seg_rows.  A CTA works through a segment row by row
+  // (a chain of about 2 us per row), so the launch takes rounds * (rows + 1) steps, the extra one for the two halo rows that a
+  // segment reads again; a last round that leaves every second CTA slot empty runs at 0.65 of the time (2.1 us per row with
+  // one CTA on an SM, 3.2 us with two).  The shortest of these wins: about 40 rows for a batch, but 12 for one image of
+  // 160 x 160, which left 68 SMs without an item at 40.
   const int Ho = 2 * Hs, strips = (2 * Ws + DW_SW - 1) / DW_SW;
-  const int segs = (Ho + 39) / 40, seg_rows = (Ho + segs - 1) / segs;
+  int segs = 1;
+  double best = 0.0;
+  for (int n = 1; n <= (Ho + 3) / 4; ++n) {
+    const int rows = (Ho + n - 1) / n;
+    const int64_t items = (int64_t)strips * n * B, slots = 2 * sms, rem = items % slots;
+    const double cost = ((double)(items / slots) + (rem == 0 ? 0.0 : rem <= sms ? 0.65 : 1.0)) * (rows + 1);
+    if (n == 1 || cost < best) {
+      best = cost;
+      segs = n;
+    }
+  }
+  const int seg_rows = (Ho + segs - 1) / segs;
+  segs = (Ho + seg_rows - 1) / seg_rows;                 // no empty segments
   const int64_t total = (int64_t)strips * segs * B;
   KF_REQUIRE(total < (1ll << 31), "kf_dw_ln: too many strips");
   const int grid = (int)(total < 2 * sms ? total : 2 * sms);
