@@ -44,6 +44,7 @@ extern "C" {
 #define KF_Q_GELU 1        /* x <- gelu_erf(x + bias[col]) before quantising                         */
 #define KF_Q_ROUND_BF16 2  /* round the (LN / GELU) value to bf16 before quantising                  */
 #define KF_Q_RECIP_DIV 4   /* amax/448, amax/6 as multiply by the fp32 reciprocal (torch-on-CUDA rule) */
+#define KF_Q_IN_BF16 256   /* kf_ln_quant only: x points to bf16 values                              */
 #define KF_Q_FAST_NV4 64   /* QUANT epilogue to nv4 only: block scale and element division through approximate
                               reciprocals instead of the IEEE divisions of the bit specification (opt-in; a code moves
                               only where the exact quotient lies within an ulp of a rounding boundary) */
@@ -88,6 +89,15 @@ KF_API int kf_quant_rows(int fmt, int in_dtype, const void* x, int64_t ldx, int 
  * lnq (infer-opt/round14_fp4_full/impl/lnq14.cu:85-130,158). */
 KF_API int kf_ln_quant(int fmt, const float* x, const float* w, const float* b, float eps, int M, int d,
                 const float* ts, int flags, void* q, void* sf, float* y_dbg, void* stream);
+
+/* Dynamic per-tensor scale of an NVFP4 operand, measured on the device in one launch: *ts = factor * max|v| (1 when the
+ * maximum is zero or NaN) over v = x [M, K] (row stride ldx, K a multiple of 32; with KF_Q_GELU over v = gelu_erf(x)), or
+ * over v = bf16(LayerNorm(x)) for contiguous f32 | bf16 x [M, d].  factor = 1/2688 is the exact scale amax / (6 * 448).
+ * ws: two 32-bit words of device memory, zero before the first use; a call leaves them zero.  Calls that share ws must be
+ * ordered.  Counterpart: the dynamic activation scale of the emulated model (infer-opt/round10_lowp_probe/impl/quant_ref.py:131-154). */
+KF_API int kf_amax_scale(int in_dtype, const void* x, int64_t ldx, int M, int K, int flags, float factor, float* ts, void* ws, void* stream);
+KF_API int kf_ln_amax_scale(int in_dtype, const void* x, const float* w, const float* b, float eps, int M, int d, float factor,
+                            float* ts, void* ws, void* stream);
 
 /* LayerNorm to a 16-bit tensor: x fp32 [M, d] -> y bf16 | f16 [M, d].
  * Replaces ln_bf16 (infer-opt/round14_fp4_full/impl/ln14.cu:23-58,67) and ln16

@@ -59,6 +59,8 @@ def lib() -> C.CDLL:
         sigs = {
             "kf_quant_rows": [i32, i32, vp, i64, i32, i32, vp, vp, i32, vp, vp, vp],
             "kf_ln_quant": [i32, vp, vp, vp, f32, i32, i32, vp, i32, vp, vp, vp, vp],
+            "kf_amax_scale": [i32, vp, i64, i32, i32, i32, f32, vp, vp, vp],
+            "kf_ln_amax_scale": [i32, vp, vp, vp, f32, i32, i32, f32, vp, vp, vp],
             "kf_ln_rows": [vp, vp, vp, f32, i32, i32, i32, vp, vp],
             "kf_gemm_bs": [C.POINTER(GemmParams), vp],
             "kf_check_device_error": [],

@@ -360,13 +360,48 @@ PyObject* ln_quant(PyObject* const* v) {
   const at::Tensor& x = cuda_tensor(v[0], "x");
   const Operand out = act(v[4], "out");
   const int64_t d = x.dim() > 0 ? x.size(-1) : 0, M = d > 0 ? x.numel() / d : 0;
-  if (x.scalar_type() != at::kFloat || !x.is_contiguous() || M != out.rows || d != out.K)
-    fail("ln_quant: x must be contiguous fp32 [M=%lld, d=%lld], got [%lld, %lld] %s", (long long)out.rows, (long long)out.K, (long long)M, (long long)d,
+  const bool bf16 = x.scalar_type() == at::kBFloat16;
+  if ((x.scalar_type() != at::kFloat && !bf16) || !x.is_contiguous() || M != out.rows || d != out.K)
+    fail("ln_quant: x must be contiguous fp32 or bf16 [M=%lld, d=%lld], got [%lld, %lld] %s", (long long)out.rows, (long long)out.K, (long long)M, (long long)d,
          c10::toString(x.scalar_type()));
-  check(kf_ln_quant(out.fmt, x.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")), (float)to_float(v[3]), (int)M,
-                    (int)d, static_cast<const float*>(out.pts), (int)to_int(v[5]), out.pq, out.psf, static_cast<float*>(opt_ptr(v[6], "y_dbg")), stream()),
+  check(kf_ln_quant(out.fmt, static_cast<const float*>(x.data_ptr()), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
+                    (float)to_float(v[3]), (int)M, (int)d, static_cast<const float*>(out.pts), (int)to_int(v[5]) | (bf16 ? KF_Q_IN_BF16 : 0), out.pq, out.psf,
+                    static_cast<float*>(opt_ptr(v[6], "y_dbg")), stream()),
         "ln_quant");
   return new_ref(v[4]);
+}
+
+// ts [1] fp32 and ws (two 32-bit words, zero before the first use)
+float* scale_target(PyObject* ts, PyObject* ws, void** words) {
+  const at::Tensor &t = cuda_tensor(ts, "ts"), &w = cuda_tensor(ws, "ws");
+  need(t.scalar_type() == at::kFloat && t.numel() == 1 && w.scalar_type() == at::kInt && w.numel() >= 2 && w.is_contiguous(),
+       "amax_scale: ts must be fp32 [1] and ws contiguous int32 [2]");
+  *words = w.data_ptr();
+  return t.data_ptr<float>();
+}
+
+// x, flags, factor, ts, ws
+PyObject* amax_scale(PyObject* const* v) {
+  const at::Tensor& x = cuda_tensor(v[0], "x");
+  const int dt = dtype_code(x.scalar_type());
+  need(x.dim() == 2 && x.stride(1) == 1 && dt >= 0, "amax_scale: x must be f32 | bf16 | f16 [M, K] with a contiguous last dim");
+  void* ws;
+  float* ts = scale_target(v[3], v[4], &ws);
+  check(kf_amax_scale(dt, x.data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), (int)to_int(v[1]), (float)to_float(v[2]), ts, ws, stream()), "amax_scale");
+  return new_ref(v[3]);
+}
+
+// x, w, b, eps, factor, ts, ws
+PyObject* ln_amax_scale(PyObject* const* v) {
+  const at::Tensor& x = cuda_tensor(v[0], "x");
+  need(x.is_contiguous() && x.dim() > 0 && (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16), "ln_amax_scale: x must be contiguous fp32 or bf16");
+  const int64_t d = x.size(-1), M = x.numel() / d;
+  void* ws;
+  float* ts = scale_target(v[5], v[6], &ws);
+  check(kf_ln_amax_scale(dtype_code(x.scalar_type()), x.data_ptr(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
+                         (float)to_float(v[3]), (int)M, (int)d, (float)to_float(v[4]), ts, ws, stream()),
+        "ln_amax_scale");
+  return new_ref(v[5]);
 }
 
 // x, w, b, eps, dtype code
@@ -526,7 +561,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef g_methods[] = {KF_ENTRY(quant_rows, 4),     KF_ENTRY(ln_quant, 7),   KF_ENTRY(ln_rows, 5),  KF_ENTRY(gemm_plain, 6),     KF_ENTRY(gemm_res, 7),
                            KF_ENTRY(qkv_rope, 10),      KF_ENTRY(gemm_gelu_q, 6), KF_ENTRY(bmm_nt, 3),   KF_ENTRY(gemm_tokens, 8),    KF_ENTRY(broadcast_rows, 3),
                            KF_ENTRY(ln_tail, 8),        KF_ENTRY(attn_fwd, 3),   KF_ENTRY(attn_fwd_quant, 4), KF_ENTRY(im2col_patch16, 1), KF_ENTRY(dw_ln, 10),
-                           KF_ENTRY(semantic, 3),       {nullptr, nullptr, 0, nullptr}};
+                           KF_ENTRY(semantic, 3),       KF_ENTRY(amax_scale, 5), KF_ENTRY(ln_amax_scale, 7), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_kf_host", "native operator layer over libkf_b200.so", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -143,6 +143,27 @@ __device__ __forceinline__ float gelu_erf(float x) {
   return fmaxf(x, 0.f) - (0.5f * ax) * (p * e);         // relu(x) - 0.5*|x|*erfc(|x|/sqrt2), both signs without cancellation
 }
 
+// The same for two values: the polynomial, the products and the final sum on packed pairs (the same bits).
+__device__ __forceinline__ float2 gelu_erf_pair(float2 x) {
+  const float2 ax = make_float2(fabsf(x.x), fabsf(x.y));
+  const float2 u = mul2(ax, splat2(0.84932180028801904272f));
+  const float2 kd = fma2(splat2(0.23164189388980933f), ax, splat2(1.0f));
+  float2 k;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(k.x) : "f"(kd.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(k.y) : "f"(kd.y));
+  float2 p = fma2(k, splat2(1.061405429f), splat2(-1.453152027f));
+  p = fma2(p, k, splat2(1.421413741f));
+  p = fma2(p, k, splat2(-0.284496736f));
+  p = fma2(p, k, splat2(0.254829592f));
+  p = mul2(p, k);
+  const float2 w = mul2(make_float2(-u.x, -u.y), u);
+  float2 e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(w.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(w.y));
+  const float2 relu = make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f));
+  return fma2(mul2(ax, splat2(-0.5f)), mul2(p, e), relu);
+}
+
 // GELU (exact-erf definition) of two values for the fused GEMM epilogues, which are short of XU (MUFU) throughput: one
 // exponential per value and no reciprocal.  gelu(x) = relu(x) - |x| * Phi(-|x|) with the normal tail written as
 // Phi(-a) = 2^(-a^2 * log2(e)/2 + Q(a)); Q is smooth and logarithm-like (Q(0) = -1) and a degree-7 least-squares fit on

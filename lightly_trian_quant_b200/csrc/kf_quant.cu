@@ -14,39 +14,41 @@
 namespace kf {
 
 // ------------------------------------------------------------------------------------------------ loads
-template <typename T>
-__device__ __forceinline__ void load16(const T* p, float (&v)[16]);
-
-template <>
-__device__ __forceinline__ void load16<float>(const float* p, float (&v)[16]) {
-  const float4* p4 = reinterpret_cast<const float4*>(p);
-  float4 a = __ldg(p4), b = __ldg(p4 + 1), c = __ldg(p4 + 2), d = __ldg(p4 + 3);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  v[8] = c.x; v[9] = c.y; v[10] = c.z; v[11] = c.w; v[12] = d.x; v[13] = d.y; v[14] = d.z; v[15] = d.w;
-}
-
-template <>
-__device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[16]) {
-  const uint4* p4 = reinterpret_cast<const uint4*>(p);
-  uint4 a = __ldg(p4), b = __ldg(p4 + 1);
-  uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    v[2 * i] = __uint_as_float(w[i] << 16);
-    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+// 32 bytes of read-once input as eight words: one 256-bit load where the address allows it (`wide`), else two of 128 bits.
+__device__ __forceinline__ void load32b(const void* p, bool wide, uint32_t* w) {
+  if (wide) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = __ldg(static_cast<const uint4*>(p)), b = __ldg(static_cast<const uint4*>(p) + 1);
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
   }
 }
+// two 16-bit values (first one in the low half) as floats
+template <typename T>
+__device__ __forceinline__ float2 unpack2(uint32_t w) {
+  if constexpr (std::is_same<T, __half>::value) return __half22float2(*reinterpret_cast<__half2*>(&w));
+  else return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
 
-template <>
-__device__ __forceinline__ void load16<__half>(const __half* p, float (&v)[16]) {
-  const uint4* p4 = reinterpret_cast<const uint4*>(p);
-  uint4 a = __ldg(p4), b = __ldg(p4 + 1);
-  uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+// 32 consecutive elements, all loads issued before the first conversion
+template <typename T>
+__device__ __forceinline__ void load32(const T* p, bool wide, float (&v)[32]) {
+  constexpr int PIECES = (int)sizeof(T);                  // of 32 bytes: 4 of fp32, 2 of a 16-bit type
+  uint32_t w[8 * PIECES];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float2 f = __half22float2(*reinterpret_cast<__half2*>(&w[i]));
-    v[2 * i] = f.x;
-    v[2 * i + 1] = f.y;
+  for (int i = 0; i < PIECES; ++i) load32b(reinterpret_cast<const uint8_t*>(p) + 32 * i, wide, w + 8 * i);
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(w[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 f = unpack2<T>(w[i]);
+      v[2 * i] = f.x;
+      v[2 * i + 1] = f.y;
+    }
   }
 }
 
@@ -62,80 +64,161 @@ __device__ __forceinline__ uint32_t gather_sf_word(int byte, int lane) {
 }
 
 // ------------------------------------------------------------------------------------------------ row quantiser
-// One thread = 16 consecutive elements of one row.  mx8 / mx4: two adjacent lanes share a 1x32 block, eight lanes one
-// scale word; nv4: one lane = one 1x16 block, four lanes one scale word.
+// One thread = 32 consecutive elements of one row: one mx block, or two nv4 blocks whose scalars go through the packed-pair
+// quantiser of the GEMM epilogue.  No maximum crosses lanes; two (nv4) or four (mx) lanes share one scale word.
+// Bound by HBM.  With 16 elements per thread (two lanes per mx block, the nv4 divisions scalar) the NVFP4 form was bound by
+// instruction issue: 51 360 x 4096 bf16 139 us = 3.9 TB/s, now 108 us = 5.0 TB/s.
 template <typename T, int FMT>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, const float* __restrict__ ts_ptr,
-                                                         const float* __restrict__ bias, int flags, uint8_t* __restrict__ q,
+                                                         const float* __restrict__ bias, int flags, int wide, uint8_t* __restrict__ q,
                                                          uint8_t* __restrict__ sf, int64_t items_valid, int64_t items_total) {
   const int lane = threadIdx.x & 31;
-  const int per_row = K >> 4;
+  const int per_row = K >> 5;
   int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool in_pad = w < items_total;          // inside the padded row range (scale bytes must be written)
   const bool valid = w < items_valid;           // a real row
   // 32-bit index arithmetic (the host checks that the item count fits); a power-of-two row length needs no division
   const uint32_t w32 = (uint32_t)w;
-  int row, c16;
+  int row, c32;
   if ((per_row & (per_row - 1)) == 0) {
     row = (int)(w32 >> (31 - __clz(per_row)));
-    c16 = (int)(w32 & (uint32_t)(per_row - 1));
+    c32 = (int)(w32 & (uint32_t)(per_row - 1));
   } else {
     row = (int)(w32 / (uint32_t)per_row);
-    c16 = (int)(w32 - (uint32_t)row * (uint32_t)per_row);
+    c32 = (int)(w32 - (uint32_t)row * (uint32_t)per_row);
   }
-  float v[16];
+  float v[32];
   if (valid) {
-    load16<T>(x + (int64_t)row * ldx + c16 * 16, v);
+    load32<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, v);
   } else {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = 0.f;
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+  }
+  if constexpr (FMT == KF_FMT_NV4 && std::is_same<T, __half>::value) {
+    // The corrected quotient of a negative zero is a positive one (code 0, the bit rule says 8).  fp16 inputs reach -0 by
+    // underflow of ordinary values; a magnitude below any fp16 one takes its place.
+    if (!(flags & KF_Q_GELU)) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(v[i]) == 0x80000000u ? -1e-20f : v[i];
+    }
   }
   const Nv4Scale ts = nv4_scale(FMT == KF_FMT_NV4 ? __ldg(ts_ptr) : 1.f);
-  if (flags & KF_Q_GELU) {
-    if (valid) {
-      const float4* b4 = reinterpret_cast<const float4*>(bias + c16 * 16);
+  if ((flags & KF_Q_GELU) && valid) {
+    const float4* b4 = reinterpret_cast<const float4*>(bias + c32 * 32);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float4 bb = __ldg(b4 + i);
-        v[4 * i] = gelu_erf(v[4 * i] + bb.x);
-        v[4 * i + 1] = gelu_erf(v[4 * i + 1] + bb.y);
-        v[4 * i + 2] = gelu_erf(v[4 * i + 2] + bb.z);
-        v[4 * i + 3] = gelu_erf(v[4 * i + 3] + bb.w);
-      }
+    for (int i = 0; i < 32; i += 4) {
+      const float4 bb = __ldg(b4 + (i >> 2));
+      const float2 a = gelu_erf_pair(add2(make_float2(v[i], v[i + 1]), make_float2(bb.x, bb.y)));
+      const float2 c = gelu_erf_pair(add2(make_float2(v[i + 2], v[i + 3]), make_float2(bb.z, bb.w)));
+      v[i] = a.x;
+      v[i + 1] = a.y;
+      v[i + 2] = c.x;
+      v[i + 3] = c.y;
     }
   }
   if (flags & KF_Q_ROUND_BF16) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = bf16_round(v[i]);
+    for (int i = 0; i < 32; i += 2) {
+      const float2 a = bf16_round2(make_float2(v[i], v[i + 1]));
+      v[i] = a.x;
+      v[i + 1] = a.y;
+    }
   }
-  float amax = 0.f;
+  float am0 = 0.f, am1 = 0.f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) amax = amax_nan(amax, fabsf(v[i]));
+  for (int i = 0; i < 16; i += 2) {
+    am0 = max3(am0, fabsf(v[i]), fabsf(v[i + 1]));
+    am1 = max3(am1, fabsf(v[16 + i]), fabsf(v[17 + i]));
+  }
   const bool div_true = !(flags & KF_Q_RECIP_DIV);
-  int byte;
-  if (FMT == KF_FMT_MX8) {
-    amax = amax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  const float(&va)[16] = *reinterpret_cast<const float(*)[16]>(&v[0]);
+  const float(&vb)[16] = *reinterpret_cast<const float(*)[16]>(&v[16]);
+  if constexpr (FMT == KF_FMT_NV4) {
     uint32_t o[4];
-    quant_mx8<16>(v, amax, div_true, o, byte);
-    if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * K + c16 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-  } else if (FMT == KF_FMT_MX4) {
-    amax = amax_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    uint32_t o[2];
-    quant_mx4<16>(v, amax, div_true, o, byte);
-    if (valid) *reinterpret_cast<uint2*>(q + (int64_t)row * (K >> 1) + c16 * 8) = make_uint2(o[0], o[1]);
+    int by0, by1;
+    quant_nv4_pair16(va, am0, vb, am1, ts, div_true, o, by0, by1);
+    if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * (K >> 1) + c32 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+    const uint32_t pk = valid ? (uint32_t)(by0 | (by1 << 8)) : 0u;
+    const uint32_t up = __shfl_xor_sync(0xffffffffu, pk, 1);           // on an even lane: the bytes of the word's other two blocks
+    if (in_pad && (lane & 1) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, 2 * c32, K >> 6)) = pk | (up << 16);
   } else {
-    uint32_t o[2];
-    quant_nv4<16>(v, amax, ts, div_true, o, byte);
-    if (valid) *reinterpret_cast<uint2*>(q + (int64_t)row * (K >> 1) + c16 * 8) = make_uint2(o[0], o[1]);
+    const float amax = amax_nan(am0, am1);
+    int byte;
+    if constexpr (FMT == KF_FMT_MX8) {
+      uint32_t o[8];
+      quant_mx8<16>(va, amax, div_true, o, byte);
+      quant_mx8<16>(vb, amax, div_true, o + 4, byte);
+      if (valid) {
+        uint4* dst = reinterpret_cast<uint4*>(q + (int64_t)row * K + c32 * 32);
+        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+    } else {
+      uint32_t o[4];
+      quant_mx4<16>(va, amax, div_true, o, byte);
+      quant_mx4<16>(vb, amax, div_true, o + 2, byte);
+      if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * (K >> 1) + c32 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    if (!valid) byte = 0;
+    const uint32_t word = gather_sf_word<1>(byte, lane);
+    if (in_pad && (lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, c32, K >> 7)) = word;
   }
-  if (!valid) byte = 0;
-  constexpr int STEP = (FMT == KF_FMT_NV4) ? 1 : 2;                 // lanes per k-block
-  uint32_t word = gather_sf_word<STEP>(byte, lane);
-  if (in_pad && (lane & (4 * STEP - 1)) == 0) {
-    int kb = (FMT == KF_FMT_NV4) ? c16 : (c16 >> 1);
-    int nkb4 = (FMT == KF_FMT_NV4) ? (K >> 6) : (K >> 7);
-    *reinterpret_cast<uint32_t*>(sf + sf_offset(row, kb, nkb4)) = word;
+}
+
+// ------------------------------------------------------------------------------------------------ dynamic per-tensor scale
+// The per-tensor scale of an NVFP4 operand measured on the values about to be quantised: ts = factor * max|v| (1 when that is
+// zero or NaN), in one launch: block maxima meet in an atomic maximum on the bit patterns (non-negative floats order as
+// integers, a NaN above them all), the last block writes ts and leaves the workspace (two words, zero before the first
+// use) as it found it.  As six to nine elementwise launches with fp32 copies it was most of a swapped block: 6420 rows of
+// ViT-B, four Linears: 457 -> 178 us.
+__device__ __forceinline__ void amax_finish(float am, float factor, float* ts, uint32_t* ws) {
+  __shared__ uint32_t part[32];
+  uint32_t bits = __float_as_uint(am);
+  bits = __reduce_max_sync(0xffffffffu, bits);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  if (lane == 0) part[warp] = bits;
+  __syncthreads();
+  if (warp != 0) return;
+  bits = __reduce_max_sync(0xffffffffu, lane < nwarps ? part[lane] : 0u);
+  if (lane != 0) return;
+  atomicMax(&ws[0], bits);
+  __threadfence();
+  if (atomicAdd(&ws[1], 1u) == gridDim.x - 1) {
+    const float peak = __uint_as_float(atomicExch(&ws[0], 0u));
+    ws[1] = 0;
+    *ts = peak > 0.f ? peak * factor : 1.f;
   }
+}
+
+// |gelu(x)| with the exact-erf definition, in the form the framework's eager GELU evaluates
+__device__ __forceinline__ float gelu_abs(float x) { return fabsf(x * 0.5f * (1.0f + erff(x * 0.70710678118654752440f))); }
+
+// max |v| or max |gelu(v)| over a matrix.  |gelu(v)| <= |v|, so an element is evaluated only when |v| is above the thread's
+// maximum so far: a few per thread instead of all (the GELU of 20 M values would take longer than reading them).
+template <typename T, bool GELU>
+__global__ void __launch_bounds__(256) amax_scale_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, int wide, float factor, float* __restrict__ ts,
+                                                         uint32_t* __restrict__ ws) {
+  const uint32_t per_row = K >> 5, total = (uint32_t)M * per_row;
+  float am = 0.f;
+  for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+    const uint32_t row = i / per_row, c = i - row * per_row;
+    float v[32];
+    load32<T>(x + (int64_t)row * ldx + c * 32, wide != 0, v);
+    if (GELU) {
+      // the piece's largest value first: most others then fail the test
+      float top = v[0];
+#pragma unroll
+      for (int j = 1; j < 32; ++j) top = fmaxf(top, v[j]);
+      if (!(fabsf(top) <= am)) am = amax_nan(am, gelu_abs(top));
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (!(fabsf(v[j]) <= am)) am = amax_nan(am, gelu_abs(v[j]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) am = max3(am, fabsf(v[j]), fabsf(v[j + 1]));
+    }
+  }
+  amax_finish(fabsf(am), factor, ts, ws);
 }
 
 // ------------------------------------------------------------------------------------------------ LayerNorm (+ quant)
@@ -168,24 +251,27 @@ __device__ __forceinline__ void ln_affine_load(const float* __restrict__ w, cons
   }
 }
 
+// four consecutive values of a row: 16 bytes of fp32 or 8 of bf16
+template <bool FROM_SMEM, typename TI>
+__device__ __forceinline__ float4 ln_load4(const TI* p) {
+  if constexpr (sizeof(TI) == 4) {
+    return FROM_SMEM ? *reinterpret_cast<const float4*>(p) : __ldg(reinterpret_cast<const float4*>(p));
+  } else {
+    const uint2 u = FROM_SMEM ? *reinterpret_cast<const uint2*>(p) : __ldg(reinterpret_cast<const uint2*>(p));
+    const float2 a = unpack2<TI>(u.x), b = unpack2<TI>(u.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+}
+
 // LayerNorm of one row with the affine parameters already in registers (the persistent kernels load them once per
 // warp: re-reading them per row doubles the load instructions of a kernel that is otherwise one pass over x).
-template <int NV, bool FROM_SMEM = false, int LAY = LAY_CHUNK>
-__device__ __forceinline__ void ln_row(const float* xr, const float (&ww)[NV][8], const float (&bb)[NV][8], float eps,
+template <int NV, bool FROM_SMEM = false, int LAY = LAY_CHUNK, typename TI = float>
+__device__ __forceinline__ void ln_row(const TI* xr, const float (&ww)[NV][8], const float (&bb)[NV][8], float eps,
                                        int lane, bool valid, float (&v)[NV][8]) {
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     if (valid) {
-      const float4* pa = reinterpret_cast<const float4*>(xr + ln_piece_offset<LAY>(i, 0, lane));
-      const float4* pc = reinterpret_cast<const float4*>(xr + ln_piece_offset<LAY>(i, 1, lane));
-      float4 a, c;
-      if (FROM_SMEM) {
-        a = *pa;
-        c = *pc;
-      } else {
-        a = __ldg(pa);
-        c = __ldg(pc);
-      }
+      const float4 a = ln_load4<FROM_SMEM>(xr + ln_piece_offset<LAY>(i, 0, lane)), c = ln_load4<FROM_SMEM>(xr + ln_piece_offset<LAY>(i, 1, lane));
       v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w; v[i][4] = c.x; v[i][5] = c.y; v[i][6] = c.z; v[i][7] = c.w;
     } else {
 #pragma unroll
@@ -237,16 +323,16 @@ __device__ __forceinline__ void ln_row(const float* xr, const float (&ww)[NV][8]
 // register-staged loads cannot (they stop while the warp computes).
 constexpr int LNQ_RING = 3;
 
-template <int NV, int FMT>
-__global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps,
+template <int NV, int FMT, typename TI>
+__global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps,
                                                        int M, int rows_pad, const float* __restrict__ ts_ptr, int flags, uint8_t* __restrict__ q,
                                                        uint8_t* __restrict__ sf, float* __restrict__ y_dbg, unsigned int* err) {
   constexpr int D = NV * 256;
   extern __shared__ __align__(128) uint8_t lsm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* ring = reinterpret_cast<float*>(lsm) + (size_t)warp * LNQ_RING * D;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(lsm + (size_t)4 * LNQ_RING * D * 4) + warp * LNQ_RING;
-  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(lsm + (size_t)4 * LNQ_RING * D * 4 + 4 * LNQ_RING * 8);
+  TI* ring = reinterpret_cast<TI*>(lsm) + (size_t)warp * LNQ_RING * D;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(lsm + (size_t)4 * LNQ_RING * D * sizeof(TI)) + warp * LNQ_RING;
+  volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(lsm + (size_t)4 * LNQ_RING * D * sizeof(TI) + 4 * LNQ_RING * 8);
   pdl_launch_dependents();                        // the next kernel of the stream may take the SMs this grid leaves
   if (threadIdx.x == 0) *abort_flag = 0;
   if (lane == 0) {
@@ -260,8 +346,8 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const fl
   auto issue = [&](int k) {                       // lane 0: start the copy of this warp's k-th row into slot k % RING
     const int r = gw + k * W;
     if (r < M) {
-      mbar_expect_tx(&bars[k % LNQ_RING], D * 4);
-      bulk_load_1d(ring + (size_t)(k % LNQ_RING) * D, x + (int64_t)r * D, D * 4, &bars[k % LNQ_RING]);
+      mbar_expect_tx(&bars[k % LNQ_RING], D * sizeof(TI));
+      bulk_load_1d(ring + (size_t)(k % LNQ_RING) * D, x + (int64_t)r * D, D * sizeof(TI), &bars[k % LNQ_RING]);
     }
   };
   if (lane == 0)
@@ -392,6 +478,24 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const fl
   }
 }
 
+// Dynamic per-tensor scale of the LayerNorm of x, rounded to bf16 as the quantiser behind it will see it (no output tensor).
+template <int NV, typename TI>
+__global__ void __launch_bounds__(128) ln_amax_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps, int M, float factor,
+                                                      float* __restrict__ ts, uint32_t* __restrict__ ws) {
+  constexpr int D = NV * 256;
+  const int lane = threadIdx.x & 31;
+  float ww[NV][8], bb[NV][8], v[NV][8], am = 0.f;
+  ln_affine_load<NV>(w, b, lane, ww, bb);
+  for (int row = blockIdx.x * 4 + (threadIdx.x >> 5); row < M; row += gridDim.x * 4) {
+    ln_row<NV>(x + (int64_t)row * D, ww, bb, eps, lane, true, v);
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) am = max3(am, fabsf(v[i][j]), fabsf(v[i][j + 1]));
+  }
+  amax_finish(bf16_round(am), factor, ts, ws);               // rounding is monotone: the maximum of the rounded values
+}
+
 template <int NV, typename TO>
 __global__ void __launch_bounds__(128) ln_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps,
                                                       int M, TO* __restrict__ y) {
@@ -485,23 +589,42 @@ __global__ void __launch_bounds__(256) broadcast_rows_kernel(const float4* __res
 }
 
 // ------------------------------------------------------------------------------------------------ host launchers
+static int rows_32b_aligned(const void* x, int64_t pitch_bytes) { return ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)pitch_bytes) & 31) == 0; }   // 256-bit loads
+
+template <typename T>
+static int launch_amax_scale(const void* x, int64_t ldx, int M, int K, bool gelu, float factor, float* ts, void* ws, cudaStream_t st) {
+  const int64_t total = (int64_t)M * (K / 32);
+  KF_REQUIRE(total + (1 << 20) < (1ll << 32), "kf_amax_scale: M*K/32 = %lld work items do not fit the 32-bit index", (long long)total);
+  int sms = 0;
+  const int rc = device_sm_count(&sms);
+  if (rc != KF_OK) return rc;
+  // one round of resident blocks at most: every block ends with one atomic on the same word
+  const unsigned grid = (unsigned)((total + 255) / 256 < 4 * sms ? (total + 255) / 256 : 4 * sms);
+  const int wide = rows_32b_aligned(x, ldx * (int64_t)sizeof(T));
+  const T* xp = static_cast<const T*>(x);
+  if (gelu) amax_scale_kernel<T, true><<<grid, 256, 0, st>>>(xp, ldx, M, K, wide, factor, ts, static_cast<uint32_t*>(ws));
+  else amax_scale_kernel<T, false><<<grid, 256, 0, st>>>(xp, ldx, M, K, wide, factor, ts, static_cast<uint32_t*>(ws));
+  return cuda_status(cudaGetLastError(), "kf_amax_scale launch");
+}
+
 template <typename T>
 static int launch_quant_rows(int fmt, const void* x, int64_t ldx, int M, int K, const float* ts, const float* bias, int flags, void* q, void* sf,
                              cudaStream_t st) {
-  int64_t per_row = K / 16;
+  int64_t per_row = K / 32;
   int64_t valid = (int64_t)M * per_row, total = (int64_t)((M + 127) / 128 * 128) * per_row;
-  KF_REQUIRE(total + 256 < (1ll << 32), "kf_quant_rows: M*K/16 = %lld work items do not fit the 32-bit index", (long long)total);
+  KF_REQUIRE(total + 256 < (1ll << 32), "kf_quant_rows: M*K/32 = %lld work items do not fit the 32-bit index", (long long)total);
   unsigned grid = (unsigned)((total + 255) / 256);
   const T* xp = static_cast<const T*>(x);
+  const int wide = rows_32b_aligned(x, ldx * (int64_t)sizeof(T));
   uint8_t *qp = static_cast<uint8_t*>(q), *sp = static_cast<uint8_t*>(sf);
-  if (fmt == KF_FMT_MX8) quant_rows_kernel<T, KF_FMT_MX8><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, qp, sp, valid, total);
-  else if (fmt == KF_FMT_NV4) quant_rows_kernel<T, KF_FMT_NV4><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, qp, sp, valid, total);
-  else quant_rows_kernel<T, KF_FMT_MX4><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, qp, sp, valid, total);
+  if (fmt == KF_FMT_MX8) quant_rows_kernel<T, KF_FMT_MX8><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
+  else if (fmt == KF_FMT_NV4) quant_rows_kernel<T, KF_FMT_NV4><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
+  else quant_rows_kernel<T, KF_FMT_MX4><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
   return cuda_status(cudaGetLastError(), "kf_quant_rows launch");
 }
 
-template <int NV>
-static int launch_ln_quant(int fmt, const float* x, const float* w, const float* b, float eps, int M, const float* ts, int flags, void* q, void* sf,
+template <int NV, typename TI>
+static int launch_ln_quant(int fmt, const TI* x, const float* w, const float* b, float eps, int M, const float* ts, int flags, void* q, void* sf,
                            float* y_dbg, cudaStream_t st) {
   int rows_pad = (M + 127) / 128 * 128;
   int sms = 0;
@@ -513,7 +636,7 @@ static int launch_ln_quant(int fmt, const float* x, const float* w, const float*
   uint8_t *qp = static_cast<uint8_t*>(q), *sp = static_cast<uint8_t*>(sf);
   unsigned int* err = dev_error_ptr();
   KF_REQUIRE(err != nullptr, "kf_ln_quant: device error word unavailable");
-  const size_t smem = (size_t)4 * LNQ_RING * NV * 256 * 4 + 4 * LNQ_RING * 8 + 16;
+  const size_t smem = (size_t)4 * LNQ_RING * NV * 256 * sizeof(TI) + 4 * LNQ_RING * 8 + 16;
   static int per_sm_cached[3][64] = {};                  // per (format, device) of this row width
   auto go = [&](auto kern) {
     // persistent: as many CTAs of 4 warps as are resident at once (4 per SM up to d = 1024, fewer for wider rows); a
@@ -532,9 +655,19 @@ static int launch_ln_quant(int fmt, const float* x, const float* w, const float*
     if (grid > (unsigned)(sms * per_sm)) grid = (unsigned)(sms * per_sm);
     return cuda_status(launch_maybe_pdl(kern, dim3(grid), dim3(128), smem, st, x, w, b, eps, M, rows_pad, ts, flags, qp, sp, y_dbg, err), "kf_ln_quant launch");
   };
-  if (fmt == KF_FMT_MX8) return go(ln_quant_kernel<NV, KF_FMT_MX8>);
-  if (fmt == KF_FMT_NV4) return go(ln_quant_kernel<NV, KF_FMT_NV4>);
-  return go(ln_quant_kernel<NV, KF_FMT_MX4>);
+  if (fmt == KF_FMT_MX8) return go(ln_quant_kernel<NV, KF_FMT_MX8, TI>);
+  if (fmt == KF_FMT_NV4) return go(ln_quant_kernel<NV, KF_FMT_NV4, TI>);
+  return go(ln_quant_kernel<NV, KF_FMT_MX4, TI>);
+}
+
+template <int NV, typename TI>
+static int launch_ln_amax(const TI* x, const float* w, const float* b, float eps, int M, float factor, float* ts, void* ws, cudaStream_t st) {
+  int sms = 0;
+  const int rc = device_sm_count(&sms);
+  if (rc != KF_OK) return rc;
+  const int grid = (M + 3) / 4 < 4 * sms ? (M + 3) / 4 : 4 * sms;
+  ln_amax_kernel<NV, TI><<<grid, 128, 0, st>>>(x, w, b, eps, M, factor, ts, static_cast<uint32_t*>(ws));
+  return cuda_status(cudaGetLastError(), "kf_ln_amax_scale launch");
 }
 
 template <int NV>
@@ -551,6 +684,35 @@ static int launch_ln_tail(const float* x, const float* w, const float* b, float 
   ln_tail_kernel<NV><<<(unsigned)((M + 3) / 4), 128, 0, st>>>(x, w, b, eps, M, Ntok, Q, npre, static_cast<__nv_bfloat16*>(qb), static_cast<__nv_bfloat16*>(xb),
                                                               static_cast<const __nv_bfloat16*>(wcls), bcls, ncls1, static_cast<__nv_bfloat16*>(cl));
   return cuda_status(cudaGetLastError(), "kf_ln_tail launch");
+}
+
+template <typename TI>
+static int ln_quant_width(int fmt, const TI* x, const float* w, const float* b, float eps, int M, int d, const float* ts, int flags, void* q, void* sf, float* y_dbg,
+                          cudaStream_t st) {
+  switch (d / 256) {
+    case 1: return launch_ln_quant<1, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    case 2: return launch_ln_quant<2, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    case 3: return launch_ln_quant<3, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    case 4: return launch_ln_quant<4, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    case 5: return launch_ln_quant<5, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    case 6: return launch_ln_quant<6, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    case 7: return launch_ln_quant<7, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+    default: return launch_ln_quant<8, TI>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
+  }
+}
+
+template <typename TI>
+static int ln_amax_width(const TI* x, const float* w, const float* b, float eps, int M, int d, float factor, float* ts, void* ws, cudaStream_t st) {
+  switch (d / 256) {
+    case 1: return launch_ln_amax<1, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    case 2: return launch_ln_amax<2, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    case 3: return launch_ln_amax<3, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    case 4: return launch_ln_amax<4, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    case 5: return launch_ln_amax<5, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    case 6: return launch_ln_amax<6, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    case 7: return launch_ln_amax<7, TI>(x, w, b, eps, M, factor, ts, ws, st);
+    default: return launch_ln_amax<8, TI>(x, w, b, eps, M, factor, ts, ws, st);
+  }
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -585,16 +747,30 @@ extern "C" int kf_ln_quant(int fmt, const float* x, const float* w, const float*
   KF_REQUIRE(aligned16(x) && aligned16(w) && aligned16(b) && aligned16(q) && aligned16(sf) && aligned16(y_dbg), "kf_ln_quant: tensors must be 16-byte aligned");
   KF_REQUIRE(fmt != KF_FMT_NV4 || ts, "kf_ln_quant: nv4 needs the per-tensor scale pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  switch (d / 256) {
-    case 1: return launch_ln_quant<1>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    case 2: return launch_ln_quant<2>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    case 3: return launch_ln_quant<3>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    case 4: return launch_ln_quant<4>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    case 5: return launch_ln_quant<5>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    case 6: return launch_ln_quant<6>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    case 7: return launch_ln_quant<7>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-    default: return launch_ln_quant<8>(fmt, x, w, b, eps, M, ts, flags, q, sf, y_dbg, st);
-  }
+  if (flags & KF_Q_IN_BF16) return ln_quant_width(fmt, reinterpret_cast<const __nv_bfloat16*>(x), w, b, eps, M, d, ts, flags, q, sf, y_dbg, st);
+  return ln_quant_width(fmt, x, w, b, eps, M, d, ts, flags, q, sf, y_dbg, st);
+}
+
+extern "C" int kf_amax_scale(int in_dtype, const void* x, int64_t ldx, int M, int K, int flags, float factor, float* ts, void* ws, void* stream) {
+  KF_REQUIRE(in_dtype == KF_F32 || in_dtype == KF_BF16 || in_dtype == KF_F16, "kf_amax_scale: unknown input dtype %d", in_dtype);
+  KF_REQUIRE(M > 0 && K > 0 && K % 32 == 0, "kf_amax_scale: K=%d must be a positive multiple of 32 and M=%d positive", K, M);
+  KF_REQUIRE(x && ts && ws && aligned16(x), "kf_amax_scale: tensors must be non-null and x 16-byte aligned");
+  KF_REQUIRE(ldx >= K && ldx % 8 == 0, "kf_amax_scale: row stride %lld must be >= K and a multiple of 8", (long long)ldx);
+  KF_REQUIRE((flags & ~KF_Q_GELU) == 0, "kf_amax_scale: only KF_Q_GELU is a valid flag");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool gelu = flags & KF_Q_GELU;
+  if (in_dtype == KF_F32) return launch_amax_scale<float>(x, ldx, M, K, gelu, factor, ts, ws, st);
+  if (in_dtype == KF_BF16) return launch_amax_scale<__nv_bfloat16>(x, ldx, M, K, gelu, factor, ts, ws, st);
+  return launch_amax_scale<__half>(x, ldx, M, K, gelu, factor, ts, ws, st);
+}
+
+extern "C" int kf_ln_amax_scale(int in_dtype, const void* x, const float* w, const float* b, float eps, int M, int d, float factor, float* ts, void* ws, void* stream) {
+  KF_REQUIRE(in_dtype == KF_F32 || in_dtype == KF_BF16, "kf_ln_amax_scale: x must be f32 or bf16");
+  KF_REQUIRE(M > 0 && d > 0 && d % 256 == 0 && d <= 2048, "kf_ln_amax_scale: d=%d must be a multiple of 256 up to 2048 and M=%d positive", d, M);
+  KF_REQUIRE(x && w && b && ts && ws && aligned16(x) && aligned16(w) && aligned16(b), "kf_ln_amax_scale: tensors must be non-null and 16-byte aligned");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (in_dtype == KF_BF16) return ln_amax_width(static_cast<const __nv_bfloat16*>(x), w, b, eps, M, d, factor, ts, ws, st);
+  return ln_amax_width(static_cast<const float*>(x), w, b, eps, M, d, factor, ts, ws, st);
 }
 
 extern "C" int kf_ln_rows(const float* x, const float* w, const float* b, float eps, int M, int d, int out_dtype, void* y, void* stream) {

@@ -61,23 +61,18 @@ class _Swap:
 
     def __init__(self, fmt: str):
         self.fmt = fmt
-        self.pool: Dict[tuple, ops.ActBuf] = {}      # persistent operands per (rows, K, device, role)
+        self.pool: Dict[tuple, tuple] = {}           # persistent operands per (rows, K, device, role), each with its scale's workspace
         self.slots: Dict[tuple, tuple] = {}          # unit -> (operand, leading shape) waiting for its Linear
         self.modules: List[torch.nn.Module] = []
 
-    def operand(self, rows: int, K: int, device, role: str) -> ops.ActBuf:
-        key = (rows, K, str(device), role)
-        buf = self.pool.get(key)
-        if buf is None:
-            buf = self.pool[key] = ops.ActBuf(rows, K, self.fmt, device)
-        return buf
-
-    def set_dynamic_scale(self, buf: ops.ActBuf, values: torch.Tensor) -> None:
-        """nv4 only: per-tensor scale amax / (6 * 448) of the values about to be quantised, on the device."""
-        if self.fmt != "nv4":
-            return
-        peak = values.float().abs().amax()
-        buf.ts.copy_(torch.where(peak > 0, peak / 2688.0, torch.ones_like(peak)).reshape(1))
+    def operand(self, rows: int, K: int, device, role: str) -> tuple:
+        """-> (operand, workspace of its dynamic scale; None unless the format is nv4)."""
+        key = (rows, K, device, role)
+        got = self.pool.get(key)
+        if got is None:
+            ws = torch.zeros(2, dtype=torch.int32, device=device) if self.fmt == "nv4" else None
+            got = self.pool[key] = (ops.ActBuf(rows, K, self.fmt, device), ws)
+        return got
 
     def install(self, module: torch.nn.Module, fn: Callable) -> None:
         module.forward = fn                          # instance attribute: shadows the class forward until disable()
@@ -98,19 +93,20 @@ class _Feeder:
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         sw = self.swap
         if self.how == "ln":
-            src = x.reshape(-1, x.shape[-1]).float().contiguous()
-            buf = sw.operand(src.shape[0], src.shape[1], x.device, "ln")
-            if sw.fmt == "nv4":
-                sw.set_dynamic_scale(buf, ops.ln_rows(src, self.w, self.b, self.eps, BF))
+            src = x.reshape(-1, x.shape[-1])
+            src = src.contiguous() if src.dtype in (torch.float32, BF) else src.float().contiguous()
+            buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "ln")
+            if ws is not None:
+                ops.ln_amax_scale(src, self.w, self.b, self.eps, buf.ts, ws)
             ops.ln_quant(src, self.w, self.b, self.eps, buf, round_bf16=True)
         else:
             src = _rows(x)
-            buf = sw.operand(src.shape[0], src.shape[1], x.device, "gelu")
-            zkey = (src.shape[1], str(x.device))
+            buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "gelu")
+            zkey = (src.shape[1], x.device)
             if zkey not in self.no_bias:
                 self.no_bias[zkey] = torch.zeros(src.shape[1], dtype=torch.float32, device=x.device)
-            if sw.fmt == "nv4":
-                sw.set_dynamic_scale(buf, torch.nn.functional.gelu(src.float()))
+            if ws is not None:
+                ops.amax_scale(src, buf.ts, ws, gelu=True)
             ops.quant_rows(src, buf, bias=self.no_bias[zkey], gelu=True, round_bf16=True)
         sw.slots[self.unit] = (buf, tuple(x.shape[:-1]))
         return x.new_empty(0)
@@ -138,8 +134,9 @@ class _QLinear:
         else:
             src = _rows(x)
             lead = tuple(x.shape[:-1])
-            buf = sw.operand(src.shape[0], src.shape[1], x.device, "lin")
-            sw.set_dynamic_scale(buf, src)
+            buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "lin")
+            if ws is not None:
+                ops.amax_scale(src, buf.ts, ws)
             ops.quant_rows(src, buf)
         y = ops.gemm_plain(buf, self.weight, self.bias, out_dtype=BF)
         return y.view(*lead, self.out_features)

@@ -146,13 +146,13 @@ def quantx(x: torch.Tensor, out: ActBuf, **kw) -> ActBuf:
 
 def ln_quant(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, out: ActBuf, *, round_bf16: bool = False,
              recip_div: bool = False, y_dbg: Optional[torch.Tensor] = None) -> ActBuf:
-    """LayerNorm of the fp32 residual stream x [..., d] fused with quantisation into out (ln_mx8 / lnq)."""
+    """LayerNorm of the fp32 (or bf16) stream x [..., d] fused with quantisation into out (ln_mx8 / lnq)."""
     global LAUNCHES
     LAUNCHES += 1
     args = (x, w, b, eps, out, _flags(False, round_bf16, recip_div), y_dbg)
     if TIMING is None:
         return _h.ln_quant(*args)
-    return _timed("ln_quant", _h.ln_quant, args, x.numel() * 4 + out.q.numel() + out.sf.numel())
+    return _timed("ln_quant", _h.ln_quant, args, x.numel() * x.element_size() + out.q.numel() + out.sf.numel())
 
 
 def ln_mx8(x, w, b, out: ActBuf, eps: float, **kw) -> ActBuf:
@@ -172,6 +172,23 @@ def ln_rows(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, dtype
 
 
 ln_bf16 = ln_rows
+
+
+def amax_scale(x: torch.Tensor, ts: torch.Tensor, ws: torch.Tensor, *, factor: float = 1.0 / 2688.0, gelu: bool = False) -> torch.Tensor:
+    """ts [1] = factor * max|v| (1 where that is zero or NaN), v = x [M, K] or gelu_erf(x), in one launch and without a host sync: the
+    dynamic per-tensor scale of an NVFP4 operand.  ws: int32 [2], zero before the first use (a call leaves it zero)."""
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (x, KF_Q_GELU if gelu else 0, factor, ts, ws)
+    return _h.amax_scale(*args) if TIMING is None else _timed("amax_scale", _h.amax_scale, args)
+
+
+def ln_amax_scale(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, ts: torch.Tensor, ws: torch.Tensor, *, factor: float = 1.0 / 2688.0) -> torch.Tensor:
+    """amax_scale of the bf16-rounded LayerNorm of f32 | bf16 x [..., d], which is not written anywhere."""
+    global LAUNCHES
+    LAUNCHES += 1
+    args = (x, w, b, eps, factor, ts, ws)
+    return _h.ln_amax_scale(*args) if TIMING is None else _timed("amax_scale", _h.ln_amax_scale, args)
 
 
 # ------------------------------------------------------------------------------------------------ weights and GEMMs

@@ -193,3 +193,55 @@ def test_non_finite_inputs_follow_the_reference(golden, fmt):
     nb = x.shape[1] // qo.VEC[fmt]
     s2 = qo.from_blocked(a.sf.cpu().numpy().reshape(1, -(-nb // 4), 32, 4, 4), x.shape[0], nb)
     assert np.array_equal(s2, golden[f"nonfinite/{key}_s"])
+
+
+# (rows, K, row stride): one row, a row count that ends inside a block of threads, strides that allow 256-bit loads and ones that do not
+@pytest.mark.parametrize("M,K,ld", [(1, 128, 128), (130, 768, 776), (1605, 3072, 3072)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("gelu", [False, True])
+def test_amax_scale(M, K, ld, dtype, gelu):
+    ops = _ops()
+    x = torch.randn(M, ld, generator=torch.Generator().manual_seed(M)).to(dtype).cuda()[:, :K]
+    ts, ws = torch.zeros(1, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda")
+    for scale in (1.0, 0.01, 0.0):                         # the workspace is left ready for the next call; small values: the negative side decides
+        xs = (x.float() * scale).to(dtype) if scale != 1.0 else x
+        ops.amax_scale(xs, ts, ws, gelu=gelu)
+        peak = (torch.nn.functional.gelu(xs.float()) if gelu else xs.float()).abs().amax()
+        expect = peak / 2688.0 if float(peak) > 0 else torch.ones_like(peak)
+        assert torch.allclose(ts, expect.reshape(1), rtol=1e-6, atol=0)
+        assert int(ws.abs().sum()) == 0
+    bad = x.clone()
+    bad[M // 2, K // 2] = float("nan")
+    assert float(ops.amax_scale(bad, ts, ws, gelu=gelu)) == 1.0
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("M,d", [(1, 768), (333, 1024), (2500, 256)])
+def test_ln_quant_and_scale_of_bf16_rows(fmt, M, d):
+    ops = _ops()
+    g = torch.Generator().manual_seed(d)
+    x = (torch.randn(M, d, generator=g) * 2 + 0.3).to(torch.bfloat16).cuda()
+    w, b = (torch.rand(d, generator=g) + 0.5).cuda(), (torch.randn(d, generator=g) * 0.1).cuda()
+    a, c = ops.ActBuf(M, d, fmt), ops.ActBuf(M, d, fmt)
+    if fmt == "nv4":
+        ws = torch.zeros(2, dtype=torch.int32, device="cuda")
+        for t in (x, x.float()):
+            ops.ln_amax_scale(t, w, b, 1e-6, a.ts, ws)
+            assert torch.allclose(a.ts, ops.ln_rows(x.float(), w, b, 1e-6).float().abs().amax().reshape(1) / 2688.0, rtol=1e-6, atol=0)
+        c.ts.copy_(a.ts)
+    ops.ln_quant(x, w, b, 1e-6, a, round_bf16=True)
+    ops.ln_quant(x.float(), w, b, 1e-6, c, round_bf16=True)
+    assert torch.equal(a.q, c.q) and torch.equal(a.sf, c.sf)
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_quant_rows_of_rows_without_32_byte_alignment(fmt, dtype):
+    x = torch.randn(131, 264, generator=torch.Generator().manual_seed(5)).to(dtype)
+    x[3, 9] = -0.0 if dtype == torch.float16 else 0.0
+    rows = x.cuda()[:, 8:]                                  # offset and stride are multiples of 16 bytes only
+    xn = x[:, 8:].float().numpy()
+    ts = qo.nv4_ts(xn) if fmt == "nv4" else None
+    q, sf = _run_quant(rows, fmt, ts)
+    eq, esf = _expect(xn, fmt, ts)
+    assert np.array_equal(sf, esf) and np.array_equal(q, eq)
