@@ -166,21 +166,20 @@ __device__ __forceinline__ void quant_chunk(const GemmArgs& g, const uint32_t (&
 // ------------------------------------------------------------------------------------------------ PLAIN
 // PLAIN epilogue of one 32-column chunk: the thread writes 64 (16-bit) or 128 (fp32) contiguous bytes of its row.
 __device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, uint8_t* dst_row, int n0, const float* bsm /* the chunk's 32 bias values in shared memory */) {
+  const float2 ts2 = splat2(ts);
 #pragma unroll
   for (int q = 0; q < 2; ++q) {                 // 16 columns at a time
     float v[16];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const float4 bb = g.bias ? *reinterpret_cast<const float4*>(bsm + 16 * q + 4 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float b4[4] = {bb.x, bb.y, bb.z, bb.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float a = __uint_as_float(r[16 * q + 4 * h + e]);
-        float x = (g.flags & KF_G_PRE_ROUND_BF16) ? bf16_round(a * ts) + b4[e] : fmaf(a, ts, b4[e]);   // the result may be rounded to bf16 before the bias
-        if (g.flags & KF_G_GELU) x = gelu_erf(x);
-        if (g.flags & KF_G_ROUND_BF16) x = bf16_round(x);
-        v[4 * h + e] = x;
-      }
+    for (int h = 0; h < 8; ++h) {               // packed pairs
+      const int k = 16 * q + 2 * h;
+      const float2 bb = g.bias ? *reinterpret_cast<const float2*>(bsm + k) : make_float2(0.f, 0.f);
+      const float2 a = make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1]));
+      float2 x = (g.flags & KF_G_PRE_ROUND_BF16) ? add2(bf16_round2(mul2(a, ts2)), bb) : fma2(a, ts2, bb);   // the result may be rounded to bf16 before the bias
+      if (g.flags & KF_G_GELU) x = gelu_erf_pair(x);
+      if (g.flags & KF_G_ROUND_BF16) x = bf16_round2(x);
+      v[2 * h] = x.x;
+      v[2 * h + 1] = x.y;
     }
     if (dst_row) {
       if (g.out_dtype == KF_F32) {

@@ -103,6 +103,24 @@ class VideoPipeline:
             self.h2d.wait_event(s.ev_comp)                  # the slot's previous compute has consumed dev_in
             s.dev_in.copy_(host, non_blocking=True)
             s.ev_h2d.record(self.h2d)
+        self._compute(s)
+
+    @torch.no_grad()
+    def _load_frame(self, s: _Slot, j: int, frame: torch.Tensor) -> None:
+        """Frame j of a slot: into the slot's pinned buffer, and on to the device at once.  The copy of a frame runs while the host
+        stages the next one, so a micro-batch is on the device one frame after its last host copy (staging the whole batch
+        first put another 2.3 ms in front of the first graph for 14 frames of 1900 x 1440, in every run)."""
+        s.pinned_in[j].copy_(frame)
+        with torch.cuda.stream(self.h2d):
+            if j == 0:
+                self.h2d.wait_event(s.ev_comp)              # the slot's previous compute has consumed dev_in
+            s.dev_in[j].copy_(s.pinned_in[j], non_blocking=True)
+            if j == self.B - 1:
+                s.ev_h2d.record(self.h2d)                   # by this thread: the next slot's frames follow on the same stream
+
+    @torch.no_grad()
+    def _compute(self, s: _Slot) -> None:
+        """graph -> D2H of a slot whose frames are on their way (ev_h2d)."""
         with torch.cuda.stream(self.comp):
             self.comp.wait_event(s.ev_h2d)
             self.comp.wait_event(s.ev_d2h)                  # the slot's previous labels have left dev_out
@@ -118,7 +136,7 @@ class VideoPipeline:
 
     # ------------------------------------------------------------------ streaming driver
     def run(self, source: Iterable, consumer: Optional[Callable] = None) -> dict:
-        """source yields uint8 host frames [H, W, 3] (numpy or torch; copied into the ring), whole pinned batches
+        """source yields uint8 host frames [H, W, 3] (numpy or torch; copied into the ring and sent on frame by frame), whole pinned batches
         [B, H, W, 3] (read in place) or (pinned batch, valid) pairs for a batch of which only the first `valid` frames count.
         consumer(frame_index, labels) is called in frame order from the result thread with a numpy view [h, w] of the slot's
         pinned output; it must copy what it keeps.  A last, partial batch is padded with
@@ -171,16 +189,16 @@ class VideoPipeline:
                             break
                         self.slots[k].src = None
                         t_in = time.perf_counter()
-                    self.slots[k].pinned_in[fill].copy_(t)
+                    self._load_frame(self.slots[k], fill, t)
                     fill += 1
                     if fill == self.B:
                         filled.put((k, idx, self.B, t_in))
                         idx += self.B
                         k, fill = None, 0
                 if k is not None and fill and not stop.is_set():   # tail: pad with the last frame
-                    buf = self.slots[k].pinned_in
+                    last = self.slots[k].pinned_in[fill - 1]
                     for j in range(fill, self.B):
-                        buf[j].copy_(buf[fill - 1])
+                        self._load_frame(self.slots[k], j, last)
                     filled.put((k, idx, fill, t_in))
             except Exception as e:  # noqa: BLE001
                 failed.append(e)
@@ -230,7 +248,10 @@ class VideoPipeline:
                     continue
                 gate.acquire()
                 try:
-                    self.submit(k, self.slots[k].src)
+                    if self.slots[k].src is None:
+                        self._compute(self.slots[k])
+                    else:
+                        self.submit(k, self.slots[k].src)
                 except Exception:
                     gate.release()
                     free.put(k)
