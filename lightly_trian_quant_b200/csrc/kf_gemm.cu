@@ -3,7 +3,7 @@
 //
 //   operands   K-major codes: e4m3 bytes (mx8), packed e2m1 nibbles (nv4 / mx4) or plain bf16; scale factors in
 //              the 128x4 blocked layout, one 512-byte atom per 128 rows x 4 k-blocks
-//   tile       128 x 256 output tile per CTA step (one MMA instruction is 128 x 256 x 32 K-bytes), 128 bytes of K per
+//   tile       128 x 256 output tile per CTA step (128 x 128 for launches of a few tiles: gemm_columns) (one MMA instruction is 128 x 256 x 32 K-bytes), 128 bytes of K per
 //              pipeline stage.  The tile shape is set by shared-memory bandwidth: a 128 x 128 MMA reads its 8 KB of
 //              operands in the ~68 clk it executes, which alone saturates the 128 B/clk of the shared-memory array,
 //              and the TMA writes of the next stages need the same array (measured: main loop at half the instruction
@@ -36,30 +36,41 @@
 
 namespace kf {
 
-// Depth of the operand ring, chosen per launch.  A fourth stage (54 KB) helps where the main loop is the longer chain
+// Depth of the operand ring, chosen per launch.  BN = 256: a fourth stage (54 KB) helps where the main loop is the longer chain
 // (measured at M = 22 470: fc2 K 4096 79 -> 76 us, MXFP8 fc2 116 -> 108 us, PLAIN 73 -> 69 us) and hurts where the epilogue is
 // (proj 51 -> 53 us, fc1 93 -> 98 us: the stage's shared memory comes out of the L1 the epilogue's global accesses use);
-// the ROPE kernel's table slabs leave no room for one.
-constexpr int MAX_STAGES = 4;
+// the ROPE kernel's table slabs leave no room for one.  BN = 128: the launches of a few tiles, where the fill rate is the bytes in
+// flight over the L2 latency, so all of K up to six stages (36 KB each).
+constexpr int MAX_STAGES = 6;
+template <int BN>
 static int gemm_stages(int epi, int k_tiles, int flags) {
+  if (BN == 128) {
+    const int most = epi == KF_EPI_ROPE ? 5 : 6;
+    return k_tiles < 2 ? 2 : k_tiles < most ? k_tiles : most;
+  }
   if (epi == KF_EPI_PLAIN) return (flags & KF_G_GELU) ? 3 : 4;      // PLAIN with GELU (the head's ConvTranspose GEMMs) is epilogue-bound too
   if (epi == KF_EPI_RES && k_tiles >= 8) return 4;
   return 3;
 }
 constexpr size_t GEMM_SMEM_MAX = 227 * 1024;
-template <int EPI>
-constexpr size_t gemm_smem(int stages, int vec_floats = 0) {   // operand ring + scale atoms + bias slices or vectors (+ the rotary-table slabs) + barriers
+// operand ring + scale atoms + bias slices or vectors (+ the rotary-table slabs) + barriers
+template <int EPI, int BN>
+constexpr size_t gemm_smem(int stages, int vec_floats = 0) {
   const size_t sl = (size_t)(vec_floats > EPI_WARPS * SLICE_FLOATS ? vec_floats : EPI_WARPS * SLICE_FLOATS) * 4;
-  return (size_t)stages * (TILE_BYTES + SF_STAGE_BYTES) + sl + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS * 4 : 0) + 256;
+  return (size_t)stages * (Tile<BN>::BYTES + Tile<BN>::SF_BYTES) + sl + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS * 4 : 0) + 256;
 }
+static_assert(gemm_smem<KF_EPI_ROPE, 256>(3) <= GEMM_SMEM_MAX && gemm_smem<KF_EPI_RES, 256>(4) <= GEMM_SMEM_MAX && gemm_smem<KF_EPI_ROPE, 128>(5) <= GEMM_SMEM_MAX &&
+                  gemm_smem<KF_EPI_RES, 128>(6) <= GEMM_SMEM_MAX,
+              "shared memory of the deepest rings");
 
 // ------------------------------------------------------------------------------------------------ the kernel
-template <int KIND, int EPI>
+template <int KIND, int EPI, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const GemmArgs g) {
   constexpr int ATOMS = KindTraits<KIND>::ATOMS;
   constexpr bool SCALED = KIND != KIND_BF16;
-  const int STAGES = g.stages;                            // 3 or 4: the ring depth this launch was given shared memory for
+  constexpr int TILE_BYTES = Tile<BN>::BYTES, SF_STAGE_BYTES = Tile<BN>::SF_BYTES, ACCS = Tile<BN>::ACCS;
+  const int STAGES = g.stages;                            // the ring depth this launch was given shared memory for
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* tiles = smem;
@@ -67,8 +78,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   float* slices = reinterpret_cast<float*>(sfs + (size_t)STAGES * SF_STAGE_BYTES);
   float* slabs = slices + (g.vec_floats > EPI_WARPS * SLICE_FLOATS ? g.vec_floats : EPI_WARPS * SLICE_FLOATS);   // ROPE only
   uint64_t* bars = reinterpret_cast<uint64_t*>(slabs + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS : 0));
-  uint64_t *full = bars, *empty = bars + MAX_STAGES, *tfull = bars + 2 * MAX_STAGES, *tempty = tfull + 1;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 1);
+  uint64_t *full = bars, *empty = bars + MAX_STAGES, *tfull = bars + 2 * MAX_STAGES, *tempty = tfull + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   pdl_launch_dependents();                               // the next kernel of the stream may take the SMs this grid leaves
@@ -78,8 +89,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(tfull, 1);
-    mbar_init(tempty, EPI_WARPS);
+    for (int a = 0; a < ACCS; ++a) {
+      mbar_init(&tfull[a], 1);
+      mbar_init(&tempty[a], EPI_WARPS);
+    }
     *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;     // the swizzled operand tiles need a 1024-byte aligned base
     fence_mbar_init();
     prefetch_tmap(&tmA);
@@ -112,9 +125,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const int m_blk = tile / g.n_tiles, n_blk = tile - m_blk * g.n_tiles;
-        const int w_halves = (n_blk * BN + 128 < g.N) ? 2 : 1;                // the last column tile may hold only 128 columns
+        const int w_halves = (BN == 256 && n_blk * BN + 128 < g.N) ? 2 : 1;   // the last column tile of 256 may hold only 128 columns
         int row_end;
-        const int a_row0 = tile_row0(g, m_blk, row_end), w_row0 = tile_wrow0(g, m_blk, n_blk);
+        const int a_row0 = tile_row0(g, m_blk, row_end), w_row0 = tile_wrow0(g, m_blk, n_blk * BN);
         const uint32_t tx = TILE_BYTES + (SCALED ? (1 + w_halves) * ATOMS * 512 : 0);
         for (int kt = 0; kt < g.k_tiles; ++kt) {
           if (!mbar_wait_warp(&empty[s], ph ^ 1, ctx, 1)) { ok = false; break; }
@@ -127,7 +140,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               uint8_t* sa = sfs + (size_t)s * SF_STAGE_BYTES;
               bulk_load_1d(sa, g.sfa + ((size_t)m_blk * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
               for (int h = 0; h < w_halves; ++h)
-                bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(2 * n_blk + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
+                bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(BN / 128 * n_blk + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
             }
           }
           __syncwarp();
@@ -148,17 +161,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++lt) {
         const int n_blk = tile % g.n_tiles;
-        const bool two = n_blk * BN + 128 < g.N;
-        if (!mbar_wait_warp(tempty, (lt & 1) ^ 1, ctx, 2)) break;               // the epilogue has taken the previous tile out of TMEM
+        const bool two = BN == 256 && n_blk * BN + 128 < g.N;
+        const uint32_t ac = lt % ACCS;
+        if (!mbar_wait_warp(&tempty[ac], ((lt / ACCS) & 1) ^ 1, ctx, 2)) break;   // the epilogue has taken this accumulator's previous tile out of TMEM
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base;
+        const uint32_t d_tmem = tmem_base + ac * BN;
         for (int kt = 0; kt < g.k_tiles; ++kt) {
           if (!mbar_wait_warp(&full[s], ph, ctx, 3)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + (size_t)s * TILE_BYTES);
           const uint64_t adesc = smem_desc_sw128(a_addr), bdesc = smem_desc_sw128(a_addr + A_BYTES);
-          // scale factors of this stage: A at +0 (4 columns per atom), W at +16 (8 columns per atom pair: the atom of
-          // columns 0..127 of the tile, then the atom of columns 128..255)
+          // scale factors of this stage: A at +0 (4 columns per atom), W at +16 (BN = 256: 8 columns per atom pair, the atom of
+          // columns 0..127 of the tile, then the atom of columns 128..255; BN = 128: 4 columns per atom)
+          constexpr uint32_t WS = 4 * (BN / 128);
           const uint32_t sf_t = tmem_base + TMEM_SF_COL + sb * SF_BUF_COLS;
           const uint32_t sa = smem_u32(sfs + (size_t)s * SF_STAGE_BYTES);
           if (elect_one()) {
@@ -166,8 +181,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
               for (int a = 0; a < ATOMS; ++a) {
                 tc_cp_sf(sf_t + 4 * a, smem_desc_sf(sa + a * 512));
-                tc_cp_sf(sf_t + 16 + 8 * a, smem_desc_sf(sa + (ATOMS + a) * 512));
-                if (two) tc_cp_sf(sf_t + 16 + 8 * a + 4, smem_desc_sf(sa + (2 * ATOMS + a) * 512));
+                tc_cp_sf(sf_t + 16 + WS * a, smem_desc_sf(sa + (ATOMS + a) * 512));
+                if (two) tc_cp_sf(sf_t + 16 + WS * a + 4, smem_desc_sf(sa + (2 * ATOMS + a) * 512));
               }
             }
 #pragma unroll
@@ -179,13 +194,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               } else if (KIND == KIND_MX8) {      // one scale per row per MMA: byte j of the atom's 32-bit word
                 mma_mxf8(d_tmem, ad, bd, idesc_with_sf_id(IDESC, j, j), acc, sf_t, sf_t + 16);
               } else if (KIND == KIND_NV4) {      // four scales per row per MMA: atom j
-                mma_nvf4(d_tmem, ad, bd, IDESC, acc, sf_t + 4 * j, sf_t + 16 + 8 * j);
+                mma_nvf4(d_tmem, ad, bd, IDESC, acc, sf_t + 4 * j, sf_t + 16 + WS * j);
               } else {                            // two scales per row per MMA: half-word (j & 1) of atom j / 2
-                mma_mxf4(d_tmem, ad, bd, idesc_with_sf_id(IDESC, 2 * (j & 1), 2 * (j & 1)), acc, sf_t + 4 * (j >> 1), sf_t + 16 + 8 * (j >> 1));
+                mma_mxf4(d_tmem, ad, bd, idesc_with_sf_id(IDESC, 2 * (j & 1), 2 * (j & 1)), acc, sf_t + 4 * (j >> 1), sf_t + 16 + WS * (j >> 1));
               }
             }
             tc_commit(&empty[s]);
-            if (kt == g.k_tiles - 1) tc_commit(tfull);
+            if (kt == g.k_tiles - 1) tc_commit(&tfull[ac]);
           }
           __syncwarp();
           if (SCALED && ++sb == SF_BUFS) sb = 0;
@@ -197,8 +212,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ------------------------------------------------------------------ epilogue: 16 warps, warp = (TMEM lane quarter, 64-column group)
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
     if (!bad_align) {
-      const TileSched sched{(int)blockIdx.x, (int)gridDim.x, total_tiles, g.n_tiles, -1};
-      epilogue_warps<EPI>(g, sched, tmem_base, tfull, tempty, slices, slabs, ctx, warp, lane);
+      const TileSched sched{(int)blockIdx.x, (int)gridDim.x, total_tiles, g.n_tiles};
+      epilogue_warps<EPI, BN>(g, sched, tmem_base, tfull, tempty, slices, slabs, ctx, warp, lane);
     }
   }
 
@@ -294,27 +309,54 @@ int device_sm_count(int* sms) {
   return KF_OK;
 }
 
-template <int KIND, int EPI>
+template <int KIND, int EPI, int BN>
 static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs& g, int grid, cudaStream_t st) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_MAX);
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<KIND, EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_MAX);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_kernel)");
     if (dev < 64) attr_set[dev] = true;
   }
-  return cuda_status(launch_maybe_pdl(gemm_kernel<KIND, EPI>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI>(g.stages, g.vec_floats), st, tmA, tmW, g), "kf_gemm_bs launch");
+  return cuda_status(launch_maybe_pdl(gemm_kernel<KIND, EPI, BN>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats), st, tmA, tmW, g), "kf_gemm_bs launch");
 }
 
-template <int KIND>
+template <int KIND, int BN>
 static int launch_gemm_epi(int epi, const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs& g, int grid, cudaStream_t st) {
   switch (epi) {
-    case KF_EPI_PLAIN: return launch_gemm<KIND, KF_EPI_PLAIN>(tmA, tmW, g, grid, st);
-    case KF_EPI_RES: return launch_gemm<KIND, KF_EPI_RES>(tmA, tmW, g, grid, st);
-    case KF_EPI_ROPE: return launch_gemm<KIND, KF_EPI_ROPE>(tmA, tmW, g, grid, st);
-    default: return launch_gemm<KIND, KF_EPI_QUANT>(tmA, tmW, g, grid, st);
+    case KF_EPI_PLAIN: return launch_gemm<KIND, KF_EPI_PLAIN, BN>(tmA, tmW, g, grid, st);
+    case KF_EPI_RES: return launch_gemm<KIND, KF_EPI_RES, BN>(tmA, tmW, g, grid, st);
+    case KF_EPI_ROPE: return launch_gemm<KIND, KF_EPI_ROPE, BN>(tmA, tmW, g, grid, st);
+    default: return launch_gemm<KIND, KF_EPI_QUANT, BN>(tmA, tmW, g, grid, st);
   }
+}
+
+template <int BN>
+static int launch_gemm_fmt(int fmt, int epi, const CUtensorMap& tmA, const CUtensorMap& tmW, GemmArgs& g, int sms, cudaStream_t st) {
+  g.n_tiles = (g.N + BN - 1) / BN;
+  const int total = g.m_tiles * g.n_tiles, grid = total < sms ? total : sms;
+  g.stages = gemm_stages<BN>(epi, g.k_tiles, g.flags);
+  // The whole bias (+ LayerScale) vector in shared memory where a CTA works on several tiles and the ring depth leaves room for it
+  const int want = (g.bias || epi == KF_EPI_RES) ? g.N * (epi == KF_EPI_RES ? 2 : 1) : 0;
+  const size_t with = epi == KF_EPI_ROPE ? gemm_smem<KF_EPI_ROPE, BN>(g.stages, want) : gemm_smem<KF_EPI_RES, BN>(g.stages, want);
+  g.vec_floats = (want > 0 && total > grid && with <= GEMM_SMEM_MAX) ? want : 0;
+  switch (fmt) {
+    case KF_FMT_MX8: return launch_gemm_epi<KIND_MX8, BN>(epi, tmA, tmW, g, grid, st);
+    case KF_FMT_NV4: return launch_gemm_epi<KIND_NV4, BN>(epi, tmA, tmW, g, grid, st);
+    case KF_FMT_MX4: return launch_gemm_epi<KIND_MX4, BN>(epi, tmA, tmW, g, grid, st);
+    default: return launch_gemm_epi<KIND_BF16, BN>(epi, tmA, tmW, g, grid, st);
+  }
+}
+
+// Column-tile width of a launch.  256 columns need the least operand traffic per product (the tile shape comment above) and win
+// wherever there are many tiles; 128 columns cut the launch finer, take twice the SMs where the tiles do not fill the
+// chip, and keep two accumulators in tensor memory.  A round of 128-column tiles takes about 0.6 of a round of 256-column tiles,
+// so 128 wins when ceil(tiles / SMs) rounds of them are shorter: one frame's 13 row tiles x 1024 columns are one round either way
+// (104 SMs instead of 52), x 4096 columns 3 x 0.6 rounds against 2; from about five rounds on the rounding no longer pays.
+static int gemm_columns(int m_tiles, int N, int sms) {
+  const int64_t r256 = ((int64_t)m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = ((int64_t)m_tiles * (N / 128) + sms - 1) / sms;
+  return 6 * r128 < 10 * r256 ? 128 : 256;
 }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -367,10 +409,15 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   }
   const uint64_t kbytes = fmt == KF_FMT_MX8 ? (uint64_t)p->K : (fmt == KF_FMT_BF16 ? 2ull * p->K : (uint64_t)p->K / 2);
   const uint64_t w_rows = p->batch > 0 ? (uint64_t)p->batch * p->w_rows_per_batch : (uint64_t)p->N;
-  CUtensorMap tmA, tmW;
-  int st = make_tmap_2d_bytes(&tmA, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
+  const int m_tiles = p->batch > 0 ? p->batch * ((p->a_rows_per_batch + BM - 1) / BM) : (p->M + BM - 1) / BM;
+  int sms = 0;
+  int st = device_sm_count(&sms);
   if (st != KF_OK) return st;
-  st = make_tmap_2d_bytes(&tmW, p->W, w_rows, kbytes, kbytes, BN);
+  const int bn = gemm_columns(m_tiles, p->N, sms);
+  CUtensorMap tmA, tmW;
+  st = make_tmap_2d_bytes(&tmA, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
+  if (st != KF_OK) return st;
+  st = make_tmap_2d_bytes(&tmW, p->W, w_rows, kbytes, kbytes, bn);
   if (st != KF_OK) return st;
   GemmArgs g{};
   g.sfa = static_cast<const uint8_t*>(p->SFA);
@@ -380,37 +427,18 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   g.M = p->M; g.N = p->N; g.K = p->K;
   g.Ntok = p->Ntok; g.prefix = p->prefix; g.H = p->H; g.d = p->H * 64;
   g.out_dtype = p->out_dtype; g.flags = p->flags; g.out_fmt = p->out_fmt;
-  g.m_tiles = (p->M + BM - 1) / BM; g.n_tiles = (p->N + BN - 1) / BN; g.k_tiles = (int)(kbytes / BKB);
+  g.m_tiles = m_tiles; g.k_tiles = (int)(kbytes / BKB);
   if (p->batch > 0) {
     g.m_tiles_pb = (p->a_rows_per_batch + BM - 1) / BM;
     g.a_rows_pb = p->a_rows_per_batch;
     g.w_rows_pb = p->w_rows_per_batch;
-    g.m_tiles = p->batch * g.m_tiles_pb;
   }
   g.nkb4 = fmt == KF_FMT_BF16 ? 0 : p->K / (4 * fmt_vec(fmt));
-  g.stages = gemm_stages(epi, g.k_tiles, p->flags);
-  {
-    // the whole bias (+ LayerScale) vector in shared memory where the ring depth of this launch leaves room for it
-    const int want = (p->bias || epi == KF_EPI_RES) ? p->N * (epi == KF_EPI_RES ? 2 : 1) : 0;
-    const size_t rest = (size_t)g.stages * (TILE_BYTES + SF_STAGE_BYTES) + (epi == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS * 4 : 0) + 256;
-    const size_t vec_bytes = (size_t)(want > EPI_WARPS * SLICE_FLOATS ? want : EPI_WARPS * SLICE_FLOATS) * 4;
-    g.vec_floats = (want > 0 && rest + vec_bytes <= GEMM_SMEM_MAX) ? want : 0;
-  }
   const bool maps_rows = epi == KF_EPI_PLAIN || epi == KF_EPI_RES;
   g.row_group = maps_rows ? p->out_row_group : 0; g.row_stride = p->out_row_stride; g.row_offset = p->out_row_offset;
   g.y_dbg = epi == KF_EPI_QUANT ? p->y_dbg : nullptr;
   g.err = dev_error_ptr();
   KF_REQUIRE(g.err != nullptr, "kf_gemm_bs: device error word unavailable");
-  int sms = 0;
-  st = device_sm_count(&sms);
-  if (st != KF_OK) return st;
-  const int total = g.m_tiles * g.n_tiles;
-  const int grid = total < sms ? total : sms;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  switch (fmt) {
-    case KF_FMT_MX8: return launch_gemm_epi<KIND_MX8>(epi, tmA, tmW, g, grid, cs);
-    case KF_FMT_NV4: return launch_gemm_epi<KIND_NV4>(epi, tmA, tmW, g, grid, cs);
-    case KF_FMT_MX4: return launch_gemm_epi<KIND_MX4>(epi, tmA, tmW, g, grid, cs);
-    default: return launch_gemm_epi<KIND_BF16>(epi, tmA, tmW, g, grid, cs);
-  }
+  return bn == 128 ? launch_gemm_fmt<128>(fmt, epi, tmA, tmW, g, sms, cs) : launch_gemm_fmt<256>(fmt, epi, tmA, tmW, g, sms, cs);
 }

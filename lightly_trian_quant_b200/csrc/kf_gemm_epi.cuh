@@ -15,9 +15,18 @@
 namespace kf {
 
 constexpr int KIND_MX8 = KF_FMT_MX8, KIND_NV4 = KF_FMT_NV4, KIND_MX4 = KF_FMT_MX4, KIND_BF16 = KF_FMT_BF16;
-constexpr int BM = 128, BN = 256, BKB = 128;          // tile rows, tile columns, K bytes per stage
-constexpr int A_BYTES = BM * BKB, TILE_BYTES = (BM + BN) * BKB;   // 16 KB of A, then 32 KB of W per stage
-constexpr int SF_STAGE_BYTES = 6144;                   // up to 4 atoms for A, then up to 4 + 4 for the two 128-row halves of W
+constexpr int BM = 128, BKB = 128;                     // tile rows, K bytes per stage
+constexpr int A_BYTES = BM * BKB;
+// Column-tile widths BN = 256 and BN = 128 (kf_gemm.cu says when which): bytes of one operand stage (16 KB of A, then 32 or
+// 16 KB of W), bytes of its scale atoms (up to 4 for A, then up to 4 for every 128 rows of W), accumulators that fit the 256
+// tensor-memory columns in front of the scale factors, and columns of one epilogue warp (16 warps = 4 row quarters x 4).
+template <int BN>
+struct Tile {
+  static constexpr int BYTES = (BM + BN) * BKB;
+  static constexpr int SF_BYTES = (1 + BN / 128) * 4 * 512;
+  static constexpr int ACCS = 256 / BN;
+  static constexpr int CW = BN / 4;
+};
 constexpr int EPI_WARPS = 16;
 constexpr int EPI_WARP0 = 4;                           // warps 0..3: TMA producer, MMA issuer, two spares
 constexpr int GEMM_THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
@@ -200,15 +209,18 @@ __device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&
 // warp's 64 columns go to its shared-memory slice with one coalesced load per tile (the kernel's shared memory leaves
 // little L1: a load inside the chunk loops would be an L2 round trip); the chunk loops then read them as broadcast
 // float4s.  The store into the slice waits for the load, an L2 round trip at the head of the tile.
-template <int EPI>
+template <int EPI, int COUNT /* 64 or 32 values */>
 __device__ __forceinline__ void epilogue_slice_stage(const GemmArgs& g, int n0, float* slice, int lane) {
   if (n0 >= g.N) return;
+  const bool on = 2 * lane < COUNT;
   float2 b2 = make_float2(0.f, 0.f), g2 = make_float2(0.f, 0.f);
-  if (g.bias) b2 = __ldg(reinterpret_cast<const float2*>(g.bias + n0) + lane);
-  if (EPI == KF_EPI_RES) g2 = __ldg(reinterpret_cast<const float2*>(g.gamma + n0) + lane);
+  if (on && g.bias) b2 = __ldg(reinterpret_cast<const float2*>(g.bias + n0) + lane);
+  if (on && EPI == KF_EPI_RES) g2 = __ldg(reinterpret_cast<const float2*>(g.gamma + n0) + lane);
   __syncwarp();                                // every lane has finished reading the previous tile's values
-  reinterpret_cast<float2*>(slice)[lane] = b2;
-  if (EPI == KF_EPI_RES) reinterpret_cast<float2*>(slice + 64)[lane] = g2;
+  if (on) {
+    reinterpret_cast<float2*>(slice)[lane] = b2;
+    if (EPI == KF_EPI_RES) reinterpret_cast<float2*>(slice + 64)[lane] = g2;
+  }
   __syncwarp();
 }
 
@@ -246,17 +258,20 @@ __device__ __forceinline__ void rope_slab_store(float* slab, int tid, const Rope
 __device__ __forceinline__ void quarter_barrier(int quarter) { asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory"); }
 
 // ------------------------------------------------------------------------------------------------ the fused epilogues
-// One epilogue warp's share of a tile: rows rbase..rbase+31 (thread `lane` holds row rbase + lane of the accumulator),
-// columns n0..n0+63 (r0 = first 32, r1 = last 32).  `slice` / `gslice` point at the bias / LayerScale values of these 64 columns in shared memory.
-template <int EPI>
-__device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r0)[32], uint32_t (&r1)[32], float ts, const Nv4Scale& sco, int rbase, int n0,
-                                              const float* slice, const float* gslice /* RES: the LayerScale values of the warp's 64 columns */,
+// One epilogue warp's share of a tile: rows rbase..rbase+31 (thread `lane` holds row rbase + lane of the accumulator) and W
+// columns in r.  W = 64: columns n0..n0+63.  W = 32: columns n0..n0+31; ROPE then holds half of the rotation pairs of the
+// head that starts at n0, columns j0..j0+15 in r[0..15] and 32+j0..32+j0+15 in r[16..31].
+// `slice` / `gslice` point at the bias / LayerScale values of the columns from n0 in shared memory.
+template <int EPI, int W>
+__device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W], float ts, const Nv4Scale& sco, int rbase, int n0, int j0,
+                                              const float* slice, const float* gslice /* RES: the LayerScale values of the warp's columns */,
                                               const float* slab /* ROPE: the quarter's table rows in shared memory, or null */, int lane,
-                                              int m_end /* first row past the product: M, or the end of the tile's product in a batched launch */) {
+                                              int m_end /* first row past the product: M, or the end of the tile's product in a batched launch */,
+                                              const F8* res_ahead /* RES, W = 32: the row's residual values, already requested */) {
   const int m = rbase + lane;
   if (EPI == KF_EPI_ROPE) {
     // the 64 columns of this warp are one head of q, k or v and the thread's 64 values are one [token, head] row of the
-    // output: r0 = first half, r1 = second half of the rotation pairs, so the rotary embedding needs no data exchange:
+    // output: first half of r = first, second half = second columns of the rotation pairs, so the rotary embedding needs no data exchange:
     //   lo' = lo*cos_lo - hi*sin_lo (tables of columns 0..31), hi' = hi*cos_hi + lo*sin_hi (tables of columns 32..63).
     // With KF_G_ROPE_HALF the table row of every token of the warp's quarter is already in shared memory (rope_slab_*).
     if (m >= g.M) return;
@@ -271,29 +286,30 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r0)[
     uint32_t wlo[8], whi[8];                    // 16 output columns of each half: stored as soon as they are complete
     const float2 ts2 = splat2(ts);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {               // 4 rotation pairs at a time (few values live: the thread already holds 64 accumulators)
+    for (int c = 0; c < W / 8; ++c) {           // 4 rotation pairs at a time (few values live: the thread already holds W accumulators)
       float2 lo[2], hi[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int j = 4 * c + 2 * e;
-        lo[e] = fma2(make_float2(__uint_as_float(r0[j]), __uint_as_float(r0[j + 1])), ts2, *reinterpret_cast<const float2*>(slice + j));
-        hi[e] = fma2(make_float2(__uint_as_float(r1[j]), __uint_as_float(r1[j + 1])), ts2, *reinterpret_cast<const float2*>(slice + 32 + j));
+        lo[e] = fma2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), ts2, *reinterpret_cast<const float2*>(slice + j0 + j));
+        hi[e] = fma2(make_float2(__uint_as_float(r[W / 2 + j]), __uint_as_float(r[W / 2 + j + 1])), ts2, *reinterpret_cast<const float2*>(slice + 32 + j0 + j));
       }
       float2 ol[2] = {lo[0], lo[1]}, oh[2] = {hi[0], hi[1]};
       if (rot) {
+        const int ct = (j0 >> 2) + c;           // 16-byte piece of the table row
         float4 s4, c4;                          // sin / cos of the 4 pairs: first for the lo outputs, then for the hi outputs
         if (slab != nullptr) {                  // both halves of the tables are the same 32 values
-          s4 = *reinterpret_cast<const float4*>(srow + ((c ^ (lane & 7)) << 2));
-          c4 = *reinterpret_cast<const float4*>(srow + (((c + 8) ^ (lane & 7)) << 2));
+          s4 = *reinterpret_cast<const float4*>(srow + ((ct ^ (lane & 7)) << 2));
+          c4 = *reinterpret_cast<const float4*>(srow + (((ct + 8) ^ (lane & 7)) << 2));
         } else {
-          s4 = ldg4_nc(sn + 4 * c);
-          c4 = ldg4_nc(cs + 4 * c);
+          s4 = ldg4_nc(sn + 4 * ct);
+          c4 = ldg4_nc(cs + 4 * ct);
         }
         ol[0] = fma2(hi[0], make_float2(-s4.x, -s4.y), mul2(lo[0], make_float2(c4.x, c4.y)));
         ol[1] = fma2(hi[1], make_float2(-s4.z, -s4.w), mul2(lo[1], make_float2(c4.z, c4.w)));
         if (slab == nullptr) {
-          s4 = ldg4_nc(sn + 32 + 4 * c);
-          c4 = ldg4_nc(cs + 32 + 4 * c);
+          s4 = ldg4_nc(sn + 32 + 4 * ct);
+          c4 = ldg4_nc(cs + 32 + 4 * ct);
         }
         oh[0] = fma2(hi[0], make_float2(c4.x, c4.y), mul2(lo[0], make_float2(s4.x, s4.y)));
         oh[1] = fma2(hi[1], make_float2(c4.z, c4.w), mul2(lo[1], make_float2(s4.z, s4.w)));
@@ -304,13 +320,13 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r0)[
         whi[2 * (c & 3) + e] = pack2(oh[e].x, oh[e].y, g.out_dtype);
       }
       if ((c & 3) == 3) {
-        stg8w(dst + 32 * (c >> 2), wlo);
-        stg8w(dst + 64 + 32 * (c >> 2), whi);
+        stg8w(dst + 2 * j0 + 32 * (c >> 2), wlo);
+        stg8w(dst + 64 + 2 * j0 + 32 * (c >> 2), whi);
       }
     }
   } else if (EPI == KF_EPI_RES) {
-    // out = R + gamma * (acc*ts + bias) on the thread's 256 contiguous bytes of the fp32 residual row: eight 32-byte pieces,
-    // four residual loads in flight ahead of the arithmetic.
+    // out = R + gamma * (acc*ts + bias) on the thread's 256 (or 128) contiguous bytes of the fp32 residual row: 32-byte pieces,
+    // four residual loads in flight ahead of the arithmetic (W = 32: all of them since before the accumulator was complete).
     if (m >= g.M) return;
     const float* rrow = g.R + (size_t)m * g.N + n0;
     const int64_t orow = g.row_group > 0 ? (int64_t)(m / g.row_group) * g.row_stride + g.row_offset + m % g.row_group : m;   // the output may be a longer stream
@@ -318,12 +334,12 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r0)[
     const float2 ts2 = splat2(ts);
     F8 rr[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) rr[c] = ldg8_stream(rrow + 8 * c);
+    for (int c = 0; c < 4; ++c) rr[c] = W == 32 ? res_ahead[c] : ldg8_stream(rrow + 8 * c);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const uint32_t* acc = c < 4 ? &r0[8 * c] : &r1[8 * (c - 4)];
+    for (int c = 0; c < W / 8; ++c) {
+      const uint32_t* acc = &r[8 * c];
       const F8 cur = rr[c & 3];
-      if (c + 4 < 8) rr[c & 3] = ldg8_stream(rrow + 8 * (c + 4));
+      if (c + 4 < W / 8) rr[c & 3] = ldg8_stream(rrow + 8 * (c + 4));
       float o[8];
 #pragma unroll
       for (int e = 0; e < 8; e += 2) {
@@ -341,16 +357,16 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r0)[
       const int64_t orow = g.row_group > 0 ? (int64_t)(m / g.row_group) * g.row_stride + g.row_offset + m % g.row_group : m;
       dst_row = static_cast<uint8_t*>(g.C) + (size_t)orow * g.N * (g.out_dtype == KF_F32 ? 4 : 2);
     }
-    plain_chunk(g, r0, ts, dst_row, n0, slice);
-    plain_chunk(g, r1, ts, dst_row, n0 + 32, slice + 32);
+#pragma unroll
+    for (int c = 0; c < W; c += 32) plain_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, dst_row, n0 + c, slice + c);
   } else {   // KF_EPI_QUANT: gelu(acc*ts + bias) -> codes + blocked scales of format out_fmt
-    quant_chunk(g, r0, ts, sco, m, n0, slice);
-    quant_chunk(g, r1, ts, sco, m, n0 + 32, slice + 32);
+#pragma unroll
+    for (int c = 0; c < W; c += 32) quant_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, sco, m, n0 + c, slice + c);
   }
 }
 
 // First A / C row of row tile m_blk and the first row past its product (batched launches: row tiles never straddle two
-// products, the last tile of a product is cut at the product's end); the first W row of column tile n_blk.
+// products, the last tile of a product is cut at the product's end); the first W row of the column tile that starts at n0.
 __device__ __forceinline__ int tile_row0(const GemmArgs& g, int m_blk, int& row_end) {
   if (g.m_tiles_pb > 0) {
     const int b = m_blk / g.m_tiles_pb, mt = m_blk - b * g.m_tiles_pb;
@@ -360,37 +376,31 @@ __device__ __forceinline__ int tile_row0(const GemmArgs& g, int m_blk, int& row_
   row_end = g.M;
   return m_blk * BM;
 }
-__device__ __forceinline__ int tile_wrow0(const GemmArgs& g, int m_blk, int n_blk) {
-  return (g.m_tiles_pb > 0 ? (m_blk / g.m_tiles_pb) * g.w_rows_pb : 0) + n_blk * BN;
-}
+__device__ __forceinline__ int tile_wrow0(const GemmArgs& g, int m_blk, int n0) { return (g.m_tiles_pb > 0 ? (m_blk / g.m_tiles_pb) * g.w_rows_pb : 0) + n0; }
 
 // ------------------------------------------------------------------------------------------------ tile schedules and the epilogue warps' loop
-// The i-th tile of a persistent CTA: tiles start, start + step, ... of the row-major tile grid (n_fixed < 0), or a fixed
-// column block with the row blocks start, start + step, ... (a weight-stationary schedule).
+// The i-th tile of a persistent CTA: tiles start, start + step, ... of the row-major tile grid.
 struct TileSched {
-  int start, step, total, n_tiles, n_fixed;     // n_fixed < 0: row-major walk over (m, n); else the column block every tile uses
+  int start, step, total, n_tiles;
   __device__ __forceinline__ bool get(int i, int& m_blk, int& n_blk) const {
     const int idx = start + i * step;
     if (idx >= total) return false;
-    if (n_fixed >= 0) {
-      m_blk = idx;
-      n_blk = n_fixed;
-    } else {
-      m_blk = idx / n_tiles;
-      n_blk = idx - m_blk * n_tiles;
-    }
+    m_blk = idx / n_tiles;
+    n_blk = idx - m_blk * n_tiles;
     return true;
   }
 };
 
-// Body of the 16 epilogue warps (warp = (TMEM lane quarter, 64-column group)): per tile, stage the bias slice (and fetch the
-// rotary-table rows), wait for the accumulator, take the warp's 32 x 64 piece into registers, hand TMEM back at once and
+// Body of the 16 epilogue warps (warp = (TMEM lane quarter, 64- or 32-column group)): per tile, stage the bias slice (and fetch
+// the rotary-table rows), wait for the accumulator, take the warp's piece into registers, hand TMEM back at once and
 // run the fused epilogue on the registers while the next tile's main loop fills the accumulator again.
-template <int EPI>
+template <int EPI, int BN>
 __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSched& sched, uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty, float* slices,
                                                float* slabs, const WaitCtx& ctx, int warp, int lane) {
+  constexpr int W = Tile<BN>::CW, ACCS = Tile<BN>::ACCS;
+  constexpr bool PAIRS = EPI == KF_EPI_ROPE && W == 32;       // two warps share a head: its column pairs 0..15 and 16..31
   const int quarter = warp & 3;                 // TMEM lanes 32*quarter .. +31 are the ones this warp may read
-  const int cg = (warp - EPI_WARP0) >> 2;       // which 64-column group of the 256-column tile
+  const int cg = (warp - EPI_WARP0) >> 2;       // which column group of the tile
   float* slice = slices + (warp - EPI_WARP0) * SLICE_FLOATS;
   // Where the launch left room for it, the bias vector (and the LayerScale vector) is brought into shared memory once per
   // CTA instead of 64 values per warp and tile: that load was an L2 round trip (400-700 clk) at the head of every tile of
@@ -408,28 +418,44 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSche
   if (g.ts_a) ts *= __ldg(g.ts_a);
   if (g.ts_w) ts *= __ldg(g.ts_w);
   const Nv4Scale sco = nv4_scale((EPI == KF_EPI_QUANT && g.out_fmt == KF_FMT_NV4) ? __ldg(g.tso) : 1.f);   // once per CTA: every global load here is an L2 round trip
-  const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + cg * 64;
+  const int col = PAIRS ? (cg >> 1) * 64 : cg * W, j0 = PAIRS ? (cg & 1) * 16 : 0;
+  const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + col + j0;
   int m_blk, n_blk;
   for (int lt = 0; sched.get(lt, m_blk, n_blk); ++lt) {
     int row_end;
     const int rbase = tile_row0(g, m_blk, row_end) + quarter * 32;
-    const int n0 = n_blk * BN + cg * 64;        // first column of this warp's group
-    uint32_t r0[32], r1[32];
-    if (!vec) epilogue_slice_stage<EPI>(g, n0, slice, lane);
+    const int n0 = n_blk * BN + col;            // first column of this warp's group (or of its head)
+    const int acc = lt % ACCS;
+    const uint32_t taddr = taddr0 + acc * BN;
+    uint32_t r[W];
+    if (!vec) epilogue_slice_stage<EPI, PAIRS ? 64 : W>(g, n0, slice, lane);
     const float* bsl = vec ? slices + n0 : slice;
     const float* gsl = vec ? slices + g.N + n0 : slice + 64;
     // ROPE with half tables: the quarter's table rows are fetched now and parked in shared memory after the wait
     const bool use_slab = EPI == KF_EPI_ROPE && (g.flags & KF_G_ROPE_HALF) != 0 && n_blk * BN < 2 * g.d;   // the tile holds q or k columns
     RopeSlabRegs tab;
     if (EPI == KF_EPI_ROPE && use_slab) rope_slab_fetch(g, rbase, cg * 32 + lane, tab);
-    if (!mbar_wait(tfull, lt & 1, ctx, 4)) break;
+    F8 res[4];
+    if (EPI == KF_EPI_RES && W == 32 && rbase + lane < g.M) {  // the residual's latency runs under the main loop
+#pragma unroll
+      for (int c = 0; c < 4; ++c) res[c] = ldg8_stream(g.R + (size_t)(rbase + lane) * g.N + n0 + 8 * c);
+    }
+    if (!mbar_wait(&tfull[acc], (lt / ACCS) & 1, ctx, 4)) break;
     tc_fence_after();
-    tmem_ld32(taddr, r0);
-    tmem_ld32(taddr + 32, r1);
+    __syncwarp();
+    if constexpr (W == 64) {
+      tmem_ld32(taddr, reinterpret_cast<uint32_t(&)[32]>(r[0]));
+      tmem_ld32(taddr + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+    } else if constexpr (PAIRS) {
+      tmem_ld16(taddr, reinterpret_cast<uint32_t(&)[16]>(r[0]));
+      tmem_ld16(taddr + 32, reinterpret_cast<uint32_t(&)[16]>(r[16]));
+    } else {
+      tmem_ld32(taddr, r);
+    }
     tmem_ld_wait();
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(tempty);                       // the accumulator is in registers: hand TMEM back
+    if (lane == 0) mbar_arrive(&tempty[acc]);                 // the accumulator is in registers: hand TMEM back
     float* slab = nullptr;
     if (EPI == KF_EPI_ROPE && use_slab) {                      // all 4 warps of the quarter take this path together (it depends on the tile only)
       slab = slabs + quarter * ROPE_SLAB_FLOATS;
@@ -438,7 +464,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSche
       quarter_barrier(quarter);
     }
     if (n0 >= g.N) continue;                                   // column group past N in the last column tile
-    epilogue_math<EPI>(g, r0, r1, ts, sco, rbase, n0, bsl, gsl, slab, lane, row_end);
+    epilogue_math<EPI, W>(g, r, ts, sco, rbase, n0, j0, bsl, gsl, slab, lane, row_end, res);
   }
 }
 
