@@ -63,7 +63,6 @@ class _Swap:
         self.fmt = fmt
         self.pool: Dict[tuple, tuple] = {}           # persistent operands per (rows, K, device, role), each with its scale's workspace
         self.slots: Dict[tuple, tuple] = {}          # unit -> (operand, leading shape) waiting for its Linear
-        self.modules: List[torch.nn.Module] = []
 
     def operand(self, rows: int, K: int, device, role: str) -> tuple:
         """-> (operand, workspace of its dynamic scale; None unless the format is nv4)."""
@@ -73,10 +72,6 @@ class _Swap:
             ws = torch.zeros(2, dtype=torch.int32, device=device) if self.fmt == "nv4" else None
             got = self.pool[key] = (ops.ActBuf(rows, K, self.fmt, device), ws)
         return got
-
-    def install(self, module: torch.nn.Module, fn: Callable) -> None:
-        module.forward = fn                          # instance attribute: shadows the class forward until disable()
-        self.modules.append(module)
 
 
 class _Feeder:
@@ -151,16 +146,24 @@ def enable(model, units, fmt: str = "mx8") -> None:
     disable(model)
     swap = _Swap(fmt)
     blocks = model.backbone.blocks
+    # The list lives on the model alone: a session that held its modules would keep itself, the model and the operand pool alive in a
+    # reference cycle until the collector finds it.
+    patched: List[torch.nn.Module] = []
+
+    def install(module: torch.nn.Module, fn: Callable) -> None:
+        module.forward = fn                      # instance attribute: shadows the class forward until disable()
+        patched.append(module)
+
     for layer, kind in sorted(wanted):
         feeder_path, how, linear_path = _UNIT_PLAN[kind]
         block = blocks[layer]
         unit = (layer, kind)
         if feeder_path is not None:
             feeder = _resolve(block, feeder_path)
-            swap.install(feeder, _Feeder(swap, unit, how, feeder))
+            install(feeder, _Feeder(swap, unit, how, feeder))
         lin = _resolve(block, linear_path)
-        swap.install(lin, _QLinear(swap, unit, lin))
-    setattr(model, _ATTR, swap.modules)
+        install(lin, _QLinear(swap, unit, lin))
+    setattr(model, _ATTR, patched)
 
 
 def disable(model) -> None:
