@@ -156,7 +156,7 @@ def main():
     ap.add_argument("--size", type=int, default=SIZE, help="input side in pixels (default 640)")
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--pdl", action="store_true", help="launch the block kernels with programmatic dependent launch (default: plain stream order)")
+    ap.add_argument("--pdl", action="store_true", help="programmatic dependent launch for every launch (default: only for launches over few rows)")
     args = ap.parse_args()
     rank, world, local = int(os.environ.get("RANK", 0)), int(os.environ.get("WORLD_SIZE", 1)), int(os.environ.get("LOCAL_RANK", 0))
     if args.impl == "reference":

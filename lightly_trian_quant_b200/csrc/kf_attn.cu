@@ -612,7 +612,7 @@ static int attn_launch(int dtype, const void* qkv, void* O, int B, int N, int H,
   if (sst != KF_OK) return sst;
   const int slots = 2 * sms;                                  // two CTAs are resident per SM
   const int grid = items < slots ? (int)items : slots;
-  return cuda_status(launch_maybe_pdl(kern, dim3(grid), dim3(AT_THREADS), (size_t)AT_SMEM, static_cast<cudaStream_t>(stream), tq, tk, tv, a),
+  return cuda_status(launch_maybe_pdl((int64_t)B * N, kern, dim3(grid), dim3(AT_THREADS), (size_t)AT_SMEM, static_cast<cudaStream_t>(stream), tq, tk, tv, a),
                      "kf_attn_fwd launch");
 }
 

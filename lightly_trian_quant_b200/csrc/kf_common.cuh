@@ -17,7 +17,7 @@ namespace kf {
 void set_error(const char* fmt, ...);
 int cuda_status(cudaError_t e, const char* what);
 int device_sm_count(int* sms);   // multiprocessor count of the current device (cached)
-bool pdl_enabled();              // kf_set_pdl: launch the block kernels with programmatic dependent launch
+bool pdl_for(int64_t rows, cudaStream_t st);   // programmatic dependent launch for a launch over this many rows?
 
 // Programmatic dependent launch: a kernel lets its successor's CTAs start on SMs it no longer occupies (its partial last
 // wave, its teardown) and the successor runs its prologue (barrier set-up, TMEM allocation, descriptor prefetch) there; the
@@ -26,9 +26,9 @@ bool pdl_enabled();              // kf_set_pdl: launch the block kernels with pr
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// <<<grid, block, smem, stream>>> with the programmatic-stream-serialization attribute when PDL is enabled
+// <<<grid, block, smem, stream>>>, with the programmatic-stream-serialization attribute where pdl_for(rows) says so
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_maybe_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+inline cudaError_t launch_maybe_pdl(int64_t rows, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -38,7 +38,7 @@ inline cudaError_t launch_maybe_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bl
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = pdl_for(rows, st) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

@@ -319,7 +319,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmW, const Gem
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_kernel)");
     if (dev < 64) attr_set[dev] = true;
   }
-  return cuda_status(launch_maybe_pdl(gemm_kernel<KIND, EPI, BN>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats), st, tmA, tmW, g), "kf_gemm_bs launch");
+  return cuda_status(launch_maybe_pdl(g.M, gemm_kernel<KIND, EPI, BN>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats), st, tmA, tmW, g), "kf_gemm_bs launch");
 }
 
 template <int KIND, int BN>
@@ -351,12 +351,13 @@ static int launch_gemm_fmt(int fmt, int epi, const CUtensorMap& tmA, const CUten
 
 // Column-tile width of a launch.  256 columns need the least operand traffic per product (the tile shape comment above) and win
 // wherever there are many tiles; 128 columns cut the launch finer, take twice the SMs where the tiles do not fill the
-// chip, and keep two accumulators in tensor memory.  A round of 128-column tiles takes about 0.6 of a round of 256-column tiles,
-// so 128 wins when ceil(tiles / SMs) rounds of them are shorter: one frame's 13 row tiles x 1024 columns are one round either way
-// (104 SMs instead of 52), x 4096 columns 3 x 0.6 rounds against 2; from about five rounds on the rounding no longer pays.
-static int gemm_columns(int m_tiles, int N, int sms) {
+// chip, and keep two accumulators in tensor memory.  A round of 128-column tiles takes about 0.6 of a round of 256-column tiles
+// (0.7 for PLAIN, whose epilogue is too short to hide the larger operand traffic: MXFP8 1605 x 1024 x 4096 13.4 us in 3 rounds
+// against 12.8 in 2), so 128 wins when ceil(tiles / SMs) rounds of them are shorter: one frame's 13 row tiles x 1024 columns are one round either way
+// (104 SMs instead of 52), x 4096 columns 3 x 0.6 rounds against 2 (fc1 NVFP4 14.6 -> 12.1 us, proj / fc2 13.9 -> 8.8 us on average); from about five rounds on the rounding no longer pays.
+static int gemm_columns(int m_tiles, int N, int sms, bool plain) {
   const int64_t r256 = ((int64_t)m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = ((int64_t)m_tiles * (N / 128) + sms - 1) / sms;
-  return 6 * r128 < 10 * r256 ? 128 : 256;
+  return (plain ? 7 : 6) * r128 < 10 * r256 ? 128 : 256;
 }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -413,7 +414,7 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   int sms = 0;
   int st = device_sm_count(&sms);
   if (st != KF_OK) return st;
-  const int bn = gemm_columns(m_tiles, p->N, sms);
+  const int bn = gemm_columns(m_tiles, p->N, sms, epi == KF_EPI_PLAIN);
   CUtensorMap tmA, tmW;
   st = make_tmap_2d_bytes(&tmA, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
   if (st != KF_OK) return st;

@@ -10,6 +10,8 @@ namespace kf {
 // GEMM against the Conv2d weight [d, 3, 16, 16] viewed as [d, 768].  One thread moves 16 pixels (32 bytes) of one
 // patch row.
 __global__ void __launch_bounds__(256) im2col16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, int B, int S) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int g = S >> 4;
   const int64_t total = (int64_t)B * g * g * 48;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -109,6 +111,8 @@ __global__ void __launch_bounds__(256, 2)
 dw_ln_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ bias, const float* __restrict__ dww, const float* __restrict__ lnw,
              const float* __restrict__ lnb, __nv_bfloat16* __restrict__ out, int Hs, int Ws, int C_arg, float eps, int pre_act, int strips, int segs,
              int seg_rows, int total_items) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t dsm[];
   const int C = CT ? CT : C_arg;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nwarps = blockDim.x >> 5;
@@ -486,9 +490,9 @@ extern "C" int kf_im2col_patch16(const void* x, void* out, int B, int S, void* s
   if (B == 0) return KF_OK;
   KF_REQUIRE(x && out && al16(x) && al16(out), "kf_im2col_patch16: tensors must be non-null and 16-byte aligned");
   const int64_t total = (int64_t)B * (S / 16) * (S / 16) * 48;
-  im2col16_kernel<<<(unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(x),
-                                                                                                static_cast<__nv_bfloat16*>(out), B, S);
-  return cuda_status(cudaGetLastError(), "kf_im2col_patch16 launch");
+  return cuda_status(launch_maybe_pdl(total / 48, im2col16_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), B, S),
+                     "kf_im2col_patch16 launch");
 }
 
 extern "C" int kf_dw_ln(const void* g, const float* bias, const float* dww, const float* lnw, const float* lnb, void* out, int B, int Hs, int Ws, int C,
@@ -537,9 +541,9 @@ extern "C" int kf_dw_ln(const void* g, const float* bias, const float* dww, cons
   const int grid = (int)(total < 2 * sms ? total : 2 * sms);
   // the channel counts of the ViT-L and ViT-B heads are compiled in (pixel offsets become instruction immediates)
   auto kern = C == 1024 ? dw_ln_kernel<1024> : C == 768 ? dw_ln_kernel<768> : dw_ln_kernel<0>;
-  kern<<<grid, C / 4, smem, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(g), bias, dww, lnw, lnb, static_cast<__nv_bfloat16*>(out), Hs,
-                                                                 Ws, C, eps, pre_act, strips, segs, seg_rows, (int)total);
-  return cuda_status(cudaGetLastError(), "kf_dw_ln launch");
+  return cuda_status(launch_maybe_pdl((int64_t)B * Hs * Ws, kern, dim3(grid), dim3(C / 4), smem, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(g), bias,
+                                      dww, lnw, lnb, static_cast<__nv_bfloat16*>(out), Hs, Ws, C, eps, pre_act, strips, segs, seg_rows, (int)total),
+                     "kf_dw_ln launch");
 }
 
 extern "C" int kf_semantic(const void* mask_logits, const void* class_logits, int B, int Q, int ncls, int HW, float* scores, uint8_t* labels, void* stream) {
@@ -626,8 +630,9 @@ extern "C" int kf_patch_embed_static(const void* x, const void* w, const float* 
   if (rc != KF_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t total = rows * 48;
-  im2col16_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(scratch), B, S);
-  rc = cuda_status(cudaGetLastError(), "kf_patch_embed_static gather launch");
+  rc = cuda_status(launch_maybe_pdl(rows, im2col16_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(x),
+                                    static_cast<__nv_bfloat16*>(scratch), B, S),
+                   "kf_patch_embed_static gather launch");
   if (rc != KF_OK) return rc;
   kf_gemm_params p = {};
   p.fmt = KF_FMT_BF16;

@@ -72,6 +72,8 @@ template <typename T, int FMT>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, const float* __restrict__ ts_ptr,
                                                          const float* __restrict__ bias, int flags, int wide, uint8_t* __restrict__ q,
                                                          uint8_t* __restrict__ sf, int64_t items_valid, int64_t items_total) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int per_row = K >> 5;
   int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -198,6 +200,8 @@ __device__ __forceinline__ float gelu_abs(float x) { return fabsf(x * 0.5f * (1.
 template <typename T, bool GELU>
 __global__ void __launch_bounds__(256) amax_scale_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, int wide, float factor, float* __restrict__ ts,
                                                          uint32_t* __restrict__ ws) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint32_t per_row = K >> 5, total = (uint32_t)M * per_row;
   float am = 0.f;
   for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
@@ -482,6 +486,8 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI
 template <int NV, typename TI>
 __global__ void __launch_bounds__(128) ln_amax_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps, int M, float factor,
                                                       float* __restrict__ ts, uint32_t* __restrict__ ws) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int D = NV * 256;
   const int lane = threadIdx.x & 31;
   float ww[NV][8], bb[NV][8], v[NV][8], am = 0.f;
@@ -499,6 +505,8 @@ __global__ void __launch_bounds__(128) ln_amax_kernel(const TI* __restrict__ x, 
 template <int NV, typename TO>
 __global__ void __launch_bounds__(128) ln_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps,
                                                       int M, TO* __restrict__ y) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int D = NV * 256;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -531,6 +539,8 @@ __global__ void __launch_bounds__(128) ln_tail_kernel(const float* __restrict__ 
                                                       int M, int Ntok, int Q, int npre, __nv_bfloat16* __restrict__ qb, __nv_bfloat16* __restrict__ xb,
                                                       const __nv_bfloat16* __restrict__ wcls, const float* __restrict__ bcls, int ncls1,
                                                       __nv_bfloat16* __restrict__ cl) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int D = NV * 256;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -581,6 +591,8 @@ __global__ void __launch_bounds__(128) ln_tail_kernel(const float* __restrict__ 
 // The query rows that join the stream for the last blocks and the cls / register rows in front of the patch tokens.
 __global__ void __launch_bounds__(256) broadcast_rows_kernel(const float4* __restrict__ src, float4* __restrict__ dst, int R, int d4, int B, int64_t img_stride4,
                                                              int64_t row_offset4) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t n = (int64_t)R * d4;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * B; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t bimg = i / n, e = i - bimg * n;
@@ -602,9 +614,10 @@ static int launch_amax_scale(const void* x, int64_t ldx, int M, int K, bool gelu
   const unsigned grid = (unsigned)((total + 255) / 256 < 4 * sms ? (total + 255) / 256 : 4 * sms);
   const int wide = rows_32b_aligned(x, ldx * (int64_t)sizeof(T));
   const T* xp = static_cast<const T*>(x);
-  if (gelu) amax_scale_kernel<T, true><<<grid, 256, 0, st>>>(xp, ldx, M, K, wide, factor, ts, static_cast<uint32_t*>(ws));
-  else amax_scale_kernel<T, false><<<grid, 256, 0, st>>>(xp, ldx, M, K, wide, factor, ts, static_cast<uint32_t*>(ws));
-  return cuda_status(cudaGetLastError(), "kf_amax_scale launch");
+  cudaError_t e;
+  if (gelu) e = launch_maybe_pdl(M, amax_scale_kernel<T, true>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, wide, factor, ts, static_cast<uint32_t*>(ws));
+  else e = launch_maybe_pdl(M, amax_scale_kernel<T, false>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, wide, factor, ts, static_cast<uint32_t*>(ws));
+  return cuda_status(e, "kf_amax_scale launch");
 }
 
 template <typename T>
@@ -617,10 +630,11 @@ static int launch_quant_rows(int fmt, const void* x, int64_t ldx, int M, int K, 
   const T* xp = static_cast<const T*>(x);
   const int wide = rows_32b_aligned(x, ldx * (int64_t)sizeof(T));
   uint8_t *qp = static_cast<uint8_t*>(q), *sp = static_cast<uint8_t*>(sf);
-  if (fmt == KF_FMT_MX8) quant_rows_kernel<T, KF_FMT_MX8><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
-  else if (fmt == KF_FMT_NV4) quant_rows_kernel<T, KF_FMT_NV4><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
-  else quant_rows_kernel<T, KF_FMT_MX4><<<grid, 256, 0, st>>>(xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
-  return cuda_status(cudaGetLastError(), "kf_quant_rows launch");
+  cudaError_t e;
+  if (fmt == KF_FMT_MX8) e = launch_maybe_pdl(M, quant_rows_kernel<T, KF_FMT_MX8>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
+  else if (fmt == KF_FMT_NV4) e = launch_maybe_pdl(M, quant_rows_kernel<T, KF_FMT_NV4>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
+  else e = launch_maybe_pdl(M, quant_rows_kernel<T, KF_FMT_MX4>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
+  return cuda_status(e, "kf_quant_rows launch");
 }
 
 template <int NV, typename TI>
@@ -653,7 +667,7 @@ static int launch_ln_quant(int fmt, const TI* x, const float* w, const float* b,
       if (dev < 64) per_sm_cached[fmt][dev] = per_sm;
     }
     if (grid > (unsigned)(sms * per_sm)) grid = (unsigned)(sms * per_sm);
-    return cuda_status(launch_maybe_pdl(kern, dim3(grid), dim3(128), smem, st, x, w, b, eps, M, rows_pad, ts, flags, qp, sp, y_dbg, err), "kf_ln_quant launch");
+    return cuda_status(launch_maybe_pdl(M, kern, dim3(grid), dim3(128), smem, st, x, w, b, eps, M, rows_pad, ts, flags, qp, sp, y_dbg, err), "kf_ln_quant launch");
   };
   if (fmt == KF_FMT_MX8) return go(ln_quant_kernel<NV, KF_FMT_MX8, TI>);
   if (fmt == KF_FMT_NV4) return go(ln_quant_kernel<NV, KF_FMT_NV4, TI>);
@@ -666,24 +680,25 @@ static int launch_ln_amax(const TI* x, const float* w, const float* b, float eps
   const int rc = device_sm_count(&sms);
   if (rc != KF_OK) return rc;
   const int grid = (M + 3) / 4 < 4 * sms ? (M + 3) / 4 : 4 * sms;
-  ln_amax_kernel<NV, TI><<<grid, 128, 0, st>>>(x, w, b, eps, M, factor, ts, static_cast<uint32_t*>(ws));
-  return cuda_status(cudaGetLastError(), "kf_ln_amax_scale launch");
+  const cudaError_t e = launch_maybe_pdl(M, ln_amax_kernel<NV, TI>, dim3(grid), dim3(128), 0, st, x, w, b, eps, M, factor, ts, static_cast<uint32_t*>(ws));
+  return cuda_status(e, "kf_ln_amax_scale launch");
 }
 
 template <int NV>
 static int launch_ln_rows(const float* x, const float* w, const float* b, float eps, int M, int out_dtype, void* y, cudaStream_t st) {
   unsigned grid = (unsigned)((M + 3) / 4);
-  if (out_dtype == KF_BF16) ln_rows_kernel<NV, __nv_bfloat16><<<grid, 128, 0, st>>>(x, w, b, eps, M, static_cast<__nv_bfloat16*>(y));
-  else ln_rows_kernel<NV, __half><<<grid, 128, 0, st>>>(x, w, b, eps, M, static_cast<__half*>(y));
-  return cuda_status(cudaGetLastError(), "kf_ln_rows launch");
+  cudaError_t e;
+  if (out_dtype == KF_BF16) e = launch_maybe_pdl(M, ln_rows_kernel<NV, __nv_bfloat16>, dim3(grid), dim3(128), 0, st, x, w, b, eps, M, static_cast<__nv_bfloat16*>(y));
+  else e = launch_maybe_pdl(M, ln_rows_kernel<NV, __half>, dim3(grid), dim3(128), 0, st, x, w, b, eps, M, static_cast<__half*>(y));
+  return cuda_status(e, "kf_ln_rows launch");
 }
 
 template <int NV>
 static int launch_ln_tail(const float* x, const float* w, const float* b, float eps, int M, int Ntok, int Q, int npre, void* qb, void* xb, const void* wcls,
                           const float* bcls, int ncls1, void* cl, cudaStream_t st) {
-  ln_tail_kernel<NV><<<(unsigned)((M + 3) / 4), 128, 0, st>>>(x, w, b, eps, M, Ntok, Q, npre, static_cast<__nv_bfloat16*>(qb), static_cast<__nv_bfloat16*>(xb),
+  const cudaError_t e = launch_maybe_pdl(M, ln_tail_kernel<NV>, dim3((M + 3) / 4), dim3(128), 0, st, x, w, b, eps, M, Ntok, Q, npre, static_cast<__nv_bfloat16*>(qb), static_cast<__nv_bfloat16*>(xb),
                                                               static_cast<const __nv_bfloat16*>(wcls), bcls, ncls1, static_cast<__nv_bfloat16*>(cl));
-  return cuda_status(cudaGetLastError(), "kf_ln_tail launch");
+  return cuda_status(e, "kf_ln_tail launch");
 }
 
 template <typename TI>
@@ -823,7 +838,7 @@ extern "C" int kf_broadcast_rows(const float* src, float* dst, int R, int d, int
   const int64_t n = (int64_t)R * (d / 4) * B;
   int grid = (int)((n + 255) / 256);
   if (grid > 148 * 8) grid = 148 * 8;
-  broadcast_rows_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), R, d / 4, B, img_stride / 4,
+  const cudaError_t e = launch_maybe_pdl(img_stride / d * B, broadcast_rows_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream), reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), R, d / 4, B, img_stride / 4,
                                                                             row_offset * (d / 4));
-  return cuda_status(cudaGetLastError(), "kf_broadcast_rows launch");
+  return cuda_status(e, "kf_broadcast_rows launch");
 }

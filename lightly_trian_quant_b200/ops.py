@@ -193,7 +193,7 @@ def ln_amax_scale(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float,
 
 # ------------------------------------------------------------------------------------------------ weights and GEMMs
 def set_pdl(on: bool) -> None:
-    """Programmatic dependent launch for the block kernels (off by default); results are the same either way.
+    """Programmatic dependent launch: True = every launch, False (default) = launches over few rows; results are the same either way.
     Counterpart: set_pdl (infer-opt/round13_mxfp8_full/impl/mx13.cu:282)."""
     check(_lib.lib().kf_set_pdl(1 if on else 0), "kf_set_pdl")
 

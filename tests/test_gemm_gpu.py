@@ -307,3 +307,57 @@ def test_batched_products_match_one_launch_per_product(B, Q, P, K):
         assert torch.equal(out[b], one)
     ref = torch.bmm(a.float(), w.float().transpose(1, 2))
     assert go.rel_fro(out.float().cpu().numpy(), ref.cpu().numpy()) < 4e-3
+
+
+# The two column-tile widths: a launch of 148 row tiles takes 256-column tiles (N = 640: the last one holds 128 columns), the same
+# rows in a launch of their own 128-column tiles.  First image, and the last one, which ends inside a row tile.
+@pytest.mark.parametrize("fmt", FMTS + ["bf16"])
+def test_column_tile_widths_agree(fmt):
+    ops = _ops()
+    B, Ntok, prefix, H = 37, 511, 5, 4                      # 18 907 rows
+    M, K = B * Ntok, 256 if fmt != "bf16" else 192
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x = rnd(M, K).to(torch.bfloat16)
+
+    def operand(rows):
+        if fmt == "bf16":
+            return rows.contiguous()
+        a = ops.ActBuf(rows.shape[0], K, fmt)
+        if fmt == "nv4":
+            a.ts.fill_(0.003)
+        return ops.quant_rows(rows, a)
+
+    def launches(rows, res, n_img):
+        a = operand(rows)
+        out = [ops.gemm_plain(a, W, bias, gelu=True, out_dtype=torch.float32), ops.gemm_plain(a, W, None, out_dtype=torch.float16),
+               ops.gemm_res(a, W, bias, gamma, res)]
+        for tables, half in ((general, False), (axial, True)):
+            out.append(ops.qkv_rope(a, Wq, bias_q, *tables, Ntok, prefix, H, half_tables=half).transpose(0, 1).reshape(n_img, -1))
+        if fmt != "bf16":
+            for ofmt in FMTS:
+                q = ops.ActBuf(rows.shape[0], 640, ofmt)
+                if ofmt == "nv4":
+                    q.ts.fill_(0.002)
+                ops.gemm_gelu_q(a, W, bias, q, round_bf16=True)
+                out += [q.q, q.sf]
+        ops.check_device_error()
+        return out
+
+    W, Wq = ops.QWeight(rnd(640, K) * 0.05, fmt), ops.QWeight(rnd(3 * H * 64, K) * 0.05, fmt)
+    bias, bias_q, gamma = rnd(640) * 0.1, rnd(3 * H * 64) * 0.1, rnd(640)
+    general = (rnd(Ntok - prefix, 64), rnd(Ntok - prefix, 64))
+    axial = tuple(torch.cat((t[:, :32], t[:, :32]), dim=1).contiguous() for t in general)
+    res = rnd(M, 640)
+    big = launches(x, res, B)
+    for b in (0, B - 1):
+        rows = slice(b * Ntok, (b + 1) * Ntok)
+        small = launches(x[rows], res[rows].contiguous(), 1)
+        for i, (u, v) in enumerate(zip(big, small)):
+            if u.dim() == 1:                                # blocked scales: the first image starts on a row-tile boundary
+                if b == 0:
+                    n = 3 * v.numel() // 4                  # its three whole row tiles
+                    assert torch.equal(u[:n], v[:n]), i
+                continue
+            part = u[b:b + 1] if u.shape[0] == B else u[rows]
+            assert torch.equal(part, v), i
