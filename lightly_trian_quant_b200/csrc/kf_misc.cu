@@ -40,8 +40,8 @@ __global__ void __launch_bounds__(256) im2col16_kernel(const __nv_bfloat16* __re
 // 16-byte cp.async copies (zero fill outside the image) that run two rows ahead, across item boundaries too; every
 // row is fetched once per strip and used for three output rows.  Per output row a thread reads its 4 channels of the
 // 3 x 10 window (30 8-byte shared loads), accumulates the 8 pixels in tap order on packed fp32 pairs, rounds to bf16,
-// and the LayerNorm sums of the 8 pixels are reduced over the CTA (a transposing butterfly inside the warp, then one
-// shared-memory exchange per statistic); the thread normalises and stores its own 8 bytes of each pixel, so no conv
+// and the LayerNorm statistics of the 8 pixels are reduced over the CTA (transposing butterflies inside the warp, then one
+// shared-memory exchange); the thread normalises and stores its own 8 bytes of each pixel, so no conv
 // result goes through shared memory and a warp's stores are 256 contiguous bytes.
 constexpr int DW_SW = 8, DW_HALO = DW_SW + 2, DW_RING = 5;
 
@@ -72,10 +72,8 @@ __device__ __forceinline__ DwItem dw_item(int item, int strips, int segs, int se
   return r;
 }
 
-// sums of v[0..7] over all threads of the CTA, returned in v for every thread.  red: 64 floats of shared memory that no
-// other exchange uses between the two barriers around this call.
-__device__ __forceinline__ void dw_block_sum8(float (&v)[8], float* red, int warp, int lane, int nwarps) {
-  // transposing butterfly: after the three halving steps lane l holds the partial sum of pixel l >> 2
+// Sums of v[0..7] over the warp by a transposing butterfly: lane l returns the sum of v[l >> 2].
+__device__ __forceinline__ float dw_warp_sum8(const float (&v)[8], int lane) {
   float a[4], b[2];
   bool hi = lane & 16;
 #pragma unroll
@@ -93,17 +91,9 @@ __device__ __forceinline__ void dw_block_sum8(float (&v)[8], float* red, int war
   float c = (hi ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, hi ? b[0] : b[1], 4);
   c += __shfl_xor_sync(0xffffffffu, c, 2);
   c += __shfl_xor_sync(0xffffffffu, c, 1);
-  if ((lane & 3) == 0) red[warp * 8 + (lane >> 2)] = c;
-  __syncthreads();
-  float tot = 0.f;
-  if (lane < 8) {
-#pragma unroll
-    for (int w = 0; w < 8; ++w)
-      if (w < nwarps) tot += red[w * 8 + lane];
-  }
-#pragma unroll
-  for (int p = 0; p < 8; ++p) v[p] = __shfl_sync(0xffffffffu, tot, p);
+  return c;
 }
+constexpr int DW_RED_FLOATS = 2 * 8 * 8 * 2;             // (mean, squared deviations) of 8 warps x 8 pixels, then (mean, 1/sigma) of the 8 pixels per warp
 
 // CT: the channel count as a compile-time constant (0 = use the run-time argument)
 template <int CT>
@@ -119,7 +109,8 @@ dw_ln_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ bias
   const int Ho = 2 * Hs, Wo = 2 * Ws;
   const int row_bytes = DW_HALO * C * 2;
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dsm);
-  float* red = reinterpret_cast<float*>(dsm + DW_RING * row_bytes);       // two exchange areas of 64 floats
+  float2* red = reinterpret_cast<float2*>(dsm + DW_RING * row_bytes);
+  float2* stat = red + 64 + warp * 8;
 
   // the thread's channels: tap weights, LayerNorm parameters, bias
   float2 w[9][2];
@@ -220,7 +211,9 @@ dw_ln_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ bias
             }
           }
         }
-        // ---- LayerNorm over the channels of each of the 8 pixels, statistics on the bf16-rounded conv outputs
+        // ---- LayerNorm over the channels of each of the 8 pixels, statistics on the bf16-rounded conv outputs: mean and squared
+        // deviations of the warp's 128 channels first (two-pass, inside the warp), then one exchange that combines the warps:
+        // M2 = sum M2_w + 128 * sum (mean_w - mean)^2.  One block-wide exchange per row instead of one per statistic.
         float s8[8];
 #pragma unroll
         for (int p = 0; p < DW_SW; ++p) {
@@ -229,23 +222,41 @@ dw_ln_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ bias
           const float2 s2 = add2(acc[p][0], acc[p][1]);
           s8[p] = s2.x + s2.y;
         }
-        dw_block_sum8(s8, red, warp, lane, nwarps);
+        const float wmean = dw_warp_sum8(s8, lane) * (1.0f / 128.0f);          // of pixel lane >> 2
 #pragma unroll
         for (int p = 0; p < DW_SW; ++p) {
-          const float2 nm = splat2(-s8[p] * invC);
-          acc[p][0] = add2(acc[p][0], nm);
-          acc[p][1] = add2(acc[p][1], nm);
-          const float2 q2 = fma2(acc[p][1], acc[p][1], mul2(acc[p][0], acc[p][0]));
+          const float2 nm = splat2(-__shfl_sync(0xffffffffu, wmean, 4 * p));
+          const float2 d0 = add2(acc[p][0], nm), d1 = add2(acc[p][1], nm);
+          const float2 q2 = fma2(d1, d1, mul2(d0, d0));
           s8[p] = q2.x + q2.y;
         }
-        dw_block_sum8(s8, red + 64, warp, lane, nwarps);
+        const float wm2 = dw_warp_sum8(s8, lane);
+        if ((lane & 3) == 0) red[warp * 8 + (lane >> 2)] = make_float2(wmean, wm2);
+        __syncthreads();
+        if (lane < 8) {                                       // lane = pixel
+          float2 part[8];
+          float mean = 0.f, m2 = 0.f;
+#pragma unroll
+          for (int w8 = 0; w8 < 8; ++w8) {
+            part[w8] = w8 < nwarps ? red[w8 * 8 + lane] : make_float2(0.f, 0.f);
+            mean += part[w8].x;
+          }
+          mean *= 128.0f * invC;
+#pragma unroll
+          for (int w8 = 0; w8 < 8; ++w8) {
+            const float d = part[w8].x - mean;
+            if (w8 < nwarps) m2 += fmaf(128.0f * d, d, part[w8].y);
+          }
+          stat[lane] = make_float2(mean, rsqrtf(m2 * invC + eps));
+        }
+        __syncwarp();
         __nv_bfloat16* orow = out + (((int64_t)T.b * Ho + Y) * Wo + T.X0) * C + t * 4;
 #pragma unroll
         for (int p = 0; p < DW_SW; ++p) {
           if (T.X0 + p < Wo) {
-            const float2 rstd = splat2(rsqrtf(s8[p] * invC + eps));
-            const __nv_bfloat162 h0 = __float22bfloat162_rn(fma2(mul2(acc[p][0], rstd), gw0, gb0));
-            const __nv_bfloat162 h1 = __float22bfloat162_rn(fma2(mul2(acc[p][1], rstd), gw1, gb1));
+            const float2 mr = stat[p], nm = splat2(-mr.x), rstd = splat2(mr.y);
+            const __nv_bfloat162 h0 = __float22bfloat162_rn(fma2(mul2(add2(acc[p][0], nm), rstd), gw0, gb0));
+            const __nv_bfloat162 h1 = __float22bfloat162_rn(fma2(mul2(add2(acc[p][1], nm), rstd), gw1, gb1));
             *reinterpret_cast<uint2*>(orow + (int64_t)p * C) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
           }
         }
@@ -502,12 +513,12 @@ extern "C" int kf_dw_ln(const void* g, const float* bias, const float* dww, cons
   if (B == 0) return KF_OK;
   KF_REQUIRE(g && (bias || pre_act) && dww && lnw && lnb && out && al16(g) && al16(out) && al16(lnw) && al16(lnb) && al16(dww) && al16(bias),
              "kf_dw_ln: tensors must be non-null and 16-byte aligned");
-  const size_t smem = (size_t)DW_RING * DW_HALO * C * 2 + 2 * 64 * sizeof(float);
+  const size_t smem = (size_t)DW_RING * DW_HALO * C * 2 + DW_RED_FLOATS * sizeof(float);
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !attr_set[dev]) {
-    const int big = (int)((size_t)DW_RING * DW_HALO * 1024 * 2 + 2 * 64 * sizeof(float));
+    const int big = (int)((size_t)DW_RING * DW_HALO * 1024 * 2 + DW_RED_FLOATS * sizeof(float));
     cudaError_t e = cudaFuncSetAttribute(dw_ln_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(dw_ln_kernel<768>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(dw_ln_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
