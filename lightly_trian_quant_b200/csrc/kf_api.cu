@@ -23,12 +23,12 @@ int cuda_status(cudaError_t e, const char* what) {
 
 // Programmatic dependent launch is taken where the launches are short: the successor's start-up (about 2 us of launch, barrier and
 // tensor-memory set-up) then runs under its predecessor.  Measured, whole models, plain -> dependent: ViT-B 256 px called eagerly
-// 782 -> 695 us, ViT-L 640 px one frame captured 1950 -> 1876 us; ViT-B 640 px eager, three images, 2298 -> 2126 us (launch gaps
+// 782 -> 635 us, ViT-L 640 px one frame captured 1950 -> 1883 us; ViT-B 640 px eager, three images, 2298 -> 2052 us (launch gaps
 // of the eager stream); captured graphs of 3210 rows are level and of 6420 rows and more 1 to 2 % slower, hence the two lines.
 static bool g_pdl = false;                            // kf_set_pdl(1): every launch
 bool pdl_for(int64_t rows, cudaStream_t st) {
   if (g_pdl || rows <= 2048) return true;
-  if (rows > 5120) return false;
+  if (rows > 20480) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }

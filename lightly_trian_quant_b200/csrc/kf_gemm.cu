@@ -43,9 +43,9 @@ namespace kf {
 // flight over the L2 latency, so all of K up to six stages (36 KB each).
 constexpr int MAX_STAGES = 6;
 template <int BN>
-static int gemm_stages(int epi, int k_tiles, int flags) {
+static int gemm_stages(int epi, int k_tiles, int flags, bool res_tma) {
   if (BN == 128) {
-    const int most = epi == KF_EPI_ROPE ? 5 : 6;
+    const int most = epi == KF_EPI_ROPE ? 5 : res_tma ? 4 : 6;
     return k_tiles < 2 ? 2 : k_tiles < most ? k_tiles : most;
   }
   if (epi == KF_EPI_PLAIN) return (flags & KF_G_GELU) ? 3 : 4;      // PLAIN with GELU (the head's ConvTranspose GEMMs) is epilogue-bound too
@@ -53,20 +53,23 @@ static int gemm_stages(int epi, int k_tiles, int flags) {
   return 3;
 }
 constexpr size_t GEMM_SMEM_MAX = 227 * 1024;
-// operand ring + scale atoms + bias slices or vectors (+ the rotary-table slabs) + barriers
+// operand ring + scale atoms + bias slices or vectors (+ the rotary-table slabs, + the residual boxes) + barriers
 template <int EPI, int BN>
-constexpr size_t gemm_smem(int stages, int vec_floats = 0) {
+constexpr size_t gemm_smem(int stages, int vec_floats = 0, bool res_tma = false) {
   const size_t sl = (size_t)(vec_floats > EPI_WARPS * SLICE_FLOATS ? vec_floats : EPI_WARPS * SLICE_FLOATS) * 4;
-  return (size_t)stages * (Tile<BN>::BYTES + Tile<BN>::SF_BYTES) + sl + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS * 4 : 0) + 256;
+  return (size_t)stages * (Tile<BN>::BYTES + Tile<BN>::SF_BYTES) + sl + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS * 4 : 0) +
+         (res_tma ? EPI_WARPS * RES_BOX_BYTES : 0) + 384;
 }
 static_assert(gemm_smem<KF_EPI_ROPE, 256>(3) <= GEMM_SMEM_MAX && gemm_smem<KF_EPI_RES, 256>(4) <= GEMM_SMEM_MAX && gemm_smem<KF_EPI_ROPE, 128>(5) <= GEMM_SMEM_MAX &&
-                  gemm_smem<KF_EPI_RES, 128>(6) <= GEMM_SMEM_MAX,
+                  gemm_smem<KF_EPI_RES, 128>(6) <= GEMM_SMEM_MAX &&
+                  gemm_smem<KF_EPI_RES, 128>(4, 0, true) <= GEMM_SMEM_MAX,
               "shared memory of the deepest rings");
 
 // ------------------------------------------------------------------------------------------------ the kernel
 template <int KIND, int EPI, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const GemmArgs g) {
+gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmR,
+            const __grid_constant__ CUtensorMap tmC, const GemmArgs g) {
   constexpr int ATOMS = KindTraits<KIND>::ATOMS;
   constexpr bool SCALED = KIND != KIND_BF16;
   constexpr int TILE_BYTES = Tile<BN>::BYTES, SF_STAGE_BYTES = Tile<BN>::SF_BYTES, ACCS = Tile<BN>::ACCS;
@@ -74,15 +77,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* tiles = smem;
-  uint8_t* sfs = smem + (size_t)STAGES * TILE_BYTES;
+  uint8_t* boxes = smem + (size_t)STAGES * TILE_BYTES;                                  // RES through shared memory only; 1024-byte aligned
+  uint8_t* sfs = boxes + (EPI == KF_EPI_RES && BN == 128 && g.res_tma ? EPI_WARPS * RES_BOX_BYTES : 0);
   float* slices = reinterpret_cast<float*>(sfs + (size_t)STAGES * SF_STAGE_BYTES);
   float* slabs = slices + (g.vec_floats > EPI_WARPS * SLICE_FLOATS ? g.vec_floats : EPI_WARPS * SLICE_FLOATS);   // ROPE only
   uint64_t* bars = reinterpret_cast<uint64_t*>(slabs + (EPI == KF_EPI_ROPE ? 4 * ROPE_SLAB_FLOATS : 0));
   uint64_t *full = bars, *empty = bars + MAX_STAGES, *tfull = bars + 2 * MAX_STAGES, *tempty = tfull + 2;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* box_full = tempty + 2;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(box_full + EPI_WARPS);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
-  pdl_launch_dependents();                               // the next kernel of the stream may take the SMs this grid leaves
   const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -93,6 +97,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       mbar_init(&tfull[a], 1);
       mbar_init(&tempty[a], EPI_WARPS);
     }
+    if (EPI == KF_EPI_RES && BN == 128)
+      for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&box_full[w], 1);
     *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;     // the swizzled operand tiles need a 1024-byte aligned base
     fence_mbar_init();
     prefetch_tmap(&tmA);
@@ -213,10 +219,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
     if (!bad_align) {
       const TileSched sched{(int)blockIdx.x, (int)gridDim.x, total_tiles, g.n_tiles};
-      epilogue_warps<EPI, BN>(g, sched, tmem_base, tfull, tempty, slices, slabs, ctx, warp, lane);
+      epilogue_warps<EPI, BN>(g, sched, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tmR, &tmC, ctx, warp, lane);
     }
   }
 
+  pdl_launch_dependents();                               // only now: see kf_common.cuh
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
@@ -309,8 +316,12 @@ int device_sm_count(int* sms) {
   return KF_OK;
 }
 
+struct GemmMaps {
+  CUtensorMap A, W, R, C;                                 // R, C: the residual and the output of a RES launch through shared memory, else copies of A
+};
+
 template <int KIND, int EPI, int BN>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs& g, int grid, cudaStream_t st) {
+static int launch_gemm(const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -319,33 +330,33 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmW, const Gem
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_kernel)");
     if (dev < 64) attr_set[dev] = true;
   }
-  return cuda_status(launch_maybe_pdl(g.M, gemm_kernel<KIND, EPI, BN>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats), st, tmA, tmW, g), "kf_gemm_bs launch");
+  return cuda_status(launch_maybe_pdl(g.M, gemm_kernel<KIND, EPI, BN>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats, g.res_tma != 0), st, tm.A, tm.W, tm.R, tm.C, g), "kf_gemm_bs launch");
 }
 
 template <int KIND, int BN>
-static int launch_gemm_epi(int epi, const CUtensorMap& tmA, const CUtensorMap& tmW, const GemmArgs& g, int grid, cudaStream_t st) {
+static int launch_gemm_epi(int epi, const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
   switch (epi) {
-    case KF_EPI_PLAIN: return launch_gemm<KIND, KF_EPI_PLAIN, BN>(tmA, tmW, g, grid, st);
-    case KF_EPI_RES: return launch_gemm<KIND, KF_EPI_RES, BN>(tmA, tmW, g, grid, st);
-    case KF_EPI_ROPE: return launch_gemm<KIND, KF_EPI_ROPE, BN>(tmA, tmW, g, grid, st);
-    default: return launch_gemm<KIND, KF_EPI_QUANT, BN>(tmA, tmW, g, grid, st);
+    case KF_EPI_PLAIN: return launch_gemm<KIND, KF_EPI_PLAIN, BN>(tm, g, grid, st);
+    case KF_EPI_RES: return launch_gemm<KIND, KF_EPI_RES, BN>(tm, g, grid, st);
+    case KF_EPI_ROPE: return launch_gemm<KIND, KF_EPI_ROPE, BN>(tm, g, grid, st);
+    default: return launch_gemm<KIND, KF_EPI_QUANT, BN>(tm, g, grid, st);
   }
 }
 
 template <int BN>
-static int launch_gemm_fmt(int fmt, int epi, const CUtensorMap& tmA, const CUtensorMap& tmW, GemmArgs& g, int sms, cudaStream_t st) {
+static int launch_gemm_fmt(int fmt, int epi, const GemmMaps& tm, GemmArgs& g, int sms, cudaStream_t st) {
   g.n_tiles = (g.N + BN - 1) / BN;
   const int total = g.m_tiles * g.n_tiles, grid = total < sms ? total : sms;
-  g.stages = gemm_stages<BN>(epi, g.k_tiles, g.flags);
+  g.stages = gemm_stages<BN>(epi, g.k_tiles, g.flags, g.res_tma != 0);
   // The whole bias (+ LayerScale) vector in shared memory where a CTA works on several tiles and the ring depth leaves room for it
   const int want = (g.bias || epi == KF_EPI_RES) ? g.N * (epi == KF_EPI_RES ? 2 : 1) : 0;
-  const size_t with = epi == KF_EPI_ROPE ? gemm_smem<KF_EPI_ROPE, BN>(g.stages, want) : gemm_smem<KF_EPI_RES, BN>(g.stages, want);
+  const size_t with = epi == KF_EPI_ROPE ? gemm_smem<KF_EPI_ROPE, BN>(g.stages, want) : gemm_smem<KF_EPI_RES, BN>(g.stages, want, g.res_tma != 0);
   g.vec_floats = (want > 0 && total > grid && with <= GEMM_SMEM_MAX) ? want : 0;
   switch (fmt) {
-    case KF_FMT_MX8: return launch_gemm_epi<KIND_MX8, BN>(epi, tmA, tmW, g, grid, st);
-    case KF_FMT_NV4: return launch_gemm_epi<KIND_NV4, BN>(epi, tmA, tmW, g, grid, st);
-    case KF_FMT_MX4: return launch_gemm_epi<KIND_MX4, BN>(epi, tmA, tmW, g, grid, st);
-    default: return launch_gemm_epi<KIND_BF16, BN>(epi, tmA, tmW, g, grid, st);
+    case KF_FMT_MX8: return launch_gemm_epi<KIND_MX8, BN>(epi, tm, g, grid, st);
+    case KF_FMT_NV4: return launch_gemm_epi<KIND_NV4, BN>(epi, tm, g, grid, st);
+    case KF_FMT_MX4: return launch_gemm_epi<KIND_MX4, BN>(epi, tm, g, grid, st);
+    default: return launch_gemm_epi<KIND_BF16, BN>(epi, tm, g, grid, st);
   }
 }
 
@@ -359,6 +370,10 @@ static int gemm_columns(int m_tiles, int N, int sms, bool plain) {
   const int64_t r256 = ((int64_t)m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = ((int64_t)m_tiles * (N / 128) + sms - 1) / sms;
   return (plain ? 7 : 6) * r128 < 10 * r256 ? 128 : 256;
 }
+
+// RES launches that move the residual through shared memory (128-column tiles): those of many rounds, where its bandwidth counts
+// and the box of the next tile travels under the present one.
+static bool gemm_res_boxes(int fmt, int m_tiles, int N, int sms) { return (int64_t)m_tiles * (N / 128) >= 3 * (int64_t)sms; }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static bool al32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }   // 256-bit global accesses of the epilogues
@@ -414,12 +429,20 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   int sms = 0;
   int st = device_sm_count(&sms);
   if (st != KF_OK) return st;
-  const int bn = gemm_columns(m_tiles, p->N, sms, epi == KF_EPI_PLAIN);
-  CUtensorMap tmA, tmW;
-  st = make_tmap_2d_bytes(&tmA, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
+  const bool res_tma = epi == KF_EPI_RES && p->out_row_group == 0 && gemm_res_boxes(fmt, m_tiles, p->N, sms);
+  const int bn = res_tma ? 128 : gemm_columns(m_tiles, p->N, sms, epi == KF_EPI_PLAIN);
+  GemmMaps tm;
+  st = make_tmap_2d_bytes(&tm.A, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
   if (st != KF_OK) return st;
-  st = make_tmap_2d_bytes(&tmW, p->W, w_rows, kbytes, kbytes, bn);
+  st = make_tmap_2d_bytes(&tm.W, p->W, w_rows, kbytes, kbytes, bn);
   if (st != KF_OK) return st;
+  tm.R = tm.C = tm.A;
+  if (res_tma) {
+    st = make_tmap_2d_bytes(&tm.R, p->R, (uint64_t)p->M, 4ull * p->N, 4ull * p->N, 32);
+    if (st != KF_OK) return st;
+    st = make_tmap_2d_bytes(&tm.C, p->C, (uint64_t)p->M, 4ull * p->N, 4ull * p->N, 32);
+    if (st != KF_OK) return st;
+  }
   GemmArgs g{};
   g.sfa = static_cast<const uint8_t*>(p->SFA);
   g.sfw = static_cast<const uint8_t*>(p->SFW);
@@ -437,9 +460,10 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   g.nkb4 = fmt == KF_FMT_BF16 ? 0 : p->K / (4 * fmt_vec(fmt));
   const bool maps_rows = epi == KF_EPI_PLAIN || epi == KF_EPI_RES;
   g.row_group = maps_rows ? p->out_row_group : 0; g.row_stride = p->out_row_stride; g.row_offset = p->out_row_offset;
+  g.res_tma = res_tma;
   g.y_dbg = epi == KF_EPI_QUANT ? p->y_dbg : nullptr;
   g.err = dev_error_ptr();
   KF_REQUIRE(g.err != nullptr, "kf_gemm_bs: device error word unavailable");
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  return bn == 128 ? launch_gemm_fmt<128>(fmt, epi, tmA, tmW, g, sms, cs) : launch_gemm_fmt<256>(fmt, epi, tmA, tmW, g, sms, cs);
+  return bn == 128 ? launch_gemm_fmt<128>(fmt, epi, tm, g, sms, cs) : launch_gemm_fmt<256>(fmt, epi, tm, g, sms, cs);
 }

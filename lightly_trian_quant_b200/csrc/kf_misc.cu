@@ -10,7 +10,6 @@ namespace kf {
 // GEMM against the Conv2d weight [d, 3, 16, 16] viewed as [d, 768].  One thread moves 16 pixels (32 bytes) of one
 // patch row.
 __global__ void __launch_bounds__(256) im2col16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, int B, int S) {
-  pdl_launch_dependents();
   pdl_wait();
   const int g = S >> 4;
   const int64_t total = (int64_t)B * g * g * 48;
@@ -101,7 +100,6 @@ __global__ void __launch_bounds__(256, 2)
 dw_ln_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ bias, const float* __restrict__ dww, const float* __restrict__ lnw,
              const float* __restrict__ lnb, __nv_bfloat16* __restrict__ out, int Hs, int Ws, int C_arg, float eps, int pre_act, int strips, int segs,
              int seg_rows, int total_items) {
-  pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) uint8_t dsm[];
   const int C = CT ? CT : C_arg;

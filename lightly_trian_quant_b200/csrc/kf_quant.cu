@@ -72,7 +72,6 @@ template <typename T, int FMT>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, const float* __restrict__ ts_ptr,
                                                          const float* __restrict__ bias, int flags, int wide, uint8_t* __restrict__ q,
                                                          uint8_t* __restrict__ sf, int64_t items_valid, int64_t items_total) {
-  pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int per_row = K >> 5;
@@ -200,7 +199,6 @@ __device__ __forceinline__ float gelu_abs(float x) { return fabsf(x * 0.5f * (1.
 template <typename T, bool GELU>
 __global__ void __launch_bounds__(256) amax_scale_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, int wide, float factor, float* __restrict__ ts,
                                                          uint32_t* __restrict__ ws) {
-  pdl_launch_dependents();
   pdl_wait();
   const uint32_t per_row = K >> 5, total = (uint32_t)M * per_row;
   float am = 0.f;
@@ -486,7 +484,6 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI
 template <int NV, typename TI>
 __global__ void __launch_bounds__(128) ln_amax_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps, int M, float factor,
                                                       float* __restrict__ ts, uint32_t* __restrict__ ws) {
-  pdl_launch_dependents();
   pdl_wait();
   constexpr int D = NV * 256;
   const int lane = threadIdx.x & 31;
@@ -505,7 +502,6 @@ __global__ void __launch_bounds__(128) ln_amax_kernel(const TI* __restrict__ x, 
 template <int NV, typename TO>
 __global__ void __launch_bounds__(128) ln_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps,
                                                       int M, TO* __restrict__ y) {
-  pdl_launch_dependents();
   pdl_wait();
   constexpr int D = NV * 256;
   const int lane = threadIdx.x & 31;
@@ -539,7 +535,6 @@ __global__ void __launch_bounds__(128) ln_tail_kernel(const float* __restrict__ 
                                                       int M, int Ntok, int Q, int npre, __nv_bfloat16* __restrict__ qb, __nv_bfloat16* __restrict__ xb,
                                                       const __nv_bfloat16* __restrict__ wcls, const float* __restrict__ bcls, int ncls1,
                                                       __nv_bfloat16* __restrict__ cl) {
-  pdl_launch_dependents();
   pdl_wait();
   constexpr int D = NV * 256;
   const int lane = threadIdx.x & 31;
@@ -591,7 +586,6 @@ __global__ void __launch_bounds__(128) ln_tail_kernel(const float* __restrict__ 
 // The query rows that join the stream for the last blocks and the cls / register rows in front of the patch tokens.
 __global__ void __launch_bounds__(256) broadcast_rows_kernel(const float4* __restrict__ src, float4* __restrict__ dst, int R, int d4, int B, int64_t img_stride4,
                                                              int64_t row_offset4) {
-  pdl_launch_dependents();
   pdl_wait();
   const int64_t n = (int64_t)R * d4;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * B; i += (int64_t)gridDim.x * blockDim.x) {
