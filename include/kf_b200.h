@@ -62,6 +62,8 @@ extern "C" {
 #define KF_G_ROPE_HALF 128 /* ROPE: the caller guarantees that columns 32..63 of sin / cos repeat columns 0..31 (the axial
                               tables of DINOv3 are the angle vector concatenated with itself); lets the kernel keep the table
                               rows of a tile in shared memory.  Without the flag both halves are read as given. */
+#define KF_G_W_STATIC 512  /* the caller guarantees that no kernel of this library still running on the stream writes W or SFW (weights
+                              laid out once): under dependent launch the kernel may read them before its predecessor is done */
 
 /* Library version and the SM architecture the kernels were built for ("sm_100a"). */
 KF_API const char* kf_version(void);

@@ -146,6 +146,8 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
 }
 
 // ------------------------------------------------------------------------------------------------ GEMM
+// A weight container (ops.QWeight) holds codes that the row quantiser or torch wrote, or a copy of a bf16 tensor: kernels that signal
+// their successors only by ending, so KF_G_W_STATIC holds for every launch with one.  bmm_nt takes activations and does not claim it.
 // A side, W side and the common fields; returns M
 int64_t gemm_fill(kf_gemm_params& p, PyObject* a, const Operand& W, int epi) {
   int64_t M;
@@ -184,7 +186,7 @@ PyObject* gemm_plain(PyObject* const* v) {
   const float* bias = f32_vec(v[2], W.rows, "bias");
   const int64_t M = gemm_fill(p, v[0], W, KF_EPI_PLAIN);
   p.bias = bias;
-  p.flags = (int)to_int(v[5]);
+  p.flags = (int)to_int(v[5]) | KF_G_W_STATIC;
   if (v[3] == Py_None) {
     p.out_dtype = (int)to_int(v[4]);
     at::Tensor out = empty({M, W.rows}, dtype_of(p.out_dtype), W.q->device());
@@ -208,6 +210,7 @@ PyObject* gemm_res(PyObject* const* v) {
   const int64_t M = gemm_fill(p, v[0], W, KF_EPI_RES);
   p.bias = bias;
   p.gamma = gamma;
+  p.flags = KF_G_W_STATIC;
   p.R = f32_vec(v[4], M * W.rows, "res");
   p.out_dtype = KF_F32;
   if (v[5] == Py_None) {
@@ -253,7 +256,7 @@ PyObject* qkv_rope(PyObject* const* v) {
   p.prefix = (int)prefix;
   p.H = (int)H;
   p.out_dtype = (int)to_int(v[8]);
-  p.flags = (int)to_int(v[9]);
+  p.flags = (int)to_int(v[9]) | KF_G_W_STATIC;
   at::Tensor out = empty({3, M / Ntok, Ntok, H, 64}, dtype_of(p.out_dtype), W.q->device());
   p.C = out.data_ptr();
   gemm_run(p, "qkv_rope");
@@ -276,7 +279,7 @@ PyObject* gemm_gelu_q(PyObject* const* v) {
   p.Qo = out.pq;
   p.SFo = out.psf;
   p.tso = static_cast<const float*>(out.pts);
-  p.flags = (int)to_int(v[4]);
+  p.flags = (int)to_int(v[4]) | KF_G_W_STATIC;
   gemm_run(p, "gemm_gelu_q");
   return new_ref(v[3]);
 }
@@ -332,7 +335,7 @@ PyObject* gemm_tokens(PyObject* const* v) {
   p.out_row_group = (int)to_int(v[4]);
   p.out_row_stride = (int)to_int(v[5]);
   p.out_row_offset = (int)to_int(v[6]);
-  p.flags = (int)to_int(v[7]);
+  p.flags = (int)to_int(v[7]) | KF_G_W_STATIC;
   gemm_run(p, "gemm_tokens");
   return new_ref(v[3]);
 }

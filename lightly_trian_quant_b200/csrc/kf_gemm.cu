@@ -111,7 +111,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();                                            // set-up done: from here on global memory of the predecessors is read and written
+  // Set-up done: from here on global memory of the predecessors is read and written.  The producer may ask for weights first.
+  const bool w_early = (g.flags & KF_G_W_STATIC) != 0;
+  if (warp != 0 || !w_early) pdl_wait();
   const uint32_t tmem_base = *tmem_holder;
   const WaitCtx ctx{abort_flag, g.err};
   const int total_tiles = g.m_tiles * g.n_tiles;
@@ -124,34 +126,47 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (warp < EPI_WARP0) {
     setmaxnreg_dec<EPI == KF_EPI_ROPE ? REGS_LEAN_ROPE : REGS_LEAN>();
     if (bad_align) {
-      // nothing is issued; fall through to the teardown
+      if (warp == 0 && w_early) pdl_wait();              // nothing is issued; fall through to the teardown
     } else if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       uint32_t s = 0, ph = 0;
       bool ok = true;
+      // Weights that no running predecessor writes (KF_G_W_STATIC): the W part of the first tile's stages is requested before the
+      // wait for the predecessor, so its way from HBM runs under the predecessor's end.
+      int early = 0;
+      auto load_w = [&](uint32_t st, int kt, int m_blk, int n_blk, int w_halves, uint32_t tx) {
+        mbar_expect_tx(&full[st], tx);
+        tma_load_2d(tiles + (size_t)st * TILE_BYTES + A_BYTES, &tmW, kt * BKB, tile_wrow0(g, m_blk, n_blk * BN), &full[st]);   // rows past the end of W are filled with zeros
+        if (SCALED) {
+          uint8_t* sa = sfs + (size_t)st * SF_STAGE_BYTES;
+          for (int h = 0; h < w_halves; ++h)
+            bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(BN / 128 * n_blk + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[st]);
+        }
+      };
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const int m_blk = tile / g.n_tiles, n_blk = tile - m_blk * g.n_tiles;
         const int w_halves = (BN == 256 && n_blk * BN + 128 < g.N) ? 2 : 1;   // the last column tile of 256 may hold only 128 columns
         int row_end;
-        const int a_row0 = tile_row0(g, m_blk, row_end), w_row0 = tile_wrow0(g, m_blk, n_blk * BN);
+        const int a_row0 = tile_row0(g, m_blk, row_end);
         const uint32_t tx = TILE_BYTES + (SCALED ? (1 + w_halves) * ATOMS * 512 : 0);
+        if (w_early && tile == (int)blockIdx.x) {
+          early = g.k_tiles < STAGES ? g.k_tiles : STAGES;
+          if (elect_one())
+            for (int kt = 0; kt < early; ++kt) load_w(kt, kt, m_blk, n_blk, w_halves, tx);
+          __syncwarp();
+          pdl_wait();
+        }
         for (int kt = 0; kt < g.k_tiles; ++kt) {
           if (!mbar_wait_warp(&empty[s], ph ^ 1, ctx, 1)) { ok = false; break; }
           if (elect_one()) {
-            mbar_expect_tx(&full[s], tx);
-            uint8_t* ta = tiles + (size_t)s * TILE_BYTES;
-            tma_load_2d(ta, &tmA, kt * BKB, a_row0, &full[s]);
-            tma_load_2d(ta + A_BYTES, &tmW, kt * BKB, w_row0, &full[s]);       // rows past the end of W are filled with zeros
-            if (SCALED) {
-              uint8_t* sa = sfs + (size_t)s * SF_STAGE_BYTES;
-              bulk_load_1d(sa, g.sfa + ((size_t)m_blk * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
-              for (int h = 0; h < w_halves; ++h)
-                bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(BN / 128 * n_blk + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
-            }
+            if (kt >= early) load_w(s, kt, m_blk, n_blk, w_halves, tx);
+            tma_load_2d(tiles + (size_t)s * TILE_BYTES, &tmA, kt * BKB, a_row0, &full[s]);
+            if (SCALED) bulk_load_1d(sfs + (size_t)s * SF_STAGE_BYTES, g.sfa + ((size_t)m_blk * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
           }
           __syncwarp();
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
+        early = 0;
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issuer
@@ -364,16 +379,21 @@ static int launch_gemm_fmt(int fmt, int epi, const GemmMaps& tm, GemmArgs& g, in
 // wherever there are many tiles; 128 columns cut the launch finer, take twice the SMs where the tiles do not fill the
 // chip, and keep two accumulators in tensor memory.  A round of 128-column tiles takes about 0.6 of a round of 256-column tiles
 // (0.7 for PLAIN, whose epilogue is too short to hide the larger operand traffic: MXFP8 1605 x 1024 x 4096 13.4 us in 3 rounds
-// against 12.8 in 2), so 128 wins when ceil(tiles / SMs) rounds of them are shorter: one frame's 13 row tiles x 1024 columns are one round either way
+// against 12.8 in 2; 0.505 for QUANT on 4-bit operands, which is as slow as its epilogue in either form, M = 22 470 92.6 -> 90.2 us),
+// so 128 wins when ceil(tiles / SMs) rounds of them are shorter: one frame's 13 row tiles x 1024 columns are one round either way
 // (104 SMs instead of 52), x 4096 columns 3 x 0.6 rounds against 2 (fc1 NVFP4 14.6 -> 12.1 us, proj / fc2 13.9 -> 8.8 us on average); from about five rounds on the rounding no longer pays.
-static int gemm_columns(int m_tiles, int N, int sms, bool plain) {
+static int gemm_columns(int fmt, int epi, int m_tiles, int N, int sms) {
   const int64_t r256 = ((int64_t)m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = ((int64_t)m_tiles * (N / 128) + sms - 1) / sms;
-  return (plain ? 7 : 6) * r128 < 10 * r256 ? 128 : 256;
+  const bool fp4 = fmt == KF_FMT_NV4 || fmt == KF_FMT_MX4;
+  const int permille = epi == KF_EPI_PLAIN ? 700 : epi == KF_EPI_QUANT && fp4 ? 505 : 600;
+  return permille * r128 < 1000 * r256 ? 128 : 256;
 }
 
 // RES launches that move the residual through shared memory (128-column tiles): those of many rounds, where its bandwidth counts
 // and the box of the next tile travels under the present one.
-static bool gemm_res_boxes(int fmt, int m_tiles, int N, int sms) { return (int64_t)m_tiles * (N / 128) >= 3 * (int64_t)sms; }
+// Not for a long K: the 128-column tiles then cost more operand traffic than the boxes save (M = 22 470, NVFP4: K 1024, 4 stages,
+// 45 -> 33 us, but K 4096, 16 stages, 67 -> 77 us; MXFP8 x 768: K 768, 6 stages, 38.6 -> 27.6, K 3072, 24 stages, 64.7 -> 77).
+static bool gemm_res_boxes(int k_tiles, int m_tiles, int N, int sms) { return k_tiles <= 8 && (int64_t)m_tiles * (N / 128) >= 3 * (int64_t)sms; }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static bool al32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }   // 256-bit global accesses of the epilogues
@@ -429,8 +449,8 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   int sms = 0;
   int st = device_sm_count(&sms);
   if (st != KF_OK) return st;
-  const bool res_tma = epi == KF_EPI_RES && p->out_row_group == 0 && gemm_res_boxes(fmt, m_tiles, p->N, sms);
-  const int bn = res_tma ? 128 : gemm_columns(m_tiles, p->N, sms, epi == KF_EPI_PLAIN);
+  const bool res_tma = epi == KF_EPI_RES && p->out_row_group == 0 && gemm_res_boxes((int)(kbytes / BKB), m_tiles, p->N, sms);
+  const int bn = res_tma ? 128 : gemm_columns(fmt, epi, m_tiles, p->N, sms);
   GemmMaps tm;
   st = make_tmap_2d_bytes(&tm.A, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
   if (st != KF_OK) return st;

@@ -215,6 +215,8 @@ class QWeight:
         self.fmt = fmt
         if fmt == "bf16":
             self.q = W.to(torch.bfloat16).contiguous()
+            if self.q.data_ptr() == W.data_ptr():
+                self.q = self.q.clone()            # a copy of its own: the GEMM reads weights ahead of its predecessor's end
             self.sf = None
             self.ts = None
             return
