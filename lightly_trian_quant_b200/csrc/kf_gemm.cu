@@ -116,7 +116,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (warp != 0 || !w_early) pdl_wait();
   const uint32_t tmem_base = *tmem_holder;
   const WaitCtx ctx{abort_flag, g.err};
-  const int total_tiles = g.m_tiles * g.n_tiles;
   const bool bad_align = *abort_flag != 0 || g.err[0] != 0;   // misaligned tiles, or an earlier CTA / launch already failed: skip the work
   if (*abort_flag != 0 && threadIdx.x == 0 && atomicCAS(&g.err[0], 0u, (unsigned)(-KF_ERR_DEVICE_WAIT)) == 0u) {
     g.err[1] = 100;
@@ -134,34 +133,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       // Weights that no running predecessor writes (KF_G_W_STATIC): the W part of the first tile's stages is requested before the
       // wait for the predecessor, so its way from HBM runs under the predecessor's end.
       int early = 0;
-      auto load_w = [&](uint32_t st, int kt, int m_blk, int n_blk, int w_halves, uint32_t tx) {
+      auto load_w = [&](uint32_t st, int kt, const WorkItem& w, int w_halves, uint32_t tx) {
         mbar_expect_tx(&full[st], tx);
-        tma_load_2d(tiles + (size_t)st * TILE_BYTES + A_BYTES, &tmW, kt * BKB, tile_wrow0(g, m_blk, n_blk * BN), &full[st]);   // rows past the end of W are filled with zeros
+        // rows past the end of W are filled with zeros; a half tile has a map of its own with boxes of 128 rows
+        tma_load_2d(tiles + (size_t)st * TILE_BYTES + A_BYTES, BN == 256 && w.cols == 128 ? &tmR : &tmW, kt * BKB, tile_wrow0(g, w.m_blk, w.n0), &full[st]);
         if (SCALED) {
           uint8_t* sa = sfs + (size_t)st * SF_STAGE_BYTES;
           for (int h = 0; h < w_halves; ++h)
-            bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(BN / 128 * n_blk + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[st]);
+            bulk_load_1d(sa + (1 + h) * ATOMS * 512, g.sfw + ((size_t)(w.n0 / 128 + h) * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[st]);
         }
       };
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        const int m_blk = tile / g.n_tiles, n_blk = tile - m_blk * g.n_tiles;
-        const int w_halves = (BN == 256 && n_blk * BN + 128 < g.N) ? 2 : 1;   // the last column tile of 256 may hold only 128 columns
+      for (int idx = blockIdx.x; idx < g.items && ok; idx += gridDim.x) {
+        const WorkItem w = work_item<BN>(g, idx);
+        const int w_halves = (BN == 256 && w.cols == BN && w.n0 + 128 < g.N) ? 2 : 1;   // the last column tile of 256 may hold only 128 columns
         int row_end;
-        const int a_row0 = tile_row0(g, m_blk, row_end);
-        const uint32_t tx = TILE_BYTES + (SCALED ? (1 + w_halves) * ATOMS * 512 : 0);
-        if (w_early && tile == (int)blockIdx.x) {
+        const int a_row0 = tile_row0(g, w.m_blk, row_end);
+        const uint32_t tx = A_BYTES + w.cols * BKB + (SCALED ? (1 + w_halves) * ATOMS * 512 : 0);
+        if (w_early && idx == (int)blockIdx.x) {
           early = g.k_tiles < STAGES ? g.k_tiles : STAGES;
           if (elect_one())
-            for (int kt = 0; kt < early; ++kt) load_w(kt, kt, m_blk, n_blk, w_halves, tx);
+            for (int kt = 0; kt < early; ++kt) load_w(kt, kt, w, w_halves, tx);
           __syncwarp();
           pdl_wait();
         }
         for (int kt = 0; kt < g.k_tiles; ++kt) {
           if (!mbar_wait_warp(&empty[s], ph ^ 1, ctx, 1)) { ok = false; break; }
           if (elect_one()) {
-            if (kt >= early) load_w(s, kt, m_blk, n_blk, w_halves, tx);
+            if (kt >= early) load_w(s, kt, w, w_halves, tx);
             tma_load_2d(tiles + (size_t)s * TILE_BYTES, &tmA, kt * BKB, a_row0, &full[s]);
-            if (SCALED) bulk_load_1d(sfs + (size_t)s * SF_STAGE_BYTES, g.sfa + ((size_t)m_blk * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
+            if (SCALED) bulk_load_1d(sfs + (size_t)s * SF_STAGE_BYTES, g.sfa + ((size_t)w.m_blk * g.nkb4 + (size_t)kt * ATOMS) * 512, ATOMS * 512, &full[s]);
           }
           __syncwarp();
           if (++s == STAGES) { s = 0; ph ^= 1; }
@@ -174,15 +174,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       // K-bytes.  One thread issues both, so the hardware runs them in order (an MMA sees the copies in front of it, a copy
       // does not overtake the MMAs that read the buffer's previous contents) and overlaps them: twelve copies and four
       // MMAs take the time of the MMAs alone.
-      constexpr uint32_t IDESC = KIND == KIND_BF16 ? idesc_f16(1, BN)
-                                 : KIND == KIND_MX8 ? idesc_bs(0, 1, BN)
-                                 : KIND == KIND_NV4 ? idesc_bs(1, 0, BN)
-                                                    : idesc_bs(1, 1, BN);
+      constexpr auto idesc_n = [](int n) {
+        return KIND == KIND_BF16 ? idesc_f16(1, n) : KIND == KIND_MX8 ? idesc_bs(0, 1, n) : KIND == KIND_NV4 ? idesc_bs(1, 0, n) : idesc_bs(1, 1, n);
+      };
       uint32_t s = 0, ph = 0, lt = 0, sb = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++lt) {
-        const int n_blk = tile % g.n_tiles;
-        const bool two = BN == 256 && n_blk * BN + 128 < g.N;
+      for (int idx = blockIdx.x; idx < g.items && ok; idx += gridDim.x, ++lt) {
+        const WorkItem w = work_item<BN>(g, idx);
+        const bool two = BN == 256 && w.cols == BN && w.n0 + 128 < g.N;
+        const uint32_t IDESC = w.cols == BN ? idesc_n(BN) : idesc_n(128);
         const uint32_t ac = lt % ACCS;
         if (!mbar_wait_warp(&tempty[ac], ((lt / ACCS) & 1) ^ 1, ctx, 2)) break;   // the epilogue has taken this accumulator's previous tile out of TMEM
         tc_fence_after();
@@ -233,8 +233,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ------------------------------------------------------------------ epilogue: 16 warps, warp = (TMEM lane quarter, 64-column group)
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
     if (!bad_align) {
-      const TileSched sched{(int)blockIdx.x, (int)gridDim.x, total_tiles, g.n_tiles};
-      epilogue_warps<EPI, BN>(g, sched, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tmR, &tmC, ctx, warp, lane);
+      epilogue_warps<EPI, BN>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tmR, &tmC, ctx, warp, lane);
     }
   }
 
@@ -332,7 +331,7 @@ int device_sm_count(int* sms) {
 }
 
 struct GemmMaps {
-  CUtensorMap A, W, R, C;                                 // R, C: the residual and the output of a RES launch through shared memory, else copies of A
+  CUtensorMap A, W, R, C;                                 // R, C: the residual and the output of a RES launch through shared memory; R: W in boxes of 128 rows for half tiles
 };
 
 template <int KIND, int EPI, int BN>
@@ -358,10 +357,20 @@ static int launch_gemm_epi(int epi, const GemmMaps& tm, const GemmArgs& g, int g
   }
 }
 
+// A last round of 256-column tiles that fills at most half of the SMs is cut into halves of 128 columns: the round then takes about
+// 0.6 of its time (one frame's 13 x 16 tiles are 1.6 rounds instead of 2, M = 22 470 x 3072 14.6 instead of 15).  Number of tiles cut.
+static int split_tiles(int total, int N, int sms) {
+  const int rest = total % sms;
+  return total > sms && 2 * rest <= sms && N % 256 == 0 ? rest : 0;
+}
+
 template <int BN>
 static int launch_gemm_fmt(int fmt, int epi, const GemmMaps& tm, GemmArgs& g, int sms, cudaStream_t st) {
   g.n_tiles = (g.N + BN - 1) / BN;
   const int total = g.m_tiles * g.n_tiles, grid = total < sms ? total : sms;
+  const int split = BN == 256 ? split_tiles(total, g.N, sms) : 0;
+  g.full_tiles = total - split;
+  g.items = total + split;
   g.stages = gemm_stages<BN>(epi, g.k_tiles, g.flags, g.res_tma != 0);
   // The whole bias (+ LayerScale) vector in shared memory where a CTA works on several tiles and the ring depth leaves room for it
   const int want = (g.bias || epi == KF_EPI_RES) ? g.N * (epi == KF_EPI_RES ? 2 : 1) : 0;
@@ -380,13 +389,14 @@ static int launch_gemm_fmt(int fmt, int epi, const GemmMaps& tm, GemmArgs& g, in
 // chip, and keep two accumulators in tensor memory.  A round of 128-column tiles takes about 0.6 of a round of 256-column tiles
 // (0.7 for PLAIN, whose epilogue is too short to hide the larger operand traffic: MXFP8 1605 x 1024 x 4096 13.4 us in 3 rounds
 // against 12.8 in 2; 0.505 for QUANT on 4-bit operands, which is as slow as its epilogue in either form, M = 22 470 92.6 -> 90.2 us),
-// so 128 wins when ceil(tiles / SMs) rounds of them are shorter: one frame's 13 row tiles x 1024 columns are one round either way
-// (104 SMs instead of 52), x 4096 columns 3 x 0.6 rounds against 2 (fc1 NVFP4 14.6 -> 12.1 us, proj / fc2 13.9 -> 8.8 us on average); from about five rounds on the rounding no longer pays.
+// so 128 wins where its rounds are the shorter sum: one frame's 13 row tiles x 1024 columns are one round either way (104 SMs instead
+// of 52: proj / fc2 NVFP4 13.9 -> 8.8 us on average).
 static int gemm_columns(int fmt, int epi, int m_tiles, int N, int sms) {
-  const int64_t r256 = ((int64_t)m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = ((int64_t)m_tiles * (N / 128) + sms - 1) / sms;
+  const int t256 = m_tiles * ((N + 255) / 256), t128 = m_tiles * (N / 128);
   const bool fp4 = fmt == KF_FMT_NV4 || fmt == KF_FMT_MX4;
   const int permille = epi == KF_EPI_PLAIN ? 700 : epi == KF_EPI_QUANT && fp4 ? 505 : 600;
-  return permille * r128 < 1000 * r256 ? 128 : 256;
+  const int64_t cost256 = 1000 * (int64_t)(t256 / sms) + (t256 % sms == 0 ? 0 : split_tiles(t256, N, sms) ? 600 : 1000), cost128 = (int64_t)permille * ((t128 + sms - 1) / sms);
+  return cost128 <= cost256 ? 128 : 256;
 }
 
 // RES launches that move the residual through shared memory (128-column tiles): those of many rounds, where its bandwidth counts
@@ -457,6 +467,10 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   st = make_tmap_2d_bytes(&tm.W, p->W, w_rows, kbytes, kbytes, bn);
   if (st != KF_OK) return st;
   tm.R = tm.C = tm.A;
+  if (bn == 256 && split_tiles(m_tiles * ((p->N + 255) / 256), p->N, sms)) {
+    st = make_tmap_2d_bytes(&tm.R, p->W, w_rows, kbytes, kbytes, 128);   // the half tiles' W boxes
+    if (st != KF_OK) return st;
+  }
   if (res_tma) {
     st = make_tmap_2d_bytes(&tm.R, p->R, (uint64_t)p->M, 4ull * p->N, 4ull * p->N, 32);
     if (st != KF_OK) return st;

@@ -47,6 +47,7 @@ struct GemmArgs {
   int Ntok, prefix, H, d;
   int out_dtype, flags, out_fmt;
   int m_tiles, n_tiles, k_tiles, nkb4, stages;
+  int full_tiles, items;                   // work items: full_tiles whole tiles, then the remaining tiles of the last round as two 128-column halves each
   int row_group, row_stride, row_offset;   // PLAIN, RES: output row = (m / group) * stride + offset + m % group (group 0: identity)
   int m_tiles_pb, a_rows_pb, w_rows_pb;    // batched products (m_tiles_pb > 0): row tiles, A rows and W rows per product
   int vec_floats;                          // > 0: the whole bias vector (and for RES the LayerScale vector behind it) sits in shared memory for the launch
@@ -398,23 +399,31 @@ __device__ __forceinline__ int tile_row0(const GemmArgs& g, int m_blk, int& row_
 __device__ __forceinline__ int tile_wrow0(const GemmArgs& g, int m_blk, int n0) { return (g.m_tiles_pb > 0 ? (m_blk / g.m_tiles_pb) * g.w_rows_pb : 0) + n0; }
 
 // ------------------------------------------------------------------------------------------------ tile schedules and the epilogue warps' loop
-// The i-th tile of a persistent CTA: tiles start, start + step, ... of the row-major tile grid.
-struct TileSched {
-  int start, step, total, n_tiles;
-  __device__ __forceinline__ bool get(int i, int& m_blk, int& n_blk) const {
-    const int idx = start + i * step;
-    if (idx >= total) return false;
-    m_blk = idx / n_tiles;
-    n_blk = idx - m_blk * n_tiles;
-    return true;
-  }
+// Work item idx of a launch: columns n0 .. n0 + cols - 1 of row tile m_blk.  Items are the tiles in row-major order; the tiles of a
+// last round that would leave more than half of the SMs empty come as two halves of 128 columns (BN = 256, kf_gemm.cu).
+struct WorkItem {
+  int m_blk, n0, cols;
 };
+template <int BN>
+__device__ __forceinline__ WorkItem work_item(const GemmArgs& g, int idx) {
+  int tile = idx, half = 0, cols = BN;
+  if (BN == 256 && idx >= g.full_tiles) {
+    tile = g.full_tiles + ((idx - g.full_tiles) >> 1);
+    half = (idx - g.full_tiles) & 1;
+    cols = 128;
+  }
+  WorkItem w;
+  w.m_blk = tile / g.n_tiles;
+  w.n0 = (tile - w.m_blk * g.n_tiles) * BN + half * 128;
+  w.cols = cols;
+  return w;
+}
 
 // Body of the 16 epilogue warps (warp = (TMEM lane quarter, 64- or 32-column group)): per tile, stage the bias slice (and fetch
 // the rotary-table rows), wait for the accumulator, take the warp's piece into registers, hand TMEM back at once and
 // run the fused epilogue on the registers while the next tile's main loop fills the accumulator again.
 template <int EPI, int BN>
-__device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSched& sched, uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty, float* slices,
+__device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty, float* slices,
                                                float* slabs, uint8_t* boxes, uint64_t* box_full, const CUtensorMap* tmR, const CUtensorMap* tmC, const WaitCtx& ctx, int warp,
                                                int lane) {
   constexpr int W = Tile<BN>::CW, ACCS = Tile<BN>::ACCS;
@@ -440,26 +449,27 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSche
   const Nv4Scale sco = nv4_scale((EPI == KF_EPI_QUANT && g.out_fmt == KF_FMT_NV4) ? __ldg(g.tso) : 1.f);   // once per CTA: every global load here is an L2 round trip
   const int col = PAIRS ? (cg >> 1) * 64 : cg * W, j0 = PAIRS ? (cg & 1) * 16 : 0;
   const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + col + j0;
-  int m_blk, n_blk;
   // RES through shared memory: this warp's box and its barrier; the box of the next tile is requested when the present one has left
   const bool boxed = EPI == KF_EPI_RES && W == 32 && g.res_tma != 0;
   uint8_t* box = boxes + (warp - EPI_WARP0) * RES_BOX_BYTES;
   uint64_t* bfull = box_full + (warp - EPI_WARP0);
   uint32_t bph = 0;
-  auto box_load = [&](int i) {
-    int mb, nb;
-    if (!sched.get(i, mb, nb)) return;
-    const int row = mb * BM + quarter * 32;
+  auto box_load = [&](int idx) {
+    if (idx >= g.items) return;
+    const WorkItem w = work_item<BN>(g, idx);
+    const int row = w.m_blk * BM + quarter * 32;
     if (row < g.M && lane == 0) {
       mbar_expect_tx(bfull, RES_BOX_BYTES);
-      tma_load_2d(box, tmR, (nb * BN + col) * 4, row, bfull);
+      tma_load_2d(box, tmR, (w.n0 + col) * 4, row, bfull);
     }
   };
-  if (boxed) box_load(0);
-  for (int lt = 0; sched.get(lt, m_blk, n_blk); ++lt) {
+  if (boxed) box_load(blockIdx.x);
+  int lt = 0;
+  for (int idx = blockIdx.x; idx < g.items; idx += gridDim.x, ++lt) {
+    const WorkItem item = work_item<BN>(g, idx);
     int row_end;
-    const int rbase = tile_row0(g, m_blk, row_end) + quarter * 32;
-    const int n0 = n_blk * BN + col;            // first column of this warp's group (or of its head)
+    const int rbase = tile_row0(g, item.m_blk, row_end) + quarter * 32;
+    const int n0 = item.n0 + col;               // first column of this warp's group (or of its head)
     const int acc = lt % ACCS;
     const uint32_t taddr = taddr0 + acc * BN;
     uint32_t r[W];
@@ -467,7 +477,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSche
     const float* bsl = vec ? slices + n0 : slice;
     const float* gsl = vec ? slices + g.N + n0 : slice + 64;
     // ROPE with half tables: the quarter's table rows are fetched now and parked in shared memory after the wait
-    const bool use_slab = EPI == KF_EPI_ROPE && (g.flags & KF_G_ROPE_HALF) != 0 && n_blk * BN < 2 * g.d;   // the tile holds q or k columns
+    const bool use_slab = EPI == KF_EPI_ROPE && (g.flags & KF_G_ROPE_HALF) != 0 && item.n0 < 2 * g.d;   // the tile holds q or k columns
     RopeSlabRegs tab;
     if (EPI == KF_EPI_ROPE && use_slab) rope_slab_fetch(g, rbase, cg * 32 + lane, tab);
     F8 res[4];
@@ -498,7 +508,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSche
       rope_slab_store(slab, cg * 32 + lane, tab);
       quarter_barrier(quarter);
     }
-    if (n0 >= g.N) continue;                                   // column group past N in the last column tile
+    if (n0 >= g.N || col >= item.cols) continue;               // column group past N in the last column tile, or past a half tile
     if constexpr (EPI == KF_EPI_RES && W == 32) {
       if (boxed) {
         if (rbase < g.M) {
@@ -513,7 +523,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, const TileSche
             bulk_wait_read();
           }
         }
-        box_load(lt + 1);
+        box_load(idx + gridDim.x);
         __syncwarp();
         continue;
       }

@@ -361,3 +361,35 @@ def test_column_tile_widths_agree(fmt):
                 continue
             part = u[b:b + 1] if u.shape[0] == B else u[rows]
             assert torch.equal(part, v), i
+
+
+# Launches whose last round is cut into half tiles: 149 row tiles x 256 columns (one tile cut), 13 x 16 tiles (60 cut); every row block
+# against a launch of its own, which has whole tiles.
+@pytest.mark.parametrize("fmt", FMTS + ["bf16"])
+@pytest.mark.parametrize("M,N,K", [(149 * 128 - 3, 256, 512), (1605, 4096, 1024)])
+def test_last_round_in_half_tiles(fmt, M, N, K):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(12)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    W = ops.QWeight(torch.randn(N, K, generator=g, device="cuda") * 0.05, fmt)
+    bias, gamma = torch.randn(N, generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda")
+    res = torch.randn(M, N, generator=g, device="cuda")
+
+    def launches(rows, r):
+        a = rows.contiguous()
+        if fmt != "bf16":
+            a = ops.ActBuf(rows.shape[0], K, fmt)
+            if fmt == "nv4":
+                a.ts.fill_(0.003)
+            ops.quant_rows(rows, a)
+        out = [ops.gemm_plain(a, W, bias, out_dtype=torch.float32), ops.gemm_res(a, W, bias, gamma, r.contiguous())]
+        if fmt != "bf16":
+            q = ops.ActBuf(rows.shape[0], N, "mx8")
+            out.append(ops.gemm_gelu_q(a, W, bias, q).q)
+        ops.check_device_error()
+        return out
+
+    big = launches(x, res)
+    for r0, r1 in ((0, 128), (M // 2, M // 2 + 200), (M - 130, M)):
+        for i, (u, v) in enumerate(zip(big, launches(x[r0:r1], res[r0:r1]))):
+            assert torch.equal(u[r0:r1], v), (r0, i)
