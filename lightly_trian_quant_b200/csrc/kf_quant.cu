@@ -194,8 +194,15 @@ __device__ __forceinline__ void amax_finish(float am, float factor, float* ts, u
 // |gelu(x)| with the exact-erf definition, in the form the framework's eager GELU evaluates
 __device__ __forceinline__ float gelu_abs(float x) { return fabsf(x * 0.5f * (1.0f + erff(x * 0.70710678118654752440f))); }
 
-// max |v| or max |gelu(v)| over a matrix.  |gelu(v)| <= |v|, so an element is evaluated only when |v| is above the thread's
-// maximum so far: a few per thread instead of all (the GELU of 20 M values would take longer than reading them).
+// max |v| or max |gelu(v)| over a matrix.  GELU rises for v >= 0 and stays within 0.17 of zero below, so of 32 values only the largest is
+// evaluated, and the negative ones only while nothing above 0.17 has been seen (the GELU of 20 M values takes longer than reading
+// them: 6420 x 3072 bf16 28 us with a test per value).  NaN and -Inf give NaN, as the eager GELU does.
+constexpr float GELU_NEG_MAX = 0.17f;                      // above |gelu(-0.7518)| = 0.16997
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float y;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
 template <typename T, bool GELU>
 __global__ void __launch_bounds__(256) amax_scale_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, int wide, float factor, float* __restrict__ ts,
                                                          uint32_t* __restrict__ ws) {
@@ -207,14 +214,22 @@ __global__ void __launch_bounds__(256) amax_scale_kernel(const T* __restrict__ x
     float v[32];
     load32<T>(x + (int64_t)row * ldx + c * 32, wide != 0, v);
     if (GELU) {
-      // the piece's largest value first: most others then fail the test
-      float top = v[0];
+      float top = v[0], low = v[0];
 #pragma unroll
-      for (int j = 1; j < 32; ++j) top = fmaxf(top, v[j]);
-      if (!(fabsf(top) <= am)) am = amax_nan(am, gelu_abs(top));
+      for (int j = 0; j < 32; j += 2) {
+        top = max3(top, v[j], v[j + 1]);
+        low = min3(low, v[j], v[j + 1]);
+      }
+      if (!(low >= -3.402823466e38f)) {
+        am = __int_as_float(0x7fc00000);
+      } else {
+        if (top > am) am = fmaxf(am, gelu_abs(top));
+        if (am < GELU_NEG_MAX && -low > am) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (!(fabsf(v[j]) <= am)) am = amax_nan(am, gelu_abs(v[j]));
+          for (int j = 0; j < 32; ++j)
+            if (-v[j] > am) am = fmaxf(am, gelu_abs(v[j]));
+        }
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < 32; j += 2) am = max3(am, fabsf(v[j]), fabsf(v[j + 1]));
