@@ -44,6 +44,8 @@ extern "C" {
 #define KF_Q_GELU 1        /* x <- gelu_erf(x + bias[col]) before quantising                         */
 #define KF_Q_ROUND_BF16 2  /* round the (LN / GELU) value to bf16 before quantising                  */
 #define KF_Q_RECIP_DIV 4   /* amax/448, amax/6 as multiply by the fp32 reciprocal (torch-on-CUDA rule) */
+#define KF_Q_STATIC_AFFINE 1024 /* kf_ln_quant: no kernel of this library still running on the stream writes w or b (parameters
+                                  laid out once): under dependent launch they may be read before the predecessor is done */
 #define KF_Q_IN_BF16 256   /* kf_ln_quant only: x points to bf16 values                              */
 #define KF_Q_FAST_NV4 64   /* QUANT epilogue to nv4 only: block scale and element division through approximate
                               reciprocals instead of the IEEE divisions of the bit specification (opt-in; a code moves

@@ -16,7 +16,7 @@ HEADERS = sorted((PKG.parent / "include").glob("*.h"))
 
 KF_FMT = {"mx8": 0, "nv4": 1, "mx4": 2, "bf16": 3}
 KF_DT = {"f32": 0, "bf16": 1, "f16": 2}
-KF_Q_GELU, KF_Q_ROUND_BF16, KF_Q_RECIP_DIV, KF_Q_FAST_NV4 = 1, 2, 4, 64
+KF_Q_GELU, KF_Q_ROUND_BF16, KF_Q_RECIP_DIV, KF_Q_FAST_NV4, KF_Q_STATIC_AFFINE = 1, 2, 4, 64, 1024
 
 KF_EPI = {"plain": 0, "res": 1, "rope": 2, "quant": 3}
 KF_G_GELU, KF_G_ROUND_BF16, KF_G_PRE_ROUND_BF16, KF_G_ROPE_HALF = 8, 16, 32, 128

@@ -357,6 +357,12 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI
     fence_mbar_init();
   }
   __syncthreads();
+  constexpr bool BLK16 = FMT == KF_FMT_NV4 && NV == 4;   // d = 1024 in NVFP4: a lane owns whole 16-value blocks
+  constexpr int LAY = BLK16 ? LAY_BLK16 : LAY_SWAP;
+  float ww[NV][8], bb[NV][8];
+  // the affine parameters of a model are no predecessor's output: their L2 round trip runs under the predecessor's end
+  const bool early = (flags & KF_Q_STATIC_AFFINE) != 0;
+  if (early) ln_affine_load<NV, LAY>(w, b, lane, ww, bb);
   pdl_wait();                                     // from here on global memory of the predecessors is read and written
   const WaitCtx ctx{abort_flag, err};
   const int W = gridDim.x * 4, gw = blockIdx.x * 4 + warp;
@@ -369,10 +375,7 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI
   };
   if (lane == 0)
     for (int k = 0; k < LNQ_RING; ++k) issue(k);
-  constexpr bool BLK16 = FMT == KF_FMT_NV4 && NV == 4;   // d = 1024 in NVFP4: a lane owns whole 16-value blocks
-  constexpr int LAY = BLK16 ? LAY_BLK16 : LAY_SWAP;
-  float ww[NV][8], bb[NV][8];
-  ln_affine_load<NV, LAY>(w, b, lane, ww, bb);
+  if (!early) ln_affine_load<NV, LAY>(w, b, lane, ww, bb);
   const Nv4Scale ts = nv4_scale(FMT == KF_FMT_NV4 ? __ldg(ts_ptr) : 1.f);
   const bool div_true = !(flags & KF_Q_RECIP_DIV);
   const bool rb = flags & KF_Q_ROUND_BF16;

@@ -93,7 +93,7 @@ class _Feeder:
             buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "ln")
             if ws is not None:
                 ops.ln_amax_scale(src, self.w, self.b, self.eps, buf.ts, ws)
-            ops.ln_quant(src, self.w, self.b, self.eps, buf, round_bf16=True)
+            ops.ln_quant(src, self.w, self.b, self.eps, buf, round_bf16=True, static_affine=True)
         else:
             src = _rows(x)
             buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "gelu")

@@ -145,11 +145,12 @@ def quantx(x: torch.Tensor, out: ActBuf, **kw) -> ActBuf:
 
 
 def ln_quant(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, out: ActBuf, *, round_bf16: bool = False,
-             recip_div: bool = False, y_dbg: Optional[torch.Tensor] = None) -> ActBuf:
-    """LayerNorm of the fp32 (or bf16) stream x [..., d] fused with quantisation into out (ln_mx8 / lnq)."""
+             recip_div: bool = False, y_dbg: Optional[torch.Tensor] = None, static_affine: bool = False) -> ActBuf:
+    """LayerNorm of the fp32 (or bf16) stream x [..., d] fused with quantisation into out (ln_mx8 / lnq).
+    static_affine=True promises that w and b are parameters, not the output of an operator in flight."""
     global LAUNCHES
     LAUNCHES += 1
-    args = (x, w, b, eps, out, _flags(False, round_bf16, recip_div), y_dbg)
+    args = (x, w, b, eps, out, _flags(False, round_bf16, recip_div) | (_lib.KF_Q_STATIC_AFFINE if static_affine else 0), y_dbg)
     if TIMING is None:
         return _h.ln_quant(*args)
     return _timed("ln_quant", _h.ln_quant, args, x.numel() * x.element_size() + out.q.numel() + out.sf.numel())

@@ -129,7 +129,7 @@ def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, cali
     if cal and nv4:
         set_ts(L.ts_ln1, ops.ln_rows(x, L.ln1_w, L.ln1_b, L.ln1_eps, BF))
     a, a2, a3, f = L.operands(M, x.device)
-    ops.ln_quant(x, L.ln1_w, L.ln1_b, L.ln1_eps, a, round_bf16=round_bf16)
+    ops.ln_quant(x, L.ln1_w, L.ln1_b, L.ln1_eps, a, round_bf16=round_bf16, static_affine=True)
     qkv = ops.qkv_rope(a, L.qkv, L.bqkv, sin, cos, N, prefix, heads, out_dtype=attn_dtype, half_tables=half_tables)
     # ---- attention with its output quantised in the epilogue -> proj (gamma + residual, in place on the stream)
     if cal and nv4:
@@ -139,7 +139,7 @@ def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, cali
     # ---- LN2 + quant -> fc1 (GELU + quantise-out) -> fc2 (gamma + residual)
     if cal and nv4:
         set_ts(L.ts_ln2, ops.ln_rows(x, L.ln2_w, L.ln2_b, L.ln2_eps, BF))
-    ops.ln_quant(x, L.ln2_w, L.ln2_b, L.ln2_eps, a3, round_bf16=round_bf16)
+    ops.ln_quant(x, L.ln2_w, L.ln2_b, L.ln2_eps, a3, round_bf16=round_bf16, static_affine=True)
     if cal and nv4:
         set_ts(L.ts_g, ops.gemm_plain(a3, L.fc1, L.b1, gelu=True))
     ops.gemm_gelu_q(a3, L.fc1, L.b1, f, round_bf16=round_bf16)
