@@ -105,6 +105,37 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int out_dtype) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// Stores the warp's 32 rows of 128 bytes (lane = row, w = its four 32-byte pieces) as whole lines: inside every four lanes the pieces are
+// transposed (4 x 4), then a store instruction covers eight rows of 128 bytes instead of 32 pieces of 32 bytes in 32 lines, whose
+// look-ups had L1 71 % busy in the ROPE epilogue, the unit the operand ring fills through (qkv NVFP4 M = 22 470: 66 -> 60 us, MXFP8
+// x 768 55 -> 52 us).  The same for PLAIN (435 -> 449 us, instruction-bound) and for the residual of RES (level) did not pay.
+// base: the 128 bytes of row 0; rows from `rows` on are not written.
+__device__ __forceinline__ void store_rows128(uint32_t (&w)[32], uint8_t* base, size_t row_bytes, int rows, int lane) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {                  // -> w[8 * (2j + e)]: piece 2j + b0 of row e of the lane's pair
+      const uint32_t a = w[16 * j + q], b = w[16 * j + 8 + q];
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, b0 ? a : b, 1);
+      w[16 * j + q] = b0 ? got : a;
+      w[16 * j + 8 + q] = b0 ? b : got;
+    }
+#pragma unroll
+  for (int e = 0; e < 2; ++e)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {                  // -> w[8 * k]: piece 2 * b1 + b0 of row k of the lane's four
+      const uint32_t a = w[8 * e + q], b = w[16 + 8 * e + q];
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, b1 ? a : b, 2);
+      w[8 * e + q] = b1 ? got : a;
+      w[16 + 8 * e + q] = b1 ? b : got;
+    }
+  const int row0 = lane & ~3;
+  uint8_t* p = base + (size_t)row0 * row_bytes + (lane & 3) * 32;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (row0 + k < rows) stg8w(p + k * row_bytes, &w[8 * k]);
+}
 // ------------------------------------------------------------------------------------------------ QUANT
 // QUANT epilogue of one 32-column chunk: the thread owns columns n0..n0+31 of row m = two nv4 blocks or one mx block, so
 // block maxima need no shuffles and the per-block scale arithmetic is paid once per 16 / 32 values.
@@ -276,16 +307,16 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
     // output: first half of r = first, second half = second columns of the rotation pairs, so the rotary embedding needs no data exchange:
     //   lo' = lo*cos_lo - hi*sin_lo (tables of columns 0..31), hi' = hi*cos_hi + lo*sin_hi (tables of columns 32..63).
     // With KF_G_ROPE_HALF the table row of every token of the warp's quarter is already in shared memory (rope_slab_*).
-    if (m >= g.M) return;
+    if (W == 32 && m >= g.M) return;            // W = 64: all lanes take part in the stores
     const int which = n0 / g.d, h = (n0 - which * g.d) >> 6;
     const int b = m / g.Ntok, t = m - b * g.Ntok;
     const int nbatch = g.M / g.Ntok;
-    const bool rot = which < 2 && t >= g.prefix;
+    const bool rot = which < 2 && t >= g.prefix && m < g.M;
     const float* sn = g.sin + (size_t)(rot ? t - g.prefix : 0) * 64;
     const float* cs = g.cos + (size_t)(rot ? t - g.prefix : 0) * 64;
     const float* srow = slab + lane * 64;
     uint8_t* dst = static_cast<uint8_t*>(g.C) + ((((size_t)which * nbatch + b) * g.Ntok + t) * g.H + h) * 128;
-    uint32_t wlo[8], whi[8];                    // 16 output columns of each half: stored as soon as they are complete
+    uint32_t wo[W == 64 ? 32 : 16];             // packed output: the columns of the first half, then those of the second
     const float2 ts2 = splat2(ts);
 #pragma unroll
     for (int c = 0; c < W / 8; ++c) {           // 4 rotation pairs at a time (few values live: the thread already holds W accumulators)
@@ -318,13 +349,15 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
       }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        wlo[2 * (c & 3) + e] = pack2(ol[e].x, ol[e].y, g.out_dtype);
-        whi[2 * (c & 3) + e] = pack2(oh[e].x, oh[e].y, g.out_dtype);
+        wo[2 * c + e] = pack2(ol[e].x, ol[e].y, g.out_dtype);
+        wo[W / 4 + 2 * c + e] = pack2(oh[e].x, oh[e].y, g.out_dtype);
       }
-      if ((c & 3) == 3) {
-        stg8w(dst + 2 * j0 + 32 * (c >> 2), wlo);
-        stg8w(dst + 64 + 2 * j0 + 32 * (c >> 2), whi);
-      }
+    }
+    if constexpr (W == 64) {                    // rows of the output are [token, head] rows: row m of a third of q / k / v is b * Ntok + t = m
+      store_rows128(wo, static_cast<uint8_t*>(g.C) + (((size_t)which * g.M + rbase) * g.H + h) * 128, (size_t)g.H * 128, g.M - rbase, lane);
+    } else {
+      stg8w(dst + 2 * j0, wo);
+      stg8w(dst + 64 + 2 * j0, wo + 8);
     }
   } else if (EPI == KF_EPI_RES) {
     // out = R + gamma * (acc*ts + bias) on the thread's 256 (or 128) contiguous bytes of the fp32 residual row: 32-byte pieces,
