@@ -167,68 +167,41 @@ __device__ __forceinline__ float quant_values16(const GemmArgs& g, const uint32_
   return am;
 }
 
-// o: the chunk's codes (four words of nibbles, eight of bytes), returned: its scale bytes (nv4 two, else one), block 0 lowest.
-__device__ __forceinline__ uint32_t quant_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, const Nv4Scale& sco /* per-tensor scale of an nv4 output */, int m, int n0,
-                                                const float* bsm /* the chunk's 32 bias values in shared memory */, uint32_t* o) {
+__device__ __forceinline__ void quant_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, const Nv4Scale& sco /* per-tensor scale of an nv4 output */, int m, int n0,
+                                            const float* bsm /* the chunk's 32 bias values in shared memory */) {
   const bool div_true = !(g.flags & KF_Q_RECIP_DIV);
-  float* dbg = (g.y_dbg != nullptr && m < g.M) ? g.y_dbg + (size_t)m * g.N + n0 : nullptr;
+  const bool ok = m < g.M;
+  float* dbg = (g.y_dbg != nullptr && ok) ? g.y_dbg + (size_t)m * g.N + n0 : nullptr;
   int by0, by1;
-  float va[16], vb[16];
-  const float am0 = quant_values16(g, r, 0, ts, bsm, dbg, va), am1 = quant_values16(g, r, 1, ts, bsm, dbg, vb);
   if (g.out_fmt == KF_FMT_NV4) {
+    uint32_t o[4];
+    float va[16], vb[16];
+    const float am0 = quant_values16(g, r, 0, ts, bsm, dbg, va), am1 = quant_values16(g, r, 1, ts, bsm, dbg, vb);
     if (g.flags & KF_Q_FAST_NV4) {
       quant_nv4_fast<16>(va, am0, sco.ts, sco.rcp_ts, o, by0);
       quant_nv4_fast<16>(vb, am1, sco.ts, sco.rcp_ts, o + 2, by1);
     } else {
       quant_nv4_pair16(va, am0, vb, am1, sco, div_true, o, by0, by1);
     }
-    return (uint32_t)(by0 | (by1 << 8));
+    if (ok) *reinterpret_cast<uint4*>(g.Qo + (size_t)m * (g.N >> 1) + (n0 >> 1)) = make_uint4(o[0], o[1], o[2], o[3]);
+    // two scale bytes of this row for the chunk (rows beyond M inside the last tile get zeros)
+    *reinterpret_cast<uint16_t*>(g.SFo + sf_offset(m, n0 >> 4, g.N >> 6)) = ok ? (uint16_t)(by0 | (by1 << 8)) : (uint16_t)0;
+    return;
   }
-  const float am = amax_nan(am0, am1);
+  float va[16], vb[16];
+  const float am = amax_nan(quant_values16(g, r, 0, ts, bsm, dbg, va), quant_values16(g, r, 1, ts, bsm, dbg, vb));
   if (g.out_fmt == KF_FMT_MX8) {
+    uint32_t o[8];
     quant_mx8<16>(va, am, div_true, o, by0);
     quant_mx8<16>(vb, am, div_true, o + 4, by0);
+    if (ok) stg8w(g.Qo + (size_t)m * g.N + n0, o);
+    g.SFo[sf_offset(m, n0 >> 5, g.N >> 7)] = ok ? (uint8_t)by0 : (uint8_t)0;
   } else {
+    uint32_t o[4];
     quant_mx4<16>(va, am, div_true, o, by0);
     quant_mx4<16>(vb, am, div_true, o + 2, by0);
-  }
-  return (uint32_t)by0;
-}
-
-// The W columns of a thread: codes in whole 32-byte sectors and the scale bytes of 64 columns together (W = 64), rows beyond M inside the
-// last tile get zero scale bytes.
-template <int W>
-__device__ __forceinline__ void quant_columns(const GemmArgs& g, const uint32_t (&r)[W], float ts, const Nv4Scale& sco, int m, int n0, const float* bsm) {
-  const bool ok = m < g.M;
-  uint32_t by = 0;
-  if (g.out_fmt == KF_FMT_MX8) {
-#pragma unroll
-    for (int c = 0; c < W; c += 32) {
-      uint32_t o[8];
-      by |= quant_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, sco, m, n0 + c, bsm + c, o) << (c / 4);
-      if (ok) stg8w(g.Qo + (size_t)m * g.N + n0 + c, o);
-    }
-  } else {
-    uint32_t o[W / 8];
-#pragma unroll
-    for (int c = 0; c < W; c += 32)
-      by |= quant_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, sco, m, n0 + c, bsm + c, o + c / 8) << (g.out_fmt == KF_FMT_NV4 ? c / 2 : c / 4);
-    uint8_t* q = g.Qo + (size_t)m * (g.N >> 1) + (n0 >> 1);
-    if constexpr (W == 64) {
-      if (ok) stg8w(q, o);
-    } else {
-      if (ok) *reinterpret_cast<uint4*>(q) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-  }
-  if (!ok) by = 0;
-  if (g.out_fmt == KF_FMT_NV4) {
-    uint8_t* p = g.SFo + sf_offset(m, n0 >> 4, g.N >> 6);
-    if (W == 64) *reinterpret_cast<uint32_t*>(p) = by;
-    else *reinterpret_cast<uint16_t*>(p) = (uint16_t)by;
-  } else {
-    uint8_t* p = g.SFo + sf_offset(m, n0 >> 5, g.N >> 7);
-    if (W == 64) *reinterpret_cast<uint16_t*>(p) = (uint16_t)by;
-    else *p = (uint8_t)by;
+    if (ok) *reinterpret_cast<uint4*>(g.Qo + (size_t)m * (g.N >> 1) + (n0 >> 1)) = make_uint4(o[0], o[1], o[2], o[3]);
+    g.SFo[sf_offset(m, n0 >> 5, g.N >> 7)] = ok ? (uint8_t)by0 : (uint8_t)0;
   }
 }
 
@@ -422,7 +395,8 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
 #pragma unroll
     for (int c = 0; c < W; c += 32) plain_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, dst_row, n0 + c, slice + c);
   } else {   // KF_EPI_QUANT: gelu(acc*ts + bias) -> codes + blocked scales of format out_fmt
-    quant_columns<W>(g, r, ts, sco, m, n0, slice);
+#pragma unroll
+    for (int c = 0; c < W; c += 32) quant_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, sco, m, n0 + c, slice + c);
   }
 }
 
