@@ -78,13 +78,6 @@ __device__ __forceinline__ F8 ldg8_stream(const float* p) {   // 32-byte aligned
                : "l"(p));
   return r;
 }
-__device__ __forceinline__ F8 ldg8_nc(const float* p) {       // read-only data shared by several warps (rotary tables)
-  F8 r;
-  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
-               : "l"(p));
-  return r;
-}
 __device__ __forceinline__ float4 ldg4_nc(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ void stg8(void* p, float a, float b, float c, float d, float e, float f, float g, float h) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h)
