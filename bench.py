@@ -177,7 +177,7 @@ def main():
 
     from lightly_trian_quant_b200 import modeldef, ops, sharding, stack
 
-    ops.set_pdl(args.pdl)
+    ops.set_pdl(True if args.pdl else None)
     cfg = modeldef.VIT_L if args.arch == "vit_l" else modeldef.VIT_B
     size = args.size
     if size != SIZE and "+s" not in args.variant:

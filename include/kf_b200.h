@@ -249,10 +249,14 @@ KF_API int kf_tensor_peak_probe(int fmt, int n, int iters, int sf_copies, double
 KF_API int kf_attn_fwd_quant(int dtype, const void* qkv, int B, int N, int H, float pre, int out_fmt, void* Qo, void* SFo,
                              const float* tso, int flags, void* stream);
 
-/* Programmatic dependent launch: 1 = every launch, 0 (default) = launches over few rows, where it is the faster form (kf_api.cu).
- * Results are the same either way.
+/* Programmatic dependent launch, process-wide: KF_PDL_OFF = plain stream order, KF_PDL_ALL (and any other non-zero value) = every
+ * launch, KF_PDL_AUTO (the state before the first call) = launches over few rows, where it is the faster form (kf_api.cu).
+ * Results are the same in all three.
  * Counterpart: set_pdl(bool) (infer-opt/round13_mxfp8_full/impl/mx13.cu:282). */
-KF_API int kf_set_pdl(int on);
+#define KF_PDL_OFF 0
+#define KF_PDL_ALL 1
+#define KF_PDL_AUTO (-1)
+KF_API int kf_set_pdl(int mode);
 
 /* Reads (and clears) the device error word that kernels with bounded waits write when a wait runs out.
  * Synchronises the device.  Returns KF_OK, or KF_ERR_DEVICE_WAIT with where/block in the error string.

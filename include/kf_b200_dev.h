@@ -22,6 +22,9 @@ KF_API int kf_fill_rate_probe(const void* src, long long span, int stage_bytes, 
  * No reference counterpart. */
 KF_API int kf_selftest_rcp(int exponent, unsigned int* mismatches, void* stream);
 
+/* 1 when a launch over this many rows on this stream would use programmatic dependent launch (kf_set_pdl), else 0. */
+KF_API int kf_pdl_choice(int64_t rows, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

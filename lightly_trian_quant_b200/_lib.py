@@ -18,6 +18,7 @@ KF_FMT = {"mx8": 0, "nv4": 1, "mx4": 2, "bf16": 3}
 KF_DT = {"f32": 0, "bf16": 1, "f16": 2}
 KF_Q_GELU, KF_Q_ROUND_BF16, KF_Q_RECIP_DIV, KF_Q_FAST_NV4, KF_Q_STATIC_AFFINE = 1, 2, 4, 64, 1024
 
+KF_PDL = {"off": 0, "all": 1, "auto": -1}
 KF_EPI = {"plain": 0, "res": 1, "rope": 2, "quant": 3}
 KF_G_GELU, KF_G_ROUND_BF16, KF_G_PRE_ROUND_BF16, KF_G_ROPE_HALF = 8, 16, 32, 128
 
@@ -63,6 +64,8 @@ def lib() -> C.CDLL:
             "kf_ln_amax_scale": [i32, vp, vp, vp, f32, i32, i32, f32, vp, vp, vp],
             "kf_ln_rows": [vp, vp, vp, f32, i32, i32, i32, vp, vp],
             "kf_gemm_bs": [C.POINTER(GemmParams), vp],
+            "kf_set_pdl": [i32],
+            "kf_pdl_choice": [i64, vp],
             "kf_check_device_error": [],
             "kf_attn_fwd": [i32, vp, vp, i32, i32, i32, f32, vp],
             "kf_tensor_peak_probe": [i32, i32, i32, i32, C.POINTER(C.c_double), vp],

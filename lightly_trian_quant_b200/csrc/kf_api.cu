@@ -1,7 +1,9 @@
 // Status plumbing of the C-ABI: thread-local last-error text, CUDA error mapping, version, scale-tensor sizes.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
+#include "../../include/kf_b200_dev.h"
 #include "kf_sm100.cuh"
 
 namespace kf {
@@ -25,9 +27,11 @@ int cuda_status(cudaError_t e, const char* what) {
 // tensor-memory set-up) then runs under its predecessor.  Measured, whole models, plain -> dependent: ViT-B 256 px called eagerly
 // 782 -> 635 us, ViT-L 640 px one frame captured 1950 -> 1883 us; ViT-B 640 px eager, three images, 2298 -> 2052 us (launch gaps
 // of the eager stream); captured graphs of 3210 rows are level and of 6420 rows and more 1 to 2 % slower, hence the two lines.
-static bool g_pdl = false;                            // kf_set_pdl(1): every launch
+static std::atomic<int> g_pdl{KF_PDL_AUTO};            // kf_set_pdl
 bool pdl_for(int64_t rows, cudaStream_t st) {
-  if (g_pdl || rows <= 2048) return true;
+  const int mode = g_pdl.load(std::memory_order_relaxed);
+  if (mode != KF_PDL_AUTO) return mode == KF_PDL_ALL;
+  if (rows <= 2048) return true;
   if (rows > 20480) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
@@ -61,10 +65,12 @@ extern "C" int kf_check_device_error(void) {
   return KF_ERR_DEVICE_WAIT;
 }
 
-extern "C" int kf_set_pdl(int on) {
-  kf::g_pdl = on != 0;
+extern "C" int kf_set_pdl(int mode) {
+  kf::g_pdl.store(mode == KF_PDL_AUTO || mode == KF_PDL_OFF ? mode : KF_PDL_ALL, std::memory_order_relaxed);
   return KF_OK;
 }
+
+extern "C" int kf_pdl_choice(int64_t rows, void* stream) { return kf::pdl_for(rows, static_cast<cudaStream_t>(stream)) ? 1 : 0; }
 
 extern "C" const char* kf_version(void) { return "kf_b200 0.1 sm_100a"; }
 

@@ -193,10 +193,10 @@ def ln_amax_scale(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float,
 
 
 # ------------------------------------------------------------------------------------------------ weights and GEMMs
-def set_pdl(on: bool) -> None:
-    """Programmatic dependent launch: True = every launch, False (default) = launches over few rows; results are the same either way.
-    Counterpart: set_pdl (infer-opt/round13_mxfp8_full/impl/mx13.cu:282)."""
-    check(_lib.lib().kf_set_pdl(1 if on else 0), "kf_set_pdl")
+def set_pdl(on: Optional[bool]) -> None:
+    """Programmatic dependent launch: True = every launch, False = none (plain stream order), None = launches over few rows, which is how
+    the package starts; results are the same in all three.  Counterpart: set_pdl (infer-opt/round13_mxfp8_full/impl/mx13.cu:282)."""
+    check(_lib.lib().kf_set_pdl(_lib.KF_PDL["auto" if on is None else "all" if on else "off"]), "kf_set_pdl")
 
 
 def check_device_error() -> None:

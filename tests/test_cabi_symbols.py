@@ -59,6 +59,25 @@ def test_set_pdl_switch(built_lib):
     ops.set_pdl(False)
 
 
+def test_dependent_launch_modes(built_lib):
+    """False means plain stream order for every size, True dependent launch for every size, None the choice by rows."""
+    from lightly_trian_quant_b200 import _lib, ops
+
+    L = _lib.lib()
+    choices = lambda: [L.kf_pdl_choice(rows, None) for rows in (1, 2048, 1 << 20)]  # noqa: E731
+    try:
+        ops.set_pdl(None)
+        assert choices() == [1, 1, 0]
+        ops.set_pdl(False)
+        assert choices() == [0, 0, 0]
+        ops.set_pdl(True)
+        assert choices() == [1, 1, 1]
+        ops.set_pdl(None)
+        assert choices() == [1, 1, 0]
+    finally:
+        ops.set_pdl(None)
+
+
 def test_gemm_params_mirror_matches_the_header(built_lib, tmp_path):
     """the ctypes mirror of kf_gemm_params has the size and the field offsets the C compiler gives the header's struct."""
     import ctypes as C
