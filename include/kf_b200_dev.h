@@ -22,6 +22,10 @@ KF_API int kf_fill_rate_probe(const void* src, long long span, int stage_bytes, 
  * No reference counterpart. */
 KF_API int kf_selftest_rcp(int exponent, unsigned int* mismatches, void* stream);
 
+/* Self-test of the failure path: a one-thread launch that lets its successor start under dependent launch, waits delay_us (0..1000)
+ * and sets the device error word the way a bounded wait that ran out does (kf_check_device_error).  No reference counterpart. */
+KF_API int kf_selftest_raise_error(int delay_us, void* stream);
+
 /* 1 when a launch over this many rows on this stream would use programmatic dependent launch (kf_set_pdl), else 0. */
 KF_API int kf_pdl_choice(int64_t rows, void* stream);
 

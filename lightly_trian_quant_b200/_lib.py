@@ -66,6 +66,7 @@ def lib() -> C.CDLL:
             "kf_gemm_bs": [C.POINTER(GemmParams), vp],
             "kf_set_pdl": [i32],
             "kf_pdl_choice": [i64, vp],
+            "kf_selftest_raise_error": [i32, vp],
             "kf_check_device_error": [],
             "kf_attn_fwd": [i32, vp, vp, i32, i32, i32, f32, vp],
             "kf_tensor_peak_probe": [i32, i32, i32, i32, C.POINTER(C.c_double), vp],

@@ -50,7 +50,22 @@ unsigned int* dev_error_ptr() {
   return static_cast<unsigned int*>(p);
 }
 
+// A launch that lets its successor start, takes delay_us and then fails: the error word as a bounded wait that ran out leaves it.
+__global__ void raise_error_kernel(unsigned int* err, int delay_us) {
+  pdl_launch_dependents();
+  for (int i = 0; i < delay_us; ++i) __nanosleep(1000);
+  if (atomicCAS(&err[0], 0u, (unsigned)(-KF_ERR_DEVICE_WAIT)) == 0u) err[1] = 200;
+}
+
 }  // namespace kf
+
+extern "C" int kf_selftest_raise_error(int delay_us, void* stream) {
+  KF_REQUIRE(delay_us >= 0 && delay_us <= 1000, "kf_selftest_raise_error: delay of %d us", delay_us);
+  unsigned int* err = kf::dev_error_ptr();
+  KF_REQUIRE(err != nullptr, "kf_selftest_raise_error: device error word unavailable");
+  kf::raise_error_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(err, delay_us);
+  return kf::cuda_status(cudaGetLastError(), "kf_selftest_raise_error launch");
+}
 
 extern "C" int kf_check_device_error(void) {
   cudaError_t e = cudaDeviceSynchronize();

@@ -152,7 +152,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&p_full[i], 128);
       mbar_init(&o_full[i], 1);                           // PV(G) completes o_full[G % 3]: a waiter is never more than one phase behind
     }
-    *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;   // the swizzled tiles need a 1024-byte aligned base
+    *abort_flag = 0u;
     fence_mbar_init();
   }
   if (warp == 5) {
@@ -165,8 +165,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   pdl_wait();                                            // set-up done: from here on global memory of the predecessors is read and written
   const uint32_t tmem_base = *tmem_holder;
   const WaitCtx ctx{abort_flag, a.err};
-  const bool bad_align = *abort_flag != 0 || a.err[0] != 0;   // misaligned tiles, or an earlier CTA / launch already failed: skip the work
-  if (*abort_flag != 0 && threadIdx.x == 0 && atomicCAS(&a.err[0], 0u, 99u) == 0u) {
+  const bool bad_align = (smem_u32(smem) & 1023u) != 0;  // the swizzled tiles need a 1024-byte aligned base; the same answer in every thread
+  if (bad_align && threadIdx.x == 0 && atomicCAS(&a.err[0], 0u, 99u) == 0u) {
     a.err[1] = 100;
     a.err[2] = blockIdx.x;
   }
@@ -183,7 +183,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       prefetch_tmap(&tmV);
     }
     uint32_t G = 0;
-    bool ok = true;
+    // Has an earlier launch failed?  The producer alone looks, once: without its loads the other roles' waits end with the abort flag.
+    bool ok = !__any_sync(0xffffffffu, *static_cast<volatile unsigned int*>(a.err) != 0u);
+    if (!ok) *abort_flag = 1u;
     for (int it = 0; it < n_my && ok; ++it) {
       const Item I = item_of(it);
       const int qb = it & 1;

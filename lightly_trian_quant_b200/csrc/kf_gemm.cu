@@ -99,7 +99,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
     if (EPI == KF_EPI_RES && BN == 128)
       for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&box_full[w], 1);
-    *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;     // the swizzled operand tiles need a 1024-byte aligned base
+    *abort_flag = 0u;
     fence_mbar_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmW);
@@ -116,8 +116,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (warp != 0 || !w_early) pdl_wait();
   const uint32_t tmem_base = *tmem_holder;
   const WaitCtx ctx{abort_flag, g.err};
-  const bool bad_align = *abort_flag != 0 || g.err[0] != 0;   // misaligned tiles, or an earlier CTA / launch already failed: skip the work
-  if (*abort_flag != 0 && threadIdx.x == 0 && atomicCAS(&g.err[0], 0u, (unsigned)(-KF_ERR_DEVICE_WAIT)) == 0u) {
+  const bool bad_align = (smem_u32(smem) & 1023u) != 0;   // the swizzled operand tiles need a 1024-byte aligned base; the same answer in every thread
+  if (bad_align && threadIdx.x == 0 && atomicCAS(&g.err[0], 0u, (unsigned)(-KF_ERR_DEVICE_WAIT)) == 0u) {
     g.err[1] = 100;
     g.err[2] = blockIdx.x;
   }
@@ -129,7 +129,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     } else if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       uint32_t s = 0, ph = 0;
-      bool ok = true;
+      // Has an earlier launch failed?  The producer alone looks, once, before it requests anything: without its loads no barrier of the
+      // other roles completes and the abort flag ends their waits.  A look of every warp at a word that another launch may write
+      // in between would let some roles run and others not.
+      bool ok = !__any_sync(0xffffffffu, *static_cast<volatile unsigned int*>(g.err) != 0u);
+      if (!ok) {
+        *abort_flag = 1u;
+        if (w_early) pdl_wait();
+      }
       // Weights that no running predecessor writes (KF_G_W_STATIC): the W part of the first tile's stages is requested before the
       // wait for the predecessor, so its way from HBM runs under the predecessor's end.
       int early = 0;

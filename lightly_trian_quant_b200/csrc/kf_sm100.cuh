@@ -69,7 +69,7 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// Waits for the phase with the given parity.  Never spins forever: after about two seconds (or when another role of
+// Waits for the phase with the given parity (a completed phase passes also when the abort flag is up).  Never spins forever: after about two seconds (or when another role of
 // this CTA has already given up) it records where it stopped in the error word, raises the CTA-wide abort flag and
 // returns false; callers then skip their remaining work and fall through to the common teardown.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, uint32_t where) {

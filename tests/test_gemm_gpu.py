@@ -393,3 +393,45 @@ def test_last_round_in_half_tiles(fmt, M, N, K):
     for r0, r1 in ((0, 128), (M // 2, M // 2 + 200), (M - 130, M)):
         for i, (u, v) in enumerate(zip(big, launches(x[r0:r1], res[r0:r1]))):
             assert torch.equal(u[r0:r1], v), (r0, i)
+
+
+# the error word is already set when the kernel starts (delay 0), or is set by the predecessor while the kernel, started early under dependent
+# launch, has requested its weights (delay 200 us); 16 operand stages are more than the ring holds, one stage is less; 9600 rows take the residual through shared memory
+@pytest.mark.parametrize("delay", [0, 200])
+@pytest.mark.parametrize("M,K", [(320, 256), (320, 4096), (9600, 256)])
+def test_a_failed_predecessor_does_not_stall_the_launch(M, K, delay):
+    """every role of the GEMM and attention kernels comes to the same decision when an earlier launch has failed: the launch ends well inside
+    the two seconds of a bounded wait, and the next one is whole again."""
+    import time
+
+    from lightly_trian_quant_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    N, H, Ntok = 768, 4, 160
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    a = ops.quant_rows(x, ops.ActBuf(M, K, "nv4"))
+    W = ops.QWeight(torch.randn(N, K, generator=g, device="cuda") * 0.02, "nv4")
+    bias = torch.randn(N, generator=g, device="cuda")
+    res = torch.randn(M, N, generator=g, device="cuda")
+    tab = torch.randn(2, Ntok, 64, generator=g, device="cuda")
+    out = ops.ActBuf(M, N, "nv4")
+    qkv = torch.randn(3, M // Ntok, Ntok, H, 64, generator=g, device="cuda").bfloat16()
+    calls = [
+        lambda: ops.gemm_plain(a, W, bias),
+        lambda: ops.gemm_res(a, W, bias, bias, res),
+        lambda: ops.qkv_rope(a, W, bias, tab[0], tab[1], Ntok, 0, H),
+        lambda: ops.gemm_gelu_q(a, W, bias, out).q.clone(),
+        lambda: ops.attn_fwd(qkv),
+    ]
+    ops.set_pdl(True)
+    for call in calls:
+        ref = call()
+        ops.check_device_error()
+        t0 = time.perf_counter()
+        _lib.check(_lib.lib().kf_selftest_raise_error(delay, torch.cuda.current_stream().cuda_stream), "kf_selftest_raise_error")
+        call()
+        with pytest.raises(_lib.KfError, match="wait site 200"):
+            ops.check_device_error()
+        assert time.perf_counter() - t0 < 1.0
+        assert torch.equal(call(), ref)
+        ops.check_device_error()
