@@ -44,8 +44,7 @@ extern "C" {
 #define KF_Q_GELU 1        /* x <- gelu_erf(x + bias[col]) before quantising                         */
 #define KF_Q_ROUND_BF16 2  /* round the (LN / GELU) value to bf16 before quantising                  */
 #define KF_Q_RECIP_DIV 4   /* amax/448, amax/6 as multiply by the fp32 reciprocal (torch-on-CUDA rule) */
-#define KF_Q_STATIC_AFFINE 1024 /* kf_ln_quant: no kernel of this library still running on the stream writes w or b (parameters
-                                  laid out once): under dependent launch they may be read before the predecessor is done */
+#define KF_Q_STATIC_AFFINE 1024 /* kf_ln_quant: the caller guarantees for w and b what KF_G_W_STATIC guarantees for W and SFW */
 #define KF_Q_IN_BF16 256   /* kf_ln_quant only: x points to bf16 values                              */
 #define KF_Q_FAST_NV4 64   /* QUANT epilogue to nv4 only: block scale and element division through approximate
                               reciprocals instead of the IEEE divisions of the bit specification (opt-in; a code moves
@@ -64,8 +63,10 @@ extern "C" {
 #define KF_G_ROPE_HALF 128 /* ROPE: the caller guarantees that columns 32..63 of sin / cos repeat columns 0..31 (the axial
                               tables of DINOv3 are the angle vector concatenated with itself); lets the kernel keep the table
                               rows of a tile in shared memory.  Without the flag both halves are read as given. */
-#define KF_G_W_STATIC 512  /* the caller guarantees that no kernel of this library still running on the stream writes W or SFW (weights
-                              laid out once): under dependent launch the kernel may read them before its predecessor is done */
+#define KF_G_W_STATIC 512  /* the caller guarantees that every write of W and SFW was complete and visible before the launch in front of
+                              this one on the stream began its work (the host has synchronised with it, or that launch itself ran
+                              behind it): under dependent launch the kernel reads them before that launch has ended, so the
+                              launch in front must not be the one that writes them */
 
 /* Library version and the SM architecture the kernels were built for ("sm_100a"). */
 KF_API const char* kf_version(void);

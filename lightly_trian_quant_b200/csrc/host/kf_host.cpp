@@ -22,7 +22,7 @@
 namespace {
 
 PyObject* g_error = nullptr;                                   // KfError
-PyObject *s_M, *s_N, *s_K, *s_fmt, *s_q, *s_sf, *s_ts;         // interned attribute names
+PyObject *s_M, *s_N, *s_K, *s_fmt, *s_q, *s_sf, *s_ts, *s_settled;         // interned attribute names
 PyObject* g_fmt_names[4];                                      // interned "mx8", "nv4", "mx4", "bf16": index = KF_FMT_*
 
 struct Failed {};                                              // a Python exception is set
@@ -92,7 +92,7 @@ int fmt_code(PyObject* name) {
 struct Operand {                                               // ActBuf or QWeight
   int fmt;
   int64_t rows, K;
-  const at::Tensor* q;
+  const at::Tensor *q, *sf;                                    // sf: null for bf16
   void *pq, *psf, *pts;
 };
 
@@ -103,7 +103,9 @@ Operand operand(PyObject* o, PyObject* rows_attr, const char* what) {
   r.fmt = fmt_code(attr(o, s_fmt));
   r.q = &cuda_tensor(attr(o, s_q), what);
   r.pq = r.q->data_ptr();
-  r.psf = opt_ptr(attr(o, s_sf), what);
+  PyObject* sf = attr(o, s_sf);
+  r.sf = sf == Py_None ? nullptr : &cuda_tensor(sf, what);
+  r.psf = r.sf ? r.sf->data_ptr() : nullptr;
   r.pts = opt_ptr(attr(o, s_ts), what);
   return r;
 }
@@ -146,8 +148,34 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
 }
 
 // ------------------------------------------------------------------------------------------------ GEMM
-// A weight container (ops.QWeight) holds codes that the row quantiser or torch wrote, or a copy of a bf16 tensor: kernels that signal
-// their successors only by ending, so KF_G_W_STATIC holds for every launch with one.  bmm_nt takes activations and does not claim it.
+// KF_G_W_STATIC lets the kernel read weights before the wait that makes the predecessor's writes visible, so it is claimed only for
+// weights whose writes the host has seen complete and that nothing has written since: `settled` is the sum of the version counters of q
+// and sf at that moment (ops.QWeight), None where the host did not wait.  torch counts its in-place writes, writable() those of
+// the operators here; an object without the attribute claims nothing.  bmm_nt takes activations and does not claim it either.
+bool weight_settled(PyObject* o, const at::Tensor& q, const at::Tensor* sf) {
+  PyObject* v = PyObject_GetAttr(o, s_settled);
+  if (!v) {
+    if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw Failed{};
+    PyErr_Clear();
+    return false;
+  }
+  const bool claimed = v != Py_None;
+  const long long seen = claimed ? PyLong_AsLongLong(v) : 0;
+  Py_DECREF(v);
+  if (seen == -1 && PyErr_Occurred()) throw Failed{};
+  if (!claimed || q.is_inference() || (sf && sf->is_inference())) return false;      // an inference tensor has no version counter
+  return (int64_t)q._version() + (sf ? (int64_t)sf->_version() : 0) == seen;
+}
+int w_static(PyObject* o, const Operand& W) { return weight_settled(o, *W.q, W.sf) ? KF_G_W_STATIC : 0; }
+
+// out is about to be written: counted as torch counts an in-place operation
+void writable(const at::Tensor& out) {
+  if (!out.is_inference()) out.unsafeGetTensorImpl()->bump_version();
+}
+void writable(const Operand& out) {
+  writable(*out.q);
+  if (out.sf) writable(*out.sf);
+}
 // A side, W side and the common fields; returns M
 int64_t gemm_fill(kf_gemm_params& p, PyObject* a, const Operand& W, int epi) {
   int64_t M;
@@ -186,7 +214,7 @@ PyObject* gemm_plain(PyObject* const* v) {
   const float* bias = f32_vec(v[2], W.rows, "bias");
   const int64_t M = gemm_fill(p, v[0], W, KF_EPI_PLAIN);
   p.bias = bias;
-  p.flags = (int)to_int(v[5]) | KF_G_W_STATIC;
+  p.flags = (int)to_int(v[5]) | w_static(v[1], W);
   if (v[3] == Py_None) {
     p.out_dtype = (int)to_int(v[4]);
     at::Tensor out = empty({M, W.rows}, dtype_of(p.out_dtype), W.q->device());
@@ -197,6 +225,7 @@ PyObject* gemm_plain(PyObject* const* v) {
   const at::Tensor& out = cuda_tensor(v[3], "out");
   p.out_dtype = dtype_code(out.scalar_type());
   p.C = out.data_ptr();
+  writable(out);
   gemm_run(p, "gemm_plain");
   return new_ref(v[3]);
 }
@@ -210,7 +239,7 @@ PyObject* gemm_res(PyObject* const* v) {
   const int64_t M = gemm_fill(p, v[0], W, KF_EPI_RES);
   p.bias = bias;
   p.gamma = gamma;
-  p.flags = KF_G_W_STATIC;
+  p.flags = w_static(v[1], W);
   p.R = f32_vec(v[4], M * W.rows, "res");
   p.out_dtype = KF_F32;
   if (v[5] == Py_None) {
@@ -232,6 +261,7 @@ PyObject* gemm_res(PyObject* const* v) {
     p.out_row_offset = offset;
   }
   p.C = out.data_ptr();
+  writable(out);
   gemm_run(p, "gemm_res");
   return new_ref(v[5]);
 }
@@ -256,7 +286,7 @@ PyObject* qkv_rope(PyObject* const* v) {
   p.prefix = (int)prefix;
   p.H = (int)H;
   p.out_dtype = (int)to_int(v[8]);
-  p.flags = (int)to_int(v[9]) | KF_G_W_STATIC;
+  p.flags = (int)to_int(v[9]) | w_static(v[1], W);
   at::Tensor out = empty({3, M / Ntok, Ntok, H, 64}, dtype_of(p.out_dtype), W.q->device());
   p.C = out.data_ptr();
   gemm_run(p, "qkv_rope");
@@ -279,7 +309,8 @@ PyObject* gemm_gelu_q(PyObject* const* v) {
   p.Qo = out.pq;
   p.SFo = out.psf;
   p.tso = static_cast<const float*>(out.pts);
-  p.flags = (int)to_int(v[4]) | KF_G_W_STATIC;
+  p.flags = (int)to_int(v[4]) | w_static(v[1], W);
+  writable(out);
   gemm_run(p, "gemm_gelu_q");
   return new_ref(v[3]);
 }
@@ -298,6 +329,7 @@ PyObject* bmm_nt(PyObject* const* v) {
     out = cuda_tensor(v[2], "out");
     if (out.dim() != 3 || out.size(0) != B || out.size(1) != Q || out.size(2) != P || out.scalar_type() != at::kBFloat16 || !out.is_contiguous())
       fail("bmm_nt: out must be contiguous bf16 [%lld, %lld, %lld]", (long long)B, (long long)Q, (long long)P);
+    writable(out);
   }
   kf_gemm_params p = {};
   p.fmt = KF_FMT_BF16;
@@ -335,7 +367,8 @@ PyObject* gemm_tokens(PyObject* const* v) {
   p.out_row_group = (int)to_int(v[4]);
   p.out_row_stride = (int)to_int(v[5]);
   p.out_row_offset = (int)to_int(v[6]);
-  p.flags = (int)to_int(v[7]) | KF_G_W_STATIC;
+  p.flags = (int)to_int(v[7]) | w_static(v[1], W);
+  writable(out);
   gemm_run(p, "gemm_tokens");
   return new_ref(v[3]);
 }
@@ -352,6 +385,7 @@ PyObject* quant_rows(PyObject* const* v) {
   }
   const int dt = dtype_code(x.scalar_type());
   if (dt < 0) fail("quant_rows: unsupported dtype %s", c10::toString(x.scalar_type()));
+  writable(out);
   check(kf_quant_rows(out.fmt, dt, x.data_ptr(), x.stride(0), (int)out.rows, (int)out.K, static_cast<const float*>(out.pts),
                       static_cast<const float*>(opt_ptr(v[2], "bias")), (int)to_int(v[3]), out.pq, out.psf, stream()),
         "quant_rows");
@@ -367,6 +401,7 @@ PyObject* ln_quant(PyObject* const* v) {
   if ((x.scalar_type() != at::kFloat && !bf16) || !x.is_contiguous() || M != out.rows || d != out.K)
     fail("ln_quant: x must be contiguous fp32 or bf16 [M=%lld, d=%lld], got [%lld, %lld] %s", (long long)out.rows, (long long)out.K, (long long)M, (long long)d,
          c10::toString(x.scalar_type()));
+  writable(out);
   check(kf_ln_quant(out.fmt, static_cast<const float*>(x.data_ptr()), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
                     (float)to_float(v[3]), (int)M, (int)d, static_cast<const float*>(out.pts), (int)to_int(v[5]) | (bf16 ? KF_Q_IN_BF16 : 0), out.pq, out.psf,
                     static_cast<float*>(opt_ptr(v[6], "y_dbg")), stream()),
@@ -474,6 +509,7 @@ PyObject* attn_fwd(PyObject* const* v) {
   const at::Tensor& qkv = qkv_tensor(v[0], "attn_fwd: qkv must be contiguous [3, B, N, H, 64] bf16 or f16");
   const int64_t B = qkv.size(1), N = qkv.size(2), H = qkv.size(3);
   at::Tensor out = v[2] == Py_None ? empty({B, N, H * 64}, qkv.scalar_type(), qkv.device()) : cuda_tensor(v[2], "out");
+  if (v[2] != Py_None) writable(out);
   check(kf_attn_fwd(dtype_code(qkv.scalar_type()), qkv.data_ptr(), out.data_ptr(), (int)B, (int)N, (int)H, (float)to_float(v[1]), stream()), "attn_fwd");
   return v[2] == Py_None ? THPVariable_Wrap(std::move(out)) : new_ref(v[2]);
 }
@@ -485,6 +521,7 @@ PyObject* attn_fwd_quant(PyObject* const* v) {
   const int64_t B = qkv.size(1), N = qkv.size(2), H = qkv.size(3);
   if (out.rows != B * N || out.K != H * 64)
     fail("attn_fwd_quant: out must be [%lld, %lld], got [%lld, %lld]", (long long)(B * N), (long long)(H * 64), (long long)out.rows, (long long)out.K);
+  writable(out);
   check(kf_attn_fwd_quant(dtype_code(qkv.scalar_type()), qkv.data_ptr(), (int)B, (int)N, (int)H, (float)to_float(v[2]), out.fmt, out.pq, out.psf,
                           static_cast<const float*>(out.pts), (int)to_int(v[3]), stream()),
         "attn_fwd_quant");
@@ -536,6 +573,12 @@ PyObject* semantic(PyObject* const* v) {
   return t;
 }
 
+// a weight: does the next GEMM with it read it ahead of its predecessor's end?
+PyObject* reads_weight_early(PyObject* const* v) {
+  PyObject* sf = attr(v[0], s_sf);
+  return PyBool_FromLong(weight_settled(v[0], tensor(attr(v[0], s_q), "weight"), sf == Py_None ? nullptr : &tensor(sf, "weight")));
+}
+
 // ------------------------------------------------------------------------------------------------ module
 template <PyObject* (*F)(PyObject* const*), int ARGS>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -564,7 +607,8 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef g_methods[] = {KF_ENTRY(quant_rows, 4),     KF_ENTRY(ln_quant, 7),   KF_ENTRY(ln_rows, 5),  KF_ENTRY(gemm_plain, 6),     KF_ENTRY(gemm_res, 7),
                            KF_ENTRY(qkv_rope, 10),      KF_ENTRY(gemm_gelu_q, 6), KF_ENTRY(bmm_nt, 3),   KF_ENTRY(gemm_tokens, 8),    KF_ENTRY(broadcast_rows, 3),
                            KF_ENTRY(ln_tail, 8),        KF_ENTRY(attn_fwd, 3),   KF_ENTRY(attn_fwd_quant, 4), KF_ENTRY(im2col_patch16, 1), KF_ENTRY(dw_ln, 10),
-                           KF_ENTRY(semantic, 3),       KF_ENTRY(amax_scale, 5), KF_ENTRY(ln_amax_scale, 7), {nullptr, nullptr, 0, nullptr}};
+                           KF_ENTRY(semantic, 3),       KF_ENTRY(amax_scale, 5), KF_ENTRY(ln_amax_scale, 7),
+                           KF_ENTRY(reads_weight_early, 1), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_kf_host", "native operator layer over libkf_b200.so", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
@@ -582,6 +626,7 @@ PyMODINIT_FUNC PyInit__kf_host() {
   s_q = PyUnicode_InternFromString("q");
   s_sf = PyUnicode_InternFromString("sf");
   s_ts = PyUnicode_InternFromString("ts");
+  s_settled = PyUnicode_InternFromString("settled");
   const char* names[4] = {"mx8", "nv4", "mx4", "bf16"};
   for (int i = 0; i < 4; ++i) g_fmt_names[i] = PyUnicode_InternFromString(names[i]);
   return PyModule_Create(&g_module);

@@ -137,7 +137,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         *abort_flag = 1u;
         if (w_early) pdl_wait();
       }
-      // Weights that no running predecessor writes (KF_G_W_STATIC): the W part of the first tile's stages is requested before the
+      // Weights whose writes the host has seen complete (KF_G_W_STATIC): the W part of the first tile's stages is requested before the
       // wait for the predecessor, so its way from HBM runs under the predecessor's end.
       int early = 0;
       auto load_w = [&](uint32_t st, int kt, const WorkItem& w, int w_halves, uint32_t tx) {

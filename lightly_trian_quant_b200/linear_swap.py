@@ -83,6 +83,10 @@ class _Feeder:
             self.w = module.weight.detach().float().contiguous()
             self.b = module.bias.detach().float().contiguous()
             self.eps = module.eps
+            # copies of its own that the host has seen complete may be read ahead of the predecessor's end; the model's own tensors may
+            # be written by anyone
+            own = self.w.data_ptr() != module.weight.data_ptr() and self.b.data_ptr() != module.bias.data_ptr()
+            self.static = own and ops.settled(self.w, self.b) is not None
         self.no_bias: Dict[tuple, torch.Tensor] = {}   # the GELU quantiser wants a bias vector: zeros, made once per width
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
@@ -93,7 +97,7 @@ class _Feeder:
             buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "ln")
             if ws is not None:
                 ops.ln_amax_scale(src, self.w, self.b, self.eps, buf.ts, ws)
-            ops.ln_quant(src, self.w, self.b, self.eps, buf, round_bf16=True, static_affine=True)
+            ops.ln_quant(src, self.w, self.b, self.eps, buf, round_bf16=True, static_affine=self.static)
         else:
             src = _rows(x)
             buf, ws = sw.operand(src.shape[0], src.shape[1], x.device, "gelu")

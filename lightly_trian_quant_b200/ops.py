@@ -147,7 +147,8 @@ def quantx(x: torch.Tensor, out: ActBuf, **kw) -> ActBuf:
 def ln_quant(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, out: ActBuf, *, round_bf16: bool = False,
              recip_div: bool = False, y_dbg: Optional[torch.Tensor] = None, static_affine: bool = False) -> ActBuf:
     """LayerNorm of the fp32 (or bf16) stream x [..., d] fused with quantisation into out (ln_mx8 / lnq).
-    static_affine=True promises that w and b are parameters, not the output of an operator in flight."""
+    static_affine=True promises that every write of w and b was complete before the launch in front of this one began its work:
+    they are then read before that launch has ended."""
     global LAUNCHES
     LAUNCHES += 1
     args = (x, w, b, eps, out, _flags(False, round_bf16, recip_div) | (_lib.KF_Q_STATIC_AFFINE if static_affine else 0), y_dbg)
@@ -204,11 +205,23 @@ def check_device_error() -> None:
     check(_lib.lib().kf_check_device_error(), "kf_check_device_error")
 
 
+def settled(*tensors: torch.Tensor) -> Optional[int]:
+    """Waits until the writes of these tensors on the current stream are complete; -> the sum of their version counters, or None
+    under graph capture and for inference tensors (which have no counter)."""
+    if torch.cuda.is_current_stream_capturing() or any(t.is_inference() for t in tensors):
+        return None
+    torch.cuda.current_stream(tensors[0].device).synchronize()
+    return sum(t._version for t in tensors)
+
+
 class QWeight:
-    """Weight [N, K] (nn.Linear layout) quantised once along K with 1-D block scales; fmt "bf16" keeps a bf16 copy.
+    """Weight [N, K] (nn.Linear layout) quantised once along K with 1-D block scales; fmt "bf16" keeps it in bf16.
     nv4: exact per-tensor scale ts = amax/(6*448) computed once on the host cores (IEEE division).
     Counterparts: MXW (infer-opt/round13_mxfp8_full/impl/mx13.py:74-84), Lin / FP4Linear weights
-    (infer-opt/round14_fp4_full/impl/stack14b.py:55-66, fp4util.py:114-131)."""
+    (infer-opt/round14_fp4_full/impl/stack14b.py:55-66, fp4util.py:114-131).
+
+    The constructor waits for the quantisation (not under graph capture): a GEMM may then request the weights ahead of its
+    predecessor's end, as long as nothing has written q or sf since, by their version counters."""
 
     def __init__(self, W: torch.Tensor, fmt: str, ts: Optional[torch.Tensor] = None):
         _need_cuda(W)
@@ -216,10 +229,9 @@ class QWeight:
         self.fmt = fmt
         if fmt == "bf16":
             self.q = W.to(torch.bfloat16).contiguous()
-            if self.q.data_ptr() == W.data_ptr():
-                self.q = self.q.clone()            # a copy of its own: the GEMM reads weights ahead of its predecessor's end
             self.sf = None
             self.ts = None
+            self.settled = settled(self.q)
             return
         Wf = W.float().contiguous()
         buf = ActBuf(self.N, self.K, fmt, device=W.device)
@@ -232,6 +244,7 @@ class QWeight:
             buf.ts.copy_(ts.reshape(1))
         quant_rows(Wf, buf)
         self.q, self.sf, self.ts = buf.q, buf.sf, buf.ts
+        self.settled = settled(self.q, self.sf)
 
 
 MXW = QWeight

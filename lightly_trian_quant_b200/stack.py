@@ -108,10 +108,12 @@ class Layer:
 
 
 def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, calib: Calib, *, round_bf16: bool, attn_dtype, half_tables: bool = False,
-              grow_into: torch.Tensor = None) -> torch.Tensor:
+              grow_into: torch.Tensor = None, static_ln1: bool = False) -> torch.Tensor:
     """x fp32 [B, N, d] (updated in place) -> x.  grow_into (fp32 [B, N + Q, d], optional): the block's result is written
     behind the first Q rows of every image of this longer stream instead (the fc2 epilogue maps the rows), which is then
-    returned: how the query tokens join the stream without a copy of it."""
+    returned: how the query tokens join the stream without a copy of it.  static_ln1: the launch in front is not the one that wrote
+    the first LayerNorm's parameters (model_fn: always a kernel of the patch embedding or of the block before).  The second LayerNorm has
+    the projection in front of it."""
     B, N, d = x.shape
     M = B * N
     fmt = L.fmt
@@ -129,7 +131,7 @@ def block_fwd(x: torch.Tensor, L: Layer, sin, cos, prefix: int, heads: int, cali
     if cal and nv4:
         set_ts(L.ts_ln1, ops.ln_rows(x, L.ln1_w, L.ln1_b, L.ln1_eps, BF))
     a, a2, a3, f = L.operands(M, x.device)
-    ops.ln_quant(x, L.ln1_w, L.ln1_b, L.ln1_eps, a, round_bf16=round_bf16, static_affine=True)
+    ops.ln_quant(x, L.ln1_w, L.ln1_b, L.ln1_eps, a, round_bf16=round_bf16, static_affine=static_ln1)
     qkv = ops.qkv_rope(a, L.qkv, L.bqkv, sin, cos, N, prefix, heads, out_dtype=attn_dtype, half_tables=half_tables)
     # ---- attention with its output quantised in the epilogue -> proj (gamma + residual, in place on the stream)
     if cal and nv4:
@@ -269,7 +271,7 @@ def make_model_fn(model, fmt: str, *, image_size: int = 640, round_bf16: bool = 
             elif i == first_joint == 0:                   # every block is a joint block: no fc2 in front to do the move
                 t = torch.cat((queries[None].expand(t.shape[0], -1, -1), t), dim=1).contiguous()
             t = block_fwd(t, layers[i], sin, cos, t.shape[1] - P, heads, calib, round_bf16=round_bf16, attn_dtype=attn_dtype, half_tables=half_tables,
-                          grow_into=grow)
+                          grow_into=grow, static_ln1=True)
         out = head(t, grid)
         calib.on = False
         return out

@@ -134,3 +134,29 @@ def test_host_checks_of_the_head_kernels(built_lib):
         ops.bmm_nt(a, w)                                     # CPU tensors
     with pytest.raises(KfError):
         ops.bmm_nt(a.float(), w)                             # wrong dtype (checked before the device)
+
+
+def test_weights_are_read_early_only_while_settled(built_lib):
+    """a GEMM may request weights ahead of its predecessor's end only if the host has seen them complete and nothing has written them since."""
+    import types
+
+    import torch
+
+    from lightly_trian_quant_b200 import _lib
+
+    early = _lib.host().reads_weight_early
+    q, sf = torch.zeros(128, 64, dtype=torch.uint8), torch.zeros(512, dtype=torch.uint8)
+    w = types.SimpleNamespace(N=128, K=128, fmt="nv4", q=q, sf=sf, ts=None)
+    assert not early(w)                                      # a container that claims nothing
+    w.settled = None
+    assert not early(w)
+    w.settled = q._version + sf._version
+    assert early(w)
+    sf.add_(1)                                               # written in place since
+    assert not early(w)
+    w.settled = q._version + sf._version
+    q.view(-1)[3:5].zero_()                                  # through a view
+    assert not early(w)
+    with torch.inference_mode():
+        w.q, w.sf, w.settled = torch.zeros(128, 64), None, 0
+    assert not early(w)

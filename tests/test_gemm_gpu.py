@@ -435,3 +435,46 @@ def test_a_failed_predecessor_does_not_stall_the_launch(M, K, delay):
         assert time.perf_counter() - t0 < 1.0
         assert torch.equal(call(), ref)
         ops.check_device_error()
+
+
+@pytest.mark.parametrize("fmt", FMTS + ["bf16"])
+@pytest.mark.parametrize("M", [1, 300, 2304])
+def test_weights_written_right_before_the_launch(fmt, M):
+    """construct a weight and call at once, rewrite its tensors in place and call at once: the results are those of plain stream order."""
+    from lightly_trian_quant_b200 import _lib
+
+    ops = _ops()
+    N, K = 512, 1024
+    early = _lib.host().reads_weight_early
+    a, W0, _, _ = _quant_pair(_mk_x(M, K, 5), _mk_w(N, K, 6), fmt)
+    ws = [_mk_w(N, K, 7 + i).cuda() for i in range(4)]
+    ops.set_pdl(False)
+    plain = []
+    for w in ws:
+        W = ops.QWeight(w, fmt)
+        torch.cuda.synchronize()
+        plain.append(ops.gemm_plain(a, W))
+        torch.cuda.synchronize()
+    ops.set_pdl(True)
+    for _ in range(5):
+        held = [ops.QWeight(w, fmt) for w in ws]
+        one = ops.QWeight(ws[0].clone(), fmt)
+        assert early(one)
+        for w, W, ref in zip(ws, held, plain):
+            assert torch.equal(ops.gemm_plain(a, ops.QWeight(w, fmt)), ref)
+            one.q.copy_(W.q)
+            if fmt != "bf16":
+                one.sf.copy_(W.sf)
+            if fmt == "nv4":
+                one.ts.copy_(W.ts)
+            assert not early(one)
+            assert torch.equal(ops.gemm_plain(a, one), ref)
+    if fmt != "bf16":                                        # an operator of the package writes the container
+        buf = ops.ActBuf(N, K, fmt)
+        one.q, one.sf, one.ts = buf.q, buf.sf, buf.ts
+        one.settled = ops.settled(buf.q, buf.sf)
+        if fmt == "nv4":
+            buf.ts.copy_(held[1].ts)
+        ops.quant_rows(ws[1].float(), buf)
+        assert not early(one) and torch.equal(ops.gemm_plain(a, one), plain[1])
+    ops.check_device_error()

@@ -348,3 +348,47 @@ def test_linear_swap_enable_disable(fmt):
     ml3, _ = model(x)
     linear_swap.disable(model)
     assert mo.cosine(ml3.float().cpu(), ml0.cpu()) > 0.9
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_early_reads_give_plain_stream_order(dtype):
+    """parameters and weights that the kernels read ahead of their predecessor's end (Linear swap, one block, whole model) against plain stream
+    order; LayerNorm parameters rewritten right before the call included."""
+    from lightly_trian_quant_b200 import linear_swap
+
+    modeldef, ops, stack = _mods()
+    cfg = modeldef.EoMTConfig(**TINY)
+    model = modeldef.build_model(cfg, 0, "stress", "cuda").to(dtype)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(2, 41, cfg.dim, generator=g, device="cuda")
+    img = torch.rand(2, 3, 64, 64, generator=g, device="cuda").to(BF)
+    norms = [torch.rand(cfg.dim, generator=g, device="cuda").to(dtype) + 0.5 for _ in range(3)]
+    sin, cos = (t.float().contiguous() for t in model.backbone.rope_embed(H=6, W=6))
+
+    def outputs(fmt):
+        blk = model.backbone.blocks[0]
+        out = []
+        blk.norm1.weight.copy_(norms[2])
+        for n in norms:
+            linear_swap.enable(model, [(0, "qkv"), (0, "fc1")], fmt)
+            blk.norm1.weight.copy_(n)
+            out.append(blk.attn.qkv(blk.norm1(x.to(dtype))).clone())
+            linear_swap.disable(model)
+            L, cal = stack.Layer(blk, fmt), stack.Calib()
+            stack.block_fwd(x.clone(), L, sin, cos, 5, cfg.heads, cal, round_bf16=True, attn_dtype=BF)
+            cal.on = False
+            L.ln1_w.copy_(n)
+            out.append(stack.block_fwd(x.clone(), L, sin, cos, 5, cfg.heads, cal, round_bf16=True, attn_dtype=BF))
+        fn, _ = stack.make_variant("tiny", model, f"b200_{fmt}+s64")
+        fn(img)
+        blk.norm1.weight.copy_(norms[0])
+        return out + [t.clone() for t in fn(img)]
+
+    for fmt in ("mx8", "nv4"):
+        ops.set_pdl(False)
+        ref = outputs(fmt)
+        ops.set_pdl(True)
+        for _ in range(3):
+            for got, want in zip(outputs(fmt), ref):
+                assert torch.equal(got, want)
+    ops.check_device_error()
