@@ -52,6 +52,17 @@ const at::Tensor& cuda_tensor(PyObject* o, const char* what) {
   return t;
 }
 
+[[noreturn]] void divides_by_zero(const char* what) {          // what Python arithmetic on the shapes raises
+  PyErr_SetString(PyExc_ZeroDivisionError, what);
+  throw Failed{};
+}
+
+// rows of x seen as [rows, d]
+int64_t rows_of(const at::Tensor& x, int64_t d, const char* what) {
+  if (d == 0) divides_by_zero(what);
+  return x.numel() / d;
+}
+
 // pointer of an optional CUDA tensor (None = null)
 void* opt_ptr(PyObject* o, const char* what) { return o == Py_None ? nullptr : cuda_tensor(o, what).data_ptr(); }
 
@@ -230,6 +241,31 @@ PyObject* gemm_plain(PyObject* const* v) {
   return new_ref(v[3]);
 }
 
+// (group, stride, offset) as any iterable of three integers
+struct RowMap {
+  int group, stride, offset;
+};
+RowMap row_map(PyObject* o) {
+  PyObject* seq = PySequence_Fast(o, "gemm_res: row_map must be (group, stride, offset)");
+  if (!seq) throw Failed{};
+  int value[3] = {0, 0, 0};
+  bool ok = PySequence_Fast_GET_SIZE(seq) == 3;
+  if (!ok) PyErr_Format(PyExc_ValueError, "gemm_res: row_map must be (group, stride, offset), got %zd values", PySequence_Fast_GET_SIZE(seq));
+  for (int i = 0; ok && i < 3; ++i) {
+    const long n = PyLong_AsLong(PySequence_Fast_GET_ITEM(seq, i));
+    ok = !(n == -1 && PyErr_Occurred());
+    if (ok && n != (int)n) {
+      PyErr_Format(PyExc_OverflowError, "gemm_res: row_map value %ld does not fit a 32-bit integer", n);
+      ok = false;
+    }
+    value[i] = (int)n;
+  }
+  Py_DECREF(seq);
+  if (!ok) throw Failed{};
+  if (value[0] == 0) divides_by_zero("gemm_res: row_map with a group of 0 rows");
+  return {value[0], value[1], value[2]};
+}
+
 // a, W, bias, gamma, res, out | None, row_map | None
 PyObject* gemm_res(PyObject* const* v) {
   const Operand W = weight(v[1]);
@@ -252,13 +288,12 @@ PyObject* gemm_res(PyObject* const* v) {
   const at::Tensor& out = cuda_tensor(v[5], "out");
   need(out.scalar_type() == at::kFloat && out.is_contiguous(), "gemm_res: out must be contiguous fp32");
   if (v[6] != Py_None) {
-    int group, stride, offset;
-    if (!PyTuple_Check(v[6]) || !PyArg_ParseTuple(v[6], "iii", &group, &stride, &offset)) throw Failed{};
-    if (M % group || out.numel() != (M / group) * stride * W.rows || offset + group > stride)
-      fail("gemm_res: row mapping (%d, %d, %d) does not fit M=%lld rows into %lld output rows", group, stride, offset, (long long)M, (long long)(out.numel() / W.rows));
-    p.out_row_group = group;
-    p.out_row_stride = stride;
-    p.out_row_offset = offset;
+    const RowMap m = row_map(v[6]);
+    if (M % m.group || out.numel() != (M / m.group) * m.stride * W.rows || (int64_t)m.offset + m.group > m.stride)
+      fail("gemm_res: row mapping (%d, %d, %d) does not fit M=%lld rows into an output of %lld values", m.group, m.stride, m.offset, (long long)M, (long long)out.numel());
+    p.out_row_group = m.group;
+    p.out_row_stride = m.stride;
+    p.out_row_offset = m.offset;
   }
   p.C = out.data_ptr();
   writable(out);
@@ -433,7 +468,7 @@ PyObject* amax_scale(PyObject* const* v) {
 PyObject* ln_amax_scale(PyObject* const* v) {
   const at::Tensor& x = cuda_tensor(v[0], "x");
   need(x.is_contiguous() && x.dim() > 0 && (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16), "ln_amax_scale: x must be contiguous fp32 or bf16");
-  const int64_t d = x.size(-1), M = x.numel() / d;
+  const int64_t d = x.size(-1), M = rows_of(x, d, "ln_amax_scale: x has a last dimension of 0");
   void* ws;
   float* ts = scale_target(v[5], v[6], &ws);
   check(kf_ln_amax_scale(dtype_code(x.scalar_type()), x.data_ptr(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
@@ -446,7 +481,7 @@ PyObject* ln_amax_scale(PyObject* const* v) {
 PyObject* ln_rows(PyObject* const* v) {
   const at::Tensor& x = cuda_tensor(v[0], "x");
   need(x.scalar_type() == at::kFloat && x.is_contiguous() && x.dim() > 0, "ln_rows: x must be contiguous fp32");
-  const int64_t d = x.size(-1), M = x.numel() / d;
+  const int64_t d = x.size(-1), M = rows_of(x, d, "ln_rows: x has a last dimension of 0");
   const int dt = (int)to_int(v[4]);
   at::Tensor y = empty(x.sizes(), dtype_of(dt), x.device());
   check(kf_ln_rows(x.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")), (float)to_float(v[3]), (int)M, (int)d, dt,
@@ -461,7 +496,7 @@ PyObject* broadcast_rows(PyObject* const* v) {
   need(src.scalar_type() == at::kFloat && dst.scalar_type() == at::kFloat && src.is_contiguous() && dst.is_contiguous() && dst.dim() == 3 && src.dim() > 0 &&
            src.size(-1) == dst.size(2),
        "broadcast_rows: src [R, d] and dst [B, Ntok, d] must be contiguous fp32");
-  const int64_t d = dst.size(2), R = src.numel() / d;
+  const int64_t d = dst.size(2), R = rows_of(src, d, "broadcast_rows: src and dst have a last dimension of 0");
   check(kf_broadcast_rows(src.data_ptr<float>(), dst.data_ptr<float>(), (int)R, (int)d, (int)dst.size(0), dst.size(1) * d, to_int(v[2]), stream()), "broadcast_rows");
   return new_ref(v[1]);
 }

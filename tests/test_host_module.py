@@ -1,0 +1,55 @@
+"""The native operator module (csrc/host/kf_host.cpp): bad arguments end as Python errors, containers may be any object with the attributes, other
+threads run while an operator is inside the library."""
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+
+def _res_case(M=6, N=128, K=256):
+    from lightly_trian_quant_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    W = ops.QWeight(torch.randn(N, K, generator=g, device="cuda") * 0.05, "bf16")
+    vec = torch.randn(N, generator=g, device="cuda")
+    return a, W, vec, torch.randn(M, N, generator=g, device="cuda")
+
+
+@gpu
+@pytest.mark.parametrize("row_map,error", [
+    ((0, 5, 2), ZeroDivisionError), ([0, 0, 0], ZeroDivisionError), ((3, 5), ValueError), ((3, 5, 2, 1), ValueError), (7, TypeError),
+    ((3.0, 5, 2), TypeError), ((1 << 40, 5, 2), OverflowError), ((4, 5, 1), RuntimeError), ((-3, 5, 2), RuntimeError)])
+def test_bad_row_maps_are_python_errors(row_map, error):
+    from lightly_trian_quant_b200 import ops
+
+    a, W, vec, res = _res_case()
+    with pytest.raises(error):
+        ops.gemm_res(a, W, vec, vec, res, out=torch.zeros(2, 5, 128, device="cuda"), row_map=row_map)
+
+
+@gpu
+@pytest.mark.parametrize("kind", [tuple, list, iter])
+def test_row_map_takes_any_iterable(kind):
+    from lightly_trian_quant_b200 import ops
+
+    a, W, vec, res = _res_case()
+    plain = ops.gemm_res(a, W, vec, vec, res)
+    out = torch.zeros(2, 5, 128, device="cuda")
+    ops.gemm_res(a, W, vec, vec, res, out=out, row_map=kind((3, 5, 2)))
+    assert torch.equal(out[:, 2:].reshape(6, 128), plain) and not out[:, :2].any()
+
+
+@gpu
+def test_empty_last_dimension_is_a_python_error():
+    from lightly_trian_quant_b200 import ops
+
+    none = torch.zeros(3, 0, device="cuda")
+    with pytest.raises(ZeroDivisionError):
+        ops.ln_rows(none, none, none, 1e-5)
+    with pytest.raises(ZeroDivisionError):
+        ops.ln_amax_scale(none, none, none, 1e-5, torch.ones(1, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda"))
+    with pytest.raises(ZeroDivisionError):
+        ops.broadcast_rows(none, torch.zeros(2, 3, 0, device="cuda"), 0)
+    with pytest.raises(ops.KfError):
+        ops.ln_quant(none, none, none, 1e-5, ops.ActBuf(3, 256, "mx8"))
