@@ -63,14 +63,28 @@ int64_t rows_of(const at::Tensor& x, int64_t d, const char* what) {
   return x.numel() / d;
 }
 
+at::Tensor opt_tensor(PyObject* o, const char* what) { return o == Py_None ? at::Tensor() : cuda_tensor(o, what); }
 // pointer of an optional CUDA tensor (None = null)
 void* opt_ptr(PyObject* o, const char* what) { return o == Py_None ? nullptr : cuda_tensor(o, what).data_ptr(); }
 
-PyObject* attr(PyObject* o, PyObject* name) {
+// An owned reference: an attribute may be a property, whose value nobody else holds.
+class Ref {
+ public:
+  explicit Ref(PyObject* p) : p_(p) {}
+  Ref(Ref&& o) noexcept : p_(o.p_) { o.p_ = nullptr; }
+  Ref(const Ref&) = delete;
+  Ref& operator=(const Ref&) = delete;
+  ~Ref() { Py_XDECREF(p_); }
+  operator PyObject*() const { return p_; }
+
+ private:
+  PyObject* p_;
+};
+
+Ref attr(PyObject* o, PyObject* name) {
   PyObject* v = PyObject_GetAttr(o, name);
   if (!v) throw Failed{};
-  Py_DECREF(v);                                                // the container keeps it alive for the duration of the call
-  return v;
+  return Ref(v);
 }
 
 int64_t to_int(PyObject* o) {
@@ -100,10 +114,10 @@ int fmt_code(PyObject* name) {
   fail("unknown operand format %R", name);
 }
 
-struct Operand {                                               // ActBuf or QWeight
+struct Operand {                                               // ActBuf or QWeight; holds its tensors until the launch is made
   int fmt;
   int64_t rows, K;
-  const at::Tensor *q, *sf;                                    // sf: null for bf16
+  at::Tensor q, sf, ts;                                        // sf: undefined for bf16, ts: undefined unless nv4
   void *pq, *psf, *pts;
 };
 
@@ -112,12 +126,12 @@ Operand operand(PyObject* o, PyObject* rows_attr, const char* what) {
   r.rows = to_int(attr(o, rows_attr));
   r.K = to_int(attr(o, s_K));
   r.fmt = fmt_code(attr(o, s_fmt));
-  r.q = &cuda_tensor(attr(o, s_q), what);
-  r.pq = r.q->data_ptr();
-  PyObject* sf = attr(o, s_sf);
-  r.sf = sf == Py_None ? nullptr : &cuda_tensor(sf, what);
-  r.psf = r.sf ? r.sf->data_ptr() : nullptr;
-  r.pts = opt_ptr(attr(o, s_ts), what);
+  r.q = cuda_tensor(attr(o, s_q), what);
+  r.pq = r.q.data_ptr();
+  r.sf = opt_tensor(attr(o, s_sf), what);
+  r.psf = r.sf.defined() ? r.sf.data_ptr() : nullptr;
+  r.ts = opt_tensor(attr(o, s_ts), what);
+  r.pts = r.ts.defined() ? r.ts.data_ptr() : nullptr;
   return r;
 }
 Operand act(PyObject* o, const char* what) { return operand(o, s_M, what); }
@@ -163,7 +177,7 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
 // weights whose writes the host has seen complete and that nothing has written since: `settled` is the sum of the version counters of q
 // and sf at that moment (ops.QWeight), None where the host did not wait.  torch counts its in-place writes, writable() those of
 // the operators here; an object without the attribute claims nothing.  bmm_nt takes activations and does not claim it either.
-bool weight_settled(PyObject* o, const at::Tensor& q, const at::Tensor* sf) {
+bool weight_settled(PyObject* o, const at::Tensor& q, const at::Tensor& sf) {
   PyObject* v = PyObject_GetAttr(o, s_settled);
   if (!v) {
     if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw Failed{};
@@ -174,18 +188,18 @@ bool weight_settled(PyObject* o, const at::Tensor& q, const at::Tensor* sf) {
   const long long seen = claimed ? PyLong_AsLongLong(v) : 0;
   Py_DECREF(v);
   if (seen == -1 && PyErr_Occurred()) throw Failed{};
-  if (!claimed || q.is_inference() || (sf && sf->is_inference())) return false;      // an inference tensor has no version counter
-  return (int64_t)q._version() + (sf ? (int64_t)sf->_version() : 0) == seen;
+  if (!claimed || q.is_inference() || (sf.defined() && sf.is_inference())) return false;      // an inference tensor has no version counter
+  return (int64_t)q._version() + (sf.defined() ? (int64_t)sf._version() : 0) == seen;
 }
-int w_static(PyObject* o, const Operand& W) { return weight_settled(o, *W.q, W.sf) ? KF_G_W_STATIC : 0; }
+int w_static(PyObject* o, const Operand& W) { return weight_settled(o, W.q, W.sf) ? KF_G_W_STATIC : 0; }
 
 // out is about to be written: counted as torch counts an in-place operation
 void writable(const at::Tensor& out) {
   if (!out.is_inference()) out.unsafeGetTensorImpl()->bump_version();
 }
 void writable(const Operand& out) {
-  writable(*out.q);
-  if (out.sf) writable(*out.sf);
+  writable(out.q);
+  if (out.sf.defined()) writable(out.sf);
 }
 // A side, W side and the common fields; returns M
 int64_t gemm_fill(kf_gemm_params& p, PyObject* a, const Operand& W, int epi) {
@@ -228,7 +242,7 @@ PyObject* gemm_plain(PyObject* const* v) {
   p.flags = (int)to_int(v[5]) | w_static(v[1], W);
   if (v[3] == Py_None) {
     p.out_dtype = (int)to_int(v[4]);
-    at::Tensor out = empty({M, W.rows}, dtype_of(p.out_dtype), W.q->device());
+    at::Tensor out = empty({M, W.rows}, dtype_of(p.out_dtype), W.q.device());
     p.C = out.data_ptr();
     gemm_run(p, "gemm_plain");
     return THPVariable_Wrap(std::move(out));
@@ -322,7 +336,7 @@ PyObject* qkv_rope(PyObject* const* v) {
   p.H = (int)H;
   p.out_dtype = (int)to_int(v[8]);
   p.flags = (int)to_int(v[9]) | w_static(v[1], W);
-  at::Tensor out = empty({3, M / Ntok, Ntok, H, 64}, dtype_of(p.out_dtype), W.q->device());
+  at::Tensor out = empty({3, M / Ntok, Ntok, H, 64}, dtype_of(p.out_dtype), W.q.device());
   p.C = out.data_ptr();
   gemm_run(p, "qkv_rope");
   return THPVariable_Wrap(std::move(out));
@@ -610,8 +624,8 @@ PyObject* semantic(PyObject* const* v) {
 
 // a weight: does the next GEMM with it read it ahead of its predecessor's end?
 PyObject* reads_weight_early(PyObject* const* v) {
-  PyObject* sf = attr(v[0], s_sf);
-  return PyBool_FromLong(weight_settled(v[0], tensor(attr(v[0], s_q), "weight"), sf == Py_None ? nullptr : &tensor(sf, "weight")));
+  const Ref q = attr(v[0], s_q), sf = attr(v[0], s_sf);
+  return PyBool_FromLong(weight_settled(v[0], tensor(q, "weight"), sf == Py_None ? at::Tensor() : tensor(sf, "weight")));
 }
 
 // ------------------------------------------------------------------------------------------------ module

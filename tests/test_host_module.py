@@ -53,3 +53,72 @@ def test_empty_last_dimension_is_a_python_error():
         ops.broadcast_rows(none, torch.zeros(2, 3, 0, device="cuda"), 0)
     with pytest.raises(ops.KfError):
         ops.ln_quant(none, none, none, 1e-5, ops.ActBuf(3, 256, "mx8"))
+
+
+PROPERTY_PROBE = """
+import types
+import torch
+from lightly_trian_quant_b200 import _lib
+
+log = []
+
+class Rows:
+    def __index__(self):
+        log.append("used")
+        return 128
+    def __del__(self):
+        log.append("freed")
+
+class Weight:
+    K, fmt, sf, ts = 256, "bf16", None, None
+    @property
+    def N(self):
+        return Rows()
+    @property
+    def q(self):
+        return torch.zeros(128, 256, dtype=torch.bfloat16)
+
+try:
+    _lib.host().gemm_plain(torch.zeros(1, 256, dtype=torch.bfloat16), Weight(), None, None, 1, 0)
+except _lib.KfError as e:
+    assert "CUDA" in str(e)
+else:
+    raise SystemExit("a CPU tensor was taken")
+assert log == ["used", "freed"], log
+"""
+
+
+def test_attribute_values_live_until_they_are_used():
+    """a container's attribute may be a property whose value nobody else holds (in a process of its own: a use after free may end it)."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    from lightly_trian_quant_b200 import build
+
+    build.build()
+    r = subprocess.run([sys.executable, "-c", PROPERTY_PROBE], capture_output=True, text=True, cwd=Path(__file__).resolve().parents[1])
+    assert r.returncode == 0, (r.returncode, r.stderr)
+
+
+@gpu
+def test_containers_with_property_attributes():
+    """operands whose every attribute access makes a new tensor give the bits of the package's own containers."""
+    from lightly_trian_quant_b200 import ops
+
+    class Fresh:
+        def __init__(self, held):
+            self.held = held
+
+        def __getattr__(self, name):
+            t = getattr(self.held, name)
+            return t.clone() if isinstance(t, torch.Tensor) else t
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.randn(300, 512, generator=g, device="cuda").bfloat16()
+    a = ops.quant_rows(x, ops.ActBuf(300, 512, "nv4"))
+    W = ops.QWeight(torch.randn(384, 512, generator=g, device="cuda") * 0.05, "nv4")
+    want = ops.gemm_plain(a, W)
+    for _ in range(20):
+        assert torch.equal(ops.gemm_plain(Fresh(a), Fresh(W)), want)
+    ops.check_device_error()
