@@ -174,22 +174,25 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
 
 // ------------------------------------------------------------------------------------------------ GEMM
 // KF_G_W_STATIC lets the kernel read weights before the wait that makes the predecessor's writes visible, so it is claimed only for
-// weights whose writes the host has seen complete and that nothing has written since: `settled` is the sum of the version counters of q
-// and sf at that moment (ops.QWeight), None where the host did not wait.  torch counts its in-place writes, writable() those of
-// the operators here; an object without the attribute claims nothing.  bmm_nt takes activations and does not claim it either.
+// weights whose writes the host has seen complete and that nothing has written since: `settled` is (q, sf, sum of their version counters)
+// at that moment (ops.settled), None where the host did not wait.  torch counts its in-place writes, writable() those of the operators
+// here; other tensors in the place of those two, or an object without the attribute, claim nothing.  bmm_nt takes activations and does
+// not claim it either.
 bool weight_settled(PyObject* o, const at::Tensor& q, const at::Tensor& sf) {
-  PyObject* v = PyObject_GetAttr(o, s_settled);
-  if (!v) {
+  PyObject* p = PyObject_GetAttr(o, s_settled);
+  if (!p) {
     if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw Failed{};
     PyErr_Clear();
     return false;
   }
-  const bool claimed = v != Py_None;
-  const long long seen = claimed ? PyLong_AsLongLong(v) : 0;
-  Py_DECREF(v);
-  if (seen == -1 && PyErr_Occurred()) throw Failed{};
-  if (!claimed || q.is_inference() || (sf.defined() && sf.is_inference())) return false;      // an inference tensor has no version counter
-  return (int64_t)q._version() + (sf.defined() ? (int64_t)sf._version() : 0) == seen;
+  const Ref seen(p);
+  if (!PyTuple_Check(p) || PyTuple_GET_SIZE(p) != 3) return false;
+  auto same = [&](Py_ssize_t i, const at::Tensor& t) {
+    PyObject* held = PyTuple_GET_ITEM(p, i);
+    return t.defined() ? THPVariable_Check(held) && THPVariable_Unpack(held).is_same(t) : held == Py_None;
+  };
+  if (!same(0, q) || !same(1, sf) || q.is_inference() || (sf.defined() && sf.is_inference())) return false;   // an inference tensor has no version counter
+  return (int64_t)q._version() + (sf.defined() ? (int64_t)sf._version() : 0) == to_int(PyTuple_GET_ITEM(p, 2));
 }
 int w_static(PyObject* o, const Operand& W) { return weight_settled(o, W.q, W.sf) ? KF_G_W_STATIC : 0; }
 

@@ -205,13 +205,14 @@ def check_device_error() -> None:
     check(_lib.lib().kf_check_device_error(), "kf_check_device_error")
 
 
-def settled(*tensors: torch.Tensor) -> Optional[int]:
-    """Waits until the writes of these tensors on the current stream are complete; -> the sum of their version counters, or None
-    under graph capture and for inference tensors (which have no counter)."""
-    if torch.cuda.is_current_stream_capturing() or any(t.is_inference() for t in tensors):
+def settled(q: torch.Tensor, sf: Optional[torch.Tensor] = None) -> Optional[tuple]:
+    """Waits until the writes of these tensors on the current stream are complete; -> (q, sf, sum of their version counters), or None under
+    graph capture and for inference tensors (which have no counter)."""
+    ts = [t for t in (q, sf) if t is not None]
+    if torch.cuda.is_current_stream_capturing() or any(t.is_inference() for t in ts):
         return None
-    torch.cuda.current_stream(tensors[0].device).synchronize()
-    return sum(t._version for t in tensors)
+    torch.cuda.current_stream(q.device).synchronize()
+    return q, sf, sum(t._version for t in ts)
 
 
 class QWeight:
@@ -221,7 +222,15 @@ class QWeight:
     (infer-opt/round14_fp4_full/impl/stack14b.py:55-66, fp4util.py:114-131).
 
     The constructor waits for the quantisation (not under graph capture): a GEMM may then request the weights ahead of its
-    predecessor's end, as long as nothing has written q or sf since, by their version counters."""
+    predecessor's end, as long as nothing has written q or sf since, by their version counters, or put others in their place."""
+
+    def __setattr__(self, name, value):
+        if name in ("q", "sf"):
+            super().__setattr__("settled", None)       # also: the tensors of the past are not held
+        super().__setattr__(name, value)
+
+    def __getstate__(self):
+        return {**self.__dict__, "settled": None}          # the tensors of a copy have been written since
 
     def __init__(self, W: torch.Tensor, fmt: str, ts: Optional[torch.Tensor] = None):
         _need_cuda(W)

@@ -150,13 +150,42 @@ def test_weights_are_read_early_only_while_settled(built_lib):
     assert not early(w)                                      # a container that claims nothing
     w.settled = None
     assert not early(w)
-    w.settled = q._version + sf._version
+    claim = lambda: (q, sf, q._version + sf._version)  # noqa: E731
+    w.settled = claim()
     assert early(w)
     sf.add_(1)                                               # written in place since
     assert not early(w)
-    w.settled = q._version + sf._version
+    w.settled = claim()
     q.view(-1)[3:5].zero_()                                  # through a view
     assert not early(w)
-    with torch.inference_mode():
-        w.q, w.sf, w.settled = torch.zeros(128, 64), None, 0
+    w.settled = claim()
+    for name in ("q", "sf"):                                 # another tensor with the same counter in its place
+        old = getattr(w, name)
+        setattr(w, name, old.clone())
+        while getattr(w, name)._version < old._version:
+            getattr(w, name).add_(0)
+        assert not early(w)
+        setattr(w, name, old)
+        assert early(w)
+    w.sf = None
     assert not early(w)
+    with torch.inference_mode():
+        q = w.q = torch.zeros(128, 64)
+        w.settled = (q, None, 0)
+    assert not early(w)
+
+
+def test_a_weight_forgets_its_settled_tensors(built_lib):
+    """assigning q or sf of a QWeight takes the claim back, and does not keep the old tensors alive; a copy makes no claim."""
+    import copy
+
+    import torch
+
+    from lightly_trian_quant_b200 import ops
+
+    W = ops.QWeight.__new__(ops.QWeight)
+    W.q, W.sf = torch.zeros(4, dtype=torch.uint8), None
+    W.settled = (W.q, None, 0)
+    assert copy.deepcopy(W).settled is None and copy.copy(W).settled is None and torch.equal(copy.deepcopy(W).q, W.q)
+    W.q = torch.ones(4, dtype=torch.uint8)
+    assert W.settled is None

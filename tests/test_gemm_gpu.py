@@ -473,6 +473,7 @@ def test_weights_written_right_before_the_launch(fmt, M):
         buf = ops.ActBuf(N, K, fmt)
         one.q, one.sf, one.ts = buf.q, buf.sf, buf.ts
         one.settled = ops.settled(buf.q, buf.sf)
+        assert early(one)
         if fmt == "nv4":
             buf.ts.copy_(held[1].ts)
         ops.quant_rows(ws[1].float(), buf)
