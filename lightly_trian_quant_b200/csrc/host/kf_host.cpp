@@ -155,7 +155,30 @@ void check(int status, const char* what) {
   if (status != 0) fail("%s failed with status %d: %s", what, status, kf_last_error_string());
 }
 
+// Other threads run while this one is inside an allocation or the library: a launch blocks when the stream's queue is full.
+class Unlocked {
+ public:
+  Unlocked() : state_(PyEval_SaveThread()) {}
+  Unlocked(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state_); }
+
+ private:
+  PyThreadState* state_;
+};
+
+// fn(args...) of the C-ABI without the interpreter lock; the arguments have been worked out with it
+template <typename... P, typename... A>
+void launch(const char* what, int (*fn)(P...), A... args) {
+  int status;
+  {
+    const Unlocked unlocked;
+    status = fn(args...);
+  }
+  check(status, what);
+}
+
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, at::Device device) {
+  const Unlocked unlocked;
   return at::Tensor(at::detail::empty_cuda(sizes, dtype, device, std::nullopt));
 }
 
@@ -233,7 +256,7 @@ int64_t gemm_fill(kf_gemm_params& p, PyObject* a, const Operand& W, int epi) {
   return M;
 }
 
-void gemm_run(const kf_gemm_params& p, const char* what) { check(kf_gemm_bs(&p, stream()), what); }
+void gemm_run(const kf_gemm_params& p, const char* what) { launch(what, kf_gemm_bs, &p, stream()); }
 
 // a, W, bias, out | None, out dtype code, flags
 PyObject* gemm_plain(PyObject* const* v) {
@@ -297,7 +320,11 @@ PyObject* gemm_res(PyObject* const* v) {
   p.out_dtype = KF_F32;
   if (v[5] == Py_None) {
     if (v[6] != Py_None) fail("gemm_res: a row mapping needs the output tensor");
-    at::Tensor out = at::empty_like(tensor(v[4], "res"));
+    const at::Tensor& res = tensor(v[4], "res");
+    at::Tensor out = [&] {
+      const Unlocked unlocked;
+      return at::empty_like(res);
+    }();
     p.C = out.data_ptr();
     gemm_run(p, "gemm_res");
     return THPVariable_Wrap(std::move(out));
@@ -438,9 +465,8 @@ PyObject* quant_rows(PyObject* const* v) {
   const int dt = dtype_code(x.scalar_type());
   if (dt < 0) fail("quant_rows: unsupported dtype %s", c10::toString(x.scalar_type()));
   writable(out);
-  check(kf_quant_rows(out.fmt, dt, x.data_ptr(), x.stride(0), (int)out.rows, (int)out.K, static_cast<const float*>(out.pts),
-                      static_cast<const float*>(opt_ptr(v[2], "bias")), (int)to_int(v[3]), out.pq, out.psf, stream()),
-        "quant_rows");
+  launch("quant_rows", kf_quant_rows, out.fmt, dt, x.data_ptr(), x.stride(0), (int)out.rows, (int)out.K, static_cast<const float*>(out.pts),
+         static_cast<const float*>(opt_ptr(v[2], "bias")), (int)to_int(v[3]), out.pq, out.psf, stream());
   return new_ref(v[1]);
 }
 
@@ -454,10 +480,9 @@ PyObject* ln_quant(PyObject* const* v) {
     fail("ln_quant: x must be contiguous fp32 or bf16 [M=%lld, d=%lld], got [%lld, %lld] %s", (long long)out.rows, (long long)out.K, (long long)M, (long long)d,
          c10::toString(x.scalar_type()));
   writable(out);
-  check(kf_ln_quant(out.fmt, static_cast<const float*>(x.data_ptr()), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
-                    (float)to_float(v[3]), (int)M, (int)d, static_cast<const float*>(out.pts), (int)to_int(v[5]) | (bf16 ? KF_Q_IN_BF16 : 0), out.pq, out.psf,
-                    static_cast<float*>(opt_ptr(v[6], "y_dbg")), stream()),
-        "ln_quant");
+  launch("ln_quant", kf_ln_quant, out.fmt, static_cast<const float*>(x.data_ptr()), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
+         (float)to_float(v[3]), (int)M, (int)d, static_cast<const float*>(out.pts), (int)to_int(v[5]) | (bf16 ? KF_Q_IN_BF16 : 0), out.pq, out.psf,
+         static_cast<float*>(opt_ptr(v[6], "y_dbg")), stream());
   return new_ref(v[4]);
 }
 
@@ -477,7 +502,7 @@ PyObject* amax_scale(PyObject* const* v) {
   need(x.dim() == 2 && x.stride(1) == 1 && dt >= 0, "amax_scale: x must be f32 | bf16 | f16 [M, K] with a contiguous last dim");
   void* ws;
   float* ts = scale_target(v[3], v[4], &ws);
-  check(kf_amax_scale(dt, x.data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), (int)to_int(v[1]), (float)to_float(v[2]), ts, ws, stream()), "amax_scale");
+  launch("amax_scale", kf_amax_scale, dt, x.data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), (int)to_int(v[1]), (float)to_float(v[2]), ts, ws, stream());
   return new_ref(v[3]);
 }
 
@@ -488,9 +513,8 @@ PyObject* ln_amax_scale(PyObject* const* v) {
   const int64_t d = x.size(-1), M = rows_of(x, d, "ln_amax_scale: x has a last dimension of 0");
   void* ws;
   float* ts = scale_target(v[5], v[6], &ws);
-  check(kf_ln_amax_scale(dtype_code(x.scalar_type()), x.data_ptr(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
-                         (float)to_float(v[3]), (int)M, (int)d, (float)to_float(v[4]), ts, ws, stream()),
-        "ln_amax_scale");
+  launch("ln_amax_scale", kf_ln_amax_scale, dtype_code(x.scalar_type()), x.data_ptr(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")),
+         (float)to_float(v[3]), (int)M, (int)d, (float)to_float(v[4]), ts, ws, stream());
   return new_ref(v[5]);
 }
 
@@ -501,9 +525,8 @@ PyObject* ln_rows(PyObject* const* v) {
   const int64_t d = x.size(-1), M = rows_of(x, d, "ln_rows: x has a last dimension of 0");
   const int dt = (int)to_int(v[4]);
   at::Tensor y = empty(x.sizes(), dtype_of(dt), x.device());
-  check(kf_ln_rows(x.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")), (float)to_float(v[3]), (int)M, (int)d, dt,
-                   y.data_ptr(), stream()),
-        "ln_rows");
+  launch("ln_rows", kf_ln_rows, x.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")), (float)to_float(v[3]), (int)M, (int)d, dt,
+         y.data_ptr(), stream());
   return THPVariable_Wrap(std::move(y));
 }
 
@@ -514,7 +537,7 @@ PyObject* broadcast_rows(PyObject* const* v) {
            src.size(-1) == dst.size(2),
        "broadcast_rows: src [R, d] and dst [B, Ntok, d] must be contiguous fp32");
   const int64_t d = dst.size(2), R = rows_of(src, d, "broadcast_rows: src and dst have a last dimension of 0");
-  check(kf_broadcast_rows(src.data_ptr<float>(), dst.data_ptr<float>(), (int)R, (int)d, (int)dst.size(0), dst.size(1) * d, to_int(v[2]), stream()), "broadcast_rows");
+  launch("broadcast_rows", kf_broadcast_rows, src.data_ptr<float>(), dst.data_ptr<float>(), (int)R, (int)d, (int)dst.size(0), dst.size(1) * d, to_int(v[2]), stream());
   return new_ref(v[1]);
 }
 
@@ -538,9 +561,8 @@ PyObject* ln_tail(PyObject* const* v) {
     bcls = bc.data_ptr<float>();
     cl = empty({B * Q, wc.size(0)}, at::kBFloat16, x.device());
   }
-  check(kf_ln_tail(x.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")), (float)to_float(v[3]), (int)B, (int)Ntok,
-                   (int)Q, (int)npre, (int)d, qb.data_ptr(), xb.data_ptr(), wcls, bcls, ncls1, ncls1 ? cl.data_ptr() : nullptr, stream()),
-        "ln_tail");
+  launch("ln_tail", kf_ln_tail, x.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[1], "w")), static_cast<const float*>(opt_ptr(v[2], "b")), (float)to_float(v[3]), (int)B, (int)Ntok,
+         (int)Q, (int)npre, (int)d, qb.data_ptr(), xb.data_ptr(), wcls, bcls, ncls1, ncls1 ? cl.data_ptr() : nullptr, stream());
   if (!ncls1) return pair(std::move(qb), std::move(xb));
   PyObject* t = PyTuple_New(3);
   PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(qb)));
@@ -562,7 +584,7 @@ PyObject* attn_fwd(PyObject* const* v) {
   const int64_t B = qkv.size(1), N = qkv.size(2), H = qkv.size(3);
   at::Tensor out = v[2] == Py_None ? empty({B, N, H * 64}, qkv.scalar_type(), qkv.device()) : cuda_tensor(v[2], "out");
   if (v[2] != Py_None) writable(out);
-  check(kf_attn_fwd(dtype_code(qkv.scalar_type()), qkv.data_ptr(), out.data_ptr(), (int)B, (int)N, (int)H, (float)to_float(v[1]), stream()), "attn_fwd");
+  launch("attn_fwd", kf_attn_fwd, dtype_code(qkv.scalar_type()), qkv.data_ptr(), out.data_ptr(), (int)B, (int)N, (int)H, (float)to_float(v[1]), stream());
   return v[2] == Py_None ? THPVariable_Wrap(std::move(out)) : new_ref(v[2]);
 }
 
@@ -574,9 +596,8 @@ PyObject* attn_fwd_quant(PyObject* const* v) {
   if (out.rows != B * N || out.K != H * 64)
     fail("attn_fwd_quant: out must be [%lld, %lld], got [%lld, %lld]", (long long)(B * N), (long long)(H * 64), (long long)out.rows, (long long)out.K);
   writable(out);
-  check(kf_attn_fwd_quant(dtype_code(qkv.scalar_type()), qkv.data_ptr(), (int)B, (int)N, (int)H, (float)to_float(v[2]), out.fmt, out.pq, out.psf,
-                          static_cast<const float*>(out.pts), (int)to_int(v[3]), stream()),
-        "attn_fwd_quant");
+  launch("attn_fwd_quant", kf_attn_fwd_quant, dtype_code(qkv.scalar_type()), qkv.data_ptr(), (int)B, (int)N, (int)H, (float)to_float(v[2]), out.fmt, out.pq, out.psf,
+         static_cast<const float*>(out.pts), (int)to_int(v[3]), stream());
   return new_ref(v[1]);
 }
 
@@ -588,7 +609,7 @@ PyObject* im2col_patch16(PyObject* const* v) {
        "im2col_patch16: x must be contiguous bf16 [B, 3, S, S]");
   const int64_t B = x.size(0), S = x.size(2), g = S / 16;
   at::Tensor out = empty({B * g * g, 768}, at::kBFloat16, x.device());
-  check(kf_im2col_patch16(x.data_ptr(), out.data_ptr(), (int)B, (int)S, stream()), "im2col_patch16");
+  launch("im2col_patch16", kf_im2col_patch16, x.data_ptr(), out.data_ptr(), (int)B, (int)S, stream());
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -601,9 +622,8 @@ PyObject* dw_ln(PyObject* const* v) {
            (v[1] != Py_None || pre),
        "dw_ln: g must be contiguous bf16 [B*Hs*Ws, 4C] and dww fp32 [9, C]");
   at::Tensor out = empty({B, 2 * Hs, 2 * Ws, C}, at::kBFloat16, g.device());
-  check(kf_dw_ln(g.data_ptr(), static_cast<const float*>(opt_ptr(v[1], "bias")), dww.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[3], "lnw")),
-                 static_cast<const float*>(opt_ptr(v[4], "lnb")), out.data_ptr(), (int)B, (int)Hs, (int)Ws, (int)C, (float)to_float(v[8]), pre ? 1 : 0, stream()),
-        "dw_ln");
+  launch("dw_ln", kf_dw_ln, g.data_ptr(), static_cast<const float*>(opt_ptr(v[1], "bias")), dww.data_ptr<float>(), static_cast<const float*>(opt_ptr(v[3], "lnw")),
+         static_cast<const float*>(opt_ptr(v[4], "lnb")), out.data_ptr(), (int)B, (int)Hs, (int)Ws, (int)C, (float)to_float(v[8]), pre ? 1 : 0, stream());
   return THPVariable_Wrap(std::move(out));
 }
 
@@ -616,8 +636,7 @@ PyObject* semantic(PyObject* const* v) {
   const bool want = truth(v[2]);
   at::Tensor labels = empty({B, h, w}, at::kByte, ml.device()), scores;
   if (want) scores = empty({B, ncls1, h, w}, at::kFloat, ml.device());
-  check(kf_semantic(ml.data_ptr(), cl.data_ptr(), (int)B, (int)Q, (int)ncls1 - 1, (int)(h * w), want ? scores.data_ptr<float>() : nullptr, labels.data_ptr<uint8_t>(), stream()),
-        "semantic");
+  launch("semantic", kf_semantic, ml.data_ptr(), cl.data_ptr(), (int)B, (int)Q, (int)ncls1 - 1, (int)(h * w), want ? scores.data_ptr<float>() : nullptr, labels.data_ptr<uint8_t>(), stream());
   if (want) return pair(std::move(labels), std::move(scores));
   PyObject* t = PyTuple_New(2);
   PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(labels)));

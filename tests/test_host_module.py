@@ -122,3 +122,49 @@ def test_containers_with_property_attributes():
     for _ in range(20):
         assert torch.equal(ops.gemm_plain(Fresh(a), Fresh(W)), want)
     ops.check_device_error()
+
+
+@gpu
+def test_other_threads_run_while_a_launch_waits():
+    """a launch blocks while the queue of its stream is full; another Python thread runs meanwhile.  One fp64 product of a few tenths of a second, then
+    more launches than the queue holds: the longest gap between the other thread's steps stays far below the longest launch."""
+    import threading
+    import time
+
+    from lightly_trian_quant_b200 import ops
+
+    n = 16384
+    big = torch.ones(n, n, dtype=torch.float64, device="cuda")
+    out = torch.empty_like(big)
+    x = torch.randn(128, 256, device="cuda")
+    buf = ops.ActBuf(128, 256, "mx8")
+    ops.quant_rows(x, buf)
+    torch.mm(big[:256], big, out=out[:256])                   # the library's first call is out of the way
+    torch.cuda.synchronize()
+    gaps, stop = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps[0] = max(gaps[0], now - last)
+            last = now
+
+    t = threading.Thread(target=tick)
+    t.start()
+    longest = 0.0
+    try:
+        torch.mm(big, big, out=out)
+        for _ in range(3000):
+            t0 = time.perf_counter()
+            ops.quant_rows(x, buf)
+            longest = max(longest, time.perf_counter() - t0)
+    finally:
+        stop.set()
+        t.join()
+    torch.cuda.synchronize()
+    ops.check_device_error()
+    print(f"longest launch {longest * 1e3:.0f} ms, longest gap of the other thread {gaps[0] * 1e3:.1f} ms")
+    assert longest > 0.05, "the queue never filled: the test shows nothing"
+    assert gaps[0] < 0.5 * longest
