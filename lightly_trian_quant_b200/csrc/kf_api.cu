@@ -24,15 +24,20 @@ int cuda_status(cudaError_t e, const char* what) {
 }
 
 // Programmatic dependent launch is taken where the launches are short: the successor's start-up (about 2 us of launch, barrier and
-// tensor-memory set-up) then runs under its predecessor.  Measured, whole models, plain -> dependent: ViT-B 256 px called eagerly
-// 782 -> 635 us, ViT-L 640 px one frame captured 1950 -> 1883 us; ViT-B 640 px eager, three images, 2298 -> 2052 us (launch gaps
-// of the eager stream); captured graphs of 3210 rows are level and of 6420 rows and more 1 to 2 % slower, hence the two lines.
+// tensor-memory set-up) then runs under its predecessor.  Over many rows the successor's CTAs, waiting on the SMs, cost more than that.
+// Outside a capture it also hides the launch gaps of the stream, so the line lies higher.  Whole models of 640 px images, change of the time from
+// plain to dependent (ViT-B MXFP8 / ViT-L NVFP4 / ViT-B bf16):
+//   rows        1605               3210           4815               6420   9630          12 840         16 050        19 260
+//   captured    -8.3 -7.3 -2.7 %   -3.2 -1.7 %    -4.2 -1.5 -0.8 %   +1.0   +2.5 +2.6 %   +2.3    +1.0   +3.3 +1.8 %   +4.3 +3.3 +1.9 %
+//   eager       -22 -20 -15 %      -12 -11 %      -12 -8.4 -8.8 %    -5.3   -4.2 -2.0 %   -1.1    -2.3   +0.0 +0.4 %   +2.4 +1.7 +0.4 %
+// and ViT-B 256 px (261 rows) eager 846 -> 612 us.
+constexpr int64_t PDL_ROWS_CAPTURED = 5120, PDL_ROWS_EAGER = 14336;
 static std::atomic<int> g_pdl{KF_PDL_AUTO};            // kf_set_pdl
 bool pdl_for(int64_t rows, cudaStream_t st) {
   const int mode = g_pdl.load(std::memory_order_relaxed);
   if (mode != KF_PDL_AUTO) return mode == KF_PDL_ALL;
-  if (rows <= 2048) return true;
-  if (rows > 20480) return false;
+  if (rows <= PDL_ROWS_CAPTURED) return true;
+  if (rows > PDL_ROWS_EAGER) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }

@@ -392,3 +392,34 @@ def test_early_reads_give_plain_stream_order(dtype):
             for got, want in zip(outputs(fmt), ref):
                 assert torch.equal(got, want)
     ops.check_device_error()
+
+
+def test_dependent_launch_lines_by_rows():
+    """the choice by rows, inside and outside a capture, at its lines; a model between them gives the bits of plain stream order in both forms."""
+    from lightly_trian_quant_b200 import _lib
+
+    modeldef, ops, stack = _mods()
+    L = _lib.lib()
+    rows = (1, 5120, 5121, 14336, 14337)
+    choices = lambda: [L.kf_pdl_choice(r, torch.cuda.current_stream().cuda_stream) for r in rows]  # noqa: E731
+    ops.set_pdl(None)
+    assert choices() == [1, 1, 1, 1, 0]
+    cfg = modeldef.EoMTConfig(**TINY)
+    fn, _ = stack.make_variant("tiny", modeldef.build_model(cfg, 0, "stress", "cuda"), "b200_nv4+s64")
+    x = torch.rand(170, 3, 64, 64, generator=torch.Generator().manual_seed(9)).to(BF).cuda()      # 3570 rows, 9010 with the queries
+    fn(x)
+    ops.set_pdl(False)
+    ref = [t.clone() for t in fn(x)]
+    ops.set_pdl(None)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        inside = choices()
+        out = fn(x)
+    assert inside == [1, 1, 0, 0, 0]
+    for _ in range(10):
+        graph.replay()
+        assert torch.equal(out[0], ref[0]) and torch.equal(out[1], ref[1])
+        eager = fn(x)
+        assert torch.equal(eager[0], ref[0]) and torch.equal(eager[1], ref[1])
+    ops.check_device_error()
