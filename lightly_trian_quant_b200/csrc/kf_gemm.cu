@@ -408,8 +408,15 @@ static int gemm_columns(int fmt, int epi, int m_tiles, int N, int sms) {
 
 // RES launches that move the residual through shared memory (128-column tiles): those of many rounds, where its bandwidth counts
 // and the box of the next tile travels under the present one.
-// Not for a long K: the 128-column tiles then cost more operand traffic than the boxes save (M = 22 470, NVFP4: K 1024, 4 stages,
-// 45 -> 33 us, but K 4096, 16 stages, 67 -> 77 us; MXFP8 x 768: K 768, 6 stages, 38.6 -> 27.6, K 3072, 24 stages, 64.7 -> 77).
+// Not for a long K: the 128-column tiles then cost more operand traffic than the boxes save.  Without -> with boxes, in place, operands from HBM,
+// us at M = 9630, 22 470 and 51 360:
+//    4 stages  NVFP4 1024 x 1024   26.8 -> 20.8   47.4 -> 37.3   97.6 -> 76.8
+//    6 stages  MXFP8  768 x  768   24.7 -> 21.1   41.3 -> 36.6   80.5 -> 70.8
+//    8 stages  MXFP8 1024 x 1024   30.7 -> 30.0   55.6 -> 56.2  116.8 -> 112.4     NVFP4 1024 x 2048  33.6 -> 32.5  60.5 -> 61.2  120.4 -> 116.6
+//   10 stages  MXFP8 1024 x 1280   33.9 -> 34.1   62.6 -> 63.8  127.8 -> 130.2
+//   12 stages  bf16   768 x  768   31.9 -> 30.5   55.8 -> 55.6  107.2 -> 109.3     NVFP4  768 x 3072  34.9 -> 31.9  60.6 -> 59.5  109.5 -> 116.8
+//   16 stages  NVFP4 1024 x 4096   41.0 -> 45.9   74.7 -> 88.5  157.4 -> 176.9
+// Faster up to 6 stages, level at 8, with the sign changing from row count to row count up to 12, slower from there: the line is after 8.
 static bool gemm_res_boxes(int k_tiles, int m_tiles, int N, int sms) { return k_tiles <= 8 && (int64_t)m_tiles * (N / 128) >= 3 * (int64_t)sms; }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
