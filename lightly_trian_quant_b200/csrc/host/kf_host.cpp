@@ -6,7 +6,7 @@
 // Here an operator costs its launch (about 2 us), one allocation where it returns a new tensor and about 1 us for the rest.
 //
 // Containers are the Python ones: an operand is any object with the attributes M, K, fmt, q, sf, ts (ops.ActBuf), a weight any
-// object with N, K, fmt, q, sf, ts (ops.QWeight).  Errors are KfError of the package.
+// object with N, K, fmt, q, sf, ts and optionally settled (ops.QWeight).  Errors are KfError of the package.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 

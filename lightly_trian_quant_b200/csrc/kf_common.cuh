@@ -22,7 +22,8 @@ bool pdl_for(int64_t rows, cudaStream_t st);   // programmatic dependent launch 
 // Programmatic dependent launch: a kernel lets its successor's CTAs start on SMs it no longer occupies (its partial last
 // wave, its teardown) and the successor runs its prologue (barrier set-up, TMEM allocation, descriptor prefetch) there; the
 // successor must not touch global memory before pdl_wait(), which returns when every predecessor grid has completed
-// and its writes are visible.  Both are no-ops for a kernel launched without the attribute.
+// and its writes are visible; the exceptions are parameters whose writes the caller vouches for (KF_G_W_STATIC,
+// KF_Q_STATIC_AFFINE).  Both are no-ops for a kernel launched without the attribute.
 // Where a kernel signals: LayerNorm + quantise and attention on entry (their successors are GEMMs, which find no room on an SM before
 // its CTA leaves), the GEMM at the end of its work (a successor's CTAs that wait beside it slow it down: ViT-B 256 px eager 687 us with
 // the signal on entry, 635 us at the end), the short streaming kernels not at all (the end of the grid is the signal).

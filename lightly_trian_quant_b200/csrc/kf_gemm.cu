@@ -25,7 +25,7 @@
 //              ROPE   bias + rotary embedding of q,k + relayout      -> bf16 | f16 [3,B,Ntok,H,64]   (qkv)
 //              QUANT  gelu(acc*ts + bias) quantised again            -> codes [M,N] + blocked scales (fc1 -> fc2)
 //              all four work in the TMEM row layout (a thread owns 64 consecutive columns of one row) and touch global
-//              memory in whole 32-byte sectors (kf_gemm_epi.cuh)
+//              memory in whole 32-byte sectors or 128-byte lines (kf_gemm_epi.cuh)
 //
 // Replaces (reference checkout paths): infer-opt/round13_mxfp8_full/impl/mgx_core.cu:118-444 (MXFP8, mma.sync) and
 // infer-opt/round14_fp4_full/impl/fp4g_core.cu:153-470 (NVFP4 / MXFP4, mma.sync); epilogue math per
@@ -111,7 +111,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // Set-up done: from here on global memory of the predecessors is read and written.  The producer may ask for weights first.
+  // Set-up done: from here on global memory of the predecessors is read and written.  Ahead of the wait the producer reads only the
+  // error word and weights that KF_G_W_STATIC vouches for.
   const bool w_early = (g.flags & KF_G_W_STATIC) != 0;
   if (warp != 0 || !w_early) pdl_wait();
   const uint32_t tmem_base = *tmem_holder;

@@ -6,9 +6,11 @@
 // Every epilogue works in the layout tcgen05.ld delivers: thread `lane` of a warp owns 64 consecutive columns of ONE
 // output row.  That is 128 contiguous bytes of a 16-bit output (exactly one [token, head] row of the q/k/v layout) or
 // 256 contiguous bytes of an fp32 one, which the thread moves with 256-bit global loads / stores (ld/st.global.v8): every
-// access is a whole 32-byte sector, so nothing is restaged through shared memory; the only shared memory the epilogue
-// warps use holds the bias (and LayerScale) values: the whole vector of the launch, loaded once per CTA, or a 64-value
-// slice per warp and tile where the operand ring leaves no room for the vector.
+// access is a whole 32-byte sector.  Two forms exchange data to move whole 128-byte lines instead: ROPE transposes the pieces of every
+// four rows between lanes (store_rows128), RES launches of many rounds and a short K update the residual in shared memory, where
+// it comes and goes as TMA boxes (epilogue_res_tma).  Shared memory also holds the bias (and LayerScale) values, the whole vector of
+// the launch, loaded once per CTA, or a 64-value slice per warp and tile where the operand ring leaves no room for the vector, and
+// for ROPE the rotary-table rows of the tile.
 #pragma once
 #include "kf_sm100.cuh"
 

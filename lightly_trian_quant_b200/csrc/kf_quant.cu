@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI
   constexpr bool BLK16 = FMT == KF_FMT_NV4 && NV == 4;   // d = 1024 in NVFP4: a lane owns whole 16-value blocks
   constexpr int LAY = BLK16 ? LAY_BLK16 : LAY_SWAP;
   float ww[NV][8], bb[NV][8];
-  // the affine parameters of a model are no predecessor's output: their L2 round trip runs under the predecessor's end
+  // affine parameters whose writes the caller vouches for: their L2 round trip runs under the predecessor's end
   const bool early = (flags & KF_Q_STATIC_AFFINE) != 0;
   if (early) ln_affine_load<NV, LAY>(w, b, lane, ww, bb);
   pdl_wait();                                     // from here on global memory of the predecessors is read and written
