@@ -493,6 +493,10 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
   };
   if (boxed) box_load(blockIdx.x);
   int lt = 0;
+  // ROPE: the four warps of a quarter meet at named barriers, which have no limit.  A warp whose wait ran out therefore does not leave: it
+  // keeps company at the barriers of its remaining tiles (the same number in all four warps: they depend on the tile only) and
+  // stores nothing.
+  bool live = true;
   for (int idx = blockIdx.x; idx < g.items; idx += gridDim.x, ++lt) {
     const WorkItem item = work_item<BN>(g, idx);
     int row_end;
@@ -513,7 +517,8 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
 #pragma unroll
       for (int c = 0; c < 4; ++c) res[c] = ldg8_stream(g.R + (size_t)(rbase + lane) * g.N + n0 + 8 * c);
     }
-    if (!mbar_wait(&tfull[acc], (lt / ACCS) & 1, ctx, 4)) break;
+    if (EPI == KF_EPI_ROPE) live = live && mbar_wait_warp(&tfull[acc], (lt / ACCS) & 1, ctx, 4);
+    else if (!mbar_wait(&tfull[acc], (lt / ACCS) & 1, ctx, 4)) break;
     tc_fence_after();
     __syncwarp();
     if constexpr (W == 64) {
@@ -536,7 +541,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
       rope_slab_store(slab, cg * 32 + lane, tab);
       quarter_barrier(quarter);
     }
-    if (n0 >= g.N || col >= item.cols) continue;               // column group past N in the last column tile, or past a half tile
+    if (!live || n0 >= g.N || col >= item.cols) continue;      // column group past N in the last column tile, or past a half tile
     if constexpr (EPI == KF_EPI_RES && W == 32) {
       if (boxed) {
         if (rbase < g.M) {

@@ -413,13 +413,14 @@ def test_a_failed_predecessor_does_not_stall_the_launch(M, K, delay):
     W = ops.QWeight(torch.randn(N, K, generator=g, device="cuda") * 0.02, "nv4")
     bias = torch.randn(N, generator=g, device="cuda")
     res = torch.randn(M, N, generator=g, device="cuda")
-    tab = torch.randn(2, Ntok, 64, generator=g, device="cuda")
+    tab = torch.randn(2, Ntok, 32, generator=g, device="cuda").repeat(1, 1, 2)
     out = ops.ActBuf(M, N, "nv4")
     qkv = torch.randn(3, M // Ntok, Ntok, H, 64, generator=g, device="cuda").bfloat16()
     calls = [
         lambda: ops.gemm_plain(a, W, bias),
         lambda: ops.gemm_res(a, W, bias, bias, res),
         lambda: ops.qkv_rope(a, W, bias, tab[0], tab[1], Ntok, 0, H),
+        lambda: ops.qkv_rope(a, W, bias, tab[0], tab[1], Ntok, 0, H, half_tables=True),      # four warps meet at named barriers per tile
         lambda: ops.gemm_gelu_q(a, W, bias, out).q.clone(),
         lambda: ops.attn_fwd(qkv),
     ]
