@@ -3,31 +3,36 @@
 //
 //   input    qkv [3, B, N, H, 64] bf16 | f16 (the physical layout the qkv GEMM epilogue writes)
 //   output   O [B, N, H*64] bf16 | f16, or directly the quantised operand of the proj GEMM (kf_attn_fwd_quant)
-//   CTA      persistent, two per SM; an item is 128 query rows of one (batch, head), key tiles of 64; a CTA takes the
+//   CTA      persistent, two per SM; an item is 128 query rows of one (batch, head), key tiles of 96; a CTA takes the
 //            items blockIdx.x, blockIdx.x + gridDim.x, ... and keeps every barrier phase running across them
 //   roles    warps 0..3: softmax, one query row per thread (tcgen05.ld of the S row, running max / sum in fp32,
-//            P -> 16 bit -> tensor memory by tcgen05.st); warp 4: TMA producer (Q in two buffers, K and V in 4-deep
+//            P -> 16 bit -> tensor memory by tcgen05.st); warp 4: TMA producer (Q in two buffers, K and V in 3-deep
 //            rings, 4-D tensor maps so rows past N read zero); warp 5 issues the products (S = Q K^T: 4 MMAs of K=16
-//            from shared memory; O += P V: 4 MMAs of K=16 with P as the A operand from tensor memory and V as the
+//            from shared memory; O += P V: 6 MMAs of K=16 with P as the A operand from tensor memory and V as the
 //            MN-major B operand); warps 6 and 7 idle (they complete the second warp group, whose registers setmaxnreg
-//            hands to the softmax warps: 200 against 56).
-//   pipeline three S buffers in tensor memory, P(j) written over the first half of S(j); O accumulates over all key
-//            tiles.  One thread issues PV(j) and then S(j+3) into the same buffer: the tensor core runs them in order,
-//            so nothing waits for PV(j) to complete, and S runs two steps ahead of the softmax, also across the end of an
-//            item (the next item's Q and first K tiles are loaded by then).  The softmax warps request the next S row as
-//            soon as the registers of the present one are free and ask for its barrier half a step before they look at
-//            the answer: what bounds the kernel is their instruction stream (two of them per scheduler take 983 clk per
-//            64-key step of both in a loop of nothing else, ~1150 here: the exponentials' unit is busy for 768 of them).
+//            hands to the softmax warps: 208 against 48).
+//   pipeline two S buffers in tensor memory, P(j) written over the first half of S(j); O accumulates over all key
+//            tiles.  One thread issues PV(j) and then S(j+2) into the same buffer: the tensor core runs them in order,
+//            so nothing waits for PV(j) to complete, also across the end of an item (the next item's Q and first K tiles
+//            are loaded by then).  The softmax warps request two thirds of the next S row when two thirds of the present one
+//            are used up, and ask for its barrier a third of a step before they look at the answer.  What bounds the kernel is their
+//            instruction stream: two of them per scheduler take 1242 clk per 96-key step in a loop of nothing else (the
+//            exponentials' unit: 1152), ~1660 here, where waits, S loads, the check of the row sum and the hand-over of P add
+//            ~400 clk to every step of a warp, whatever its width.  That is why a step has 96 keys: with 64 (three S buffers, S two steps
+//            ahead, the same tensor memory) a third more of them were paid; 128 leave no room for a second S buffer, and a last
+//            tile of 128 pads the model's token counts more (1605 keys: 1632 with tiles of 96, 1664 with 64 or 128).
 //            The exponentials of a tile
 //            use the running maximum as it is; the tile's own row sum tells whether that was safe (below 2^15 no
 //            element exceeded 2^15), so no maximum is tracked in the common case; only a row whose sum came out larger
 //            finds its maximum, recomputes its P and has its O rescaled (TMEM load, multiply, store), which happens on
 //            the first tiles and then almost never; the O barriers are waited only then and at the end of an item.
-//            Measured (B 14, H 16, NVFP4 out, N 1605 / 1805; B 8, N 4101, f16, MXFP4 out; B 1, N 1605): 200 / 246 / 664 /
-//            25.8 us, against 214 / 264 / 691 / 28.3 us with an issuing warp for each product and S(j+2) behind the
-//            completion of PV(j).  Level with that, and not kept: four CTAs per SM with one S buffer each (202 / 245 /
-//            680 / 34 us), two softmax warps per row with an O each (209 / 258 / 673 / 28 us); the end of a step spread
-//            over the exponentials of the next one broke those into pieces too small to overlap (241 / 296 / 793 / 35 us).
+//            Measured, tiles of 64 -> 96 keys (B 14, H 16, N 1605, bf16 out / NVFP4 out; N 1805, NVFP4 out; B 8, N 4101, f16,
+//            MXFP4 out; B 1, N 1605, NVFP4 out): 199 -> 186 / 204 -> 194 / 250 -> 239 / 667 -> 636 / 24.7 -> 23.6 us.
+//            Not kept: the barrier asked for only where it is waited on (198 us against 194), the next row requested at the end of the
+//            step (199), five of sixteen pairs or none of every third 32 off the special-function unit (202, 202), an item's output behind the
+//            first step of the next one (203: the waits it hides are fewer than the registers it takes from the loop); with
+//            tiles of 64: four CTAs per SM with one S buffer each, two softmax warps per row with an O each, the end of a step
+//            spread over the exponentials of the next one (level or slower).
 //   numerics softmax scale 1/8 folded into exp2 (fp32; three of every four element pairs by the special-function unit,
 //            the fourth by a cubic on the FMA pipe: the unit is shared by the softmax warps of both CTAs and is the
 //            busiest pipe of the step; more than a quarter costs more issue slots than it frees); the exponent
@@ -43,18 +48,19 @@
 
 namespace kf {
 
-constexpr int AT_BM = 128, AT_BN = 64, AT_D = 64;
+constexpr int AT_BM = 128, AT_BN = 96, AT_D = 64;
 constexpr int AT_THREADS = 256;                        // warps 0..3 softmax, 4 TMA, 5 MMA issuer, 6 and 7 idle
-constexpr int AT_REGS_SOFTMAX = 200, AT_REGS_LEAN = 56; // 128 * 200 + 128 * 56 <= 256 * 128, the allocation at launch
-constexpr int AT_KV = 4;                               // K / V ring depth
+constexpr int AT_REGS_SOFTMAX = 208, AT_REGS_LEAN = 48; // 128 * 208 + 128 * 48 <= 256 * 128, the allocation at launch
+constexpr int AT_KV = 3;                               // K / V ring depth
 constexpr int AT_QTILE = AT_BM * AT_D * 2;             // 16 KB
-constexpr int AT_KTILE = AT_BN * AT_D * 2;             // 8 KB
+constexpr int AT_KTILE = AT_BN * AT_D * 2;             // 12 KB
 constexpr int AT_OFF_Q = 0, AT_OFF_K = 2 * AT_QTILE, AT_OFF_V = AT_OFF_K + AT_KV * AT_KTILE, AT_OFF_BAR = AT_OFF_V + AT_KV * AT_KTILE;
 constexpr size_t AT_SMEM = (size_t)AT_OFF_BAR + 256;
 constexpr float AT_SUM_LIMIT = 32768.f;                  // a tile's row sum above this sends the row to the exact-maximum path (the largest finite f16 is 65504)
 constexpr int AT_POLY_K = 3;                             // element pairs AT_POLY_K .. 3 of every four take the polynomial exponential
-constexpr int AT_SBUF = 3;                               // S buffers in tensor memory
-constexpr int AT_TMEM_COLS = 256, AT_COL_S = 0, AT_COL_O = AT_SBUF * 64;   // P (16-bit pairs, 32 columns) replaces the first half of its S buffer
+constexpr int AT_SBUF = 2;                               // S buffers in tensor memory
+constexpr int AT_TMEM_COLS = 256, AT_COL_S = 0, AT_COL_O = AT_SBUF * AT_BN;   // P (16-bit pairs, 48 columns) replaces the first half of its S buffer
+static_assert(AT_COL_O + AT_D <= AT_TMEM_COLS, "TMEM budget");
 
 struct AttnArgs {
   void* O;
@@ -150,7 +156,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int i = 0; i < AT_SBUF; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 128);
-      mbar_init(&o_full[i], 1);                           // PV(G) completes o_full[G % 3]: a waiter is never more than one phase behind
+      mbar_init(&o_full[i], 1);                           // PV(G) completes o_full[G % 2]: a waiter is never more than one phase behind
     }
     *abort_flag = 0u;
     fence_mbar_init();
@@ -182,7 +188,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       prefetch_tmap(&tmK);
       prefetch_tmap(&tmV);
     }
-    uint32_t G = 0;
+    uint32_t st = 0, ph = 1;                                                      // ring slot and the parity of its release
     // Has an earlier launch failed?  The producer alone looks, once: without its loads the other roles' waits end with the abort flag.
     bool ok = !__any_sync(0xffffffffu, *static_cast<volatile unsigned int*>(a.err) != 0u);
     if (!ok) *abort_flag = 1u;
@@ -194,9 +200,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mbar_expect_tx(&q_full[qb], AT_QTILE);
         tma_load_4d(smem + AT_OFF_Q + qb * AT_QTILE, &tmQ, 0, I.h, I.qt * AT_BM, I.b, &q_full[qb]);
       }
-      for (int j = 0; j < n_kt; ++j, ++G) {
-        const int st = G % AT_KV;
-        const uint32_t ph = ((G / AT_KV) & 1) ^ 1;
+      for (int j = 0; j < n_kt; ++j) {
         if (!mbar_wait_warp(&k_empty[st], ph, ctx, 11)) { ok = false; break; }      // S(G - AT_KV) is complete
         if (elect_one()) {
           mbar_expect_tx(&k_full[st], AT_KTILE);
@@ -209,30 +213,35 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tma_load_4d(smem + AT_OFF_V + st * AT_KTILE, &tmV, 0, I.h, j * AT_BN, I.b, &v_full[st]);
         }
         __syncwarp();
+        if (++st == AT_KV) {
+          st = 0;
+          ph ^= 1;
+        }
       }
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    // S(0), S(1), S(2), then PV(G) and S(G + 3) for every step.  All come from one thread, so the tensor core runs them in
-    // order: S(G + 3) overwrites the buffer of P(G) behind PV(G) without a wait for its completion.  A softmax that sees
-    // S(G + 3) complete knows that PV(G) is.  S runs two steps ahead of the softmax: issued one step ahead (two buffers) it
-    // came ~700 clk after the hand-over of P, in the middle of the step that wants to prefetch it.
+    // S(0), S(1), then PV(G) and S(G + 2) for every step.  All come from one thread, so the tensor core runs them in
+    // order: S(G + 2) overwrites the buffer of P(G) behind PV(G) without a wait for its completion.  A softmax that sees
+    // S(G + 2) complete knows that PV(G) is.  S(G + 2) comes ~700 clk after the hand-over of P(G); the softmax asks for it ~1000 clk
+    // into step G + 1.
     const uint32_t idesc_s = idesc_f16(F16 ? 0u : 1u, AT_BN);
     const uint32_t idesc_o = idesc_f16(F16 ? 0u : 1u, AT_D) | (1u << 16);     // B (= V) is MN-major
     const uint32_t t_o = tmem_base + AT_COL_O;
     const uint32_t total = (uint32_t)n_my * (uint32_t)n_kt;                  // key-tile steps of this CTA over all its items
     const bool leader = elect_one();
     uint32_t s_it = 0, s_j = 0;                                              // item and key tile of the next S product
-    auto issue_s = [&](uint32_t G, uint32_t buf) {
+    uint32_t k_st = 0, k_ph = 0;                                             // its slot in the K ring and the parity of the load
+    auto issue_s = [&](uint32_t buf) {
       const uint64_t qdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_Q + (s_it & 1) * AT_QTILE));
-      const uint64_t kdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_K + (G % AT_KV) * AT_KTILE));
+      const uint64_t kdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_K + k_st * AT_KTILE));
       const uint32_t t_s = tmem_base + AT_COL_S + buf * AT_BN;
       const bool last = s_j + 1 == (uint32_t)n_kt;
       if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) mma_f16(t_s, qdesc + 2 * kk, kdesc + 2 * kk, idesc_s, kk != 0);
+        for (int kk = 0; kk < AT_D / 16; ++kk) mma_f16(t_s, qdesc + 2 * kk, kdesc + 2 * kk, idesc_s, kk != 0);
         tc_commit(&s_full[buf]);
-        tc_commit(&k_empty[G % AT_KV]);
+        tc_commit(&k_empty[k_st]);
         if (last) tc_commit(&q_empty[s_it & 1]);                             // the item's last S product: its Q buffer is free once it completes
       }
       __syncwarp();
@@ -240,36 +249,48 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         s_j = 0;
         ++s_it;
       }
+      if (++k_st == AT_KV) {
+        k_st = 0;
+        k_ph ^= 1;
+      }
     };
     bool ok = true;
     for (uint32_t G = 0; G < AT_SBUF && G < total && ok; ++G) {
-      ok = (s_j != 0 || mbar_wait_warp(&q_full[s_it & 1], (s_it >> 1) & 1, ctx, 12)) && mbar_wait_warp(&k_full[G], 0, ctx, 13);
+      ok = (s_j != 0 || mbar_wait_warp(&q_full[s_it & 1], (s_it >> 1) & 1, ctx, 12)) && mbar_wait_warp(&k_full[k_st], k_ph, ctx, 13);
       tc_fence_after();
-      if (ok) issue_s(G, G);
+      if (ok) issue_s(G);
     }
     uint32_t j = 0, buf = 0, pph = 0;                                        // buffer of step G and the parity of its P barrier
+    uint32_t st = 0, vph = 0;                                                // V ring
     for (uint32_t G = 0; G < total && ok; ++G) {
-      const uint32_t st = G % AT_KV, g3 = G + AT_SBUF;
-      const bool more = g3 < total;
+      const bool more = G + AT_SBUF < total;
       if (more && s_j == 0 && !mbar_wait_warp(&q_full[s_it & 1], (s_it >> 1) & 1, ctx, 12)) break;
-      // P(G), V(G) and K(G + 3), asked for together: a barrier costs a round trip of 60 clk also when its phase is complete
-      if (!mbar_wait_warp3(&p_full[buf], pph, &v_full[st], (G / AT_KV) & 1, &k_full[(more ? g3 : G) % AT_KV], ((more ? g3 : G) / AT_KV) & 1, ctx, 14)) break;
+      // P(G), V(G) and the K tile of S(G + 2), asked for together: a barrier costs a round trip of 60 clk also when its phase is complete
+      if (more) {
+        if (!mbar_wait_warp3(&p_full[buf], pph, &v_full[st], vph, &k_full[k_st], k_ph, ctx, 14)) break;
+      } else {
+        if (!mbar_wait_warp3(&p_full[buf], pph, &v_full[st], vph, &v_full[st], vph, ctx, 14)) break;
+      }
       tc_fence_after();
       const uint32_t t_p = tmem_base + AT_COL_S + buf * AT_BN;
       const uint64_t vdesc = smem_desc_sw128(smem_u32(smem + AT_OFF_V + st * AT_KTILE));
       if (leader) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)         // A: 16 keys = 8 TMEM columns of P; B: 16 key rows of V = two 8-row groups of 1024 bytes
+        for (int kk = 0; kk < AT_BN / 16; ++kk)  // A: 16 keys = 8 TMEM columns of P; B: 16 key rows of V = two 8-row groups of 1024 bytes
           mma_f16_ta(t_o, t_p + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (j | (uint32_t)kk) != 0);
         tc_commit(&o_full[buf]);
         tc_commit(&v_empty[st]);
       }
       __syncwarp();
-      if (more) issue_s(g3, buf);
+      if (more) issue_s(buf);
       if (++j == (uint32_t)n_kt) j = 0;
       if (++buf == AT_SBUF) {
         buf = 0;
         pph ^= 1;
+      }
+      if (++st == AT_KV) {
+        st = 0;
+        vph ^= 1;
       }
     }
   }   // warps 6 and 7 are idle: they complete the second warp group, whose registers go to the softmax warps
@@ -317,12 +338,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const Item I = item_of(it);
     const int qt = I.qt, h = I.h, b = I.b;
     float m_run = 0.f, l_run = 0.f;
-    uint32_t ra[32], rb[32];                                     // the S row of this step: keys 0..31 and 32..63 of the tile
+    uint32_t ra[32], rb[32], rc[32];                             // the S row of this step: keys 0..31, 32..63 and 64..95 of the tile
     ok = mbar_wait(&s_full[buf], sph, ctx, 17);
     if (!ok) break;
     tc_fence_after();
     tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
     tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
+    tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 64, rc);
     for (int j = 0; j < n_kt; ++j) {
       const uint32_t t_s = t_lane + AT_COL_S + buf * AT_BN, cur = buf, cph = sph;
       if (++buf == AT_SBUF) {
@@ -331,29 +353,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const bool prefetch = j + 1 < n_kt;                        // the next step of this item
       const int kbase = j * AT_BN;
-      // asked for here, looked at half a step later: S(G + 1) was issued more than a step ago and is nearly always there
-      const bool ready = mbar_test_wait(&s_full[buf], sph);
       tmem_ld_wait();
       tmem_ld_fence(ra);
       tmem_ld_fence(rb);
+      tmem_ld_fence(rc);
       if (kbase + AT_BN > a.N) {
         mask_tail(ra, kbase);
         mask_tail(rb, kbase + 32);
+        mask_tail(rc, kbase + 64);
       }
-      if (j == 0) m_run = row_max(rb, row_max(ra, -INFINITY));
+      if (j == 0) m_run = row_max(rc, row_max(rb, row_max(ra, -INFINITY)));
       const float2 mn2 = splat2(-m_run * sc);
       float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-      uint32_t w[32];
+      uint32_t w[48];
       exp_half(ra, w, mn2, s0, s1);
+      // asked for here, looked at a third of a step later: S(G + 1) was issued at the end of the last step
+      const bool ready = mbar_test_wait(&s_full[buf], sph);
+      exp_half(rb, w + 16, mn2, s0, s1);
       // The next step's S row is requested as soon as the registers of this one are free
       if (prefetch) {
         if (!ready && !mbar_wait(&s_full[buf], sph, ctx, 17)) { ok = false; break; }
         __syncwarp();
         tc_fence_after();
         tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
+        tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
       }
-      exp_half(rb, w + 16, mn2, s0, s1);
-      if (prefetch) tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
+      exp_half(rc, w + 32, mn2, s0, s1);
+      if (prefetch) tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 64, rc);
       // Lazy maximum without a maximum: the exponentials of tile j > 0 use the running maximum as it is, and the tile's
       // own row sum tells whether that was safe: while it stays below 2^15 no element exceeded 2^15 (bf16 / f16 P, the
       // fp32 sums and O have room for that), so the maximum of the tile is not needed at all.  Only a row whose sum came
@@ -365,7 +391,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         uint32_t r[32];
         float mx = m_run;
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < AT_BN / 32; ++c) {
           tmem_ld32(t_s + 32 * c, r);
           tmem_ld_wait();
           tmem_ld_fence(r);
@@ -378,17 +404,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         s0 = s1 = make_float2(0.f, 0.f);
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < AT_BN / 32; ++c) {
           tmem_ld32(t_s + 32 * c, r);
           tmem_ld_wait();
           tmem_ld_fence(r);
           if (kbase + AT_BN > a.N) mask_tail(r, kbase + 32 * c);
           if (c == 0) exp_half(r, w, splat2(-m_run * sc), s0, s1);
-          else exp_half(r, w + 16, splat2(-m_run * sc), s0, s1);
+          else if (c == 1) exp_half(r, w + 16, splat2(-m_run * sc), s0, s1);
+          else exp_half(r, w + 32, splat2(-m_run * sc), s0, s1);
         }
         sum = (s0.x + s0.y) + (s1.x + s1.y);
-        // rescale O in tensor memory: PV(G - 1) must have landed first (j > 0: the first tile's sum is at most 64).  Its
-        // barrier's previous completion, PV(G - 4), is covered by S(G), which this step has read.
+        // rescale O in tensor memory: PV(G - 1) must have landed first (j > 0: the first tile's sum is at most 96).  Its
+        // barrier's previous completion, PV(G - 3), is covered by S(G), which this step has read.
         const uint32_t pb = cur == 0 ? AT_SBUF - 1 : cur - 1;
         if (!mbar_wait(&o_full[pb], cur == 0 ? cph ^ 1 : cph, ctx, 18)) { ok = false; break; }
         tc_fence_after();
@@ -403,12 +430,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
       l_run = l_run * alpha + sum;
-      tmem_st32(t_s, w);                                         // the A operand of the PV product: 64 keys = 32 columns of 16-bit pairs
+      tmem_st32(t_s, *reinterpret_cast<const uint32_t(*)[32]>(w));   // the A operand of the PV product: 96 keys = 48 columns of 16-bit pairs
+      tmem_st16(t_s + 32, w + 32);
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&p_full[cur]);
     }
-    // the item's last PV product; its barrier's previous completion, PV(G - 4), is covered by S(G - 1), which has been read
+    // the item's last PV product; its barrier's previous completion, PV(G - 3), is covered by S(G - 1), which has been read
     if (ok) ok = mbar_wait(&o_full[buf == 0 ? AT_SBUF - 1 : buf - 1], buf == 0 ? sph ^ 1 : sph, ctx, 19);
     const int n = qt * AT_BM + row;
     if (ok) {

@@ -112,9 +112,10 @@ def test_attn_fused_quantise_out(fmt):
     assert np.array_equal(out.sf.cpu().numpy(), qo.to_blocked(es).reshape(-1))
 
 
-@pytest.mark.parametrize("B,N,H", [(1, 1, 1), (40, 1, 16), (40, 64, 16), (3, 65, 2), (40, 128, 9), (2, 129, 3), (1, 192, 2), (20, 193, 16), (1, 257, 5)])
+@pytest.mark.parametrize("B,N,H", [(1, 1, 1), (40, 1, 16), (40, 64, 16), (3, 65, 2), (40, 128, 9), (2, 129, 3), (1, 192, 2), (20, 193, 16), (1, 257, 5), (2, 95, 3), (40, 96, 16), (2, 97, 3), (20, 191, 16),
+                                   (1, 289, 2)])
 def test_attn_tile_edges_and_items_shorter_than_the_pipeline(B, N, H):
-    """token counts around the 64-key and 128-query tiles, and items of one to three key tiles in a CTA that works through
+    """token counts around the 96-key (its 32-key pieces) and 128-query tiles, and items of one to three key tiles in a CTA that works through
     several: S runs ahead of the softmax across item boundaries."""
     ops = _ops()
     g = torch.Generator().manual_seed(B + N)
