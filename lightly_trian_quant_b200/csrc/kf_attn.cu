@@ -362,7 +362,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mask_tail(rb, kbase + 32);
         mask_tail(rc, kbase + 64);
       }
-      if (j == 0) m_run = row_max(rc, row_max(rb, row_max(ra, -INFINITY)));
+      if (j == 0) m_run = row_max(rb, row_max(ra, -INFINITY));
       const float2 mn2 = splat2(-m_run * sc);
       float2 s0 = make_float2(0.f, 0.f), s1 = s0;
       uint32_t w[48];
@@ -384,7 +384,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // own row sum tells whether that was safe: while it stays below 2^15 no element exceeded 2^15 (bf16 / f16 P, the
       // fp32 sums and O have room for that), so the maximum of the tile is not needed at all.  Only a row whose sum came
       // out larger (or infinite) finds its maximum, raises the running maximum, recomputes its P and has its O rescaled.
-      // The first tile has no running maximum yet and finds its own first.
+      // The first tile has no running maximum yet and takes that of its first 64 keys (the 96 of the tile would do: the 64 leave the
+      // bits of P what they were with tiles of 64).
       float sum = (s0.x + s0.y) + (s1.x + s1.y), alpha = 1.f;
       const bool need = sum > AT_SUM_LIMIT;
       if (__any_sync(0xffffffffu, need)) {                    // warp-uniform; S is still in tensor memory: P replaces it only below
@@ -414,19 +415,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           else exp_half(r, w + 32, splat2(-m_run * sc), s0, s1);
         }
         sum = (s0.x + s0.y) + (s1.x + s1.y);
-        // rescale O in tensor memory: PV(G - 1) must have landed first (j > 0: the first tile's sum is at most 96).  Its
-        // barrier's previous completion, PV(G - 3), is covered by S(G), which this step has read.
-        const uint32_t pb = cur == 0 ? AT_SBUF - 1 : cur - 1;
-        if (!mbar_wait(&o_full[pb], cur == 0 ? cph ^ 1 : cph, ctx, 18)) { ok = false; break; }
-        tc_fence_after();
+        // rescale O in tensor memory, where there is one: PV(G - 1) must have landed first.  Its barrier's previous completion,
+        // PV(G - 3), is covered by S(G), which this step has read.
+        if (j > 0) {
+          const uint32_t pb = cur == 0 ? AT_SBUF - 1 : cur - 1;
+          if (!mbar_wait(&o_full[pb], cur == 0 ? cph ^ 1 : cph, ctx, 18)) { ok = false; break; }
+          tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-          tmem_ld32(t_lane + AT_COL_O + 32 * c, r);
-          tmem_ld_wait();
-          tmem_ld_fence(r);
+          for (int c = 0; c < 2; ++c) {
+            tmem_ld32(t_lane + AT_COL_O + 32 * c, r);
+            tmem_ld_wait();
+            tmem_ld_fence(r);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-          tmem_st32(t_lane + AT_COL_O + 32 * c, r);
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+            tmem_st32(t_lane + AT_COL_O + 32 * c, r);
+          }
         }
       }
       l_run = l_run * alpha + sum;

@@ -124,3 +124,21 @@ def test_attn_tile_edges_and_items_shorter_than_the_pipeline(B, N, H):
     ops.check_device_error()
     err = go.rel_fro(out.float().cpu().numpy(), ao.attn_ref(qkv.float().numpy()))
     assert err < 4e-3, err
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lo,N", [(64, 96), (64, 300), (96, 300), (288, 300)])
+def test_attn_larger_logits_behind_the_first_keys(dtype, lo, N):
+    """keys lo .. lo + 31 hold far larger logits than those before (more than 2^15 in the exponent domain): behind the first 64 keys, whose
+    maximum the rows start with, inside the first key tile (no O to rescale yet), and in the following tiles."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(lo + N)
+    qkv = torch.randn(3, 3, N, 2, 64, generator=g)
+    qkv[1, :, lo:lo + 32] *= 12
+    qkv[0, :, ::4] *= 0.05                                  # rows that stay flat
+    qkv = qkv.to(dtype)
+    out = ops.attn_fwd(qkv.cuda())
+    ops.check_device_error()
+    assert torch.isfinite(out).all()
+    err = go.rel_fro(out.float().cpu().numpy(), ao.attn_ref(qkv.float().numpy()))
+    assert err < (4e-3 if dtype == torch.bfloat16 else 1e-3), err
