@@ -103,7 +103,8 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int out_dtype) {
 // Stores the warp's 32 rows of 128 bytes (lane = row, w = its four 32-byte pieces) as whole lines: inside every four lanes the pieces are
 // transposed (4 x 4), then a store instruction covers eight rows of 128 bytes instead of 32 pieces of 32 bytes in 32 lines, whose
 // look-ups had L1 71 % busy in the ROPE epilogue, the unit the operand ring fills through (qkv NVFP4 M = 22 470: 66 -> 60 us, MXFP8
-// x 768 55 -> 52 us).  The same for PLAIN (435 -> 449 us, instruction-bound) and for the residual of RES (level) did not pay.
+// x 768 55 -> 52 us).  PLAIN bf16 NVFP4 x 4096: 78 -> 64 us together with the forms
+// below.  For the residual of RES (level) it did not pay.
 // base: the 128 bytes of row 0; rows from `rows` on are not written.
 __device__ __forceinline__ void store_rows128(uint32_t (&w)[32], uint8_t* base, size_t row_bytes, int rows, int lane) {
   const bool b0 = lane & 1, b1 = lane & 2;
@@ -138,15 +139,17 @@ __device__ __forceinline__ void store_rows128(uint32_t (&w)[32], uint8_t* base, 
 // values gelu(acc*ts + bias), optionally rounded to bf16, which y_dbg exports for the parity tests.
 
 // values 16*h .. 16*h+15 of the chunk: bias + GELU (+ bf16 rounding), exported when asked; returns their maximum magnitude
+// FAST: rounding to bf16, no export (the forms of the model), without a test per value
+template <bool FAST>
 __device__ __forceinline__ float quant_values16(const GemmArgs& g, const uint32_t (&r)[32], int h, float ts, const float* bsm, float* dbg, float (&v)[16]) {
   const float2 ts2 = splat2(ts);
 #pragma unroll
   for (int q4 = 0; q4 < 4; ++q4) {
     const int k = 16 * h + 4 * q4;
-    const float4 bb = g.bias ? *reinterpret_cast<const float4*>(bsm + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 bb = *reinterpret_cast<const float4*>(bsm + k);   // zeros without a bias
     float2 a = gelu_erf2(fma2(make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), ts2, make_float2(bb.x, bb.y)));
     float2 b = gelu_erf2(fma2(make_float2(__uint_as_float(r[k + 2]), __uint_as_float(r[k + 3])), ts2, make_float2(bb.z, bb.w)));
-    if (g.flags & KF_Q_ROUND_BF16) {
+    if (FAST || (g.flags & KF_Q_ROUND_BF16)) {
       a = bf16_round2(a);
       b = bf16_round2(b);
     }
@@ -154,7 +157,7 @@ __device__ __forceinline__ float quant_values16(const GemmArgs& g, const uint32_
     v[4 * q4 + 1] = a.y;
     v[4 * q4 + 2] = b.x;
     v[4 * q4 + 3] = b.y;
-    if (dbg) *reinterpret_cast<float4*>(dbg + k) = make_float4(a.x, a.y, b.x, b.y);
+    if (!FAST && dbg) *reinterpret_cast<float4*>(dbg + k) = make_float4(a.x, a.y, b.x, b.y);
   }
   float am = 0.f;
 #pragma unroll
@@ -162,17 +165,21 @@ __device__ __forceinline__ float quant_values16(const GemmArgs& g, const uint32_
   return am;
 }
 
+// FMT: the output format, or -1 for the one in the arguments (with all options)
+template <int FMT>
 __device__ __forceinline__ void quant_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, const Nv4Scale& sco /* per-tensor scale of an nv4 output */, int m, int n0,
                                             const float* bsm /* the chunk's 32 bias values in shared memory */) {
   const bool div_true = !(g.flags & KF_Q_RECIP_DIV);
   const bool ok = m < g.M;
-  float* dbg = (g.y_dbg != nullptr && ok) ? g.y_dbg + (size_t)m * g.N + n0 : nullptr;
+  constexpr bool FAST = FMT >= 0;
+  const int out_fmt = FAST ? FMT : g.out_fmt;
+  float* dbg = (!FAST && g.y_dbg != nullptr && ok) ? g.y_dbg + (size_t)m * g.N + n0 : nullptr;
   int by0, by1;
-  if (g.out_fmt == KF_FMT_NV4) {
+  if (out_fmt == KF_FMT_NV4) {
     uint32_t o[4];
     float va[16], vb[16];
-    const float am0 = quant_values16(g, r, 0, ts, bsm, dbg, va), am1 = quant_values16(g, r, 1, ts, bsm, dbg, vb);
-    if (g.flags & KF_Q_FAST_NV4) {
+    const float am0 = quant_values16<FAST>(g, r, 0, ts, bsm, dbg, va), am1 = quant_values16<FAST>(g, r, 1, ts, bsm, dbg, vb);
+    if (!FAST && (g.flags & KF_Q_FAST_NV4)) {
       quant_nv4_fast<16>(va, am0, sco.ts, sco.rcp_ts, o, by0);
       quant_nv4_fast<16>(vb, am1, sco.ts, sco.rcp_ts, o + 2, by1);
     } else {
@@ -184,8 +191,8 @@ __device__ __forceinline__ void quant_chunk(const GemmArgs& g, const uint32_t (&
     return;
   }
   float va[16], vb[16];
-  const float am = amax_nan(quant_values16(g, r, 0, ts, bsm, dbg, va), quant_values16(g, r, 1, ts, bsm, dbg, vb));
-  if (g.out_fmt == KF_FMT_MX8) {
+  const float am = amax_nan(quant_values16<FAST>(g, r, 0, ts, bsm, dbg, va), quant_values16<FAST>(g, r, 1, ts, bsm, dbg, vb));
+  if (out_fmt == KF_FMT_MX8) {
     uint32_t o[8];
     quant_mx8<16>(va, am, div_true, o, by0);
     quant_mx8<16>(vb, am, div_true, o + 4, by0);
@@ -201,8 +208,25 @@ __device__ __forceinline__ void quant_chunk(const GemmArgs& g, const uint32_t (&
 }
 
 // ------------------------------------------------------------------------------------------------ PLAIN
-// PLAIN epilogue of one 32-column chunk: the thread writes 64 (16-bit) or 128 (fp32) contiguous bytes of its row.
-__device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, uint8_t* dst_row, int n0, const float* bsm /* the chunk's 32 bias values in shared memory */) {
+// PLAIN epilogue of one 32-column chunk: the thread writes 64 (16-bit) or 128 (fp32) contiguous bytes of its row.  One value pair of it:
+// MODE -1 tests the flags for every pair; the modes of the model (bf16 out) are compiled for themselves: without the tests the epilogue
+// of a 128 x 256 tile takes a third of the instructions (NVFP4, M = 22 470, N = 4096, K = 1024, bf16 out: 78 -> 64 us).
+constexpr int PL_BF16 = 0, PL_GELU = 1, PL_GELU_PRE = 2;
+template <int MODE>
+__device__ __forceinline__ float2 plain_pair(const GemmArgs& g, float2 a, float2 ts2, float2 bb) {
+  const bool pre = MODE < 0 ? (g.flags & KF_G_PRE_ROUND_BF16) != 0 : MODE == PL_GELU_PRE;
+  const bool gelu = MODE < 0 ? (g.flags & KF_G_GELU) != 0 : MODE != PL_BF16;
+  float2 x = pre ? add2(bf16_round2(mul2(a, ts2)), bb) : fma2(a, ts2, bb);   // the result may be rounded to bf16 before the bias
+  if (gelu) x = gelu_erf_pair(x);
+  if (MODE < 0 && (g.flags & KF_G_ROUND_BF16)) x = bf16_round2(x);
+  return x;
+}
+__device__ __forceinline__ int plain_mode(const GemmArgs& g) {               // the same for all tiles of a launch
+  const int f = g.flags & (KF_G_PRE_ROUND_BF16 | KF_G_GELU | KF_G_ROUND_BF16);
+  if (g.out_dtype != KF_BF16) return -1;
+  return f == 0 ? PL_BF16 : f == KF_G_GELU ? PL_GELU : f == (KF_G_GELU | KF_G_PRE_ROUND_BF16) ? PL_GELU_PRE : -1;
+}
+__device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, uint8_t* dst_row, int n0, const float* bsm /* the chunk's 32 bias values in shared memory, zeros without a bias */) {
   const float2 ts2 = splat2(ts);
 #pragma unroll
   for (int q = 0; q < 2; ++q) {                 // 16 columns at a time
@@ -210,11 +234,7 @@ __device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&
 #pragma unroll
     for (int h = 0; h < 8; ++h) {               // packed pairs
       const int k = 16 * q + 2 * h;
-      const float2 bb = g.bias ? *reinterpret_cast<const float2*>(bsm + k) : make_float2(0.f, 0.f);
-      const float2 a = make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1]));
-      float2 x = (g.flags & KF_G_PRE_ROUND_BF16) ? add2(bf16_round2(mul2(a, ts2)), bb) : fma2(a, ts2, bb);   // the result may be rounded to bf16 before the bias
-      if (g.flags & KF_G_GELU) x = gelu_erf_pair(x);
-      if (g.flags & KF_G_ROUND_BF16) x = bf16_round2(x);
+      const float2 x = plain_pair<-1>(g, make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), ts2, *reinterpret_cast<const float2*>(bsm + k));
       v[2 * h] = x.x;
       v[2 * h + 1] = x.y;
     }
@@ -229,6 +249,29 @@ __device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&
         for (int e = 0; e < 8; ++e) w[e] = pack2(v[2 * e], v[2 * e + 1], g.out_dtype);
         stg8w(dst_row + (size_t)(n0 + 16 * q) * 2, w);
       }
+    }
+  }
+}
+// bf16 output without a row mapping: the warp's 32 rows x W columns; W = 64 leaves as whole lines
+template <int MODE, int W>
+__device__ __forceinline__ void plain_rows(const GemmArgs& g, const uint32_t (&r)[W], float ts, int rbase, int n0, const float* bsm, int lane, int m_end) {
+  const float2 ts2 = splat2(ts);
+  uint32_t w[W / 2];
+#pragma unroll
+  for (int k = 0; k < W; k += 4) {
+    const float4 bb = *reinterpret_cast<const float4*>(bsm + k);
+    const float2 x = plain_pair<MODE>(g, make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), ts2, make_float2(bb.x, bb.y));
+    const float2 y = plain_pair<MODE>(g, make_float2(__uint_as_float(r[k + 2]), __uint_as_float(r[k + 3])), ts2, make_float2(bb.z, bb.w));
+    w[k / 2] = pack2(x.x, x.y, KF_BF16);
+    w[k / 2 + 1] = pack2(y.x, y.y, KF_BF16);
+  }
+  uint8_t* base = static_cast<uint8_t*>(g.C) + ((size_t)rbase * g.N + n0) * 2;
+  if constexpr (W == 64) {
+    store_rows128(w, base, (size_t)g.N * 2, m_end - rbase, lane);
+  } else {
+    if (rbase + lane < m_end) {
+      stg8w(base + (size_t)lane * g.N * 2, w);
+      stg8w(base + (size_t)lane * g.N * 2 + 32, w + 8);
     }
   }
 }
@@ -265,12 +308,16 @@ struct RopeSlabRegs {
 __device__ __forceinline__ void rope_slab_fetch(const GemmArgs& g, int rbase, int tid /* 0..127 within the quarter */, RopeSlabRegs& x) {
   const int f = tid & 15;                                            // piece of the row: 0..7 sin, 8..15 cos
   const float* tab = (f < 8 ? g.sin : g.cos) + ((f & 7) << 2);
+  int t = (rbase + (tid >> 4)) % g.Ntok;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int m = rbase + (tid >> 4) + 8 * u;
     x.v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (u != 0) {
+      t += 8;
+      if (t >= g.Ntok) t = t - g.Ntok < g.Ntok ? t - g.Ntok : t % g.Ntok;
+    }
     if (m < g.M) {
-      const int t = m % g.Ntok;
       if (t >= g.prefix) x.v[u] = __ldg(reinterpret_cast<const float4*>(tab + (size_t)(t - g.prefix) * 64));
     }
   }
@@ -290,7 +337,7 @@ __device__ __forceinline__ void quarter_barrier(int quarter) { asm volatile("bar
 // columns in r.  W = 64: columns n0..n0+63.  W = 32: columns n0..n0+31; ROPE then holds half of the rotation pairs of the
 // head that starts at n0, columns j0..j0+15 in r[0..15] and 32+j0..32+j0+15 in r[16..31].
 // `slice` / `gslice` point at the bias / LayerScale values of the columns from n0 in shared memory.
-template <int EPI, int W>
+template <int EPI, int W, int MODE = -1>
 __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W], float ts, const Nv4Scale& sco, int rbase, int n0, int j0,
                                               const float* slice, const float* gslice /* RES: the LayerScale values of the warp's columns */,
                                               const float* slab /* ROPE: the quarter's table rows in shared memory, or null */, int lane,
@@ -305,52 +352,59 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
     if (W == 32 && m >= g.M) return;            // W = 64: all lanes take part in the stores
     const int which = n0 / g.d, h = (n0 - which * g.d) >> 6;
     const int b = m / g.Ntok, t = m - b * g.Ntok;
-    const int nbatch = g.M / g.Ntok;
     const bool rot = which < 2 && t >= g.prefix && m < g.M;
-    const float* sn = g.sin + (size_t)(rot ? t - g.prefix : 0) * 64;
-    const float* cs = g.cos + (size_t)(rot ? t - g.prefix : 0) * 64;
     const float* srow = slab + lane * 64;
-    uint8_t* dst = static_cast<uint8_t*>(g.C) + ((((size_t)which * nbatch + b) * g.Ntok + t) * g.H + h) * 128;
     uint32_t wo[W == 64 ? 32 : 16];             // packed output: the columns of the first half, then those of the second
     const float2 ts2 = splat2(ts);
+    // FORM 0: no rotation (v columns), 1: every row rotates, tables in the slab, 2: row by row
+    auto columns = [&](auto form) {
+      constexpr int FORM = decltype(form)::value;
+      const float* sn = g.sin + (size_t)(rot ? t - g.prefix : 0) * 64;
+      const float* cs = g.cos + (size_t)(rot ? t - g.prefix : 0) * 64;
 #pragma unroll
-    for (int c = 0; c < W / 8; ++c) {           // 4 rotation pairs at a time (few values live: the thread already holds W accumulators)
-      float2 lo[2], hi[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int j = 4 * c + 2 * e;
-        lo[e] = fma2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), ts2, *reinterpret_cast<const float2*>(slice + j0 + j));
-        hi[e] = fma2(make_float2(__uint_as_float(r[W / 2 + j]), __uint_as_float(r[W / 2 + j + 1])), ts2, *reinterpret_cast<const float2*>(slice + 32 + j0 + j));
-      }
-      float2 ol[2] = {lo[0], lo[1]}, oh[2] = {hi[0], hi[1]};
-      if (rot) {
-        const int ct = (j0 >> 2) + c;           // 16-byte piece of the table row
-        float4 s4, c4;                          // sin / cos of the 4 pairs: first for the lo outputs, then for the hi outputs
-        if (slab != nullptr) {                  // both halves of the tables are the same 32 values
-          s4 = *reinterpret_cast<const float4*>(srow + ((ct ^ (lane & 7)) << 2));
-          c4 = *reinterpret_cast<const float4*>(srow + (((ct + 8) ^ (lane & 7)) << 2));
-        } else {
-          s4 = ldg4_nc(sn + 4 * ct);
-          c4 = ldg4_nc(cs + 4 * ct);
+      for (int c = 0; c < W / 8; ++c) {           // 4 rotation pairs at a time (few values live: the thread already holds W accumulators)
+        const float4 bl = *reinterpret_cast<const float4*>(slice + j0 + 4 * c), bh = *reinterpret_cast<const float4*>(slice + 32 + j0 + 4 * c);
+        const int j = 4 * c;
+        const float2 lo[2] = {fma2(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), ts2, make_float2(bl.x, bl.y)),
+                              fma2(make_float2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])), ts2, make_float2(bl.z, bl.w))};
+        const float2 hi[2] = {fma2(make_float2(__uint_as_float(r[W / 2 + j]), __uint_as_float(r[W / 2 + j + 1])), ts2, make_float2(bh.x, bh.y)),
+                              fma2(make_float2(__uint_as_float(r[W / 2 + j + 2]), __uint_as_float(r[W / 2 + j + 3])), ts2, make_float2(bh.z, bh.w))};
+        float2 ol[2] = {lo[0], lo[1]}, oh[2] = {hi[0], hi[1]};
+        if (FORM == 1 || (FORM == 2 && rot)) {
+          const int ct = (j0 >> 2) + c;           // 16-byte piece of the table row
+          float4 s4, c4;                          // sin / cos of the 4 pairs: first for the lo outputs, then for the hi outputs
+          if (FORM == 1 || slab != nullptr) {     // both halves of the tables are the same 32 values
+            s4 = *reinterpret_cast<const float4*>(srow + ((ct ^ (lane & 7)) << 2));
+            c4 = *reinterpret_cast<const float4*>(srow + (((ct + 8) ^ (lane & 7)) << 2));
+          } else {
+            s4 = ldg4_nc(sn + 4 * ct);
+            c4 = ldg4_nc(cs + 4 * ct);
+          }
+          ol[0] = fma2(mul2(hi[0], splat2(-1.f)), make_float2(s4.x, s4.y), mul2(lo[0], make_float2(c4.x, c4.y)));   // -hi: one packed product, exact
+          ol[1] = fma2(mul2(hi[1], splat2(-1.f)), make_float2(s4.z, s4.w), mul2(lo[1], make_float2(c4.z, c4.w)));
+          if (FORM == 2 && slab == nullptr) {
+            s4 = ldg4_nc(sn + 32 + 4 * ct);
+            c4 = ldg4_nc(cs + 32 + 4 * ct);
+          }
+          oh[0] = fma2(hi[0], make_float2(c4.x, c4.y), mul2(lo[0], make_float2(s4.x, s4.y)));
+          oh[1] = fma2(hi[1], make_float2(c4.z, c4.w), mul2(lo[1], make_float2(s4.z, s4.w)));
         }
-        ol[0] = fma2(hi[0], make_float2(-s4.x, -s4.y), mul2(lo[0], make_float2(c4.x, c4.y)));
-        ol[1] = fma2(hi[1], make_float2(-s4.z, -s4.w), mul2(lo[1], make_float2(c4.z, c4.w)));
-        if (slab == nullptr) {
-          s4 = ldg4_nc(sn + 32 + 4 * ct);
-          c4 = ldg4_nc(cs + 32 + 4 * ct);
-        }
-        oh[0] = fma2(hi[0], make_float2(c4.x, c4.y), mul2(lo[0], make_float2(s4.x, s4.y)));
-        oh[1] = fma2(hi[1], make_float2(c4.z, c4.w), mul2(lo[1], make_float2(s4.z, s4.w)));
-      }
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        wo[2 * c + e] = pack2(ol[e].x, ol[e].y, g.out_dtype);
-        wo[W / 4 + 2 * c + e] = pack2(oh[e].x, oh[e].y, g.out_dtype);
+        for (int e = 0; e < 2; ++e) {
+          wo[2 * c + e] = pack2(ol[e].x, ol[e].y, g.out_dtype);
+          wo[W / 4 + 2 * c + e] = pack2(oh[e].x, oh[e].y, g.out_dtype);
+        }
       }
-    }
+    };
+    // Which form is the same for a warp: a test per value and per-row branches around the rotation doubled the instructions of the epilogue
+    // (871 per warp and 128 x 256 tile; the rows of the cls / register tokens and of the general tables still take them)
+    if (which == 2) columns(std::integral_constant<int, 0>{});
+    else if (slab != nullptr && __all_sync(W == 64 ? 0xffffffffu : __activemask(), rot || m >= g.M)) columns(std::integral_constant<int, 1>{});
+    else columns(std::integral_constant<int, 2>{});
     if constexpr (W == 64) {                    // rows of the output are [token, head] rows: row m of a third of q / k / v is b * Ntok + t = m
       store_rows128(wo, static_cast<uint8_t*>(g.C) + (((size_t)which * g.M + rbase) * g.H + h) * 128, (size_t)g.H * 128, g.M - rbase, lane);
     } else {
+      uint8_t* dst = static_cast<uint8_t*>(g.C) + ((((size_t)which * (g.M / g.Ntok) + b) * g.Ntok + t) * g.H + h) * 128;
       stg8w(dst + 2 * j0, wo);
       stg8w(dst + 64 + 2 * j0, wo + 8);
     }
@@ -381,6 +435,8 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
       }
       stg8(crow + 8 * c, o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7]);
     }
+  } else if (EPI == KF_EPI_PLAIN && MODE >= 0) {
+    plain_rows<(MODE < 0 ? 0 : MODE), W>(g, r, ts, rbase, n0, slice, lane, m_end);
   } else if (EPI == KF_EPI_PLAIN) {
     uint8_t* dst_row = nullptr;
     if (m < m_end) {
@@ -391,7 +447,7 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
     for (int c = 0; c < W; c += 32) plain_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, dst_row, n0 + c, slice + c);
   } else {   // KF_EPI_QUANT: gelu(acc*ts + bias) -> codes + blocked scales of format out_fmt
 #pragma unroll
-    for (int c = 0; c < W; c += 32) quant_chunk(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, sco, m, n0 + c, slice + c);
+    for (int c = 0; c < W; c += 32) quant_chunk<MODE>(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, sco, m, n0 + c, slice + c);
   }
 }
 
@@ -492,6 +548,9 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
     }
   };
   if (boxed) box_load(blockIdx.x);
+  // The form of the launch's options that has an epilogue of its own, or -1: the same for every tile, tested once per tile instead of per value
+  const int mode = EPI == KF_EPI_PLAIN ? (g.row_group > 0 ? -1 : plain_mode(g))
+                   : EPI == KF_EPI_QUANT && g.y_dbg == nullptr && (g.flags & (KF_Q_ROUND_BF16 | KF_Q_FAST_NV4)) == KF_Q_ROUND_BF16 ? g.out_fmt : -1;
   int lt = 0;
   // ROPE: the four warps of a quarter meet at named barriers, which have no limit.  A warp whose wait ran out therefore does not leave: it
   // keeps company at the barriers of its remaining tiles (the same number in all four warps: they depend on the tile only) and
@@ -561,7 +620,20 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
         continue;
       }
     }
-    epilogue_math<EPI, W>(g, r, ts, sco, rbase, n0, j0, bsl, gsl, slab, lane, row_end, res);
+    auto finish = [&](auto form) { epilogue_math<EPI, W, decltype(form)::value>(g, r, ts, sco, rbase, n0, j0, bsl, gsl, slab, lane, row_end, res); };
+    if constexpr (EPI == KF_EPI_PLAIN) {
+      if (mode == PL_BF16) finish(std::integral_constant<int, PL_BF16>{});
+      else if (mode == PL_GELU) finish(std::integral_constant<int, PL_GELU>{});
+      else if (mode == PL_GELU_PRE) finish(std::integral_constant<int, PL_GELU_PRE>{});
+      else finish(std::integral_constant<int, -1>{});
+    } else if constexpr (EPI == KF_EPI_QUANT) {
+      if (mode == KF_FMT_NV4) finish(std::integral_constant<int, KF_FMT_NV4>{});
+      else if (mode == KF_FMT_MX8) finish(std::integral_constant<int, KF_FMT_MX8>{});
+      else if (mode == KF_FMT_MX4) finish(std::integral_constant<int, KF_FMT_MX4>{});
+      else finish(std::integral_constant<int, -1>{});
+    } else {
+      finish(std::integral_constant<int, -1>{});
+    }
   }
   if (boxed && lane == 0) bulk_wait_all();
 }

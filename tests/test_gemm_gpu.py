@@ -480,3 +480,67 @@ def test_weights_written_right_before_the_launch(fmt, M):
         ops.quant_rows(ws[1].float(), buf)
         assert not early(one) and torch.equal(ops.gemm_plain(a, one), plain[1])
     ops.check_device_error()
+
+
+def test_gelu_error_against_float64():
+    """bias + GELU of every bf16 value in [-40, 40] (an identity product), with a 16-bit or fp32 output and as the quantise-out exports it.
+    Bound: the largest error of the approximation in exact arithmetic with fp32 rounding (3.4e-7 for outputs, 6.3e-7 for the quantise-out),
+    that of the exponential (2^-22 of at most 0.17) and the rounding of the output."""
+    ops = _ops()
+    bits = torch.arange(0, 0x4220, dtype=torch.int32)                       # 0x4220 = bf16 of 40
+    pos = bits.to(torch.int16).view(torch.bfloat16)
+    v = torch.cat((pos, -pos))
+    a = torch.zeros(v.numel(), 64, dtype=torch.bfloat16)
+    a[:, 0] = v
+    w = torch.zeros(128, 64)
+    w[:, 0] = 1.0
+    W = ops.QWeight(w.cuda(), "bf16")
+    ref = go.gelu_erf(v.double().numpy())
+    for dt, step in ((torch.float32, 2.0 ** -24), (torch.bfloat16, 2.0 ** -8)):     # unit roundoffs
+        out = ops.gemm_plain(a.cuda(), W, gelu=True, out_dtype=dt).cpu()
+        ops.check_device_error()
+        assert torch.equal(out, out[:, :1].expand_as(out))
+        err = np.abs(out[:, 0].double().numpy() - ref)
+        assert (err <= 4.0e-7 + (step + 2.0 ** -22) * np.abs(ref)).all(), (dt, err.max())
+    y = torch.empty(v.numel(), 128, device="cuda")
+    ops.gemm_gelu_q(a.cuda(), W, None, ops.ActBuf(v.numel(), 128, "mx8"), y_dbg=y)
+    ops.check_device_error()
+    err = np.abs(y[:, 0].cpu().double().numpy() - ref)
+    assert (err <= 6.8e-7 + 2.0 ** -22 * np.abs(ref)).all(), err.max()
+
+
+# rows and columns: 128-column tiles; whole tiles of 256 columns with a partial row tile; a last column tile of 128
+@pytest.mark.parametrize("M,N", [(300, 512), (9597, 768), (9597, 640)])
+@pytest.mark.parametrize("fmt", FMTS + ["bf16"])
+def test_epilogue_forms_agree(fmt, M, N):
+    """the epilogues compiled for the options of the model (bf16 out; rounding to bf16 before the quantisation) against those that test
+    every option: an fp32 output rounded afterwards, and the quantise-out with its export."""
+    ops = _ops()
+    K = 256
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    a = x if fmt == "bf16" else ops.ActBuf(M, K, fmt)
+    if fmt == "nv4":
+        a.ts.fill_(0.003)
+    if fmt != "bf16":
+        ops.quant_rows(x, a)
+    W = ops.QWeight(torch.randn(N, K, generator=g, device="cuda") * 0.1, fmt)
+    bias = torch.randn(N, generator=g, device="cuda")
+    for b in (bias, None):
+        for kw in ({}, {"gelu": True}, {"gelu": True, "pre_round": True}):
+            general = ops.gemm_plain(a, W, b, out_dtype=torch.float32, **kw)
+            assert torch.equal(ops.gemm_plain(a, W, b, **kw), general.to(torch.bfloat16)), kw
+    if fmt == "bf16":
+        return
+    for ofmt in FMTS:
+        outs = []
+        for dbg in (None, torch.empty(M, N, device="cuda")):
+            q = ops.ActBuf(M, N, ofmt)
+            q.q.fill_(0xAA)
+            q.sf.fill_(0xAA)
+            if ofmt == "nv4":
+                q.ts.fill_(0.002)
+            ops.gemm_gelu_q(a, W, bias, q, round_bf16=True, y_dbg=dbg)
+            outs.append(q)
+        assert torch.equal(outs[0].q, outs[1].q) and torch.equal(outs[0].sf, outs[1].sf), ofmt
+    ops.check_device_error()
