@@ -277,8 +277,9 @@ struct TmapKey {
   const void* base;
   uint64_t rows, row_bytes, pitch_bytes;
   uint32_t box_rows;
+  bool atoms;                                            // rows of 128 words without a swizzle (scale atoms) instead of 128-byte boxes
   bool operator==(const TmapKey& o) const {
-    return base == o.base && rows == o.rows && row_bytes == o.row_bytes && pitch_bytes == o.pitch_bytes && box_rows == o.box_rows;
+    return base == o.base && rows == o.rows && row_bytes == o.row_bytes && pitch_bytes == o.pitch_bytes && box_rows == o.box_rows && atoms == o.atoms;
   }
 };
 struct TmapSlot {
@@ -287,13 +288,12 @@ struct TmapSlot {
   bool used;
 };
 
-int make_tmap_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch_bytes, uint32_t box_rows) {
+static int make_tmap_cached(CUtensorMap* map, const TmapKey& key) {
   constexpr int SLOTS = 256;
   static thread_local TmapSlot cache[SLOTS] = {};
-  const TmapKey key{base, rows, row_bytes, pitch_bytes, box_rows};
-  uint64_t h = reinterpret_cast<uintptr_t>(base) >> 8;
-  h ^= rows * 0x9E3779B97F4A7C15ull;
-  h ^= (row_bytes << 7) ^ box_rows;
+  uint64_t h = reinterpret_cast<uintptr_t>(key.base) >> 8;
+  h ^= key.rows * 0x9E3779B97F4A7C15ull;
+  h ^= (key.row_bytes << 7) ^ key.box_rows;
   TmapSlot& slot = cache[(h ^ (h >> 17)) % SLOTS];
   if (slot.used && slot.key == key) {
     *map = slot.map;
@@ -304,21 +304,28 @@ int make_tmap_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return KF_ERR_UNSUPPORTED;
   }
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {pitch_bytes};
-  cuuint32_t box[2] = {128, box_rows};
+  cuuint64_t dims[2] = {key.atoms ? 128 : key.row_bytes, key.rows};
+  cuuint64_t strides[1] = {key.pitch_bytes};
+  cuuint32_t box[2] = {128, key.box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = fn(map, key.atoms ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(key.base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, key.atoms ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed with CUresult %d (base %p rows %llu row_bytes %llu)", (int)r, base, (unsigned long long)rows,
-              (unsigned long long)row_bytes);
+    set_error("cuTensorMapEncodeTiled failed with CUresult %d (base %p rows %llu row_bytes %llu)", (int)r, key.base, (unsigned long long)key.rows,
+              (unsigned long long)key.row_bytes);
     return KF_ERR_BAD_ARGUMENT;
   }
   slot.key = key;
   slot.map = *map;
   slot.used = true;
   return KF_OK;
+}
+int make_tmap_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch_bytes, uint32_t box_rows) {
+  return make_tmap_cached(map, TmapKey{base, rows, row_bytes, pitch_bytes, box_rows, false});
+}
+int make_tmap_atoms(CUtensorMap* map, const void* base, uint64_t n_atoms, uint32_t atoms) {
+  return make_tmap_cached(map, TmapKey{base, n_atoms, 512, 512, atoms, true});
 }
 
 int device_sm_count(int* sms) {
@@ -337,6 +344,8 @@ int device_sm_count(int* sms) {
   *sms = n;
   return KF_OK;
 }
+
+int launch_gemm_pair(const kf_gemm_params* p, uint64_t kbytes, uint64_t w_rows, GemmArgs& g, int sms, cudaStream_t st);   // kf_gemm_pair.cu
 
 struct GemmMaps {
   CUtensorMap A, W, R, C;                                 // R, C: the residual and the output of a RES launch through shared memory; R: W in boxes of 128 rows for half tiles
@@ -407,18 +416,39 @@ static int gemm_columns(int fmt, int epi, int m_tiles, int N, int sms) {
   return cost128 <= cost256 ? 128 : 256;
 }
 
-// RES launches that move the residual through shared memory (128-column tiles): those of many rounds, where its bandwidth counts
+// RES launches that move the residual through shared memory on 128-column tiles: those of many rounds, where its bandwidth counts
 // and the box of the next tile travels under the present one.
-// Not for a long K: the 128-column tiles then cost more operand traffic than the boxes save.  Without -> with boxes, in place, operands from HBM,
-// us at M = 9630, 22 470 and 51 360:
+// Not for a long K: the 128-column tiles then cost more operand traffic than the boxes save.  256-column tiles without boxes -> 128-column
+// tiles with boxes, in place, operands from HBM, us at M = 9630, 22 470 and 51 360:
 //    4 stages  NVFP4 1024 x 1024   26.8 -> 20.8   47.4 -> 37.3   97.6 -> 76.8
 //    6 stages  MXFP8  768 x  768   24.7 -> 21.1   41.3 -> 36.6   80.5 -> 70.8
 //    8 stages  MXFP8 1024 x 1024   30.7 -> 30.0   55.6 -> 56.2  116.8 -> 112.4     NVFP4 1024 x 2048  33.6 -> 32.5  60.5 -> 61.2  120.4 -> 116.6
 //   10 stages  MXFP8 1024 x 1280   33.9 -> 34.1   62.6 -> 63.8  127.8 -> 130.2
-//   12 stages  bf16   768 x  768   31.9 -> 30.5   55.8 -> 55.6  107.2 -> 109.3     NVFP4  768 x 3072  34.9 -> 31.9  60.6 -> 59.5  109.5 -> 116.8
-//   16 stages  NVFP4 1024 x 4096   41.0 -> 45.9   74.7 -> 88.5  157.4 -> 176.9
-// Faster up to 6 stages, level at 8, with the sign changing from row count to row count up to 12, slower from there: the line is after 8.
-static bool gemm_res_boxes(int k_tiles, int m_tiles, int N, int sms) { return k_tiles <= 8 && (int64_t)m_tiles * (N / 128) >= 3 * (int64_t)sms; }
+// and against CTA pairs (captured; these boxes -> pairs; 9630, 22 470, 51 360): 4 stages NVFP4 1024 x 1024 17.6 -> 19.3, 36.1 -> 38.3, 75.1 -> 86.9;
+// 6 stages MXFP8 768 x 768 15.3 -> 16.4, 34.1 -> 33.9, 67.2 -> 70.7; 8 stages MXFP8 1024 x 1024 27.8 -> 23.9, 53.2 -> 44.3, 106.4 -> 86.1.
+// The line lies after 6 stages where pairs are possible, after 8 where they are not.
+static bool gemm_res_boxes(int k_tiles, int m_tiles, int N, int sms) {
+  return k_tiles <= (N % 256 == 0 ? 6 : 8) && (int64_t)m_tiles * (N / 128) >= 3 * (int64_t)sms;
+}
+
+// Launches that run on CTA pairs (kf_gemm_pair.cu).  A tile of a pair is twice as much to lose in a last round, and a launch of pairs starts
+// about a microsecond later (cluster launch, hand-shakes), so the line lies by rows.  One CTA -> pairs, captured launches, us at 1605, 3210, 4815, 6420 and
+// 9630 rows:
+//    PLAIN / ROPE  MXFP8 768 x 2304 (qkv)   7.7 -> 8.5  10.9 -> 11.4  13.6 -> 14.0  18.5 -> 17.9  24.2 -> 22.8
+//                  NVFP4 1024 x 3072 (qkv)  8.9 -> 9.6  11.8 -> 12.7  15.2 -> 16.5  20.3 -> 20.1  26.3 -> 26.3
+//                  NVFP4 4096 x 1024        8.1 -> 9.6  10.3 -> 10.5  14.0 -> 13.5  16.6 -> 15.4  23.3 -> 21.9
+//    QUANT         MXFP8 768 x 3072        10.1 -> 10.2 13.9 -> 13.4  17.9 -> 17.1  23.3 -> 21.9  31.0 -> 29.1
+//    bf16 operands 768 x 2304               9.5 -> 10.3 14.8 -> 14.3  17.8 -> 17.1  24.3 -> 22.1  34.8 -> 30.1
+//    RES           NVFP4 4096 x 1024        9.6 -> 13.0 15.2 -> 14.2  19.8 -> 18.3  23.5 -> 22.4  (the residual as boxes)
+// Not where the tiles do not fill the pairs (for RES half of them: without pairs its residual goes in 32-byte pieces), nor for what
+// gemm_res_boxes takes.  Few rows against many columns (the mask product: two row tiles an image, 8 x 200 x 65 536 x 1024 340 -> 261 us) count from four
+// rounds on; a batched product needs its row tiles in twos.
+static bool gemm_pairs(int fmt, int epi, int m_tiles, int m_tiles_pb, int N, int sms) {
+  if (N % 256 != 0 || m_tiles_pb % 2 != 0) return false;
+  const int64_t tiles = (int64_t)((m_tiles + 1) / 2) * (N / 256), pairs = sms / 2;
+  const bool early = epi == KF_EPI_RES || epi == KF_EPI_QUANT || fmt == KF_FMT_BF16;
+  return (m_tiles >= (early ? 24 : 48) || tiles >= 4 * pairs) && (epi == KF_EPI_RES ? 2 * tiles > pairs : tiles >= pairs);
+}
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static bool al32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }   // 256-bit global accesses of the epilogues
@@ -475,7 +505,32 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   int st = device_sm_count(&sms);
   if (st != KF_OK) return st;
   const bool res_tma = epi == KF_EPI_RES && p->out_row_group == 0 && gemm_res_boxes((int)(kbytes / BKB), m_tiles, p->N, sms);
+  const int m_tiles_pb = p->batch > 0 ? (p->a_rows_per_batch + BM - 1) / BM : 0;
+  const bool pair = !res_tma && gemm_pairs(fmt, epi, m_tiles, m_tiles_pb, p->N, sms);
   const int bn = res_tma ? 128 : gemm_columns(fmt, epi, m_tiles, p->N, sms);
+  GemmArgs g{};
+  g.sfa = static_cast<const uint8_t*>(p->SFA);
+  g.sfw = static_cast<const uint8_t*>(p->SFW);
+  g.ts_a = p->ts_a; g.ts_w = p->ts_w; g.bias = p->bias; g.gamma = p->gamma; g.R = p->R; g.sin = p->sin; g.cos = p->cos; g.tso = p->tso;
+  g.C = p->C; g.Qo = static_cast<uint8_t*>(p->Qo); g.SFo = static_cast<uint8_t*>(p->SFo);
+  g.M = p->M; g.N = p->N; g.K = p->K;
+  g.Ntok = p->Ntok; g.prefix = p->prefix; g.H = p->H; g.d = p->H * 64;
+  g.out_dtype = p->out_dtype; g.flags = p->flags; g.out_fmt = p->out_fmt;
+  g.m_tiles = m_tiles; g.k_tiles = (int)(kbytes / BKB);
+  if (p->batch > 0) {
+    g.m_tiles_pb = m_tiles_pb;
+    g.a_rows_pb = p->a_rows_per_batch;
+    g.w_rows_pb = p->w_rows_per_batch;
+  }
+  g.nkb4 = fmt == KF_FMT_BF16 ? 0 : p->K / (4 * fmt_vec(fmt));
+  const bool maps_rows = epi == KF_EPI_PLAIN || epi == KF_EPI_RES;
+  g.row_group = maps_rows ? p->out_row_group : 0; g.row_stride = p->out_row_stride; g.row_offset = p->out_row_offset;
+  g.res_tma = res_tma;
+  g.y_dbg = epi == KF_EPI_QUANT ? p->y_dbg : nullptr;
+  g.err = dev_error_ptr();
+  KF_REQUIRE(g.err != nullptr, "kf_gemm_bs: device error word unavailable");
+  cudaStream_t cs = static_cast<cudaStream_t>(stream);
+  if (pair) return launch_gemm_pair(p, kbytes, w_rows, g, sms, cs);
   GemmMaps tm;
   st = make_tmap_2d_bytes(&tm.A, p->A, (uint64_t)p->M, kbytes, kbytes, BM);
   if (st != KF_OK) return st;
@@ -492,27 +547,5 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
     st = make_tmap_2d_bytes(&tm.C, p->C, (uint64_t)p->M, 4ull * p->N, 4ull * p->N, 32);
     if (st != KF_OK) return st;
   }
-  GemmArgs g{};
-  g.sfa = static_cast<const uint8_t*>(p->SFA);
-  g.sfw = static_cast<const uint8_t*>(p->SFW);
-  g.ts_a = p->ts_a; g.ts_w = p->ts_w; g.bias = p->bias; g.gamma = p->gamma; g.R = p->R; g.sin = p->sin; g.cos = p->cos; g.tso = p->tso;
-  g.C = p->C; g.Qo = static_cast<uint8_t*>(p->Qo); g.SFo = static_cast<uint8_t*>(p->SFo);
-  g.M = p->M; g.N = p->N; g.K = p->K;
-  g.Ntok = p->Ntok; g.prefix = p->prefix; g.H = p->H; g.d = p->H * 64;
-  g.out_dtype = p->out_dtype; g.flags = p->flags; g.out_fmt = p->out_fmt;
-  g.m_tiles = m_tiles; g.k_tiles = (int)(kbytes / BKB);
-  if (p->batch > 0) {
-    g.m_tiles_pb = (p->a_rows_per_batch + BM - 1) / BM;
-    g.a_rows_pb = p->a_rows_per_batch;
-    g.w_rows_pb = p->w_rows_per_batch;
-  }
-  g.nkb4 = fmt == KF_FMT_BF16 ? 0 : p->K / (4 * fmt_vec(fmt));
-  const bool maps_rows = epi == KF_EPI_PLAIN || epi == KF_EPI_RES;
-  g.row_group = maps_rows ? p->out_row_group : 0; g.row_stride = p->out_row_stride; g.row_offset = p->out_row_offset;
-  g.res_tma = res_tma;
-  g.y_dbg = epi == KF_EPI_QUANT ? p->y_dbg : nullptr;
-  g.err = dev_error_ptr();
-  KF_REQUIRE(g.err != nullptr, "kf_gemm_bs: device error word unavailable");
-  cudaStream_t cs = static_cast<cudaStream_t>(stream);
   return bn == 128 ? launch_gemm_fmt<128>(fmt, epi, tm, g, sms, cs) : launch_gemm_fmt<256>(fmt, epi, tm, g, sms, cs);
 }

@@ -7,12 +7,12 @@
 // output row.  That is 128 contiguous bytes of a 16-bit output (exactly one [token, head] row of the q/k/v layout) or
 // 256 contiguous bytes of an fp32 one, which the thread moves with 256-bit global loads / stores (ld/st.global.v8): every
 // access is a whole 32-byte sector.  Two forms exchange data to move whole 128-byte lines instead: ROPE transposes the pieces of every
-// four rows between lanes (store_rows128), RES launches of many rounds and a short K update the residual in shared memory, where
-// it comes and goes as TMA boxes (epilogue_res_tma).  Shared memory also holds the bias (and LayerScale) values, the whole vector of
+// four rows between lanes (store_rows128), as PLAIN does with bf16; RES on CTA pairs, and RES launches of many rounds and a short K, update
+// the residual in shared memory, where it comes and goes as TMA boxes (epilogue_res_tma).  Shared memory also holds the bias (and LayerScale) values, the whole vector of
 // the launch, loaded once per CTA, or a 64-value slice per warp and tile where the operand ring leaves no room for the vector, and
 // for ROPE the rotary-table rows of the tile.
 #pragma once
-#include "kf_sm100.cuh"
+#include "kf_sm100_pair.cuh"
 
 namespace kf {
 
@@ -53,7 +53,7 @@ struct GemmArgs {
   int row_group, row_stride, row_offset;   // PLAIN, RES: output row = (m / group) * stride + offset + m % group (group 0: identity)
   int m_tiles_pb, a_rows_pb, w_rows_pb;    // batched products (m_tiles_pb > 0): row tiles, A rows and W rows per product
   int vec_floats;                          // > 0: the whole bias vector (and for RES the LayerScale vector behind it) sits in shared memory for the launch
-  int res_tma;                             // RES, BN = 128: the residual goes through shared memory by TMA boxes (epilogue_res_tma)
+  int res_tma;                             // RES, BN = 128 or CTA pairs: the residual goes through shared memory by TMA boxes (epilogue_res_tma)
   float* y_dbg;                            // QUANT: optional export of the values that were quantised (fp32 [M, N])
   unsigned int* err;
 };
@@ -451,7 +451,7 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
   }
 }
 
-// RES through shared memory, BN = 128: the warp's 32 rows x 32 columns of the residual come as one TMA box (128-byte rows, swizzled),
+// RES through shared memory: 32 rows x 32 columns of the residual (all of a warp's columns where BN = 128) come as one TMA box (128-byte rows, swizzled),
 // are updated in place in shared memory and leave as one box.  Every request is then a whole 128-byte line: a read-modify-write of
 // 22 470 x 1024 fp32 takes 33.0 us this way and 39.9 us with the 32-byte accesses of the row layout (copy: 32.7 us).
 constexpr int RES_BOX_BYTES = 32 * 128;
@@ -506,7 +506,9 @@ __device__ __forceinline__ WorkItem work_item(const GemmArgs& g, int idx) {
 // Body of the 16 epilogue warps (warp = (TMEM lane quarter, 64- or 32-column group)): per tile, stage the bias slice (and fetch
 // the rotary-table rows), wait for the accumulator, take the warp's piece into registers, hand TMEM back at once and
 // run the fused epilogue on the registers while the next tile's main loop fills the accumulator again.
-template <int EPI, int BN>
+// PAIR (CTA pairs, BN = 256): work items are counted per pair and name row tiles 2 * m_blk and 2 * m_blk + 1, one per CTA; the
+// accumulator is handed back to the leader's MMA warp.
+template <int EPI, int BN, bool PAIR = false>
 __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty, float* slices,
                                                float* slabs, uint8_t* boxes, uint64_t* box_full, const CUtensorMap* tmR, const CUtensorMap* tmC, const WaitCtx& ctx, int warp,
                                                int lane) {
@@ -534,20 +536,24 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
   const int col = PAIRS ? (cg >> 1) * 64 : cg * W, j0 = PAIRS ? (cg & 1) * 16 : 0;
   const uint32_t taddr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + col + j0;
   // RES through shared memory: this warp's box and its barrier; the box of the next tile is requested when the present one has left
-  const bool boxed = EPI == KF_EPI_RES && W == 32 && g.res_tma != 0;
+  constexpr bool BOXES = EPI == KF_EPI_RES && (W == 32 || PAIR);
+  const bool boxed = BOXES && g.res_tma != 0;
+  const int first = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, stride = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x, rank = PAIR ? (int)cluster_ctarank() : 0;
+  auto row_tile = [&](const WorkItem& w) { return PAIR ? 2 * w.m_blk + rank : w.m_blk; };
+  const uint32_t leader_tempty = PAIR ? map_to_rank(tempty, 0) : 0;
   uint8_t* box = boxes + (warp - EPI_WARP0) * RES_BOX_BYTES;
   uint64_t* bfull = box_full + (warp - EPI_WARP0);
   uint32_t bph = 0;
   auto box_load = [&](int idx) {
     if (idx >= g.items) return;
     const WorkItem w = work_item<BN>(g, idx);
-    const int row = w.m_blk * BM + quarter * 32;
-    if (row < g.M && lane == 0) {
+    const int row = row_tile(w) * BM + quarter * 32;
+    if (row < g.M && col < w.cols && lane == 0) {
       mbar_expect_tx(bfull, RES_BOX_BYTES);
       tma_load_2d(box, tmR, (w.n0 + col) * 4, row, bfull);
     }
   };
-  if (boxed) box_load(blockIdx.x);
+  if (boxed) box_load(first);
   // The form of the launch's options that has an epilogue of its own, or -1: the same for every tile, tested once per tile instead of per value
   const int mode = EPI == KF_EPI_PLAIN ? (g.row_group > 0 ? -1 : plain_mode(g))
                    : EPI == KF_EPI_QUANT && g.y_dbg == nullptr && (g.flags & (KF_Q_ROUND_BF16 | KF_Q_FAST_NV4)) == KF_Q_ROUND_BF16 ? g.out_fmt : -1;
@@ -556,10 +562,10 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
   // keeps company at the barriers of its remaining tiles (the same number in all four warps: they depend on the tile only) and
   // stores nothing.
   bool live = true;
-  for (int idx = blockIdx.x; idx < g.items; idx += gridDim.x, ++lt) {
+  for (int idx = first; idx < g.items; idx += stride, ++lt) {
     const WorkItem item = work_item<BN>(g, idx);
     int row_end;
-    const int rbase = tile_row0(g, item.m_blk, row_end) + quarter * 32;
+    const int rbase = tile_row0(g, row_tile(item), row_end) + quarter * 32;
     const int n0 = item.n0 + col;               // first column of this warp's group (or of its head)
     const int acc = lt % ACCS;
     const uint32_t taddr = taddr0 + acc * BN;
@@ -592,7 +598,10 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
     tmem_ld_wait();
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&tempty[acc]);                 // the accumulator is in registers: hand TMEM back
+    if (lane == 0) {                                          // the accumulator is in registers: hand TMEM back
+      if (PAIR) mbar_arrive_remote(leader_tempty);
+      else mbar_arrive(&tempty[acc]);
+    }
     float* slab = nullptr;
     if (EPI == KF_EPI_ROPE && use_slab) {                      // all 4 warps of the quarter take this path together (it depends on the tile only)
       slab = slabs + quarter * ROPE_SLAB_FLOATS;
@@ -601,21 +610,34 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
       quarter_barrier(quarter);
     }
     if (!live || n0 >= g.N || col >= item.cols) continue;      // column group past N in the last column tile, or past a half tile
-    if constexpr (EPI == KF_EPI_RES && W == 32) {
+    if (PAIR && rbase >= g.m_tiles * BM) continue;             // the follower's row tile past the last one
+    if constexpr (BOXES) {
       if (boxed) {
+        bool lost = false;
         if (rbase < g.M) {
-          if (!mbar_wait(bfull, bph, ctx, 5)) break;
-          bph ^= 1;
-          epilogue_res_tma(g, r, ts, bsl, gsl, box, lane);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(tmC, box, n0 * 4, rbase);
-            bulk_commit();
-            bulk_wait_read();
+#pragma unroll
+          for (int c = 0; c < W; c += 32) {                      // W = 64: two boxes, one after the other through the same 4 KB
+            if (c != 0 && lane == 0) {
+              mbar_expect_tx(bfull, RES_BOX_BYTES);
+              tma_load_2d(box, tmR, (n0 + c) * 4, rbase, bfull);
+            }
+            if (!mbar_wait(bfull, bph, ctx, 5)) {
+              lost = true;
+              break;
+            }
+            bph ^= 1;
+            epilogue_res_tma(g, reinterpret_cast<const uint32_t(&)[32]>(r[c]), ts, bsl + c, gsl + c, box, lane);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(tmC, box, (n0 + c) * 4, rbase);
+              bulk_commit();
+              bulk_wait_read();
+            }
           }
         }
-        box_load(idx + gridDim.x);
+        if (lost) break;
+        box_load(idx + stride);
         __syncwarp();
         continue;
       }

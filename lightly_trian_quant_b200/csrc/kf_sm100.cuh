@@ -291,6 +291,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn encode_tiled_fn();                         // cuTensorMapEncodeTiled from the driver, looked up once; null if it has none
 // 2-D row-major byte tensor [rows, row_bytes] with a [box_rows, 128-byte] box and the 128-byte swizzle.
 int make_tmap_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch_bytes, uint32_t box_rows);
+// Scale atoms as a 2-D tensor: one row = one 512-byte atom, box = `atoms` consecutive ones.
+int make_tmap_atoms(CUtensorMap* map, const void* base, uint64_t n_atoms, uint32_t atoms);
 int device_sm_count(int* sms);
 
 }  // namespace kf

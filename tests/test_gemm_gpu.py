@@ -291,7 +291,7 @@ def test_rate_probes_run_and_report_work():
     ops.check_device_error()
 
 
-@pytest.mark.parametrize("B,Q,P,K", [(3, 200, 1024, 256), (2, 77, 384, 128), (1, 130, 128, 64)])
+@pytest.mark.parametrize("B,Q,P,K", [(3, 200, 1024, 256), (2, 77, 384, 128), (1, 130, 128, 64), (14, 200, 1536, 128), (2, 200, 38400, 64)])
 def test_batched_products_match_one_launch_per_product(B, Q, P, K):
     """kf_gemm_bs with batch > 0 (ops.bmm_nt): every product bit-identical to its own PLAIN launch, rows of one product never
     written by the tiles of another (Q is not a multiple of the 128-row tile), and against the fp32 product."""
@@ -396,9 +396,10 @@ def test_last_round_in_half_tiles(fmt, M, N, K):
 
 
 # the error word is already set when the kernel starts (delay 0), or is set by the predecessor while the kernel, started early under dependent
-# launch, has requested its weights (delay 200 us); 16 operand stages are more than the ring holds, one stage is less; 9600 rows take the residual through shared memory
+# launch, has requested its weights (delay 200 us); 16 operand stages are more than the ring holds, one stage is less; 9600 rows take the residual through
+# shared memory (K = 256) and run on CTA pairs (the other kinds; all of them with K = 4096)
 @pytest.mark.parametrize("delay", [0, 200])
-@pytest.mark.parametrize("M,K", [(320, 256), (320, 4096), (9600, 256)])
+@pytest.mark.parametrize("M,K", [(320, 256), (320, 4096), (9600, 256), (9600, 4096)])
 def test_a_failed_predecessor_does_not_stall_the_launch(M, K, delay):
     """every role of the GEMM and attention kernels comes to the same decision when an earlier launch has failed: the launch ends well inside
     the two seconds of a bounded wait, and the next one is whole again."""
@@ -544,3 +545,61 @@ def test_epilogue_forms_agree(fmt, M, N):
             outs.append(q)
         assert torch.equal(outs[0].q, outs[1].q) and torch.equal(outs[0].sf, outs[1].sf), ofmt
     ops.check_device_error()
+
+
+# 49 row tiles (the follower of the last pair has none) x 3 column tiles = 75 tiles of 74 pairs: the last one is cut into halves; one operand stage and more than the
+# ring holds.  Row blocks of the same rows run on single CTAs.
+@pytest.mark.parametrize("fmt", FMTS + ["bf16"])
+@pytest.mark.parametrize("K", [256, 2048])
+def test_cta_pairs_against_launches_of_row_blocks(fmt, K):
+    ops = _ops()
+    B, Ntok, prefix, H, N = 3, 2089, 5, 4, 768
+    M = B * Ntok
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x = rnd(M, K).to(torch.bfloat16)
+    W = ops.QWeight(rnd(N, K) * 0.05, fmt)
+    bias, gamma, res = rnd(N), rnd(N), rnd(M, N)
+    tab = torch.cat((rnd(2, Ntok - prefix, 32),) * 2, dim=2)
+
+    def launches(r0, r1):
+        rows = x[r0:r1].contiguous()
+        a = rows
+        if fmt != "bf16":
+            a = ops.ActBuf(r1 - r0, K, fmt)
+            if fmt == "nv4":
+                a.ts.fill_(0.003)
+            ops.quant_rows(rows, a)
+        n = (r1 - r0) // Ntok
+        grown = torch.zeros(n, Ntok + 7, N, device="cuda")
+        ops.gemm_res(a, W, bias, gamma, res[r0:r1].contiguous(), out=grown, row_map=(Ntok, Ntok + 7, 7))
+        out = [ops.gemm_plain(a, W, bias), ops.gemm_plain(a, W, None, gelu=True, out_dtype=torch.float32), ops.gemm_res(a, W, bias, gamma, res[r0:r1].contiguous()),
+               grown.view(n, -1)]
+        for half in (False, True):
+            out.append(ops.qkv_rope(a, W, bias, tab[0].contiguous(), tab[1].contiguous(), Ntok, prefix, H, half_tables=half).transpose(0, 1).reshape(n, -1))
+        if fmt != "bf16":
+            for ofmt in FMTS:
+                q = ops.ActBuf(r1 - r0, N, ofmt)
+                q.sf.fill_(0xAA)
+                if ofmt == "nv4":
+                    q.ts.fill_(0.002)
+                ops.gemm_gelu_q(a, W, bias, q, round_bf16=True)
+                out += [q.q, q.sf]
+        ops.check_device_error()
+        return out
+
+    big = launches(0, M)
+    for b in range(B):
+        r0, r1 = b * Ntok, (b + 1) * Ntok
+        for i, (u, v) in enumerate(zip(big, launches(r0, r1))):
+            if u.dim() == 1:                                # blocked scales: only the first image starts on a row-tile boundary
+                n = v.numel() // 17 * 16                    # its 16 whole row tiles
+                assert b != 0 or torch.equal(u[:n], v[:n]), i
+                continue
+            assert torch.equal(u[b:b + 1] if u.shape[0] == B else u[r0:r1], v), (b, i)
+    if fmt != "bf16":                                       # scale bytes of the rows past M: zeros, as the layout asks for
+        for sf in (t for t in big if t.dim() == 1):
+            tail = sf.view(49, -1, 32, 4, 4)[48]            # [k-blocks / 4, row & 31, row >> 5, 4] of the last row tile
+            rows = torch.arange(128, device="cuda")
+            per_row = tail.permute(2, 1, 0, 3).reshape(128, -1)
+            assert not per_row[48 * 128 + rows >= M].any()
