@@ -613,6 +613,10 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
     if (PAIR && rbase >= g.m_tiles * BM) continue;             // the follower's row tile past the last one
     if constexpr (BOXES) {
       if (boxed) {
+        // The column groups take turns over about half of the next tile's main loop: 16 warps' boxes at once (64 KB of loads, then of stores,
+        // twice a tile) held up the operand loads in the same queue (NVFP4 22 470 x 4096 x 1024 61.5 -> 58.1 us, MXFP8 92 -> 90, x 768 60.7 -> 58.1;
+        // 100 ns a stage is too long for bf16: 150 -> 164 against 148.5).  Not for a CTA's last tile, where it would only come later.
+        if (PAIR && cg != 0 && idx + stride < g.items) __nanosleep(cg * g.k_tiles * 75);
         bool lost = false;
         if (rbase < g.M) {
 #pragma unroll

@@ -13,7 +13,7 @@
 //                        waits for the global stores of the tile before: 1350-1900 clk per tile from the accumulator to its hand-over instead of
 //                        110-160, which had the pair level with one CTA
 //   measured   one CTA -> pair, captured launches, M = 22 470, K x N of ViT-L (us): bf16 qkv 127 -> 107, fc1 169 -> 143, fc2 161 -> 153; MXFP8
-//              qkv 79 -> 71, proj 53 -> 44, fc1 102 -> 90, fc2 96 -> 93; NVFP4 fc1 78 -> 71, fc2 65 -> 62, plain 62 -> 55
+//              qkv 79 -> 71, proj 53 -> 44, fc1 102 -> 90, fc2 96 -> 90; NVFP4 fc1 84 -> 79, fc2 65 -> 58, plain 62 -> 55
 //
 // No load is a multicast; the two cluster barriers (start, teardown) are reached by every thread on every path, every other wait is bounded.
 // Replaces the same reference kernels as kf_gemm.cu: infer-opt/round13_mxfp8_full/impl/mgx_core.cu:118-444 and
