@@ -335,10 +335,11 @@ __device__ __forceinline__ void ln_row(const TI* xr, const float (&ww)[NV][8], c
 }
 
 // Rows are streamed through shared memory: each warp owns a ring of LNQ_RING row buffers filled by 1-D bulk copies
-// (cp.async.bulk + mbarrier), so two to three rows per warp (8-12 KB) are in flight while the warp normalises and
-// quantises the current one; with 16 warps per SM that keeps well over 100 KB of HBM reads outstanding per SM, which
-// register-staged loads cannot (they stop while the warp computes).
-constexpr int LNQ_RING = 3;
+// (cp.async.bulk + mbarrier), so one to two rows per warp (4-8 KB) are in flight while the warp normalises and
+// quantises the current one; with 16 warps per SM that keeps about 100 KB of HBM reads outstanding per SM, which
+// register-staged loads cannot (they stop while the warp computes).  A third row only costs (22 470 rows, us, 3 -> 2: NVFP4 1024 24.7 -> 22.6, 768
+// 26.7 -> 25.5; MXFP8 26.8 -> 26.1, 21.2 -> 20.6); five or six CTAs per SM spill the affine parameters (28.8, 35.1).
+constexpr int LNQ_RING = 2;
 
 template <int NV, int FMT, typename TI>
 __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float eps,
