@@ -32,13 +32,16 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
   else return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
 }
 
-// 32 consecutive elements, all loads issued before the first conversion
+// 32 consecutive elements: all loads issued together, converted when they are needed
 template <typename T>
-__device__ __forceinline__ void load32(const T* p, bool wide, float (&v)[32]) {
-  constexpr int PIECES = (int)sizeof(T);                  // of 32 bytes: 4 of fp32, 2 of a 16-bit type
-  uint32_t w[8 * PIECES];
+constexpr int LOAD32_WORDS = 8 * (int)sizeof(T);          // 32-byte pieces: 4 of fp32, 2 of a 16-bit type
+template <typename T>
+__device__ __forceinline__ void load32_raw(const T* p, bool wide, uint32_t (&w)[LOAD32_WORDS<T>]) {
 #pragma unroll
-  for (int i = 0; i < PIECES; ++i) load32b(reinterpret_cast<const uint8_t*>(p) + 32 * i, wide, w + 8 * i);
+  for (int i = 0; i < (int)sizeof(T); ++i) load32b(reinterpret_cast<const uint8_t*>(p) + 32 * i, wide, w + 8 * i);
+}
+template <typename T>
+__device__ __forceinline__ void unpack32(const uint32_t (&w)[LOAD32_WORDS<T>], float (&v)[32]) {
   if constexpr (sizeof(T) == 4) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(w[i]);
@@ -50,6 +53,12 @@ __device__ __forceinline__ void load32(const T* p, bool wide, float (&v)[32]) {
       v[2 * i + 1] = f.y;
     }
   }
+}
+template <typename T>
+__device__ __forceinline__ void load32(const T* p, bool wide, float (&v)[32]) {
+  uint32_t w[LOAD32_WORDS<T>];
+  load32_raw<T>(p, wide, w);
+  unpack32<T>(w, v);
 }
 
 // Gathers the scale bytes of 4 consecutive k-blocks (held by lanes lane0, lane0+STEP, ...) into one word on lane0.
@@ -67,33 +76,51 @@ __device__ __forceinline__ uint32_t gather_sf_word(int byte, int lane) {
 // One thread = 32 consecutive elements of one row: one mx block, or two nv4 blocks whose scalars go through the packed-pair
 // quantiser of the GEMM epilogue.  No maximum crosses lanes; two (nv4) or four (mx) lanes share one scale word.
 // Bound by HBM.  With 16 elements per thread (two lanes per mx block, the nv4 divisions scalar) the NVFP4 form was bound by
-// instruction issue: 51 360 x 4096 bf16 139 us = 3.9 TB/s, now 108 us = 5.0 TB/s.
+// instruction issue: 51 360 x 4096 bf16 139 us = 3.9 TB/s, then 103 us.  16-bit inputs: the grid is what is resident at once and a thread
+// requests its next item before it quantises the present one (half of a thread's life had no load in flight): NVFP4 103 -> 86 us = 6.3 TB/s,
+// MXFP8 102 -> 97, MXFP4 92 -> 84; 22 470 x 1024 16.5 -> 14.4; 6420 x 3072 12.8 -> 11.3.  fp32 inputs have twice the words in flight already
+// and lose the residency to the second set of registers (22 470 x 1024 20.6 -> 24.5 us): one item per thread.
 template <typename T, int FMT>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x, int64_t ldx, int M, int K, const float* __restrict__ ts_ptr,
                                                          const float* __restrict__ bias, int flags, int wide, uint8_t* __restrict__ q,
                                                          uint8_t* __restrict__ sf, int64_t items_valid, int64_t items_total) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
-  const int per_row = K >> 5;
-  int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool in_pad = w < items_total;          // inside the padded row range (scale bytes must be written)
-  const bool valid = w < items_valid;           // a real row
+  const uint32_t per_row = (uint32_t)K >> 5;
   // 32-bit index arithmetic (the host checks that the item count fits); a power-of-two row length needs no division
-  const uint32_t w32 = (uint32_t)w;
+  const bool pow2 = (per_row & (per_row - 1)) == 0;
+  const int log2_row = 31 - __clz((int)per_row);
+  auto place = [&](uint32_t w, int& row, int& c32) {
+    row = (int)(pow2 ? w >> log2_row : w / per_row);
+    c32 = (int)(pow2 ? w & (per_row - 1) : w - (uint32_t)row * per_row);
+  };
+  const Nv4Scale ts = nv4_scale(FMT == KF_FMT_NV4 ? __ldg(ts_ptr) : 1.f);
+  // Rows up to items_total exist in the blocked scale layout, those from items_valid on only get zero scale bytes.  Both counts are multiples
+  // of a row, and a warp's 32 items lie on one side of items_total as a whole (128 rows of it): whole warps run the loop.
+  const uint32_t valid_end = (uint32_t)items_valid, end = (uint32_t)items_total, stride = gridDim.x * 256u;
+  uint32_t w32 = blockIdx.x * 256u + threadIdx.x;
   int row, c32;
-  if ((per_row & (per_row - 1)) == 0) {
-    row = (int)(w32 >> (31 - __clz(per_row)));
-    c32 = (int)(w32 & (uint32_t)(per_row - 1));
-  } else {
-    row = (int)(w32 / (uint32_t)per_row);
-    c32 = (int)(w32 - (uint32_t)row * (uint32_t)per_row);
-  }
+  place(w32, row, c32);
+  constexpr bool AHEAD = sizeof(T) == 2;
+  uint32_t raw[LOAD32_WORDS<T>];
+  if (AHEAD && w32 < valid_end) load32_raw<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, raw);
+  for (;;) {
+  const bool valid = w32 < valid_end, in_pad = w32 < end;
   float v[32];
   if (valid) {
-    load32<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, v);
+    if (AHEAD) unpack32<T>(raw, v);
+    else load32<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, v);
   } else {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = 0.f;
+  }
+  // 16-bit inputs: the next item's loads travel while this one is quantised
+  const uint32_t next = w32 + stride;
+  const bool more = AHEAD && __any_sync(0xffffffffu, next < end && next >= stride);
+  int nrow = 0, nc32 = 0;
+  if (more) {
+    place(next, nrow, nc32);
+    if (next < valid_end) load32_raw<T>(x + (int64_t)nrow * ldx + nc32 * 32, wide != 0, raw);
   }
   if constexpr (FMT == KF_FMT_NV4 && std::is_same<T, __half>::value) {
     // The corrected quotient of a negative zero is a positive one (code 0, the bit rule says 8).  fp16 inputs reach -0 by
@@ -103,7 +130,6 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x
       for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(v[i]) == 0x80000000u ? -1e-20f : v[i];
     }
   }
-  const Nv4Scale ts = nv4_scale(FMT == KF_FMT_NV4 ? __ldg(ts_ptr) : 1.f);
   if ((flags & KF_Q_GELU) && valid) {
     const float4* b4 = reinterpret_cast<const float4*>(bias + c32 * 32);
 #pragma unroll
@@ -163,6 +189,11 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x
     if (!valid) byte = 0;
     const uint32_t word = gather_sf_word<1>(byte, lane);
     if (in_pad && (lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, c32, K >> 7)) = word;
+  }
+  if (!AHEAD || !more) break;
+  w32 = next;
+  row = nrow;
+  c32 = nc32;
   }
 }
 
@@ -639,15 +670,30 @@ static int launch_quant_rows(int fmt, const void* x, int64_t ldx, int M, int K, 
   int64_t per_row = K / 32;
   int64_t valid = (int64_t)M * per_row, total = (int64_t)((M + 127) / 128 * 128) * per_row;
   KF_REQUIRE(total + 256 < (1ll << 32), "kf_quant_rows: M*K/32 = %lld work items do not fit the 32-bit index", (long long)total);
-  unsigned grid = (unsigned)((total + 255) / 256);
+  int sms = 0, dev = 0;
+  const int rc = device_sm_count(&sms);
+  if (rc != KF_OK) return rc;
+  cudaGetDevice(&dev);
   const T* xp = static_cast<const T*>(x);
   const int wide = rows_32b_aligned(x, ldx * (int64_t)sizeof(T));
   uint8_t *qp = static_cast<uint8_t*>(q), *sp = static_cast<uint8_t*>(sf);
-  cudaError_t e;
-  if (fmt == KF_FMT_MX8) e = launch_maybe_pdl(M, quant_rows_kernel<T, KF_FMT_MX8>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
-  else if (fmt == KF_FMT_NV4) e = launch_maybe_pdl(M, quant_rows_kernel<T, KF_FMT_NV4>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
-  else e = launch_maybe_pdl(M, quant_rows_kernel<T, KF_FMT_MX4>, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total);
-  return cuda_status(e, "kf_quant_rows launch");
+  static int per_sm_cached[3][64] = {};                  // resident CTAs per (format, device) of this input type
+  auto go = [&](auto kern) {
+    int per_sm = dev < 64 ? per_sm_cached[fmt][dev] : 0;
+    if (per_sm == 0) {
+      const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
+      if (e != cudaSuccess) return cuda_status(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(quant_rows_kernel)");
+      if (per_sm < 1) per_sm = 1;
+      if (dev < 64) per_sm_cached[fmt][dev] = per_sm;
+    }
+    const int64_t blocks = (total + 255) / 256, resident = (int64_t)sms * per_sm;
+    const int64_t rounds = sizeof(T) == 2 ? (blocks + resident - 1) / resident : 1;
+    const unsigned grid = (unsigned)((blocks + rounds - 1) / rounds);   // equal shares
+    return cuda_status(launch_maybe_pdl(M, kern, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total), "kf_quant_rows launch");
+  };
+  if (fmt == KF_FMT_MX8) return go(quant_rows_kernel<T, KF_FMT_MX8>);
+  if (fmt == KF_FMT_NV4) return go(quant_rows_kernel<T, KF_FMT_NV4>);
+  return go(quant_rows_kernel<T, KF_FMT_MX4>);
 }
 
 template <int NV, typename TI>

@@ -245,3 +245,33 @@ def test_quant_rows_of_rows_without_32_byte_alignment(fmt, dtype):
     q, sf = _run_quant(rows, fmt, ts)
     eq, esf = _expect(xn, fmt, ts)
     assert np.array_equal(sf, esf) and np.array_equal(q, eq)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("fmt", ["mx8", "nv4", "mx4"])
+@pytest.mark.parametrize("M,K", [(9003, 2048), (9003, 768), (12929, 256)])
+def test_quant_rows_of_many_rounds(fmt, dtype, M, K):
+    """launches of more items than are resident at once (a thread works through several, 16-bit inputs one ahead), rows that end inside a
+    scale block, row lengths with and without a division: the bytes of launches of 128 rows each; scale bytes past the last row are zero."""
+    from lightly_trian_quant_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = (torch.randn(M, K + 32, generator=g, device="cuda") * 3).to(dtype)[:, :K]     # rows with a pitch
+    big = ops.ActBuf(M, K, fmt)
+    big.q.fill_(0xAA)
+    big.sf.fill_(0xAA)
+    if fmt == "nv4":
+        big.ts.fill_(0.003)
+    ops.quant_rows(x, big)
+    ops.check_device_error()
+    per = big.sf.numel() // ((M + 127) // 128)
+    for r0 in (0, 128 * (M // 256), 128 * ((M - 1) // 128)):
+        rows = x[r0:r0 + 128]
+        one = ops.ActBuf(rows.shape[0], K, fmt)
+        if fmt == "nv4":
+            one.ts.fill_(0.003)
+        ops.quant_rows(rows, one)
+        assert torch.equal(big.q[r0:r0 + 128], one.q.view_as(big.q[r0:r0 + 128])), r0
+        assert torch.equal(big.sf.view(-1)[r0 // 128 * per:(r0 // 128 + 1) * per], one.sf.view(-1)), r0
+    tail = big.sf.view(-1)[-per:].view(-1, 32, 4, 4).permute(2, 1, 0, 3).reshape(128, -1)
+    assert not tail[(M - 1) % 128 + 1:].any()
