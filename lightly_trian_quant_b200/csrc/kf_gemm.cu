@@ -66,7 +66,9 @@ static_assert(gemm_smem<KF_EPI_ROPE, 256>(3) <= GEMM_SMEM_MAX && gemm_smem<KF_EP
               "shared memory of the deepest rings");
 
 // ------------------------------------------------------------------------------------------------ the kernel
-template <int KIND, int EPI, int BN>
+// FORM: epilogue_form of the launch.  A kernel of its own for each: with all of them in one the code that a short launch fetches is scattered
+// (ViT-B 256 px: captured 575 -> 569 us, eager 615 -> 610).
+template <int KIND, int EPI, int BN, int FORM>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmR,
             const __grid_constant__ CUtensorMap tmC, const GemmArgs g) {
@@ -241,7 +243,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ------------------------------------------------------------------ epilogue: 16 warps, warp = (TMEM lane quarter, 64-column group)
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
     if (!bad_align) {
-      epilogue_warps<EPI, BN>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tmR, &tmC, ctx, warp, lane);
+      epilogue_warps<EPI, BN, false, FORM>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tmR, &tmC, ctx, warp, lane);
     }
   }
 
@@ -351,26 +353,38 @@ struct GemmMaps {
   CUtensorMap A, W, R, C;                                 // R, C: the residual and the output of a RES launch through shared memory; R: W in boxes of 128 rows for half tiles
 };
 
-template <int KIND, int EPI, int BN>
+template <int KIND, int EPI, int BN, int FORM = -1>
 static int launch_gemm(const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<KIND, EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_MAX);
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<KIND, EPI, BN, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_MAX);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_kernel)");
     if (dev < 64) attr_set[dev] = true;
   }
-  return cuda_status(launch_maybe_pdl(g.M, gemm_kernel<KIND, EPI, BN>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats, g.res_tma != 0), st, tm.A, tm.W, tm.R, tm.C, g), "kf_gemm_bs launch");
+  return cuda_status(launch_maybe_pdl(g.M, gemm_kernel<KIND, EPI, BN, FORM>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats, g.res_tma != 0), st, tm.A, tm.W, tm.R, tm.C, g), "kf_gemm_bs launch");
 }
 
 template <int KIND, int BN>
 static int launch_gemm_epi(int epi, const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
   switch (epi) {
-    case KF_EPI_PLAIN: return launch_gemm<KIND, KF_EPI_PLAIN, BN>(tm, g, grid, st);
+    case KF_EPI_PLAIN:
+      switch (epilogue_form(epi, g)) {
+        case PL_BF16: return launch_gemm<KIND, KF_EPI_PLAIN, BN, PL_BF16>(tm, g, grid, st);
+        case PL_GELU: return launch_gemm<KIND, KF_EPI_PLAIN, BN, PL_GELU>(tm, g, grid, st);
+        case PL_GELU_PRE: return launch_gemm<KIND, KF_EPI_PLAIN, BN, PL_GELU_PRE>(tm, g, grid, st);
+        default: return launch_gemm<KIND, KF_EPI_PLAIN, BN>(tm, g, grid, st);
+      }
     case KF_EPI_RES: return launch_gemm<KIND, KF_EPI_RES, BN>(tm, g, grid, st);
     case KF_EPI_ROPE: return launch_gemm<KIND, KF_EPI_ROPE, BN>(tm, g, grid, st);
-    default: return launch_gemm<KIND, KF_EPI_QUANT, BN>(tm, g, grid, st);
+    default:
+      switch (epilogue_form(epi, g)) {
+        case KF_FMT_MX8: return launch_gemm<KIND, KF_EPI_QUANT, BN, KF_FMT_MX8>(tm, g, grid, st);
+        case KF_FMT_NV4: return launch_gemm<KIND, KF_EPI_QUANT, BN, KF_FMT_NV4>(tm, g, grid, st);
+        case KF_FMT_MX4: return launch_gemm<KIND, KF_EPI_QUANT, BN, KF_FMT_MX4>(tm, g, grid, st);
+        default: return launch_gemm<KIND, KF_EPI_QUANT, BN>(tm, g, grid, st);
+      }
   }
 }
 

@@ -221,11 +221,6 @@ __device__ __forceinline__ float2 plain_pair(const GemmArgs& g, float2 a, float2
   if (MODE < 0 && (g.flags & KF_G_ROUND_BF16)) x = bf16_round2(x);
   return x;
 }
-__device__ __forceinline__ int plain_mode(const GemmArgs& g) {               // the same for all tiles of a launch
-  const int f = g.flags & (KF_G_PRE_ROUND_BF16 | KF_G_GELU | KF_G_ROUND_BF16);
-  if (g.out_dtype != KF_BF16) return -1;
-  return f == 0 ? PL_BF16 : f == KF_G_GELU ? PL_GELU : f == (KF_G_GELU | KF_G_PRE_ROUND_BF16) ? PL_GELU_PRE : -1;
-}
 __device__ __forceinline__ void plain_chunk(const GemmArgs& g, const uint32_t (&r)[32], float ts, uint8_t* dst_row, int n0, const float* bsm /* the chunk's 32 bias values in shared memory, zeros without a bias */) {
   const float2 ts2 = splat2(ts);
 #pragma unroll
@@ -503,12 +498,24 @@ __device__ __forceinline__ WorkItem work_item(const GemmArgs& g, int idx) {
   return w;
 }
 
+// The form of a launch's options that has an epilogue of its own, or -1.
+__host__ __device__ inline int epilogue_form(int epi, const GemmArgs& g) {
+  if (epi == KF_EPI_PLAIN) {
+    const int f = g.flags & (KF_G_PRE_ROUND_BF16 | KF_G_GELU | KF_G_ROUND_BF16);
+    if (g.row_group > 0 || g.out_dtype != KF_BF16) return -1;
+    return f == 0 ? PL_BF16 : f == KF_G_GELU ? PL_GELU : f == (KF_G_GELU | KF_G_PRE_ROUND_BF16) ? PL_GELU_PRE : -1;
+  }
+  if (epi == KF_EPI_QUANT) return g.y_dbg == nullptr && (g.flags & (KF_Q_ROUND_BF16 | KF_Q_FAST_NV4)) == KF_Q_ROUND_BF16 ? g.out_fmt : -1;
+  return -1;
+}
+constexpr int ANY_FORM = -2;                           // the kernel looks the form up and has the code of all of them
+
 // Body of the 16 epilogue warps (warp = (TMEM lane quarter, 64- or 32-column group)): per tile, stage the bias slice (and fetch
 // the rotary-table rows), wait for the accumulator, take the warp's piece into registers, hand TMEM back at once and
 // run the fused epilogue on the registers while the next tile's main loop fills the accumulator again.
 // PAIR (CTA pairs, BN = 256): work items are counted per pair and name row tiles 2 * m_blk and 2 * m_blk + 1, one per CTA; the
 // accumulator is handed back to the leader's MMA warp.
-template <int EPI, int BN, bool PAIR = false>
+template <int EPI, int BN, bool PAIR = false, int FORM = ANY_FORM>
 __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty, float* slices,
                                                float* slabs, uint8_t* boxes, uint64_t* box_full, const CUtensorMap* tmR, const CUtensorMap* tmC, const WaitCtx& ctx, int warp,
                                                int lane) {
@@ -554,9 +561,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
     }
   };
   if (boxed) box_load(first);
-  // The form of the launch's options that has an epilogue of its own, or -1: the same for every tile, tested once per tile instead of per value
-  const int mode = EPI == KF_EPI_PLAIN ? (g.row_group > 0 ? -1 : plain_mode(g))
-                   : EPI == KF_EPI_QUANT && g.y_dbg == nullptr && (g.flags & (KF_Q_ROUND_BF16 | KF_Q_FAST_NV4)) == KF_Q_ROUND_BF16 ? g.out_fmt : -1;
+  const int mode = FORM == ANY_FORM ? epilogue_form(EPI, g) : FORM;   // the same for every tile, tested once per tile instead of per value
   int lt = 0;
   // ROPE: the four warps of a quarter meet at named barriers, which have no limit.  A warp whose wait ran out therefore does not leave: it
   // keeps company at the barriers of its remaining tiles (the same number in all four warps: they depend on the tile only) and
@@ -647,7 +652,9 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
       }
     }
     auto finish = [&](auto form) { epilogue_math<EPI, W, decltype(form)::value>(g, r, ts, sco, rbase, n0, j0, bsl, gsl, slab, lane, row_end, res); };
-    if constexpr (EPI == KF_EPI_PLAIN) {
+    if constexpr (FORM != ANY_FORM) {
+      finish(std::integral_constant<int, FORM>{});
+    } else if constexpr (EPI == KF_EPI_PLAIN) {
       if (mode == PL_BF16) finish(std::integral_constant<int, PL_BF16>{});
       else if (mode == PL_GELU) finish(std::integral_constant<int, PL_GELU>{});
       else if (mode == PL_GELU_PRE) finish(std::integral_constant<int, PL_GELU_PRE>{});
