@@ -27,7 +27,8 @@
 //            finds its maximum, recomputes its P and has its O rescaled (TMEM load, multiply, store), which happens on
 //            the first tiles and then almost never; the O barriers are waited only then and at the end of an item.
 //            Measured, tiles of 64 -> 96 keys (B 14, H 16, N 1605, bf16 out / NVFP4 out; N 1805, NVFP4 out; B 8, N 4101, f16,
-//            MXFP4 out; B 1, N 1605, NVFP4 out): 199 -> 186 / 204 -> 194 / 250 -> 239 / 667 -> 636 / 24.7 -> 23.6 us.
+//            MXFP4 out; B 1, N 1605, NVFP4 out): 199 -> 186 / 204 -> 194 / 250 -> 239 / 667 -> 636 / 24.7 -> 23.6 us; 256-bit stores of the output
+//            where it is 32-byte aligned: 186 -> 184.3 / 191.1 -> 190.5 / 236.2 -> 235.4 us (16-byte pieces of a row per lane cost twice the look-ups).
 //            Not kept: the barrier asked for only where it is waited on (198 us against 194), the next row requested at the end of the
 //            step (199), five of sixteen pairs or none of every third 32 off the special-function unit (202, 202), an item's output behind the
 //            first step of the next one (203: the waits it hides are fewer than the registers it takes from the loop); with
@@ -70,6 +71,7 @@ struct AttnArgs {
   unsigned int* err;
   // optional fused quantisation of the output (the proj GEMM's A operand): out_fmt < 0 = off
   int out_fmt, flags;
+  int wide;         // the output is 32-byte aligned: 256-bit stores
   uint8_t *Qo, *SFo;
   const float* tso;
 };
@@ -329,6 +331,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int i = 0; i < 16; ++i) m4[i & 3] = max3(m4[i & 3], __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
       return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
     };
+    auto store32 = [&](uint8_t* dst, const uint32_t* w) {
+      if (a.wide) {
+        stg8w(dst, w);
+      } else {
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+    };
     auto mask_tail = [&](uint32_t (&r)[32], int key0) {          // columns past N never win the max and give P = 0
 #pragma unroll
       for (int i = 0; i < 32; ++i)
@@ -493,9 +503,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             quant_nv4_pair16(b0, am[k], b1, am[k + 1], tsc, div_true, o + 2 * k, by[k], by[k + 1]);
           }
           const uint32_t word = (uint32_t)by[0] | ((uint32_t)by[1] << 8) | ((uint32_t)by[2] << 16) | ((uint32_t)by[3] << 24);
-          uint4* dst = reinterpret_cast<uint4*>(a.Qo + m * (d >> 1) + h * 32);
-          dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-          dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+          store32(a.Qo + m * (d >> 1) + h * 32, o);
           *reinterpret_cast<uint32_t*>(a.SFo + sf_offset((int)m, h * 4, d >> 6)) = word;
         } else {
           uint32_t half = 0;
@@ -511,9 +519,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               uint32_t o[8];
               quant_mx8<16>(va, am, div_true, o, by);
               quant_mx8<16>(vb, am, div_true, o + 4, by);
-              uint4* dst = reinterpret_cast<uint4*>(a.Qo + m * d + h * 64 + k * 32);
-              dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-              dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+              store32(a.Qo + m * d + h * 64 + k * 32, o);
             } else {
               uint32_t o[4];
               quant_mx4<16>(va, am, div_true, o, by);
@@ -532,9 +538,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           w[i] = pack16(__uint_as_float(r0[2 * i]) * inv, __uint_as_float(r0[2 * i + 1]) * inv, F16);
           w[16 + i] = pack16(__uint_as_float(r1[2 * i]) * inv, __uint_as_float(r1[2 * i + 1]) * inv, F16);
         }
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<uint8_t*>(a.O) + (((size_t)b * a.N + n) * a.H + h) * (AT_D * 2));
+        uint8_t* dst = static_cast<uint8_t*>(a.O) + (((size_t)b * a.N + n) * a.H + h) * (AT_D * 2);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+        for (int i = 0; i < 4; ++i) store32(dst + 32 * i, w + 8 * i);
       }
     }
     }   // items
@@ -636,6 +642,7 @@ static int attn_launch(int dtype, const void* qkv, void* O, int B, int N, int H,
   a.scale_log2 = 0.125f * 1.4426950408889634f;
   a.err = dev_error_ptr();
   a.out_fmt = out_fmt; a.flags = flags; a.Qo = static_cast<uint8_t*>(Qo); a.SFo = static_cast<uint8_t*>(SFo); a.tso = tso;
+  a.wide = (reinterpret_cast<uintptr_t>(out_fmt < 0 ? O : Qo) & 31) == 0;
   KF_REQUIRE(a.err != nullptr, "kf_attn_fwd: device error word unavailable");
   const int q_tiles = (N + AT_BM - 1) / AT_BM;
   const long long items = (long long)B * H * q_tiles;

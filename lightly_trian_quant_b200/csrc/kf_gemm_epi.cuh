@@ -85,11 +85,6 @@ __device__ __forceinline__ void stg8(void* p, float a, float b, float c, float d
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h)
                : "memory");
 }
-__device__ __forceinline__ void stg8w(void* p, const uint32_t* w) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
-               "r"(w[6]), "r"(w[7])
-               : "memory");
-}
 // two fp32 -> one 32-bit word of two bf16 / f16 values (first value in the low half)
 __device__ __forceinline__ uint32_t pack2(float a, float b, int out_dtype) {
   if (out_dtype == KF_BF16) {

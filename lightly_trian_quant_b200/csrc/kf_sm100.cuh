@@ -123,6 +123,13 @@ __device__ __forceinline__ bool mbar_wait_warp3(uint64_t* b0, uint32_t p0, uint6
   return __all_sync(0xffffffffu, mbar_wait(b2, p2, ctx, where) && mbar_wait(b1, p1, ctx, where) && mbar_wait(b0, p0, ctx, where));
 }
 
+// 32 bytes to a 32-byte aligned address
+__device__ __forceinline__ void stg8w(void* p, const uint32_t* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
+               "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+
 // ------------------------------------------------------------------------------------------------ TMA / bulk copies
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),

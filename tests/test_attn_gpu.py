@@ -142,3 +142,26 @@ def test_attn_larger_logits_behind_the_first_keys(dtype, lo, N):
     assert torch.isfinite(out).all()
     err = go.rel_fro(out.float().cpu().numpy(), ao.attn_ref(qkv.float().numpy()))
     assert err < (4e-3 if dtype == torch.bfloat16 else 1e-3), err
+
+
+def test_attn_outputs_at_16_byte_alignment():
+    """outputs that are 16- but not 32-byte aligned take the narrower stores: the same bits."""
+    ops = _ops()
+    B, N, H = 2, 200, 2
+    qkv = torch.randn(3, B, N, H, 64, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    ref = ops.attn_fwd(qkv)
+    off = torch.empty(B * N * H * 64 + 8, dtype=torch.bfloat16, device="cuda")[8:].view(B, N, H * 64)
+    assert off.data_ptr() % 32 == 16
+    assert torch.equal(ops.attn_fwd(qkv, out=off), ref)
+    for fmt in ("mx8", "nv4", "mx4"):
+        outs = []
+        for shift in (0, 16):
+            q = ops.ActBuf(B * N, H * 64, fmt, device="cuda")
+            if fmt == "nv4":
+                q.ts.fill_(0.002)
+            q.q = torch.empty(q.q.numel() + shift, dtype=q.q.dtype, device="cuda")[shift:].view_as(q.q)
+            assert q.q.data_ptr() % 32 == shift
+            ops.attn_fwd_quant(qkv, q)
+            outs.append(q)
+        assert torch.equal(outs[0].q, outs[1].q) and torch.equal(outs[0].sf, outs[1].sf), fmt
+    ops.check_device_error()
