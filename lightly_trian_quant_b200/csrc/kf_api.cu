@@ -45,13 +45,13 @@ bool pdl_for(int64_t rows, cudaStream_t st) {
 __device__ unsigned int g_dev_error[4];
 
 unsigned int* dev_error_ptr() {
-  static unsigned int* cached[64] = {nullptr};
+  static PerDevice<unsigned int*> cached;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  if (dev < 64 && cached[dev]) return cached[dev];
+  if (unsigned int* known = cached.get(dev)) return known;
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_dev_error) != cudaSuccess) return nullptr;
-  if (dev < 64) cached[dev] = static_cast<unsigned int*>(p);
+  cached.put(dev, static_cast<unsigned int*>(p));
   return static_cast<unsigned int*>(p);
 }
 

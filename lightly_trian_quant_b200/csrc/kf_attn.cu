@@ -629,13 +629,14 @@ static int attn_launch(int dtype, const void* qkv, void* O, int B, int N, int H,
       {attn_fwd_kernel<1, -1>, attn_fwd_kernel<1, KF_FMT_MX8>, attn_fwd_kernel<1, KF_FMT_NV4>, attn_fwd_kernel<1, KF_FMT_MX4>}};
   const int oi = out_fmt < 0 ? 0 : out_fmt == KF_FMT_MX8 ? 1 : out_fmt == KF_FMT_NV4 ? 2 : 3;
   const KernelFn kern = table[dtype == KF_F16 ? 1 : 0][oi];
-  static bool attr_set[64][2][4] = {};
+  static PerDevice<bool> attr_set[2][4];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64 || !attr_set[dev][dtype == KF_F16 ? 1 : 0][oi]) {
+  PerDevice<bool>& ready = attr_set[dtype == KF_F16 ? 1 : 0][oi];
+  if (!ready.get(dev)) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(attn_fwd_kernel)");
-    if (dev < 64) attr_set[dev][dtype == KF_F16 ? 1 : 0][oi] = true;
+    ready.put(dev, true);
   }
   AttnArgs a{};
   a.O = O; a.B = B; a.N = N; a.H = H; a.f16 = dtype == KF_F16;

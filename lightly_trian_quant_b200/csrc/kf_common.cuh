@@ -1,6 +1,7 @@
 // Shared device/host helpers of the B200 (sm_100a) low-precision ViT path: format conversions, the 128x4 blocked
 // scale-factor addressing, status codes and the last-error string of the C-ABI.
 #pragma once
+#include <atomic>
 #include <utility>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -18,6 +19,20 @@ void set_error(const char* fmt, ...);
 int cuda_status(cudaError_t e, const char* what);
 int device_sm_count(int* sms);   // multiprocessor count of the current device (cached)
 bool pdl_for(int64_t rows, cudaStream_t st);   // programmatic dependent launch for a launch over this many rows?
+
+// A value that is worked out once per device and kept; T{} while it has not been.  Callers hold no lock (the Python layer releases the
+// interpreter's): threads that make their first call at the same time work out the same value and each stores it.
+template <typename T>
+class PerDevice {
+  static constexpr int MAX_DEVICES = 64;
+  std::atomic<T> v_[MAX_DEVICES] = {};
+
+ public:
+  T get(int dev) const { return dev >= 0 && dev < MAX_DEVICES ? v_[dev].load(std::memory_order_acquire) : T{}; }
+  void put(int dev, T value) {
+    if (dev >= 0 && dev < MAX_DEVICES) v_[dev].store(value, std::memory_order_release);
+  }
+};
 
 // Programmatic dependent launch: a kernel lets its successor's CTAs start on SMs it no longer occupies (its partial last
 // wave, its teardown) and the successor runs its prologue (barrier set-up, TMEM allocation, descriptor prefetch) there; the

@@ -30,8 +30,6 @@
 // Replaces (reference checkout paths): infer-opt/round13_mxfp8_full/impl/mgx_core.cu:118-444 (MXFP8, mma.sync) and
 // infer-opt/round14_fp4_full/impl/fp4g_core.cu:153-470 (NVFP4 / MXFP4, mma.sync); epilogue math per
 // mgx_core.cu:308-426 and fp4g_core.cu:309-382.
-#include <mutex>
-
 #include "kf_gemm_epi.cuh"
 
 namespace kf {
@@ -262,14 +260,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
 // ------------------------------------------------------------------------------------------------ host side
 EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
+  static const EncodeTiledFn fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
   return fn;
 }
 
@@ -331,18 +327,18 @@ int make_tmap_atoms(CUtensorMap* map, const void* base, uint64_t n_atoms, uint32
 }
 
 int device_sm_count(int* sms) {
-  static int cached[64] = {0};
+  static PerDevice<int> cached;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_status(e, "cudaGetDevice");
-  if (dev < 64 && cached[dev]) {
-    *sms = cached[dev];
+  int n = cached.get(dev);
+  if (n != 0) {
+    *sms = n;
     return KF_OK;
   }
-  int n = 0;
   e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_status(e, "cudaDeviceGetAttribute");
-  if (dev < 64) cached[dev] = n;
+  cached.put(dev, n);
   *sms = n;
   return KF_OK;
 }
@@ -355,13 +351,13 @@ struct GemmMaps {
 
 template <int KIND, int EPI, int BN, int FORM = -1>
 static int launch_gemm(const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
-  static bool attr_set[64] = {false};
+  static PerDevice<bool> attr_set;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64 || !attr_set[dev]) {
+  if (!attr_set.get(dev)) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<KIND, EPI, BN, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_MAX);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_kernel)");
-    if (dev < 64) attr_set[dev] = true;
+    attr_set.put(dev, true);
   }
   return cuda_status(launch_maybe_pdl(g.M, gemm_kernel<KIND, EPI, BN, FORM>, dim3(grid), dim3(GEMM_THREADS), gemm_smem<EPI, BN>(g.stages, g.vec_floats, g.res_tma != 0), st, tm.A, tm.W, tm.R, tm.C, g), "kf_gemm_bs launch");
 }

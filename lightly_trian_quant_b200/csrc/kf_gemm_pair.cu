@@ -207,13 +207,13 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
 // ------------------------------------------------------------------------------------------------ host side
 template <int KIND, int EPI>
 static int launch_pair(const PairMaps& tm, GemmArgs& g, int pairs, bool want_vec, cudaStream_t st) {
-  static bool attr_set[64] = {false};
+  static PerDevice<bool> attr_set;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64 || !attr_set[dev]) {
+  if (!attr_set.get(dev)) {
     cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM_MAX);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_pair_kernel)");
-    if (dev < 64) attr_set[dev] = true;
+    attr_set.put(dev, true);
   }
   const int vec = want_vec ? g.N * (EPI == KF_EPI_RES ? 2 : 1) : 0;
   g.vec_floats = pair_smem<KIND, EPI>(3, vec, g.res_tma != 0) <= PAIR_SMEM_MAX ? vec : 0;

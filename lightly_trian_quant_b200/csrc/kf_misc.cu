@@ -512,16 +512,16 @@ extern "C" int kf_dw_ln(const void* g, const float* bias, const float* dww, cons
   KF_REQUIRE(g && (bias || pre_act) && dww && lnw && lnb && out && al16(g) && al16(out) && al16(lnw) && al16(lnb) && al16(dww) && al16(bias),
              "kf_dw_ln: tensors must be non-null and 16-byte aligned");
   const size_t smem = (size_t)DW_RING * DW_HALO * C * 2 + DW_RED_FLOATS * sizeof(float);
-  static bool attr_set[64] = {false};
+  static PerDevice<bool> attr_set;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64 || !attr_set[dev]) {
+  if (!attr_set.get(dev)) {
     const int big = (int)((size_t)DW_RING * DW_HALO * 1024 * 2 + DW_RED_FLOATS * sizeof(float));
     cudaError_t e = cudaFuncSetAttribute(dw_ln_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(dw_ln_kernel<768>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(dw_ln_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(dw_ln_kernel)");
-    if (dev < 64) attr_set[dev] = true;
+    attr_set.put(dev, true);
   }
   int sms = 0;
   int st = device_sm_count(&sms);
@@ -600,22 +600,22 @@ namespace kf {
 // Device address of the array on the CURRENT device.  On the host the array's name is only a handle: cudaGetSymbolAddress turns
 // it into the pointer kernels and tensor maps can use.  Looked up once per device and kept.
 static int patch_rows_address(void** out) {
-  static void* cached[64] = {nullptr};
+  static PerDevice<void*> cached;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_status(e, "cudaGetDevice");
-  if (dev >= 0 && dev < 64 && cached[dev] != nullptr) {
-    *out = cached[dev];
+  void* p = cached.get(dev);
+  if (p != nullptr) {
+    *out = p;
     return KF_OK;
   }
-  void* p = nullptr;
   e = cudaGetSymbolAddress(&p, g_patch_rows);
   if (e != cudaSuccess) return cuda_status(e, "cudaGetSymbolAddress(patch rows)");
   if (p == nullptr) {
     set_error("kf_patch_embed_static: the scratch array has no device address");
     return KF_ERR_UNSUPPORTED;
   }
-  if (dev >= 0 && dev < 64) cached[dev] = p;
+  cached.put(dev, p);
   *out = p;
   return KF_OK;
 }

@@ -105,95 +105,95 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const T* __restrict__ x
   uint32_t raw[LOAD32_WORDS<T>];
   if (AHEAD && w32 < valid_end) load32_raw<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, raw);
   for (;;) {
-  const bool valid = w32 < valid_end, in_pad = w32 < end;
-  float v[32];
-  if (valid) {
-    if (AHEAD) unpack32<T>(raw, v);
-    else load32<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, v);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0.f;
-  }
-  // 16-bit inputs: the next item's loads travel while this one is quantised
-  const uint32_t next = w32 + stride;
-  const bool more = AHEAD && __any_sync(0xffffffffu, next < end && next >= stride);
-  int nrow = 0, nc32 = 0;
-  if (more) {
-    place(next, nrow, nc32);
-    if (next < valid_end) load32_raw<T>(x + (int64_t)nrow * ldx + nc32 * 32, wide != 0, raw);
-  }
-  if constexpr (FMT == KF_FMT_NV4 && std::is_same<T, __half>::value) {
-    // The corrected quotient of a negative zero is a positive one (code 0, the bit rule says 8).  fp16 inputs reach -0 by
-    // underflow of ordinary values; a magnitude below any fp16 one takes its place.
-    if (!(flags & KF_Q_GELU)) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(v[i]) == 0x80000000u ? -1e-20f : v[i];
-    }
-  }
-  if ((flags & KF_Q_GELU) && valid) {
-    const float4* b4 = reinterpret_cast<const float4*>(bias + c32 * 32);
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const float4 bb = __ldg(b4 + (i >> 2));
-      const float2 a = gelu_erf_pair(add2(make_float2(v[i], v[i + 1]), make_float2(bb.x, bb.y)));
-      const float2 c = gelu_erf_pair(add2(make_float2(v[i + 2], v[i + 3]), make_float2(bb.z, bb.w)));
-      v[i] = a.x;
-      v[i + 1] = a.y;
-      v[i + 2] = c.x;
-      v[i + 3] = c.y;
-    }
-  }
-  if (flags & KF_Q_ROUND_BF16) {
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      const float2 a = bf16_round2(make_float2(v[i], v[i + 1]));
-      v[i] = a.x;
-      v[i + 1] = a.y;
-    }
-  }
-  float am0 = 0.f, am1 = 0.f;
-#pragma unroll
-  for (int i = 0; i < 16; i += 2) {
-    am0 = max3(am0, fabsf(v[i]), fabsf(v[i + 1]));
-    am1 = max3(am1, fabsf(v[16 + i]), fabsf(v[17 + i]));
-  }
-  const bool div_true = !(flags & KF_Q_RECIP_DIV);
-  const float(&va)[16] = *reinterpret_cast<const float(*)[16]>(&v[0]);
-  const float(&vb)[16] = *reinterpret_cast<const float(*)[16]>(&v[16]);
-  if constexpr (FMT == KF_FMT_NV4) {
-    uint32_t o[4];
-    int by0, by1;
-    quant_nv4_pair16(va, am0, vb, am1, ts, div_true, o, by0, by1);
-    if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * (K >> 1) + c32 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-    const uint32_t pk = valid ? (uint32_t)(by0 | (by1 << 8)) : 0u;
-    const uint32_t up = __shfl_xor_sync(0xffffffffu, pk, 1);           // on an even lane: the bytes of the word's other two blocks
-    if (in_pad && (lane & 1) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, 2 * c32, K >> 6)) = pk | (up << 16);
-  } else {
-    const float amax = amax_nan(am0, am1);
-    int byte;
-    if constexpr (FMT == KF_FMT_MX8) {
-      uint32_t o[8];
-      quant_mx8<16>(va, amax, div_true, o, byte);
-      quant_mx8<16>(vb, amax, div_true, o + 4, byte);
-      if (valid) {
-        uint4* dst = reinterpret_cast<uint4*>(q + (int64_t)row * K + c32 * 32);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-      }
+    const bool valid = w32 < valid_end, in_pad = w32 < end;
+    float v[32];
+    if (valid) {
+      if (AHEAD) unpack32<T>(raw, v);
+      else load32<T>(x + (int64_t)row * ldx + c32 * 32, wide != 0, v);
     } else {
-      uint32_t o[4];
-      quant_mx4<16>(va, amax, div_true, o, byte);
-      quant_mx4<16>(vb, amax, div_true, o + 2, byte);
-      if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * (K >> 1) + c32 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = 0.f;
     }
-    if (!valid) byte = 0;
-    const uint32_t word = gather_sf_word<1>(byte, lane);
-    if (in_pad && (lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, c32, K >> 7)) = word;
-  }
-  if (!AHEAD || !more) break;
-  w32 = next;
-  row = nrow;
-  c32 = nc32;
+    // 16-bit inputs: the next item's loads travel while this one is quantised
+    const uint32_t next = w32 + stride;
+    const bool more = AHEAD && __any_sync(0xffffffffu, next < end && next >= stride);
+    int nrow = 0, nc32 = 0;
+    if (more) {
+      place(next, nrow, nc32);
+      if (next < valid_end) load32_raw<T>(x + (int64_t)nrow * ldx + nc32 * 32, wide != 0, raw);
+    }
+    if constexpr (FMT == KF_FMT_NV4 && std::is_same<T, __half>::value) {
+      // The corrected quotient of a negative zero is a positive one (code 0, the bit rule says 8).  fp16 inputs reach -0 by
+      // underflow of ordinary values; a magnitude below any fp16 one takes its place.
+      if (!(flags & KF_Q_GELU)) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(v[i]) == 0x80000000u ? -1e-20f : v[i];
+      }
+    }
+    if ((flags & KF_Q_GELU) && valid) {
+      const float4* b4 = reinterpret_cast<const float4*>(bias + c32 * 32);
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        const float4 bb = __ldg(b4 + (i >> 2));
+        const float2 a = gelu_erf_pair(add2(make_float2(v[i], v[i + 1]), make_float2(bb.x, bb.y)));
+        const float2 c = gelu_erf_pair(add2(make_float2(v[i + 2], v[i + 3]), make_float2(bb.z, bb.w)));
+        v[i] = a.x;
+        v[i + 1] = a.y;
+        v[i + 2] = c.x;
+        v[i + 3] = c.y;
+      }
+    }
+    if (flags & KF_Q_ROUND_BF16) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) {
+        const float2 a = bf16_round2(make_float2(v[i], v[i + 1]));
+        v[i] = a.x;
+        v[i + 1] = a.y;
+      }
+    }
+    float am0 = 0.f, am1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      am0 = max3(am0, fabsf(v[i]), fabsf(v[i + 1]));
+      am1 = max3(am1, fabsf(v[16 + i]), fabsf(v[17 + i]));
+    }
+    const bool div_true = !(flags & KF_Q_RECIP_DIV);
+    const float(&va)[16] = *reinterpret_cast<const float(*)[16]>(&v[0]);
+    const float(&vb)[16] = *reinterpret_cast<const float(*)[16]>(&v[16]);
+    if constexpr (FMT == KF_FMT_NV4) {
+      uint32_t o[4];
+      int by0, by1;
+      quant_nv4_pair16(va, am0, vb, am1, ts, div_true, o, by0, by1);
+      if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * (K >> 1) + c32 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+      const uint32_t pk = valid ? (uint32_t)(by0 | (by1 << 8)) : 0u;
+      const uint32_t up = __shfl_xor_sync(0xffffffffu, pk, 1);           // on an even lane: the bytes of the word's other two blocks
+      if (in_pad && (lane & 1) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, 2 * c32, K >> 6)) = pk | (up << 16);
+    } else {
+      const float amax = amax_nan(am0, am1);
+      int byte;
+      if constexpr (FMT == KF_FMT_MX8) {
+        uint32_t o[8];
+        quant_mx8<16>(va, amax, div_true, o, byte);
+        quant_mx8<16>(vb, amax, div_true, o + 4, byte);
+        if (valid) {
+          uint4* dst = reinterpret_cast<uint4*>(q + (int64_t)row * K + c32 * 32);
+          dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+          dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+      } else {
+        uint32_t o[4];
+        quant_mx4<16>(va, amax, div_true, o, byte);
+        quant_mx4<16>(vb, amax, div_true, o + 2, byte);
+        if (valid) *reinterpret_cast<uint4*>(q + (int64_t)row * (K >> 1) + c32 * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      if (!valid) byte = 0;
+      const uint32_t word = gather_sf_word<1>(byte, lane);
+      if (in_pad && (lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf + sf_offset(row, c32, K >> 7)) = word;
+    }
+    if (!AHEAD || !more) break;
+    w32 = next;
+    row = nrow;
+    c32 = nc32;
   }
 }
 
@@ -677,17 +677,21 @@ static int launch_quant_rows(int fmt, const void* x, int64_t ldx, int M, int K, 
   const T* xp = static_cast<const T*>(x);
   const int wide = rows_32b_aligned(x, ldx * (int64_t)sizeof(T));
   uint8_t *qp = static_cast<uint8_t*>(q), *sp = static_cast<uint8_t*>(sf);
-  static int per_sm_cached[3][64] = {};                  // resident CTAs per (format, device) of this input type
+  static PerDevice<int> resident[3];                     // CTAs per SM, per format of this input type
   auto go = [&](auto kern) {
-    int per_sm = dev < 64 ? per_sm_cached[fmt][dev] : 0;
-    if (per_sm == 0) {
-      const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
-      if (e != cudaSuccess) return cuda_status(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(quant_rows_kernel)");
-      if (per_sm < 1) per_sm = 1;
-      if (dev < 64) per_sm_cached[fmt][dev] = per_sm;
+    const int64_t blocks = (total + 255) / 256;
+    int64_t rounds = 1;
+    if (sizeof(T) == 2) {
+      int per_sm = resident[fmt].get(dev);
+      if (per_sm == 0) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
+        if (e != cudaSuccess) return cuda_status(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(quant_rows_kernel)");
+        if (per_sm < 1) per_sm = 1;
+        resident[fmt].put(dev, per_sm);
+      }
+      const int64_t slots = (int64_t)sms * per_sm;
+      rounds = (blocks + slots - 1) / slots;
     }
-    const int64_t blocks = (total + 255) / 256, resident = (int64_t)sms * per_sm;
-    const int64_t rounds = sizeof(T) == 2 ? (blocks + resident - 1) / resident : 1;
     const unsigned grid = (unsigned)((blocks + rounds - 1) / rounds);   // equal shares
     return cuda_status(launch_maybe_pdl(M, kern, dim3(grid), dim3(256), 0, st, xp, ldx, M, K, ts, bias, flags, wide, qp, sp, valid, total), "kf_quant_rows launch");
   };
@@ -710,12 +714,12 @@ static int launch_ln_quant(int fmt, const TI* x, const float* w, const float* b,
   unsigned int* err = dev_error_ptr();
   KF_REQUIRE(err != nullptr, "kf_ln_quant: device error word unavailable");
   const size_t smem = (size_t)4 * LNQ_RING * NV * 256 * sizeof(TI) + 4 * LNQ_RING * 8 + 16;
-  static int per_sm_cached[3][64] = {};                  // per (format, device) of this row width
+  static PerDevice<int> resident[3];                     // CTAs per SM, per format of this row width
   auto go = [&](auto kern) {
     // persistent: as many CTAs of 4 warps as are resident at once (4 per SM up to d = 1024, fewer for wider rows); a
     // grid beyond that would run its surplus as a second, nearly empty wave.  The attribute and the occupancy query are
     // per (kernel instance, device): worked out at the first call and kept.
-    int per_sm = dev < 64 ? per_sm_cached[fmt][dev] : 0;
+    int per_sm = resident[fmt].get(dev);
     if (per_sm == 0) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(ln_quant_kernel)");
@@ -723,7 +727,7 @@ static int launch_ln_quant(int fmt, const TI* x, const float* w, const float* b,
       if (e != cudaSuccess) return cuda_status(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(ln_quant_kernel)");
       if (per_sm < 1) per_sm = 1;
       if (per_sm > 4) per_sm = 4;
-      if (dev < 64) per_sm_cached[fmt][dev] = per_sm;
+      resident[fmt].put(dev, per_sm);
     }
     if (grid > (unsigned)(sms * per_sm)) grid = (unsigned)(sms * per_sm);
     return cuda_status(launch_maybe_pdl(M, kern, dim3(grid), dim3(128), smem, st, x, w, b, eps, M, rows_pad, ts, flags, qp, sp, y_dbg, err), "kf_ln_quant launch");

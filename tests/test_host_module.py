@@ -1,5 +1,8 @@
 """The native operator module (csrc/host/kf_host.cpp): bad arguments end as Python errors, containers may be any object with the attributes, other
 threads run while an operator is inside the library."""
+import re
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -168,3 +171,12 @@ def test_other_threads_run_while_a_launch_waits():
     print(f"longest launch {longest * 1e3:.0f} ms, longest gap of the other thread {gaps[0] * 1e3:.1f} ms")
     assert longest > 0.05, "the queue never filled: the test shows nothing"
     assert gaps[0] < 0.5 * longest
+
+
+def test_no_unordered_state_shared_between_threads():
+    """launchers run without the interpreter lock: what they keep between calls is const, per thread, or atomic (PerDevice), never a plain static."""
+    csrc = Path(__file__).resolve().parent.parent / "lightly_trian_quant_b200" / "csrc"
+    variable = re.compile(r"^\s*static\s+(?!const\b|constexpr\b|thread_local\b|std::atomic\b|PerDevice<|__device__)[\w:<>,* ]+?[\s*&](\w+)\s*(\[[^;]*)?(=[^;]*|\{[^;]*)?;")
+    plain = [f"{path.name}:{no}: {line.strip()}" for path in sorted(csrc.rglob("*.c*")) if path.suffix in (".cu", ".cuh", ".cpp")
+             for no, line in enumerate(path.read_text().splitlines(), 1) if variable.match(line)]
+    assert not plain, plain
