@@ -4,7 +4,7 @@
     python -m lightly_trian_quant_b200.build [--force] [--verbose]
 
 nvcc cross-compiles without a GPU.  Objects are cached under csrc/build/ keyed by a hash of each source and the
-shared headers, so an unchanged file is not recompiled.
+shared headers, so an unchanged file is not recompiled.  What ptxas says about registers and spills stays beside each object (.ptxas).
 """
 from __future__ import annotations
 
@@ -23,7 +23,7 @@ HOST_SRC = CSRC / "host" / "kf_host.cpp"
 HOST_LIB = PKG / ("_kf_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",
-         "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-DKF_BUILD"]
+         "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-Xptxas", "-v", "-DKF_BUILD"]
 
 
 def sources():
@@ -48,17 +48,18 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         tag = hashlib.sha256(src.read_bytes() + hh.encode()).hexdigest()[:16]
         obj = bdir / f"{src.stem}.{tag}.o"
         objs.append(obj)
-        if force or not obj.exists():
-            for old in bdir.glob(f"{src.stem}.*.o"):
+        if force or not (obj.exists() and obj.with_suffix(".ptxas").exists()):
+            for old in [*bdir.glob(f"{src.stem}.*.o"), *bdir.glob(f"{src.stem}.*.ptxas")]:
                 old.unlink()
             jobs.append((src, obj))
 
     def compile_one(job):
         src, obj = job
-        cmd = [NVCC, *FLAGS, "-c", str(src), "-o", str(obj)] + (["-Xptxas", "-v"] if verbose else [])
+        cmd = [NVCC, *FLAGS, "-c", str(src), "-o", str(obj)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+        obj.with_suffix(".ptxas").write_text(r.stderr)
         if verbose:
             print(r.stderr)
         return obj

@@ -349,7 +349,7 @@ struct GemmMaps {
   CUtensorMap A, W, R, C;                                 // R, C: the residual and the output of a RES launch through shared memory; R: W in boxes of 128 rows for half tiles
 };
 
-template <int KIND, int EPI, int BN, int FORM = -1>
+template <int KIND, int EPI, int BN, int FORM>
 static int launch_gemm(const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
   static PerDevice<bool> attr_set;
   int dev = 0;
@@ -364,24 +364,7 @@ static int launch_gemm(const GemmMaps& tm, const GemmArgs& g, int grid, cudaStre
 
 template <int KIND, int BN>
 static int launch_gemm_epi(int epi, const GemmMaps& tm, const GemmArgs& g, int grid, cudaStream_t st) {
-  switch (epi) {
-    case KF_EPI_PLAIN:
-      switch (epilogue_form(epi, g)) {
-        case PL_BF16: return launch_gemm<KIND, KF_EPI_PLAIN, BN, PL_BF16>(tm, g, grid, st);
-        case PL_GELU: return launch_gemm<KIND, KF_EPI_PLAIN, BN, PL_GELU>(tm, g, grid, st);
-        case PL_GELU_PRE: return launch_gemm<KIND, KF_EPI_PLAIN, BN, PL_GELU_PRE>(tm, g, grid, st);
-        default: return launch_gemm<KIND, KF_EPI_PLAIN, BN>(tm, g, grid, st);
-      }
-    case KF_EPI_RES: return launch_gemm<KIND, KF_EPI_RES, BN>(tm, g, grid, st);
-    case KF_EPI_ROPE: return launch_gemm<KIND, KF_EPI_ROPE, BN>(tm, g, grid, st);
-    default:
-      switch (epilogue_form(epi, g)) {
-        case KF_FMT_MX8: return launch_gemm<KIND, KF_EPI_QUANT, BN, KF_FMT_MX8>(tm, g, grid, st);
-        case KF_FMT_NV4: return launch_gemm<KIND, KF_EPI_QUANT, BN, KF_FMT_NV4>(tm, g, grid, st);
-        case KF_FMT_MX4: return launch_gemm<KIND, KF_EPI_QUANT, BN, KF_FMT_MX4>(tm, g, grid, st);
-        default: return launch_gemm<KIND, KF_EPI_QUANT, BN>(tm, g, grid, st);
-      }
-  }
+  return with_epilogue(epi, g, [&](auto e, auto form) { return launch_gemm<KIND, decltype(e)::value, BN, decltype(form)::value>(tm, g, grid, st); });
 }
 
 // A last round of 256-column tiles that fills at most half of the SMs is cut into halves of 128 columns: the round then takes about

@@ -14,6 +14,9 @@
 //                        110-160, which had the pair level with one CTA
 //   measured   one CTA -> pair, captured launches, M = 22 470, K x N of ViT-L (us): bf16 qkv 127 -> 107, fc1 169 -> 143, fc2 161 -> 153; MXFP8
 //              qkv 79 -> 71, proj 53 -> 44, fc1 102 -> 90, fc2 96 -> 90; NVFP4 fc1 84 -> 79, fc2 65 -> 58, plain 62 -> 55
+//   forms      a kernel for each (epilogue_form), as in kf_gemm.cu.  With all of them in one the bf16 kernels of PLAIN and QUANT spilled (24 and 96 bytes
+//              of loads): bf16 22 400 x 1024 x 4096 GELU 143.1 -> 140.0 us, 4815 x 768 x 3072 plain 19.9 -> 19.3, GELU 22.5 -> 20.9; MXFP8 QUANT
+//              22 470 x 768 x 3072 61.8 -> 61.1; NVFP4 QUANT and the one-form epilogues level
 //
 // No load is a multicast; the two cluster barriers (start, teardown) are reached by every thread on every path, every other wait is bounded.
 // Replaces the same reference kernels as kf_gemm.cu: infer-opt/round13_mxfp8_full/impl/mgx_core.cu:118-444 and
@@ -39,7 +42,7 @@ struct PairMaps {
   CUtensorMap A, W, Wh, SA, SW, R, C;                    // Wh: W in boxes of 64 rows for half tiles; R, C: the residual and the output of RES
 };
 
-template <int KIND, int EPI>
+template <int KIND, int EPI, int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
   constexpr int ATOMS = KindTraits<KIND>::ATOMS;
@@ -187,7 +190,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
     }
   } else {
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
-    if (!bad_align) epilogue_warps<EPI, 256, true>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tm.R, &tm.C, ctx, warp, lane);
+    if (!bad_align) epilogue_warps<EPI, 256, true, FORM>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tm.R, &tm.C, ctx, warp, lane);
   }
 
   pdl_launch_dependents();
@@ -205,13 +208,13 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-template <int KIND, int EPI>
+template <int KIND, int EPI, int FORM>
 static int launch_pair(const PairMaps& tm, GemmArgs& g, int pairs, bool want_vec, cudaStream_t st) {
   static PerDevice<bool> attr_set;
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set.get(dev)) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM_MAX);
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<KIND, EPI, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM_MAX);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(gemm_pair_kernel)");
     attr_set.put(dev, true);
   }
@@ -219,18 +222,13 @@ static int launch_pair(const PairMaps& tm, GemmArgs& g, int pairs, bool want_vec
   g.vec_floats = pair_smem<KIND, EPI>(3, vec, g.res_tma != 0) <= PAIR_SMEM_MAX ? vec : 0;
   g.stages = 2;
   while (g.stages < PAIR_MAX_STAGES && pair_smem<KIND, EPI>(g.stages + 1, g.vec_floats, g.res_tma != 0) <= PAIR_SMEM_MAX) ++g.stages;
-  return cuda_status(launch_maybe_pdl(g.M, gemm_pair_kernel<KIND, EPI>, dim3(2 * pairs), dim3(GEMM_THREADS), pair_smem<KIND, EPI>(g.stages, g.vec_floats, g.res_tma != 0), st, tm, g),
+  return cuda_status(launch_maybe_pdl(g.M, gemm_pair_kernel<KIND, EPI, FORM>, dim3(2 * pairs), dim3(GEMM_THREADS), pair_smem<KIND, EPI>(g.stages, g.vec_floats, g.res_tma != 0), st, tm, g),
                      "kf_gemm_bs (pair) launch");
 }
 
 template <int KIND>
 static int launch_pair_epi(int epi, const PairMaps& tm, GemmArgs& g, int pairs, bool want_vec, cudaStream_t st) {
-  switch (epi) {
-    case KF_EPI_PLAIN: return launch_pair<KIND, KF_EPI_PLAIN>(tm, g, pairs, want_vec, st);
-    case KF_EPI_RES: return launch_pair<KIND, KF_EPI_RES>(tm, g, pairs, want_vec, st);
-    case KF_EPI_ROPE: return launch_pair<KIND, KF_EPI_ROPE>(tm, g, pairs, want_vec, st);
-    default: return launch_pair<KIND, KF_EPI_QUANT>(tm, g, pairs, want_vec, st);
-  }
+  return with_epilogue(epi, g, [&](auto e, auto form) { return launch_pair<KIND, decltype(e)::value, decltype(form)::value>(tm, g, pairs, want_vec, st); });
 }
 
 // Called by kf_gemm_bs with validated arguments, N a multiple of 256 and, in a batched product, an even number of row tiles per product.
