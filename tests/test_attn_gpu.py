@@ -144,6 +144,32 @@ def test_attn_larger_logits_behind_the_first_keys(dtype, lo, N):
     assert err < (4e-3 if dtype == torch.bfloat16 else 1e-3), err
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_attn_one_key_far_above_the_maximum(dtype):
+    """ONE key whose logit exceeds the running maximum by 0 .. 418 in the exponent domain (1.4 more from query row to query row), in every place
+    of a group of 8 keys, behind the first 64 keys of the first tile and in later tiles: whichever way its exponential is taken, and
+    wherever that would overflow or wrap, the row has to find its maximum."""
+    ops = _ops()
+    places = [*range(64, 72), 90, 95, *range(96, 104), 197, 198, 294, 295, 296, 299]
+    B, N = len(places), 300
+    g = torch.Generator().manual_seed(11)
+    qkv = torch.randn(3, B, N, 1, 64, generator=g)
+    qkv[0, ..., :2] = (torch.arange(N) * 1.4 / (32 * 0.125 * 1.4427)).view(1, N, 1, 1) / 2
+    qkv[1, ..., :2] = 0
+    for b, p in enumerate(places):
+        qkv[1, b, p] = 0
+        qkv[1, b, p, 0, :2] = 32                            # q . k = 1.4 * row * 8 / log2(e)
+    qkv = qkv.to(dtype)
+    out = ops.attn_fwd(qkv.cuda()).cpu()
+    ops.check_device_error()
+    assert torch.isfinite(out).all()
+    ref = ao.attn_ref(qkv.float().numpy())
+    bound = 4e-3 if dtype == torch.bfloat16 else 1e-3
+    for b, p in enumerate(places):
+        err = go.rel_fro(out[b].float().numpy(), ref[b])
+        assert err < bound, (p, err)
+
+
 def test_attn_outputs_at_16_byte_alignment():
     """outputs that are 16- but not 32-byte aligned take the narrower stores: the same bits."""
     ops = _ops()
