@@ -353,7 +353,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int qt = I.qt, h = I.h, b = I.b;
     float m_run = 0.f, l_run = 0.f;
     uint32_t ra[32], rb[32], rc[32];                             // the S row of this step: keys 0..31, 32..63 and 64..95 of the tile
-    ok = mbar_wait(&s_full[buf], sph, ctx, 17);
+    ok = mbar_wait_warp(&s_full[buf], sph, ctx, 17);
     if (!ok) break;
     tc_fence_after();
     tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
@@ -387,8 +387,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       exp_half(rb, w + 16, mn2, s0, s1, t_max);
       // The next step's S row is requested as soon as the registers of this one are free
       if (prefetch) {
-        if (!ready && !mbar_wait(&s_full[buf], sph, ctx, 17)) { ok = false; break; }
-        __syncwarp();
+        if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&s_full[buf], sph, ctx, 17)) { ok = false; break; }
         tc_fence_after();
         tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
         tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
@@ -435,7 +434,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // PV(G - 3), is covered by S(G), which this step has read.
         if (j > 0) {
           const uint32_t pb = cur == 0 ? AT_SBUF - 1 : cur - 1;
-          if (!mbar_wait(&o_full[pb], cur == 0 ? cph ^ 1 : cph, ctx, 18)) { ok = false; break; }
+          if (!mbar_wait_warp(&o_full[pb], cur == 0 ? cph ^ 1 : cph, ctx, 18)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
@@ -456,7 +455,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_arrive(&p_full[cur]);
     }
     // the item's last PV product; its barrier's previous completion, PV(G - 3), is covered by S(G - 1), which has been read
-    if (ok) ok = mbar_wait(&o_full[buf == 0 ? AT_SBUF - 1 : buf - 1], buf == 0 ? sph ^ 1 : sph, ctx, 19);
+    if (ok) ok = mbar_wait_warp(&o_full[buf == 0 ? AT_SBUF - 1 : buf - 1], buf == 0 ? sph ^ 1 : sph, ctx, 19);
     const int n = qt * AT_BM + row;
     if (ok) {
       tc_fence_after();

@@ -584,9 +584,9 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
   };
   if (boxed) box_load(first);
   int lt = 0;
-  // ROPE: the four warps of a quarter meet at named barriers, which have no limit.  A warp whose wait ran out therefore does not leave: it
-  // keeps company at the barriers of its remaining tiles (the same number in all four warps: they depend on the tile only) and
-  // stores nothing.
+  // A warp takes one decision at every wait, and one whose wait for an accumulator ran out does not leave: it keeps company at the barriers
+  // of its remaining tiles, which have no limit (ROPE: the four warps of a quarter meet at named ones, as often in all four: they depend
+  // on the tile only), and stores nothing.
   bool live = true;
   for (int idx = first; idx < g.items; idx += stride, ++lt) {
     const WorkItem item = work_item<BN>(g, idx);
@@ -608,8 +608,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
 #pragma unroll
       for (int c = 0; c < 4; ++c) res[c] = ldg8_stream(g.R + (size_t)(rbase + lane) * g.N + n0 + 8 * c);
     }
-    if (EPI == KF_EPI_ROPE) live = live && mbar_wait_warp(&tfull[acc], (lt / ACCS) & 1, ctx, 4);
-    else if (!mbar_wait(&tfull[acc], (lt / ACCS) & 1, ctx, 4)) break;
+    live = live && mbar_wait_warp(&tfull[acc], (lt / ACCS) & 1, ctx, 4);
     tc_fence_after();
     __syncwarp();
     if constexpr (W == 64) {
@@ -651,7 +650,7 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
               mbar_expect_tx(bfull, RES_BOX_BYTES);
               tma_load_2d(box, tmR, (n0 + c) * 4, rbase, bfull);
             }
-            if (!mbar_wait(bfull, bph, ctx, 5)) {
+            if (!mbar_wait_warp(bfull, bph, ctx, 5)) {
               lost = true;
               break;
             }

@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(128, NV <= 4 ? 4 : 1) ln_quant_kernel(const TI
   for (int row = gw; row < rows_pad; row += W, ++k) {
   const bool valid = row < M;
   const int slot = k % LNQ_RING;
-  if (valid && !mbar_wait(&bars[slot], (k / LNQ_RING) & 1, ctx, 30)) break;
+  if (valid && !mbar_wait_warp(&bars[slot], (k / LNQ_RING) & 1, ctx, 30)) break;
   float v[NV][8];
   ln_row<NV, true, LAY>(ring + (size_t)slot * D, ww, bb, eps, lane, valid, v);
   __syncwarp();                                   // every lane has its part of the row: the slot can be refilled

@@ -110,7 +110,9 @@ __device__ __forceinline__ bool elect_one() {          // whole warp, converged
       : "=r"(p));
   return p != 0;
 }
-// mbar_wait for a converged warp: every lane returns the same answer, so the warp stays converged on a failure too.
+// mbar_wait for a converged warp: every lane returns the same answer, so the warp stays converged on a failure too.  Code of a whole warp
+// waits this way only: if the abort flag goes up while the phase completes, lanes that decide for themselves part, and those that go on
+// wait for the others at the next warp-wide instruction without a limit.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const WaitCtx& ctx, uint32_t where) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, ctx, where));
