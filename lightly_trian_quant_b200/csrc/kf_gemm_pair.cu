@@ -141,6 +141,12 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
           if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1; }
         }
       }
+      // The leader's commits to the empty barriers reach both CTAs on their own time, those of the last stages too: this CTA stays until the
+      // last one has arrived in every slot (a slot that was never filled is open from the start).
+      for (int i = 0; i < STAGES && ok; ++i) {
+        ok = mbar_wait_warp(&empty[s], ph ^ 1, ctx, 6);
+        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1; }
+      }
     } else if (warp == 1 && rank == 0) {
       // ------------------------------------------------------------------ MMA issuer (leader): the scale atoms of a stage, then its four MMAs
       constexpr auto idesc_n = [](int n) {
@@ -200,7 +206,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
   if (*abort_flag) {                 // a wait ran out: give copies still in flight time to land before the CTA exits
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
   }
-  cluster_sync_all();                // no arrival, load or MMA of the pair may target a CTA that has left
+  cluster_sync_all();                // no arrival, load or MMA of the pair may target a CTA that has left: rings drained, accumulators read
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc2(tmem_base, TMEM_COLS);
