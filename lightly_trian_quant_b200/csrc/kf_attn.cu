@@ -23,8 +23,8 @@
 //            tile of 128 pads the model's token counts more (1605 keys: 1632 with tiles of 96, 1664 with 64 or 128).
 //            The exponentials of a tile
 //            use the running maximum as it is; the tile's own row sum tells whether that was safe (below 2^15 no
-//            element exceeded 2^15; the arguments of the polynomial, which wraps, have a check of their own), so no maximum is tracked in the
-//            common case; only a row whose sum came out larger finds its maximum, recomputes its P and has its O rescaled (TMEM load, multiply, store), which happens on
+//            element exceeded 2^15), so no maximum is tracked in the common case; only a row whose sum came out larger
+//            finds its maximum, recomputes its P and has its O rescaled (TMEM load, multiply, store), which happens on
 //            the first tiles and then almost never; the O barriers are waited only then and at the end of an item.
 //            Measured, tiles of 64 -> 96 keys (B 14, H 16, N 1605, bf16 out / NVFP4 out; N 1805, NVFP4 out; B 8, N 4101, f16,
 //            MXFP4 out; B 1, N 1605, NVFP4 out): 199 -> 186 / 204 -> 194 / 250 -> 239 / 667 -> 636 / 24.7 -> 23.6 us; 256-bit stores of the output
@@ -85,15 +85,19 @@ __device__ __forceinline__ float ex2(float x) {
 // 2^t for a pair without the special-function unit: t = n + f with n = round(t) taken from the low mantissa bits of
 // t + 1.5 * 2^23 and f in [-0.5, 0.5]; 2^f by a cubic (minimax for the relative error on that interval: 7.6e-5, far
 // below the rounding of the 16-bit P it feeds); n goes into the exponent field by an integer add.  t is clamped at -126
-// (the result is then 2^-126 instead of 0: it vanishes in the 16-bit P and in the row sum alike).  All of it runs on the
+// (the result is then 2^-126 instead of 0: it vanishes in the 16-bit P and in the row sum alike) and at 127, behind which the add
+// would wrap to anything, a small or a negative number too: a row with such an element has a sum that no limit lets pass.  A t that
+// is no number passes the clamps and the add makes a huge element of it, with the same effect (a clamp that drops it would drop the key).  All of it runs on the
 // FMA and integer pipes, as packed pairs where the operation exists.
-// Above 128 the add wraps: the result may be anything, a small or a negative number too.  t_max takes up the largest t, for the caller to
-// reject those results (one three-way maximum a pair; a clamp from above would take two instructions).
-constexpr float EX2_POLY_MAX = 127.f;
-__device__ __forceinline__ float2 ex2_poly2(float2 t, float& t_max) {
-  t_max = max3(t_max, t.x, t.y);
-  t.x = fmaxf(t.x, -126.f);
-  t.y = fmaxf(t.y, -126.f);
+// Clamps and no check of the largest t: that costs an instruction less, but a register through the key loop (captured, us: B 14, H 12, N 1605, MXFP8 out
+// 137.5 against 135.3; B 1, H 16, N 1605 22.2 against 21.9).
+__device__ __forceinline__ float clamp_ex2(float t) {
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;\n\tmin.NaN.f32 %0, %0, 0f42FE0000;" : "+f"(t));   // [-126, 127]
+  return t;
+}
+__device__ __forceinline__ float2 ex2_poly2(float2 t) {
+  t.x = clamp_ex2(t.x);
+  t.y = clamp_ex2(t.y);
   const float2 r = add2(t, splat2(12582912.f));
   const float2 n = add2(r, splat2(-12582912.f));
   const float2 f = fma2(n, splat2(-1.f), t);
@@ -313,15 +317,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const Nv4Scale tsc = nv4_scale(OUT == KF_FMT_NV4 ? __ldg(a.tso) : 1.f);
     const float2 sc2 = splat2(sc);
     // P = exp2(s*sc + mneg) of 32 keys as 16-bit pairs; adds the row sum to s0 / s1.  The exponent arguments and the row
-    // sums run as packed pairs: half the issue slots of the scalar form.  t_max: the largest exponent argument of the polynomial.
-    auto exp_half = [&](const uint32_t (&r)[32], uint32_t* w, float2 mn2, float2& s0, float2& s1, float& t_max) {
+    // sums run as packed pairs: half the issue slots of the scalar form.
+    auto exp_half = [&](const uint32_t (&r)[32], uint32_t* w, float2 mn2, float2& s0, float2& s1) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float2 p[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const float2 t = fma2(make_float2(__uint_as_float(r[8 * i + 2 * k]), __uint_as_float(r[8 * i + 2 * k + 1])), sc2, mn2);
-          p[k] = k >= AT_POLY_K ? ex2_poly2(t, t_max) : make_float2(ex2(t.x), ex2(t.y));   // one pair in four off the special-function unit
+          p[k] = k >= AT_POLY_K ? ex2_poly2(t) : make_float2(ex2(t.x), ex2(t.y));   // one pair in four off the special-function unit
         }
         s0 = add2(s0, add2(p[0], p[1]));
         s1 = add2(s1, add2(p[2], p[3]));
@@ -379,12 +383,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (j == 0) m_run = row_max(rb, row_max(ra, -INFINITY));
       const float2 mn2 = splat2(-m_run * sc);
       float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-      float t_max = 0.f;
       uint32_t w[48];
-      exp_half(ra, w, mn2, s0, s1, t_max);
+      exp_half(ra, w, mn2, s0, s1);
       // asked for here, looked at a third of a step later: S(G + 1) was issued at the end of the last step
       const bool ready = mbar_test_wait(&s_full[buf], sph);
-      exp_half(rb, w + 16, mn2, s0, s1, t_max);
+      exp_half(rb, w + 16, mn2, s0, s1);
       // The next step's S row is requested as soon as the registers of this one are free
       if (prefetch) {
         if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(&s_full[buf], sph, ctx, 17)) { ok = false; break; }
@@ -392,17 +395,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld32(t_lane + AT_COL_S + buf * AT_BN, ra);
         tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 32, rb);
       }
-      exp_half(rc, w + 32, mn2, s0, s1, t_max);
+      exp_half(rc, w + 32, mn2, s0, s1);
       if (prefetch) tmem_ld32(t_lane + AT_COL_S + buf * AT_BN + 64, rc);
       // Lazy maximum without a maximum: the exponentials of tile j > 0 use the running maximum as it is, and the tile's
       // own row sum tells whether that was safe: while it stays below 2^15 no element exceeded 2^15 (bf16 / f16 P, the
       // fp32 sums and O have room for that), so the maximum of the tile is not needed at all.  That holds for the special-function unit,
-      // whose results only grow (to infinity), and for the polynomial up to EX2_POLY_MAX; behind that its own check speaks.  Only a row whose
-      // sum came out larger (or infinite, or no number) finds its maximum, raises the running maximum, recomputes its P and has its O rescaled.
+      // whose results only grow (to infinity), and for the polynomial, whose argument is clamped.  Only a row whose sum came out larger (or infinite,
+      // or no number) finds its maximum, raises the running maximum, recomputes its P and has its O rescaled.
       // The first tile has no running maximum yet and takes that of its first 64 keys (the 96 of the tile would do: the 64 leave the
       // bits of P what they were with tiles of 64).
       float sum = (s0.x + s0.y) + (s1.x + s1.y), alpha = 1.f;
-      const bool need = !(sum <= AT_SUM_LIMIT) || t_max > EX2_POLY_MAX;
+      const bool need = !(sum <= AT_SUM_LIMIT);
       if (__any_sync(0xffffffffu, need)) {                    // warp-uniform; S is still in tensor memory: P replaces it only below
         uint32_t r[32];
         float mx = m_run;
@@ -425,9 +428,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_ld_wait();
           tmem_ld_fence(r);
           if (kbase + AT_BN > a.N) mask_tail(r, kbase + 32 * c);
-          if (c == 0) exp_half(r, w, splat2(-m_run * sc), s0, s1, t_max);
-          else if (c == 1) exp_half(r, w + 16, splat2(-m_run * sc), s0, s1, t_max);
-          else exp_half(r, w + 32, splat2(-m_run * sc), s0, s1, t_max);
+          if (c == 0) exp_half(r, w, splat2(-m_run * sc), s0, s1);
+          else if (c == 1) exp_half(r, w + 16, splat2(-m_run * sc), s0, s1);
+          else exp_half(r, w + 32, splat2(-m_run * sc), s0, s1);
         }
         sum = (s0.x + s0.y) + (s1.x + s1.y);
         // rescale O in tensor memory, where there is one: PV(G - 1) must have landed first.  Its barrier's previous completion,

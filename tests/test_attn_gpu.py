@@ -170,6 +170,18 @@ def test_attn_one_key_far_above_the_maximum(dtype):
         assert err < bound, (p, err)
 
 
+def test_attn_a_key_that_is_no_number():
+    """a NaN in one key, in every place of a group of 8 keys, makes every row of its head NaN, as the softmax of the oracle does."""
+    ops = _ops()
+    B, N = 24, 300
+    qkv = torch.randn(3, B, N, 2, 64, generator=torch.Generator().manual_seed(13)).to(torch.bfloat16)
+    for b in range(B):
+        qkv[1, b, (64, 96, 200)[b // 8] + b % 8, 0, 5] = float("nan")
+    out = ops.attn_fwd(qkv.cuda()).cpu().view(B, N, 2, 64)
+    ops.check_device_error()
+    assert out[:, :, 0].isnan().all() and torch.isfinite(out[:, :, 1]).all()
+
+
 def test_attn_outputs_at_16_byte_alignment():
     """outputs that are 16- but not 32-byte aligned take the narrower stores: the same bits."""
     ops = _ops()
