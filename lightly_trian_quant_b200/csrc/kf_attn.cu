@@ -337,7 +337,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float m4[4] = {mx, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int i = 0; i < 16; ++i) m4[i & 3] = max3(m4[i & 3], __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-      return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      return amax_nan(amax_nan(m4[0], m4[1]), amax_nan(m4[2], m4[3]));
     };
     auto store32 = [&](uint8_t* dst, const uint32_t* w) {
       if (a.wide) {
