@@ -19,9 +19,9 @@ def _reports(stem):
     return out
 
 
-@pytest.mark.parametrize("stem,kernels", [("kf_gemm", 80), ("kf_gemm_pair", 40)])
+@pytest.mark.parametrize("stem,kernels", [("kf_gemm", 80), ("kf_gemm_pair", 40), ("kf_attn", 8)])
 def test_kernels_do_not_spill(stem, kernels):
-    """every instantiation keeps its values in registers: no form, format or output type is left out of the look."""
+    """every instantiation of the GEMM and attention kernels keeps its values in registers: no form, format or output type is left out of the look."""
     reports = _reports(stem)
     assert len(reports) == kernels
     assert not {k: v for k, v in reports.items() if v != (0, 0)}
