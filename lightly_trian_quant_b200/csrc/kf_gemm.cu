@@ -241,7 +241,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ------------------------------------------------------------------ epilogue: 16 warps, warp = (TMEM lane quarter, 64-column group)
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
     if (!bad_align) {
-      epilogue_warps<EPI, BN, false, FORM>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tmR, &tmC, ctx, warp, lane);
+      epilogue_warps<EPI, BN, false, FORM>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, nullptr, &tmR, &tmC, ctx, warp, lane);
     }
   }
 

@@ -445,6 +445,7 @@ __device__ __forceinline__ void epilogue_math(const GemmArgs& g, uint32_t (&r)[W
 // are updated in place in shared memory and leave as one box.  Every request is then a whole 128-byte line: a read-modify-write of
 // 22 470 x 1024 fp32 takes 33.0 us this way and 39.9 us with the 32-byte accesses of the row layout (copy: 32.7 us).
 constexpr int RES_BOX_BYTES = 32 * 128;
+constexpr int PACE_POLLS = 1000;                        // a turn that does not come within about 100 us is taken anyway: order, not correctness, hangs on it
 __device__ __forceinline__ void epilogue_res_tma(const GemmArgs& g, const uint32_t (&r)[32], float ts, const float* slice, const float* gslice, uint8_t* box, int lane) {
   const float2 ts2 = splat2(ts);
   uint8_t* row = box + lane * 128;
@@ -539,7 +540,7 @@ static int with_epilogue(int epi, const GemmArgs& g, Run&& run) {
 // accumulator is handed back to the leader's MMA warp.
 template <int EPI, int BN, bool PAIR, int FORM>
 __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_base, uint64_t* tfull, uint64_t* tempty, float* slices,
-                                               float* slabs, uint8_t* boxes, uint64_t* box_full, const CUtensorMap* tmR, const CUtensorMap* tmC, const WaitCtx& ctx, int warp,
+                                               float* slabs, uint8_t* boxes, uint64_t* box_full, const volatile uint32_t* issued /* PAIR, RES: operand stages requested so far */, const CUtensorMap* tmR, const CUtensorMap* tmC, const WaitCtx& ctx, int warp,
                                                int lane) {
   constexpr int W = Tile<BN>::CW, ACCS = Tile<BN>::ACCS;
   constexpr bool PAIRS = EPI == KF_EPI_ROPE && W == 32;       // two warps share a head: its column pairs 0..15 and 16..31
@@ -638,10 +639,18 @@ __device__ __forceinline__ void epilogue_warps(const GemmArgs& g, uint32_t tmem_
     if (PAIR && rbase >= g.m_tiles * BM) continue;             // the follower's row tile past the last one
     if constexpr (BOXES) {
       if (boxed) {
-        // The column groups take turns over about half of the next tile's main loop: 16 warps' boxes at once (64 KB of loads, then of stores,
-        // twice a tile) held up the operand loads in the same queue (NVFP4 22 470 x 4096 x 1024 61.5 -> 58.1 us, MXFP8 92 -> 90, x 768 60.7 -> 58.1;
-        // 100 ns a stage is too long for bf16: 150 -> 164 against 148.5).  Not for a CTA's last tile, where it would only come later.
-        if (PAIR && cg != 0 && idx + stride < g.items) __nanosleep(cg * g.k_tiles * 75);
+        // The column groups take turns over the next tile's main loop: 16 warps' boxes at once (64 KB of loads, then of stores, twice a
+        // tile) held up the operand loads in the same queue.  A turn is a fifth of the main loop, counted in the stages its producer has
+        // requested (which run a ring ahead of the products), so it is the same part of it in every format and at every clock.  None -> turns of
+        // 75 ns a stage -> a fifth, us: NVFP4 22 470 x 4096 x 1024 62.9 -> 60.4 -> 58.4, 51 360 rows 132.8 -> 124.7 -> 120.3, MXFP4 129.5 -> 118.1 -> 114.9,
+        // MXFP8 22 470 95.7 -> 91.2 -> 88.5, bf16 153.1 -> 151.0 -> 149.5; an eighth: NVFP4 60.2, 123.8, a third: 61.6, 126.7.  Not for a CTA's last
+        // tile, where it would only come later.
+        if (PAIR && cg != 0 && idx + stride < g.items) {
+          const uint32_t turn = (uint32_t)((lt + 1) * g.k_tiles + min(g.k_tiles, g.stages + cg * g.k_tiles / 5));
+          if (lane == 0)
+            for (int i = 0; i < PACE_POLLS && (int32_t)(*issued - turn) < 0 && !*ctx.abort_flag; ++i) __nanosleep(100);
+          __syncwarp();
+        }
         bool lost = false;
         if (rbase < g.M) {
 #pragma unroll

@@ -61,6 +61,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
   uint64_t* box_full = tempty + 1;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(box_full + EPI_WARPS);
   volatile uint32_t* abort_flag = tmem_holder + 1;
+  volatile uint32_t* issued = tmem_holder + 2;             // stages this CTA's producer has requested: what the residual boxes are paced by
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();                 // 0 = leader (issues the MMAs), 1 = follower
@@ -74,6 +75,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
     if (EPI == KF_EPI_RES)
       for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&box_full[w], 1);
     *abort_flag = 0u;
+    *issued = 0u;
     fence_mbar_init();
     prefetch_tmap(&tm.A);
     prefetch_tmap(&tm.W);
@@ -105,7 +107,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
       // nothing is issued; fall through to the teardown
     } else if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer (each CTA its own part)
-      uint32_t s = 0, ph = 0;
+      uint32_t s = 0, ph = 0, n_issued = 0;
       // Has an earlier launch failed?  The leader's producer alone looks, once, and raises the flag of both CTAs: without its arrivals no
       // stage completes, and the flags end the waits of all other roles.
       bool ok = true;
@@ -127,6 +129,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
           if (!mbar_wait_warp(&empty[s], ph ^ 1, ctx, 1)) { ok = false; break; }
           if (elect_one()) {
             if (rank == 0) mbar_expect_tx(&full[s], tx);
+            if (EPI == KF_EPI_RES) *issued = n_issued + 1;
             const uint32_t bar = leader_full + s * 8;
             uint8_t* ta = tiles + (size_t)s * PAIR_TILE_BYTES;
             tma_load_2d_pair(ta, &tm.A, kt * BKB, a_row, bar);              // rows past M read as zeros
@@ -138,6 +141,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
             }
           }
           __syncwarp();
+          ++n_issued;
           if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1; }
         }
       }
@@ -196,7 +200,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps tm, const GemmArgs g) {
     }
   } else {
     setmaxnreg_inc<EPI == KF_EPI_ROPE ? REGS_EPI_ROPE : REGS_EPI>();
-    if (!bad_align) epilogue_warps<EPI, 256, true, FORM>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, &tm.R, &tm.C, ctx, warp, lane);
+    if (!bad_align) epilogue_warps<EPI, 256, true, FORM>(g, tmem_base, tfull, tempty, slices, slabs, boxes, box_full, issued, &tm.R, &tm.C, ctx, warp, lane);
   }
 
   pdl_launch_dependents();
