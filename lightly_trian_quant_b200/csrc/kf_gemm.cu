@@ -425,22 +425,31 @@ static bool gemm_res_boxes(int k_tiles, int m_tiles, int N, int sms) {
 }
 
 // Launches that run on CTA pairs (kf_gemm_pair.cu).  A tile of a pair is twice as much to lose in a last round, and a launch of pairs starts
-// about a microsecond later (cluster launch, hand-shakes), so the line lies by rows.  One CTA -> pairs, captured launches, us at 1605, 3210, 4815, 6420 and
-// 9630 rows:
-//    PLAIN / ROPE  MXFP8 768 x 2304 (qkv)   7.7 -> 8.5  10.9 -> 11.4  13.6 -> 14.0  18.5 -> 17.9  24.2 -> 22.8
-//                  NVFP4 1024 x 3072 (qkv)  8.9 -> 9.6  11.8 -> 12.7  15.2 -> 16.5  20.3 -> 20.1  26.3 -> 26.3
-//                  NVFP4 4096 x 1024        8.1 -> 9.6  10.3 -> 10.5  14.0 -> 13.5  16.6 -> 15.4  23.3 -> 21.9
-//    QUANT         MXFP8 768 x 3072        10.1 -> 10.2 13.9 -> 13.4  17.9 -> 17.1  23.3 -> 21.9  31.0 -> 29.1
-//    bf16 operands 768 x 2304               9.5 -> 10.3 14.8 -> 14.3  17.8 -> 17.1  24.3 -> 22.1  34.8 -> 30.1
-//    RES           NVFP4 4096 x 1024        9.6 -> 13.0 15.2 -> 14.2  19.8 -> 18.3  23.5 -> 22.4  (the residual as boxes)
+// about a microsecond later (cluster launch, hand-shakes); what a pair gains is operand traffic, so it gains with the length of the main loop
+// beside the epilogue.  The line lies by row tiles and K, in stages of 128 bytes.  One CTA -> pairs, captured launches, us at 3210, 4815, 6420 and 9630 rows:
+//    PLAIN  4 stages   NVFP4 1024 x 4096   11.1 -> 10.8  14.4 -> 13.5  20.5 -> 18.2  30.7 -> 25.6     3  NVFP4  768 x 3072   8.1 -> 8.5  10.3 -> 10.7  14.3 -> 13.9  19.5 -> 18.3
+//           6          MXFP8  768 x 3072   10.6 ->  9.9  14.5 -> 12.7  20.2 -> 16.6  30.6 -> 25.2    16  NVFP4 4096 x 1024   9.9 -> 10.2 15.1 -> 14.1  17.9 -> 16.1  26.9 -> 24.3
+//    QUANT  3          NVFP4  768 x 3072   13.2 -> 13.5  17.1 -> 17.1  22.4 -> 21.9  30.1 -> 29.1     4  NVFP4 1024 x 4096  15.0 -> 15.6 21.3 -> 21.2  27.0 -> 27.2  40.6 -> 36.9
+//           6          MXFP8  768 x 3072   13.0 -> 14.1  16.7 -> 17.5  21.8 -> 22.6  31.5 -> 30.6     8  MXFP8 1024 x 4096  18.1 -> 16.6 28.6 -> 25.2  33.2 -> 32.5  47.0 -> 46.2
+//          12          bf16   768 x 3072   17.5 -> 16.6  24.3 -> 23.1  33.4 -> 28.6  44.1 -> 39.6
+//    ROPE   4          NVFP4 1024 x 3072   11.5 -> 12.4  14.9 -> 16.3  20.2 -> 19.9  26.5 -> 26.2     6  MXFP8  768 x 2304  10.5 -> 11.0 13.1 -> 13.8  19.0 -> 18.0  24.3 -> 22.3
+//           8          MXFP8 1024 x 3072   14.0 -> 14.7  19.2 -> 19.0  25.2 -> 24.4  39.0 -> 33.7    12  bf16   768 x 2304  15.1 -> 14.1 18.7 -> 16.8  26.0 -> 22.6  36.9 -> 31.2
+//    RES    1          NVFP4  256 x 1024    9.4 ->  8.8  12.1 -> 11.0  15.1 -> 13.3                  16  NVFP4 4096 x 1024  16.3 -> 15.4 20.9 -> 20.1  24.8 -> 24.2  34.5 -> 31.1   (the residual as boxes)
+// Under 3 stages the epilogue is all there is: pairs lose in ROPE (256 x 3072, 6420 rows: MXFP8 19.4 -> 22.0, NVFP4 17.5 -> 18.6), in QUANT on 8-bit
+// operands (9630: 29.2 -> 34.9) and in PLAIN (256 x 1024, 22 470: NVFP4 12.0 -> 12.8) but for many rounds (256 x 4096, 22 470: MXFP8 46.2 -> 43.3); QUANT on
+// 4-bit operands, as slow as its epilogue in either form, stays by its rows (256 x 4096, 9630: 35.5 -> 34.3).
 // Not where the tiles do not fill the pairs (for RES half of them: without pairs its residual goes in 32-byte pieces), nor for what
-// gemm_res_boxes takes.  Few rows against many columns (the mask product: two row tiles an image, 8 x 200 x 65 536 x 1024 340 -> 261 us) count from four
-// rounds on; a batched product needs its row tiles in twos.
-static bool gemm_pairs(int fmt, int epi, int m_tiles, int m_tiles_pb, int N, int sms) {
+// gemm_res_boxes takes.  PLAIN with few rows against many columns (the mask product: two row tiles an image, 8 x 200 x 65 536 x 1024 340 -> 261 us) counts from
+// four rounds on; a batched product needs its row tiles in twos.
+static bool gemm_pairs(int fmt, int epi, int k_tiles, int m_tiles, int m_tiles_pb, int N, int sms) {
   if (N % 256 != 0 || m_tiles_pb % 2 != 0) return false;
   const int64_t tiles = (int64_t)((m_tiles + 1) / 2) * (N / 256), pairs = sms / 2;
-  const bool early = epi == KF_EPI_RES || epi == KF_EPI_QUANT || fmt == KF_FMT_BF16;
-  return (m_tiles >= (early ? 24 : 48) || tiles >= 4 * pairs) && (epi == KF_EPI_RES ? 2 * tiles > pairs : tiles >= pairs);
+  if (epi == KF_EPI_RES) return m_tiles >= 24 && 2 * tiles > pairs;
+  const bool fp4 = fmt == KF_FMT_NV4 || fmt == KF_FMT_MX4;
+  if (k_tiles < 3 && (epi == KF_EPI_PLAIN ? tiles < 8 * pairs : epi == KF_EPI_ROPE || !fp4)) return false;
+  const int long_k = epi == KF_EPI_PLAIN ? 6 : epi == KF_EPI_QUANT ? 8 : 12;
+  const int rows = k_tiles >= long_k ? 24 : epi == KF_EPI_QUANT && !fp4 ? 64 : 48;
+  return tiles >= pairs && (m_tiles >= rows || (epi == KF_EPI_PLAIN && tiles >= 4 * pairs));
 }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -499,7 +508,7 @@ extern "C" int kf_gemm_bs(const kf_gemm_params* p, void* stream) {
   if (st != KF_OK) return st;
   const bool res_tma = epi == KF_EPI_RES && p->out_row_group == 0 && gemm_res_boxes((int)(kbytes / BKB), m_tiles, p->N, sms);
   const int m_tiles_pb = p->batch > 0 ? (p->a_rows_per_batch + BM - 1) / BM : 0;
-  const bool pair = !res_tma && gemm_pairs(fmt, epi, m_tiles, m_tiles_pb, p->N, sms);
+  const bool pair = !res_tma && gemm_pairs(fmt, epi, (int)(kbytes / BKB), m_tiles, m_tiles_pb, p->N, sms);
   const int bn = res_tma ? 128 : gemm_columns(fmt, epi, m_tiles, p->N, sms);
   GemmArgs g{};
   g.sfa = static_cast<const uint8_t*>(p->SFA);

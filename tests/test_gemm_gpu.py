@@ -397,9 +397,9 @@ def test_last_round_in_half_tiles(fmt, M, N, K):
 
 # the error word is already set when the kernel starts (delay 0), or is set by the predecessor while the kernel, started early under dependent
 # launch, has requested its weights (delay 200 us); 16 operand stages are more than the ring holds, one stage is less; 9600 rows take the residual through
-# shared memory (K = 256) and run on CTA pairs (the other kinds; all of them with K = 4096)
+# shared memory (K = 256; K = 768 too) and run on CTA pairs (QUANT with K = 256, the other kinds with K = 768, all of them with K = 4096)
 @pytest.mark.parametrize("delay", [0, 200])
-@pytest.mark.parametrize("M,K", [(320, 256), (320, 4096), (9600, 256), (9600, 4096)])
+@pytest.mark.parametrize("M,K", [(320, 256), (320, 4096), (9600, 256), (9600, 768), (9600, 4096)])
 def test_a_failed_predecessor_does_not_stall_the_launch(M, K, delay):
     """every role of the GEMM and attention kernels comes to the same decision when an earlier launch has failed: the launch ends well inside
     the two seconds of a bounded wait, and the next one is whole again."""
@@ -547,13 +547,14 @@ def test_epilogue_forms_agree(fmt, M, N):
     ops.check_device_error()
 
 
-# 49 row tiles (the follower of the last pair has none) x 3 column tiles = 75 tiles of 74 pairs: the last one is cut into halves; one operand stage and more than the
-# ring holds.  Row blocks of the same rows run on single CTAs.
+# 49 row tiles (the follower of the last pair has none) x 3 column tiles = 75 tiles of 74 pairs: the last one is cut into halves; more operand stages than the ring
+# holds, less (RES, and PLAIN and ROPE from three stages on), and 66 row tiles, from where QUANT on 8-bit operands runs on pairs
+# with a short K too.  Row blocks of the same rows run on single CTAs.
 @pytest.mark.parametrize("fmt", FMTS + ["bf16"])
-@pytest.mark.parametrize("K", [256, 2048])
-def test_cta_pairs_against_launches_of_row_blocks(fmt, K):
+@pytest.mark.parametrize("B,K", [(3, 256), (3, 768), (3, 2048), (4, 256), (4, 768)])
+def test_cta_pairs_against_launches_of_row_blocks(fmt, B, K):
     ops = _ops()
-    B, Ntok, prefix, H, N = 3, 2089, 5, 4, 768
+    Ntok, prefix, H, N = 2089, 5, 4, 768
     M = B * Ntok
     g = torch.Generator(device="cuda").manual_seed(K)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
@@ -599,7 +600,8 @@ def test_cta_pairs_against_launches_of_row_blocks(fmt, K):
             assert torch.equal(u[b:b + 1] if u.shape[0] == B else u[r0:r1], v), (b, i)
     if fmt != "bf16":                                       # scale bytes of the rows past M: zeros, as the layout asks for
         for sf in (t for t in big if t.dim() == 1):
-            tail = sf.view(49, -1, 32, 4, 4)[48]            # [k-blocks / 4, row & 31, row >> 5, 4] of the last row tile
+            last = (M - 1) // 128
+            tail = sf.view(last + 1, -1, 32, 4, 4)[last]    # [k-blocks / 4, row & 31, row >> 5, 4] of the last row tile
             rows = torch.arange(128, device="cuda")
             per_row = tail.permute(2, 1, 0, 3).reshape(128, -1)
-            assert not per_row[48 * 128 + rows >= M].any()
+            assert not per_row[last * 128 + rows >= M].any()
