@@ -126,6 +126,26 @@ def test_attn_tile_edges_and_items_shorter_than_the_pipeline(B, N, H):
     assert err < 4e-3, err
 
 
+@pytest.mark.parametrize("fmt", ["mx8", "nv4", "mx4"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,N,H", [(1, 1, 2), (40, 64, 16), (2, 95, 4), (40, 96, 16), (2, 97, 2), (2, 129, 4), (1, 192, 2), (20, 193, 16), (1, 261, 12), (1, 289, 2)])
+def test_attn_fused_quantise_out_at_tile_edges(fmt, dtype, B, N, H):
+    """the codes and scales of the fused output around the 96-key and 128-query tiles, and where a CTA works through several items, are those that
+    the row quantiser makes of the 16-bit output."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(B + N)
+    qkv = (torch.randn(3, B, N, H, 64, generator=g, device="cuda") * 1.5).to(dtype)
+    o = ops.attn_fwd(qkv).view(B * N, H * 64)
+    fused, rows = ops.ActBuf(B * N, H * 64, fmt, device="cuda"), ops.ActBuf(B * N, H * 64, fmt, device="cuda")
+    if fmt == "nv4":
+        for buf in (fused, rows):
+            buf.ts.fill_(float(o.float().abs().max()) / 2688.0 * 2)
+    ops.attn_fwd_quant(qkv, fused)
+    ops.quant_rows(o, rows)
+    ops.check_device_error()
+    assert torch.equal(fused.q, rows.q) and torch.equal(fused.sf, rows.sf)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("lo,N", [(64, 96), (64, 300), (96, 300), (288, 300)])
 def test_attn_larger_logits_behind_the_first_keys(dtype, lo, N):

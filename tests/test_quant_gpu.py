@@ -249,10 +249,11 @@ def test_quant_rows_of_rows_without_32_byte_alignment(fmt, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("fmt", ["mx8", "nv4", "mx4"])
-@pytest.mark.parametrize("M,K", [(9003, 2048), (9003, 768), (12929, 256)])
+@pytest.mark.parametrize("M,K", [(9003, 2048), (9003, 768), (13001, 768), (12929, 256), (41001, 256)])
 def test_quant_rows_of_many_rounds(fmt, dtype, M, K):
-    """launches of more items than are resident at once (a thread works through several, 16-bit inputs one ahead), rows that end inside a
-    scale block, row lengths with and without a division: the bytes of launches of 128 rows each; scale bytes past the last row are zero."""
+    """launches of more items than are resident at once (more than 148 x 2048 threads at 9003 x 2048, 13 001 x 768 and 41 001 x 256: a thread works
+    through several, 16-bit inputs one ahead) and of fewer, rows that end inside a scale block, row lengths with and without a
+    division: all rows have the bytes of launches of 128 rows each; scale bytes past the last row are zero."""
     from lightly_trian_quant_b200 import ops
 
     g = torch.Generator(device="cuda").manual_seed(M + K)
@@ -265,13 +266,15 @@ def test_quant_rows_of_many_rounds(fmt, dtype, M, K):
     ops.quant_rows(x, big)
     ops.check_device_error()
     per = big.sf.numel() // ((M + 127) // 128)
-    for r0 in (0, 128 * (M // 256), 128 * ((M - 1) // 128)):
+    q, sf = torch.empty_like(big.q), torch.empty_like(big.sf)
+    for r0 in range(0, M, 128):
         rows = x[r0:r0 + 128]
         one = ops.ActBuf(rows.shape[0], K, fmt)
         if fmt == "nv4":
             one.ts.fill_(0.003)
         ops.quant_rows(rows, one)
-        assert torch.equal(big.q[r0:r0 + 128], one.q.view_as(big.q[r0:r0 + 128])), r0
-        assert torch.equal(big.sf.view(-1)[r0 // 128 * per:(r0 // 128 + 1) * per], one.sf.view(-1)), r0
+        q.view(M, -1)[r0:r0 + 128] = one.q.view(rows.shape[0], -1)
+        sf.view(-1)[r0 // 128 * per:(r0 // 128 + 1) * per] = one.sf.view(-1)
+    assert torch.equal(big.q, q) and torch.equal(big.sf, sf)
     tail = big.sf.view(-1)[-per:].view(-1, 32, 4, 4).permute(2, 1, 0, 3).reshape(128, -1)
     assert not tail[(M - 1) % 128 + 1:].any()
