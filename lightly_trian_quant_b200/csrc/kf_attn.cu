@@ -29,6 +29,7 @@
 //            Measured, tiles of 64 -> 96 keys (B 14, H 16, N 1605, bf16 out / NVFP4 out; N 1805, NVFP4 out; B 8, N 4101, f16,
 //            MXFP4 out; B 1, N 1605, NVFP4 out): 199 -> 186 / 204 -> 194 / 250 -> 239 / 667 -> 636 / 24.7 -> 23.6 us; 256-bit stores of the output
 //            where it is 32-byte aligned: 186 -> 184.3 / 191.1 -> 190.5 / 236.2 -> 235.4 us (16-byte pieces of a row per lane cost twice the look-ups).
+//            Few tokens paid for the wider tiles (B 1, H 12, N 261, MXFP8 out 6.5 -> 6.7 us, captured) until the quantising forms stopped spilling: 6.15.
 //            Not kept: the barrier asked for only where it is waited on (198 us against 194), the next row requested at the end of the
 //            step (199), five of sixteen pairs or none of every third 32 off the special-function unit (202, 202), an item's output behind the
 //            first step of the next one (203: the waits it hides are fewer than the registers it takes from the loop); with
