@@ -439,17 +439,17 @@ static bool gemm_res_boxes(int k_tiles, int m_tiles, int N, int sms) {
 // operands (9630: 29.2 -> 34.9) and in PLAIN (256 x 1024, 22 470: NVFP4 12.0 -> 12.8) but for many rounds (256 x 4096, 22 470: MXFP8 46.2 -> 43.3); QUANT on
 // 4-bit operands, as slow as its epilogue in either form, stays by its rows (256 x 4096, 9630: 35.5 -> 34.3).
 // Not where the tiles do not fill the pairs (for RES half of them: without pairs its residual goes in 32-byte pieces), nor for what
-// gemm_res_boxes takes.  PLAIN with few rows against many columns (the mask product: two row tiles an image, 8 x 200 x 65 536 x 1024 340 -> 261 us) counts from
-// four rounds on; a batched product needs its row tiles in twos.
+// gemm_res_boxes takes.  Few rows against many columns (the mask product: two row tiles an image, 8 x 200 x 65 536 x 1024 340 -> 261 us) count from four
+// rounds on, but for QUANT with a short K (MXFP8 768 x 3072, 6420 rows, is that already); a batched product needs its row tiles in twos.
 static bool gemm_pairs(int fmt, int epi, int k_tiles, int m_tiles, int m_tiles_pb, int N, int sms) {
   if (N % 256 != 0 || m_tiles_pb % 2 != 0) return false;
   const int64_t tiles = (int64_t)((m_tiles + 1) / 2) * (N / 256), pairs = sms / 2;
   if (epi == KF_EPI_RES) return m_tiles >= 24 && 2 * tiles > pairs;
   const bool fp4 = fmt == KF_FMT_NV4 || fmt == KF_FMT_MX4;
   if (k_tiles < 3 && (epi == KF_EPI_PLAIN ? tiles < 8 * pairs : epi == KF_EPI_ROPE || !fp4)) return false;
-  const int long_k = epi == KF_EPI_PLAIN ? 6 : epi == KF_EPI_QUANT ? 8 : 12;
-  const int rows = k_tiles >= long_k ? 24 : epi == KF_EPI_QUANT && !fp4 ? 64 : 48;
-  return tiles >= pairs && (m_tiles >= rows || (epi == KF_EPI_PLAIN && tiles >= 4 * pairs));
+  const bool long_k = k_tiles >= (epi == KF_EPI_PLAIN ? 6 : epi == KF_EPI_QUANT ? 8 : 12);
+  const int rows = long_k ? 24 : epi == KF_EPI_QUANT && !fp4 ? 64 : 48;
+  return tiles >= pairs && (m_tiles >= rows || (tiles >= 4 * pairs && (long_k || epi != KF_EPI_QUANT)));
 }
 
 static bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
